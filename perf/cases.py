@@ -290,3 +290,100 @@ def tolerance(case):
     # sums of up to eight values carried in fp32 (another order differs by an ulp or two), rounded once to the tensor's type
     return {"float32": {"rel": 3e-7, "max": 2e-6}, "bfloat16": {"rel": 8e-3, "max": 1.6e-2},
             "float16": {"rel": 1e-3, "max": 2e-3}}[case["dtype"]]
+
+
+# ---- the same results in 64 bits, from plain torch ------------------------------------------------------
+def _padded_window(case, device):
+    n, win = case["n_fft"], case["win"]
+    left = (n - win) // 2
+    return F.pad(torch.hann_window(win, device=device).double(), (left, n - win - left))
+
+
+def _overlap_add(frames, hop):
+    """[..., frames, n_fft] to [..., n_fft + hop * (frames - 1)]."""
+    count, n = frames.shape[-2:]
+    at = (torch.arange(count, device=frames.device)[:, None] * hop + torch.arange(n, device=frames.device)).reshape(-1)
+    out = frames.new_zeros(*frames.shape[:-2], n + hop * (count - 1))
+    return out.index_add(-1, at, frames.flatten(-2))
+
+
+def _stft64(x, case):
+    n, hop = case["n_fft"], case["hop"]
+    if case["center"]:
+        x = F.pad(x[:, None], (n // 2, n // 2), mode="reflect")[:, 0]
+    spec = torch.fft.rfft(x.unfold(-1, n, hop) * _padded_window(case, x.device))
+    return (spec / math.sqrt(n) if case["normalized"] else spec).transpose(1, 2)
+
+
+def _istft64(spec, case):
+    n, hop, length = case["n_fft"], case["hop"], case["samples"]
+    win = _padded_window(case, spec.device)
+    frames = torch.fft.irfft(spec.transpose(1, 2), n=n) * win
+    if case["normalized"]:
+        frames = frames * math.sqrt(n)
+    y = _overlap_add(frames, hop)
+    env = _overlap_add((win * win).expand(spec.shape[2], n), hop)
+    y = torch.where(env > 1e-11, y / env.clamp_min(1e-11), torch.zeros_like(y))
+    y = y[:, n // 2:n // 2 + length]
+    return F.pad(y, (0, length - y.shape[-1]))
+
+
+def _adamw64(params, grads, moments, step):
+    """One step of AdamW with the default betas, eps and weight decay and lr 1e-3, in place; `step` counts from 1."""
+    for p, g, (m, v) in zip(params, grads, moments):
+        p.mul_(1 - 1e-3 * 1e-2)
+        m.mul_(0.9).add_(g, alpha=1 - 0.9)
+        v.mul_(0.999).addcmul_(g, g, value=1 - 0.999)
+        p.sub_(1e-3 / (1 - 0.9 ** step) * m / (v.sqrt() / math.sqrt(1 - 0.999 ** step) + 1e-8))
+
+
+def exact(case, seed):
+    device = _device()
+    gen = torch.Generator(device=device).manual_seed(seed)
+    kind = case["kind"]
+    if kind in ("stft", "istft"):
+        wave = (0.3 * torch.randn(case["batch"], case["samples"], generator=gen, device=device)).double()
+        spec = _spectrum(case, gen, device).to(torch.complex128)
+        x, other, fn = (wave, spec, _stft64) if kind == "stft" else (spec, wave, _istft64)
+        if not case["grad"]:
+            return fn(x, case)
+        x.requires_grad_(True)
+        out = fn(x, case)
+        (grad,) = torch.autograd.grad(out, x, other)
+        return [out.detach(), grad]
+    if kind == "adamw":
+        params = []
+        for i, o in _linears(case):
+            params.append((torch.randn(o, i, generator=gen, device=device) / math.sqrt(i)).double())
+            params.append((torch.randn(o, generator=gen, device=device) / math.sqrt(i)).double())
+        moments = [(torch.zeros_like(p), torch.zeros_like(p)) for p in params]
+        for step in (1, 2):
+            grads = [(1e-3 * torch.randn(p.shape, generator=gen, device=device)).double() for p in params]
+            _adamw64(params, grads, moments, step)
+        return {"params": params, "exp_avg": [m for m, _ in moments], "exp_avg_sq": [v for _, v in moments]}
+    if kind == "topk" or (kind == "train" and case["compression"] == "topk"):
+        return None  # which entries are sent is decided on fp32 sums: another precision sends others
+    if kind == "train":
+        torch.manual_seed(seed)
+        with torch.device(device):
+            layers = [torch.nn.Linear(i, o) for i, o in _linears(case)]
+        x = torch.randn(case["batch"], case["features"], generator=gen, device=device).double()
+        y = torch.randint(0, case["classes"], (case["batch"],), generator=gen, device=device)
+        for n, layer in enumerate(layers):
+            x = layer.double()(x if n == 0 else F.gelu(x))
+        loss = F.cross_entropy(x, y)
+        params = [p for layer in layers for p in layer.parameters()]
+        grads = list(torch.autograd.grad(loss, params))
+        weights = [p.detach() for p in params]
+        _adamw64(weights, grads, [(torch.zeros_like(p), torch.zeros_like(p)) for p in weights], 1)
+        return {"loss": loss.detach(), "weights": weights, "grads": grads}
+    ws, n = case["ranks"], case["n"]
+    count = n * ws if case["op"] == "reduce_scatter" else n
+    ins = [torch.randn(count, generator=gen, device=device).to(_DTYPES[case["dtype"]]).double() for _ in range(ws)]
+    if case["op"] == "allreduce":
+        return [sum(ins) / ws] * ws
+    if case["op"] == "reduce_scatter":
+        return list((sum(ins) / ws).chunk(ws))
+    if case["op"] == "allgather":
+        return [torch.cat(ins)] * ws
+    return [ins[0]] * ws
