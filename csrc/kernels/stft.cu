@@ -1,12 +1,15 @@
-// STFT / iSTFT kernels (sm_100a): shared-memory radix-4 Stockham FFTs of half the frame length
-// (real input / real output), several frames per CTA, twiddles computed once per CTA, with
-// the padding, windowing and scaling fused into the loads and stores, and an
-// atomics-free gather overlap-add.  See stft_api.h for the decomposition.
+// STFT / iSTFT kernels (sm_100a): register FFTs of half the frame length by a group of lanes of one
+// warp (fft_warp.cuh), with the padding, windowing and scaling fused into the loads and stores and
+// the overlap-add fused behind the inverse transform.  See stft_api.h for the decomposition.
 // Replaces the reference's one-thread-per-frame Metal FFT (reference
 // csrc/metal/shaders.metal:735-861) and its CPU-side padding and overlap-add
 // (reference csrc/transforms/StftMetalKernels.mm:158-393).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
+
+#include "kernels/fft_warp.cuh"
 #include "kernels/launch_count.h"
 #include "kernels/stft_api.h"
 
@@ -15,25 +18,17 @@ namespace kern {
 
 namespace {
 
-__device__ __forceinline__ void fill_twiddles(float2* tw, int n) {
-  for (int k = threadIdx.x; k < n / 2; k += blockDim.x) {
-    float sn, cs;
-    sincospif(2.0f * static_cast<float>(k) / static_cast<float>(n), &sn, &cs);
-    tw[k] = make_float2(cs, -sn);
-  }
-}
+constexpr int kSms = 148;
+constexpr size_t kMaxSmem = 227 << 10;    // per CTA
+constexpr size_t kSmemPerSm = 228 << 10;  // of which each CTA takes another 1 KB
 
-__device__ __forceinline__ int64_t reflect_index(int64_t i, int64_t len) {
-  // reflect without repeating the edge sample: -1 -> 1, len -> len-2
-  if (len == 1) return 0;
-  const int64_t period = 2 * (len - 1);
-  i %= period;
-  if (i < 0) i += period;
-  return i < len ? i : period - i;
+__device__ __forceinline__ float window_at(const StftWindow& w, int64_t n) {
+  const int64_t i = n - w.left;
+  return i >= 0 && i < w.len ? w.data[i] : 0.f;
 }
 
 // sum of window^2 over the frames covering padded position p
-__device__ __forceinline__ float envelope_at(const float* window, int64_t p, int n_fft, int hop, int n_frames) {
+__device__ __forceinline__ float envelope_at(const StftWindow& window, int64_t p, int n_fft, int hop, int n_frames) {
   int64_t f_hi = p / hop;
   if (f_hi > n_frames - 1) f_hi = n_frames - 1;
   int64_t f_lo = (p - n_fft + hop) / hop;  // ceil((p - n_fft + 1) / hop) for non-negative values
@@ -42,201 +37,411 @@ __device__ __forceinline__ float envelope_at(const float* window, int64_t p, int
   for (int64_t f = f_lo; f <= f_hi; ++f) {
     const int64_t n = p - f * hop;
     if (n >= 0 && n < n_fft) {
-      const float w = window[n];
+      const float w = window_at(window, n);
       e += w * w;
     }
   }
   return e;
 }
 
-// Both transforms work on REAL frames, so each frame is handled as a complex FFT of half the
-// length: z[m] = x[2m] + i x[2m+1], Z = FFT_{N/2}(z), and one pass with the twiddles W_N^k
-// separates / recombines the even and odd halves.  That halves the butterflies and the shared
-// memory per frame.  A CTA computes the twiddle table once and then loops over frames, `fpc`
-// frames at a time (several short frames keep all threads busy).
-//
-//   forward:  E[k] = (Z[k] + conj Z[h-k]) / 2,  O[k] = (Z[k] - conj Z[h-k]) / (2i),
-//             X[k] = E[k] + W_N^k O[k],  k = 0..h  (h = N/2, Z[h] = Z[0])
-//   inverse:  Z[k] = (X[k] + conj X[h-k]) + i W_N^{-k} (X[k] - conj X[h-k]),  z = IFFT_h(Z) (no 1/h),
-//             y[2m] = Re z[m], y[2m+1] = Im z[m]   (y = unnormalised inverse of the Hermitian extension)
-
-// Stockham autosort FFT over `fpc` independent transforms of length h stored back to back
-// (natural order in, natural order out: no bit-reversal pass, whose shared-memory scatter would put
-// a whole warp on one bank).  Radix-4 passes (four values per thread in registers; an odd log2(h)
-// starts with one radix-2 pass) ping-pong between `a` and `b`; every pass reads at stride h/4 and
-// writes runs of Ns consecutive values.  tw[t] = exp(-2*pi*i*t/(2h)), t < h; tw[t + h] = -tw[t].
-// Returns the buffer that holds the result.
-__device__ __forceinline__ float2 cmul_tw(float2 v, float2 w, float conj_sign) {
-  // v * (w.x + i * conj_sign * w.y): conj_sign = +1 keeps the table's forward twiddle, -1 conjugates it
-  const float wy = conj_sign * w.y;
-  return make_float2(v.x * w.x - v.y * wy, v.x * wy + v.y * w.x);
+template <int kBytes>
+__device__ __forceinline__ void copy_async(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(smem))),
+               "l"(gmem), "n"(kBytes)
+               : "memory");
 }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__device__ __forceinline__ float2* fft_half_smem(float2* a, float2* b, const float2* tw, int h, int log2h, int fpc,
-                                                 float sign) {
-  const float cs = -sign;  // sign = -1: forward (table as stored); +1: inverse (conjugated)
-  float2* src = a;
-  float2* dst = b;
-  int ns = 1;
-  if (log2h & 1) {
-    const int per = h / 2;
-    for (int jj = threadIdx.x; jj < per * fpc; jj += blockDim.x) {
-      const int f = jj >> (log2h - 1), j = jj & (per - 1);
-      const float2 v0 = src[f * h + j], v1 = src[f * h + j + per];
-      float2* d = dst + f * h + 2 * j;
-      d[0] = make_float2(v0.x + v1.x, v0.y + v1.y);
-      d[1] = make_float2(v0.x - v1.x, v0.y - v1.y);
+// Samples of a frame that reaches over the signal's ends (or, when dividing by the envelope, of one that lacks
+// neighbours), in `buf`.  Every lane prepares the pairs that it will read back; the copies are
+// asynchronous, so that a small call waits for memory once and not once per pair.
+template <int LH, bool kEnvelope>
+__device__ __forceinline__ void load_edge_frame(const FftFramesArgs& a, const float* sig, const float* win, float2* buf,
+                                                int f, int t, int reach) {
+  using F = WarpFft<LH>;
+  const int64_t start = static_cast<int64_t>(f) * a.hop - a.pad;
+  for (int r = 0; r < 2 * F::V; ++r) {
+    const int j = 2 * ((r / 2) * F::L + t) + (r & 1);
+    int64_t q = start + j;
+    if (a.reflect) {  // without repeating the edge sample; the signal is longer than the padding: one reflection
+      if (q < 0) q = -q;
+      if (q >= a.signal_len) q = 2 * a.signal_len - 2 - q;
     }
-    __syncthreads();
-    float2* t = src; src = dst; dst = t;
-    ns = 2;
+    float* dst = reinterpret_cast<float*>(buf) + j;
+    if (q >= 0 && q < a.signal_len) copy_async<4>(dst, sig + q);
+    else *dst = 0.f;
   }
-  const int quarter = h / 4;
-  for (; ns < h; ns *= 4) {
-    const int tstep = h / (2 * ns);  // exp(-2*pi*i*r*k/(4*ns)) = tw[r * k * tstep]
-    for (int jj = threadIdx.x; jj < quarter * fpc; jj += blockDim.x) {
-      const int f = jj >> (log2h - 2), j = jj & (quarter - 1);
-      const int k = j & (ns - 1);
-      const int t1 = k * tstep, t3 = 3 * t1;
-      const float2* x = src + f * h + j;
-      float2 w3 = tw[t3 < h ? t3 : t3 - h];
-      if (t3 >= h) w3 = make_float2(-w3.x, -w3.y);
-      const float2 v0 = x[0];
-      const float2 v1 = cmul_tw(x[quarter], tw[t1], cs);
-      const float2 v2 = cmul_tw(x[2 * quarter], tw[2 * t1], cs);
-      const float2 v3 = cmul_tw(x[3 * quarter], w3, cs);
-      const float2 a0 = make_float2(v0.x + v2.x, v0.y + v2.y), a1 = make_float2(v0.x - v2.x, v0.y - v2.y);
-      const float2 a2 = make_float2(v1.x + v3.x, v1.y + v3.y), a3 = make_float2(v1.x - v3.x, v1.y - v3.y);
-      const float2 r3 = make_float2(cs * a3.y, -cs * a3.x);  // -i * a3 forward, +i * a3 inverse
-      float2* d = dst + f * h + ((j - k) << 2) + k;
-      d[0] = make_float2(a0.x + a2.x, a0.y + a2.y);
-      d[ns] = make_float2(a1.x + r3.x, a1.y + r3.y);
-      d[2 * ns] = make_float2(a0.x - a2.x, a0.y - a2.y);
-      d[3 * ns] = make_float2(a1.x - r3.x, a1.y - r3.y);
-    }
-    __syncthreads();
-    float2* t = src; src = dst; dst = t;
-  }
-  return src;
-}
-
-__device__ __forceinline__ float load_sample(const FftFramesArgs& a, const float* sig, int64_t t, int n) {
-  float v = 0.f;
-  if (a.reflect) {
-    v = sig[reflect_index(t, a.signal_len)];
-  } else if (t >= 0 && t < a.signal_len) {
-    v = sig[t];
-    if (a.divide_envelope) {
-      const float e = envelope_at(a.window, t + a.pad, n, a.hop, a.n_frames);
-      v = e > 1e-11f ? v / e : 0.f;
-    }
-  }
-  return v;
-}
-
-__global__ void __launch_bounds__(256) fft_frames_kernel(const FftFramesArgs a, int log2h, int fpc) {
-  extern __shared__ float2 smem[];
-  const int n = a.n_fft, h = n / 2;
-  float2* tw = smem;        // h twiddles W_N^k
-  float2* data = smem + h;  // fpc * h values, and as many again for the ping-pong passes
-  float2* pong = data + fpc * h;
-  const int b = blockIdx.y;
-  fill_twiddles(tw, n);
-  const float* sig = a.signal + static_cast<int64_t>(b) * a.signal_len;
-  const int bins = h + 1;
-  for (int f0 = blockIdx.x * fpc; f0 < a.n_frames; f0 += gridDim.x * fpc) {
-    __syncthreads();  // twiddles ready / previous frames' bins written
-    for (int jj = threadIdx.x; jj < h * fpc; jj += blockDim.x) {
-      const int f = jj >> log2h, m = jj & (h - 1);
-      const int frame = f0 + f;
-      float v0 = 0.f, v1 = 0.f;
-      if (frame < a.n_frames) {
-        const int64_t start = static_cast<int64_t>(frame) * a.hop - a.pad;
-        const int64_t t0 = start + 2 * m;
-        if (a.reflect && start >= 0 && start + n <= a.signal_len) {  // frame inside the signal: no index folding
-          v0 = sig[t0];
-          v1 = sig[t0 + 1];
-        } else {
-          v0 = load_sample(a, sig, t0, n);
-          v1 = load_sample(a, sig, t0 + 1, n);
-        }
-        v0 *= a.window[2 * m];
-        v1 *= a.window[2 * m + 1];
+  copy_async_wait();
+  if (kEnvelope) {
+    const int before = min(reach - 1, f), after = min(reach - 1, a.n_frames - 1 - f);
+#pragma unroll 2
+    for (int r = 0; r < F::V; ++r) {
+      const int m = r * F::L + t;
+      float2 e = make_float2(0.f, 0.f);
+      for (int i = before; i >= -after; --i) {  // frame f - i, in frame order
+        const int o = 2 * m + i * a.hop;
+        if (o >= 0 && o < F::n) e.x += win[o] * win[o];
+        if (o + 1 >= 0 && o + 1 < F::n) e.y += win[o + 1] * win[o + 1];
       }
-      data[jj] = make_float2(v0, v1);
-    }
-    __syncthreads();
-    const float2* res = fft_half_smem(data, pong, tw, h, log2h, fpc, -1.0f);
-    for (int jj = threadIdx.x; jj < h * fpc; jj += blockDim.x) {
-      const int f = jj >> log2h, k = jj & (h - 1);
-      const int frame = f0 + f;
-      if (frame >= a.n_frames) continue;
-      const float2* d = res + f * h;
-      const float2 zk = d[k];
-      const float2 zm = d[(h - k) & (h - 1)];            // Z[h-k], with Z[h] = Z[0]
-      const float2 e = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-      const float2 o = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));   // (Zk - conj Zm) / (2i)
-      const float2 w = tw[k];
-      float2 v = make_float2(e.x + w.x * o.x - w.y * o.y, e.y + w.x * o.y + w.y * o.x);
-      float sc = a.scale;
-      if (a.hermitian_weights && k != 0) sc *= 2.0f;
-      if (a.hermitian_weights && k == 0) v.y = 0.f;  // imaginary parts of DC/Nyquist are ignored by an inverse real FFT
-      float2* out = reinterpret_cast<float2*>(a.out) + (static_cast<int64_t>(b) * a.n_frames + frame) * bins;
-      out[k] = make_float2(v.x * sc, v.y * sc);
-      if (k == 0) {  // Nyquist bin: X[h] = E[0] - O[0] (twiddle -1), from the same Z[0]
-        float2 vn = make_float2(e.x - o.x, e.y - o.y);
-        if (a.hermitian_weights) vn.y = 0.f;
-        out[h] = make_float2(vn.x * a.scale, vn.y * a.scale);
-      }
+      float2 v = buf[m];
+      v.x = e.x > 1e-11f ? v.x / e.x : 0.f;
+      v.y = e.y > 1e-11f ? v.y / e.y : 0.f;
+      buf[m] = v;
     }
   }
 }
 
-__global__ void __launch_bounds__(256) ifft_frames_kernel(const IfftFramesArgs a, int log2h, int fpc) {
+// Frames -> spectrum.  Bound by HBM (signal in, spectrum out) and by instruction issue, about equally: the
+// values stay in registers from the load to the store, and a persistent grid computes the twiddle and window
+// tables once per CTA.
+// 16 x 1 Mi samples, n_fft 2048, hop 512 (336 MB): 453 us with one CTA per
+// frame and five shared-memory passes, 92 us so.
+template <int LH, bool kEnvelope>
+__global__ void __launch_bounds__(256, LH <= 6 ? 4 : LH <= 8 ? 3 : LH <= 10 ? 2 : 1)
+    fft_frames_kernel(const FftFramesArgs a, int64_t total) {
+  using F = WarpFft<LH>;
   extern __shared__ float2 smem[];
-  const int n = a.n_fft, h = n / 2;
   float2* tw = smem;
-  float2* data = smem + h;
-  float2* pong = data + fpc * h;
-  const int b = blockIdx.y;
-  fill_twiddles(tw, n);
+  float2* split = tw + F::h;
+  float* win = reinterpret_cast<float*>(split + F::h / 2);
+  float* win_env = win + F::n;  // window / envelope, for frames with a full set of neighbours
+  float2* slots = reinterpret_cast<float2*>(win_env + (kEnvelope ? F::n : 0));
+  F::fill_tables(tw, split);
+  for (int j = threadIdx.x; j < F::n; j += blockDim.x) win[j] = window_at(a.window, j);
+  __syncthreads();
+  const int reach = (F::n + a.hop - 1) / a.hop;  // frames that cover a sample
+  if (kEnvelope) {
+    for (int j = threadIdx.x; j < a.hop && j < F::n; j += blockDim.x) {
+      float e = 0.f;
+      for (int i = j + (F::n - 1 - j) / a.hop * a.hop; i >= 0; i -= a.hop) e += win[i] * win[i];  // in frame order
+      for (int i = j; i < F::n; i += a.hop) win_env[i] = e > 1e-11f ? win[i] / e : 0.f;
+    }
+    __syncthreads();
+  }
+
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int sub = (threadIdx.x & 31) / F::L, t = threadIdx.x % F::L;
+  float2* buf = slots + (warp * F::kPerWarp + sub) * F::kSlot;
+  const float2* win2 = reinterpret_cast<const float2*>(kEnvelope ? win_env : win);
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * warps * F::kPerWarp;
+  for (int64_t i0 = (static_cast<int64_t>(blockIdx.x) * warps + warp) * F::kPerWarp; i0 < total; i0 += stride) {
+    const int64_t i = i0 + sub;
+    const bool live = i < total;
+    const int64_t b = live ? i / a.n_frames : 0;
+    const int f = live ? static_cast<int>(i - b * a.n_frames) : 0;
+    const float* sig = a.signal + b * a.signal_len;
+    const int64_t start = static_cast<int64_t>(f) * a.hop - a.pad;
+    bool inside = start >= 0 && start + F::n <= a.signal_len;
+    if (kEnvelope) inside = inside && f >= reach - 1 && f <= a.n_frames - reach;
+    float2 v[F::V];
+    if (inside) {
+      const float* src = sig + start;
+      if ((reinterpret_cast<uintptr_t>(src) & 7) == 0) {
+#pragma unroll
+        for (int r = 0; r < F::V; ++r) v[r] = reinterpret_cast<const float2*>(src)[r * F::L + t];
+      } else {
+#pragma unroll
+        for (int r = 0; r < F::V; ++r) v[r] = make_float2(src[2 * (r * F::L + t)], src[2 * (r * F::L + t) + 1]);
+      }
+#pragma unroll
+      for (int r = 0; r < F::V; ++r) {
+        const float2 w = win2[r * F::L + t];
+        v[r].x *= w.x;
+        v[r].y *= w.y;
+      }
+    } else {
+      load_edge_frame<LH, kEnvelope>(a, sig, win, buf, f, t, reach);
+#pragma unroll
+      for (int r = 0; r < F::V; ++r) {
+        const float2 w = reinterpret_cast<const float2*>(win)[r * F::L + t];
+        v[r] = buf[r * F::L + t];
+        v[r].x *= w.x;
+        v[r].y *= w.y;
+      }
+    }
+    __syncwarp();
+    F::transform(v, tw, buf, t);
+    float2* out = reinterpret_cast<float2*>(a.out) + (b * a.n_frames + f) * (F::h + 1);
+    const float half = 0.5f * a.scale;  // split_bins gives twice the bins
+    F::split_bins(v, split, t, [&](int k, float2 x) {
+      float sc = half;
+      if (kEnvelope) {  // gradient of an inverse real FFT: both halves of the spectrum, and real DC and Nyquist
+        sc = k == 0 || k == F::h ? half : a.scale;
+        if (k == 0 || k == F::h) x.y = 0.f;
+      }
+      if (live) out[k] = make_float2(x.x * sc, x.y * sc);
+    });
+  }
+}
+
+// Bins of one frame -> its windowed samples y (h float2) in `slot`, by one group of lanes.  A null `spec`
+// means that the slot already holds the bins.
+template <int LH>
+__device__ __forceinline__ void inverse_frame(const IfftOlaArgs& a, const float2* spec, int64_t stride_f,
+                                              const float2* tw, const float2* split, const float2* win2, float2* slot,
+                                              int t) {
+  using F = WarpFft<LH>;
   // hermitian: inverse real FFT of the one-sided bins.  Otherwise the adjoint of the forward
   // transform, Re(sum_{k<=h} X[k] e^{+2 pi i k n / N}), which equals half the inverse real FFT of the
   // same bins with the real parts of DC and Nyquist doubled.
   const float edge = a.hermitian ? 1.0f : 2.0f;
   const float post = a.hermitian ? a.scale : 0.5f * a.scale;
-  for (int f0 = blockIdx.x * fpc; f0 < a.n_frames; f0 += gridDim.x * fpc) {
-    __syncthreads();
-    for (int jj = threadIdx.x; jj < h * fpc; jj += blockDim.x) {
-      const int f = jj >> log2h, k = jj & (h - 1);
-      const int frame = f0 + f;
-      float2 z = make_float2(0.f, 0.f);
-      if (frame < a.n_frames) {
-        const float2* spec = reinterpret_cast<const float2*>(a.spec) + b * a.stride_b + frame * a.stride_t;
-        float2 xk = spec[k * a.stride_f];
-        float2 xm = spec[(h - k) * a.stride_f];
-        if (k == 0) {  // pair (DC, Nyquist): imaginary parts do not take part
-          xk = make_float2(edge * xk.x, 0.f);
-          xm = make_float2(edge * xm.x, 0.f);
+  float2 x[F::V], nyquist;
+  if (spec != nullptr) {
+#pragma unroll
+    for (int r = 0; r < F::V; ++r) x[r] = spec[(r * F::L + t) * stride_f];
+    nyquist = spec[F::h * stride_f];
+  } else {
+#pragma unroll
+    for (int r = 0; r < F::V; ++r) x[r] = slot[r * F::L + t];
+    nyquist = slot[F::h];
+  }
+  __syncwarp();
+  F::merge_bins(x, nyquist, split, t, edge);
+  F::transform(x, tw, slot, t);
+  static_for<0, F::V>([&](auto ic) {
+    constexpr int g = decltype(ic)::value / F::L, k2 = decltype(ic)::value % F::L;
+    const int m = t + F::L * g + F::V * k2;
+    const float2 z = x[F::at(g, k2)], w = win2[m];
+    slot[m] = make_float2(z.y * post * w.x, z.x * post * w.y);
+  });
+}
+
+struct OlaPlan {
+  int segments;       // CTAs per batch entry
+  int ring;           // frames held in shared memory
+  int reach;          // frames that cover a sample
+  int64_t row_base;   // row r of the padded signal is [r * hop, (r + 1) * hop)
+  int64_t rows;       // rows to emit, from row_base on
+};
+
+// The sum over the frames that cover them of N pairs of samples, 64 apart, of row `row`: pair u of a lane is
+// samples j + 64 u and the next one.  kFull: every pair lies in the row and in the frames.
+template <int N, bool kFull, bool kNorm>
+__device__ __forceinline__ void sum_pairs(const float2* slots, int slot_floats, const float* win, int n_fft, int hop,
+                                          int ring, int s, int i_hi, int i_lo, int j, float2 (&v)[N], float2 (&e)[N]) {
+#pragma unroll
+  for (int u = 0; u < N; ++u) v[u] = e[u] = make_float2(0.f, 0.f);
+  s -= i_hi;  // ring slot of frame row - i_hi
+  if (s < 0) s += ring;
+  for (int i = i_hi; i >= i_lo; --i) {  // in frame order
+    const float* y = reinterpret_cast<const float*>(slots) + static_cast<int64_t>(s) * slot_floats + i * hop + j;
+    const float* w = win + i * hop + j;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      if (kFull || (j + 64 * u < hop && j + 64 * u + i * hop < n_fft)) {
+        const float2 q = *reinterpret_cast<const float2*>(y + 64 * u);
+        v[u].x += q.x;
+        v[u].y += q.y;
+        if (kNorm) {
+          const float2 c = *reinterpret_cast<const float2*>(w + 64 * u);
+          e[u].x += c.x * c.x;
+          e[u].y += c.y * c.y;
         }
-        const float2 ep = make_float2(xk.x + xm.x, xk.y - xm.y);   // X[k] + conj X[h-k]
-        const float2 dm = make_float2(xk.x - xm.x, xk.y + xm.y);   // X[k] - conj X[h-k]
-        const float2 w = make_float2(tw[k].x, -tw[k].y);           // W_N^{-k}
-        const float2 od = make_float2(dm.x * w.x - dm.y * w.y, dm.x * w.y + dm.y * w.x);
-        z = make_float2(ep.x - od.y, ep.y + od.x);                 // E' + i O'
       }
-      data[jj] = z;
+    }
+    if (++s == ring) s = 0;
+  }
+}
+
+// Stores the finished sample q of a segment whose edges are folded.  The padded samples left of the signal are
+// stored where they will be added, before the row that adds them; those right of it are added to what an earlier
+// row stored.  Pass 1 stores, pass 2 adds; both happen within the first or the last segment.
+__device__ __forceinline__ void store_folded(const IfftOlaArgs& a, float* out, int64_t q, float v, int pass) {
+  const int64_t T = a.out_len;
+  const bool waits = q >= T - 1 - a.pad && q <= T - 2;
+  if (pass == 1) {
+    if (q < 0) out[-q] = v;
+    else if (waits) out[q] = v;
+  } else if (q >= T) {
+    const int64_t m = 2 * T - 2 - q;  // the sample that q is the mirror image of
+    if (m >= T - 1 - a.pad && m <= T - 2) out[m] += v;
+  } else if (q >= 0 && !waits) {
+    out[q] = q >= 1 && q <= a.pad ? v + out[q] : v;
+  }
+}
+
+// One row of finished samples, by one warp, two samples per lane (hop is even).  pass: 0 away from folded edges.
+template <bool kNorm>
+__device__ __forceinline__ void emit_row_pairs(const IfftOlaArgs& a, const float2* slots, int slot_floats,
+                                               const float* win, int ring, int s, int i_hi, int i_lo, int64_t q0,
+                                               float* out, int lane, int pass) {
+  constexpr int N = 4;
+  const bool paired = pass == 0 && q0 >= 0 && q0 + a.hop <= a.out_len && (reinterpret_cast<uintptr_t>(out + q0) & 7) == 0;
+  for (int c = 0; c < a.hop; c += 64 * N) {
+    const int j = c + 2 * lane;
+    float2 v[N], e[N];
+    if (c + 64 * N <= a.hop && (i_hi + 1) * a.hop <= a.n_fft)
+      sum_pairs<N, true, kNorm>(slots, slot_floats, win, a.n_fft, a.hop, ring, s, i_hi, i_lo, j, v, e);
+    else
+      sum_pairs<N, false, kNorm>(slots, slot_floats, win, a.n_fft, a.hop, ring, s, i_hi, i_lo, j, v, e);
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      if (j + 64 * u >= a.hop) break;
+      if (kNorm) {
+        v[u].x = e[u].x > 1e-11f ? v[u].x / e[u].x : 0.f;
+        v[u].y = e[u].y > 1e-11f ? v[u].y / e[u].y : 0.f;
+      }
+      const int64_t q = q0 + j + 64 * u;
+      if (paired) {
+        *reinterpret_cast<float2*>(out + q) = v[u];
+      } else if (kNorm || pass == 0) {
+        if (q >= 0 && q < a.out_len) out[q] = v[u].x;
+        if (q + 1 >= 0 && q + 1 < a.out_len) out[q + 1] = v[u].y;
+      } else {
+        store_folded(a, out, q, v[u].x, pass);
+        store_folded(a, out, q + 1, v[u].y, pass);
+      }
+    }
+  }
+}
+
+// Spectrum -> signal.  A CTA owns a run of rows (of `hop` samples), walks the frames that cover it, a batch of
+// one frame per lane group at a time, and adds each finished row up from the ring of the last frames in shared
+// memory.  Neighbouring CTAs both transform the reach - 1 frames between them; in return the frames stay on
+// the chip, which takes 8 * n_fft / hop bytes of traffic off every sample.  Bound by instruction issue, at the
+// 16 warps per SM that the ring leaves room for; two CTAs of 8 overlap one's transforms with the other's
+// barriers and loads.
+// 16 x 1 Mi samples, n_fft 2048, hop 512 (336 MB): 591 us with the frames written to memory and gathered
+// by a second kernel, 148 us so.
+// 16 x 240007 samples, n_fft 1024, hop 256, bins-major spectrum (77 MB): 247 us, 55 us so.
+template <int LH>
+__global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const IfftOlaArgs a, const OlaPlan pl) {
+  using F = WarpFft<LH>;
+  extern __shared__ float2 smem[];
+  float2* tw = smem;
+  float2* split = tw + F::h;
+  float* win = reinterpret_cast<float*>(split + F::h / 2);
+  float2* slots = reinterpret_cast<float2*>(win + F::n);
+  F::fill_tables(tw, split);
+  for (int j = threadIdx.x; j < F::n; j += blockDim.x) win[j] = window_at(a.window, j);
+  __syncthreads();
+
+  const int b = blockIdx.x / pl.segments, seg = blockIdx.x % pl.segments;
+  const int64_t row0 = pl.row_base + pl.rows * seg / pl.segments;
+  const int64_t row1 = pl.row_base + pl.rows * (seg + 1) / pl.segments;
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+  const int sub = lane / F::L, t = lane % F::L;
+  const int batch = warps * F::kPerWarp;             // frames transformed together
+  const int64_t f_begin = row0 > pl.reach - 1 ? row0 - (pl.reach - 1) : 0;
+  const int64_t f_end = row1 < a.n_frames ? row1 : a.n_frames;
+  const float2* spec = reinterpret_cast<const float2*>(a.spec) + b * a.stride_b;
+  float* out = a.out + b * a.out_len;
+  const int64_t T = a.out_len;
+  const bool at_edge = a.fold_reflect && (seg == 0 || seg == pl.segments - 1);
+  const bool direct = a.stride_f == 1;
+
+  int64_t f0 = f_begin, e0 = row0;
+  int slot0 = 0;                                     // ring slot of frame f0
+  for (;;) {
+    const int nf = f_end - f0 < batch ? static_cast<int>(f_end - f0) : batch;  // may be <= 0: rows without frames
+    if (!direct) {
+      // bins of neighbouring frames are (usually) neighbours in memory: lanes run over the frames.  The copies
+      // are asynchronous: a batch of spectra is in flight at once without a register held for it.
+      const int f = static_cast<int>(threadIdx.x) % batch, step = static_cast<int>(blockDim.x) / batch;
+      if (f < nf) {
+        const float2* src = spec + (f0 + f) * a.stride_t;
+        const int s = slot0 + f;
+        float2* slot = slots + (s >= pl.ring ? s - pl.ring : s) * F::kSlot;
+        for (int k = static_cast<int>(threadIdx.x) / batch; k <= F::h; k += step) copy_async<8>(slot + k, src + k * a.stride_f);
+      }
+      copy_async_wait();
+      __syncthreads();
+    }
+    if (warp * F::kPerWarp < nf) {
+      const int mine = warp * F::kPerWarp + sub;
+      const int s = slot0 + mine;
+      float2* slot = slots + (s >= pl.ring ? s - pl.ring : s) * F::kSlot;
+      // a group without a frame of its own repeats the last one into a slot that nothing reads
+      const int64_t f = f0 + (mine < nf ? mine : nf - 1);
+      if (LH >= 10 && direct && f + batch < f_end) {  // bring the next frame's bins as far as L2 meanwhile
+        // (n_fft 2048: 164 us without, 157 us with; shorter frames gain nothing)
+        const float2* next = spec + (f + batch) * a.stride_t;
+        for (int k = 16 * t; k <= F::h; k += 16 * F::L) prefetch_l2(next + k);
+      }
+      inverse_frame<LH>(a, direct ? spec + f * a.stride_t : nullptr, 1, tw, split,
+                        reinterpret_cast<const float2*>(win), slot, t);
     }
     __syncthreads();
-    const float2* res = fft_half_smem(data, pong, tw, h, log2h, fpc, +1.0f);
-    for (int jj = threadIdx.x; jj < h * fpc; jj += blockDim.x) {
-      const int f = jj >> log2h, m = jj & (h - 1);
-      const int frame = f0 + f;
-      if (frame >= a.n_frames) continue;
-      const float2 v = res[jj];
-      float2* out = reinterpret_cast<float2*>(a.frames + (static_cast<int64_t>(b) * a.n_frames + frame) * n);
-      out[m] = make_float2(v.x * post * a.window[2 * m], v.y * post * a.window[2 * m + 1]);
+    const bool last = f0 + batch >= f_end;
+    const int64_t e1 = last ? row1 : f0 + batch;
+
+    for (int pass = at_edge ? 1 : 2; pass <= 2; ++pass) {
+      for (int64_t row = e0 + warp; row < e1; row += warps) {
+        const int64_t q0 = row * a.hop - a.pad, q1 = q0 + a.hop;  // its output samples
+        const bool folds = at_edge && (q0 <= a.pad || q1 >= T - a.pad);
+        if (pass == 1) {  // rows that hold samples to store for later
+          if (q0 >= 0 && (q1 < T - a.pad || q0 > T - 2)) continue;
+        } else if (folds && (q1 <= 0 || (q0 >= T - 1 - a.pad && q1 < T))) {
+          continue;       // rows that held nothing else
+        }
+        const int i_lo = row < a.n_frames ? 0
+                         : row - a.n_frames + 1 < pl.reach ? static_cast<int>(row - a.n_frames + 1) : pl.reach;
+        const int i_hi = row < pl.reach - 1 ? static_cast<int>(row) : pl.reach - 1;
+        int s = i_lo < pl.reach ? slot0 + static_cast<int>(row - f0) : 0;  // slot of frame `row`
+        if (s >= pl.ring) s -= pl.ring;
+        if ((a.hop & 1) == 0) {
+          if (a.normalize_envelope)
+            emit_row_pairs<true>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, 0);
+          else
+            emit_row_pairs<false>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, folds ? pass : 0);
+          continue;
+        }
+        for (int j = lane; j < a.hop; j += 32) {
+          float v = 0.f, e = 0.f;
+          for (int i = i_hi; i >= i_lo; --i) {       // frame row - i, in frame order
+            const int si = s - i < 0 ? s - i + pl.ring : s - i, o = j + i * a.hop;
+            if (o < F::n) {
+              v += reinterpret_cast<const float*>(slots + si * F::kSlot)[o];
+              if (a.normalize_envelope) e += win[o] * win[o];
+            }
+          }
+          if (a.normalize_envelope) v = e > 1e-11f ? v / e : 0.f;
+          if (folds) store_folded(a, out, q0 + j, v, pass);
+          else if (q0 + j >= 0 && q0 + j < T) out[q0 + j] = v;
+        }
+      }
+      if (pass == 1) __syncthreads();
     }
+    if (last) break;
+    f0 += batch;
+    slot0 += batch;
+    if (slot0 >= pl.ring) slot0 -= pl.ring;
+    if (e1 > e0) e0 = e1;
+    __syncthreads();
+  }
+}
+
+// Spectrum -> windowed frames in global memory (only where ifft_ola_kernel cannot run).
+template <int LH>
+__global__ void __launch_bounds__(256, LH <= 8 ? 3 : LH <= 10 ? 2 : 1)
+    ifft_frames_kernel(const IfftOlaArgs a, float* frames, int64_t total) {
+  using F = WarpFft<LH>;
+  extern __shared__ float2 smem[];
+  float2* tw = smem;
+  float2* split = tw + F::h;
+  float* win = reinterpret_cast<float*>(split + F::h / 2);
+  float2* slots = reinterpret_cast<float2*>(win + F::n);
+  F::fill_tables(tw, split);
+  for (int j = threadIdx.x; j < F::n; j += blockDim.x) win[j] = window_at(a.window, j);
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int sub = (threadIdx.x & 31) / F::L, t = threadIdx.x % F::L;
+  float2* slot = slots + (warp * F::kPerWarp + sub) * F::kSlot;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * warps * F::kPerWarp;
+  for (int64_t i0 = (static_cast<int64_t>(blockIdx.x) * warps + warp) * F::kPerWarp; i0 < total; i0 += stride) {
+    const int64_t i = i0 + sub < total ? i0 + sub : total - 1;
+    const int64_t b = i / a.n_frames, f = i - b * a.n_frames;
+    const float2* spec = reinterpret_cast<const float2*>(a.spec) + b * a.stride_b + f * a.stride_t;
+    inverse_frame<LH>(a, spec, a.stride_f, tw, split, reinterpret_cast<const float2*>(win), slot, t);
+    __syncwarp();
+    if (i0 + sub < total) {
+      float2* dst = reinterpret_cast<float2*>(frames + i * F::n);
+      for (int m = t; m < F::h; m += F::L) dst[m] = slot[m];
+    }
+    __syncwarp();
   }
 }
 
@@ -253,9 +458,9 @@ __device__ __forceinline__ float ola_at(const float* frames, int64_t p, int n_ff
   return acc;
 }
 
-__global__ void __launch_bounds__(256) ola_gather_kernel(const OlaArgs a) {
+__global__ void __launch_bounds__(256) ola_gather_kernel(const IfftOlaArgs a, const float* all_frames) {
   const int b = blockIdx.y;
-  const float* frames = a.frames + static_cast<int64_t>(b) * a.n_frames * a.n_fft;
+  const float* frames = all_frames + static_cast<int64_t>(b) * a.n_frames * a.n_fft;
   float* out = a.out + static_cast<int64_t>(b) * a.out_len;
   const int64_t T = a.out_len;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -283,19 +488,145 @@ int ilog2(int n) {
 
 bool valid_nfft(int n) { return n >= 8 && n <= kStftMaxNfft && (n & (n - 1)) == 0; }
 
-// Frames handled together by one CTA iteration and the grid: enough frames per iteration to give
-// every thread butterflies, enough CTAs to fill the GPU a few times over, each looping over frames.
-void frame_grid(int n_fft, int n_frames, int batch, int* fpc, int* grid_x, size_t* smem) {
-  const int h = n_fft / 2;
-  int f = 2048 / h;  // 256 threads, h/4 radix-4 groups per frame and pass: two groups per thread
-  if (f < 1) f = 1;
-  if (f > 8) f = 8;
-  *fpc = f;
-  int64_t want = (static_cast<int64_t>(n_frames) + f - 1) / f;
-  int64_t cap = (148 * 8 + batch - 1) / batch;
-  if (cap < 1) cap = 1;
-  *grid_x = static_cast<int>(want < cap ? want : cap);
-  *smem = (static_cast<size_t>(h) + 2 * static_cast<size_t>(f) * h) * sizeof(float2);  // <= 48 KB at n_fft 4096
+// Dynamic shared memory above 48 KB has to be asked for, once per kernel and device.
+cudaError_t allow_smem(const void* kernel, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = uint64_t(1) << (dev & 63);
+  if (dev < 64 && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem));
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
+template <int LH>
+size_t table_bytes() { return WarpFft<LH>::kTables * sizeof(float2) + WarpFft<LH>::n * sizeof(float); }
+
+// Warps per CTA and grid of the frame-parallel kernels: as many resident CTAs as fit, each looping over
+// frames; calls too small for that spread over the SMs in CTAs of at least four warps, which share the work
+// of filling the tables.
+struct FrameGrid {
+  unsigned ctas;
+  int threads;
+  size_t smem;
+};
+template <int LH>
+FrameGrid frame_grid(int64_t total, size_t extra) {
+  using F = WarpFft<LH>;
+  const int64_t warps_wanted = (total + F::kPerWarp - 1) / F::kPerWarp;
+  const int warps = static_cast<int>(std::min<int64_t>(8, std::max<int64_t>(4, (warps_wanted + kSms - 1) / kSms)));
+  FrameGrid g;
+  g.threads = 32 * warps;
+  g.smem = table_bytes<LH>() + extra + static_cast<size_t>(warps) * F::kPerWarp * F::kSlot * sizeof(float2);
+  const int by_regs = LH <= 6 ? 4 : LH <= 8 ? 3 : LH <= 10 ? 2 : 1;
+  const int resident = static_cast<int>(std::min<size_t>(by_regs, kMaxSmem / (g.smem + 1024)));
+  g.ctas = static_cast<unsigned>(std::min<int64_t>((warps_wanted + warps - 1) / warps, kSms * std::max(1, resident)));
+  return g;
+}
+
+template <int LH, bool kEnvelope>
+cudaError_t run_fft_frames(const FftFramesArgs& a, cudaStream_t s) {
+  static std::atomic<uint64_t> smem_set{0};
+  const void* fn = reinterpret_cast<const void*>(fft_frames_kernel<LH, kEnvelope>);
+  cudaError_t e = allow_smem(fn, smem_set);
+  if (e != cudaSuccess) return e;
+  const int64_t total = static_cast<int64_t>(a.batch) * a.n_frames;
+  const FrameGrid g = frame_grid<LH>(total, kEnvelope ? WarpFft<LH>::n * sizeof(float) : 0);
+  fft_frames_kernel<LH, kEnvelope><<<g.ctas, g.threads, g.smem, s>>>(a, total);
+  return cudaGetLastError();
+}
+
+template <int LH>
+cudaError_t run_ifft_frames(const IfftOlaArgs& a, float* frames, cudaStream_t s) {
+  static std::atomic<uint64_t> smem_set{0};
+  const void* fn = reinterpret_cast<const void*>(ifft_frames_kernel<LH>);
+  cudaError_t e = allow_smem(fn, smem_set);
+  if (e != cudaSuccess) return e;
+  const int64_t total = static_cast<int64_t>(a.batch) * a.n_frames;
+  const FrameGrid g = frame_grid<LH>(total, 0);
+  ifft_frames_kernel<LH><<<g.ctas, g.threads, g.smem, s>>>(a, frames, total);
+  return cudaGetLastError();
+}
+
+// Geometry of the fused inverse: the most warps whose frames, with the reach - 1 frames before them, fit
+// shared memory; fewer if that leaves SMs without a CTA.  threads == 0: this problem takes the two-kernel path,
+// because a batch would be shorter than the overlap (tiny hops: neighbours would mostly repeat each other's
+// frames) or because the signal is so short that the two folded edges meet.
+struct OlaGrid {
+  OlaPlan plan;
+  int threads = 0;
+  size_t smem = 0;
+};
+template <int LH>
+OlaGrid ola_grid(const IfftOlaArgs& a) {
+  using F = WarpFft<LH>;
+  OlaGrid g;
+  OlaPlan& pl = g.plan;
+  const bool fold = a.fold_reflect != 0;
+  const int64_t reach = (static_cast<int64_t>(F::n) + a.hop - 1) / a.hop;
+  if ((fold && a.out_len < F::n + 2) || a.hop > (1 << 24)) return g;
+  const int64_t end = a.out_len + a.pad + (fold ? a.pad : 0);
+  pl.row_base = fold ? 0 : a.pad / a.hop;
+  pl.rows = (end + a.hop - 1) / a.hop - pl.row_base;
+  pl.reach = static_cast<int>(reach);
+  // two CTAs of 8 warps per SM before one of 16, that before whatever fits
+  static const int kChoices[][2] = {{8, 2}, {16, 1}, {8, 1}, {4, 1}};
+  for (const auto& choice : kChoices) {
+    const int warps = choice[0];
+    int resident = choice[1];
+    if (LH >= 11 && warps * resident > 8) continue;  // 255 registers
+    const int64_t batch = warps * F::kPerWarp;
+    const int64_t ring = batch + reach - 1;
+    const size_t smem = table_bytes<LH>() + static_cast<size_t>(ring) * F::kSlot * sizeof(float2);
+    if (batch < reach || resident * (smem + 1024) > kSmemPerSm) continue;
+    // a folded edge lies within one segment: reach + 1 rows are enough for either
+    const int64_t min_rows = std::max<int64_t>(fold ? reach + 1 : 1, batch - (reach - 1));
+    int64_t segments = std::max<int64_t>(1, pl.rows / min_rows);
+    segments = std::max<int64_t>(1, std::min<int64_t>(segments, static_cast<int64_t>(kSms) * resident / a.batch));
+    if (segments * a.batch > 0x7FFFFFFF) continue;
+    pl.segments = static_cast<int>(segments);
+    pl.ring = static_cast<int>(ring);
+    g.threads = 32 * warps;
+    g.smem = smem;
+    break;
+  }
+  return g;
+}
+
+template <int LH>
+cudaError_t run_ifft_ola(const IfftOlaArgs& a, const OlaGrid& g, cudaStream_t s) {
+  static std::atomic<uint64_t> smem_set{0};
+  const void* fn = reinterpret_cast<const void*>(ifft_ola_kernel<LH>);
+  cudaError_t e = allow_smem(fn, smem_set);
+  if (e != cudaSuccess) return e;
+  ifft_ola_kernel<LH><<<static_cast<unsigned>(g.plan.segments) * a.batch, g.threads, g.smem, s>>>(a, g.plan);
+  return cudaGetLastError();
+}
+
+// Calls f(std::integral_constant<int, log2(n_fft / 2)>).
+template <typename R, typename Fn>
+R for_size(int n_fft, Fn&& f) {
+  switch (ilog2(n_fft / 2)) {
+    case 2: return f(std::integral_constant<int, 2>{});
+    case 3: return f(std::integral_constant<int, 3>{});
+    case 4: return f(std::integral_constant<int, 4>{});
+    case 5: return f(std::integral_constant<int, 5>{});
+    case 6: return f(std::integral_constant<int, 6>{});
+    case 7: return f(std::integral_constant<int, 7>{});
+    case 8: return f(std::integral_constant<int, 8>{});
+    case 9: return f(std::integral_constant<int, 9>{});
+    case 10: return f(std::integral_constant<int, 10>{});
+    default: return f(std::integral_constant<int, 11>{});
+  }
+}
+
+OlaGrid ola_grid_for(const IfftOlaArgs& a) {
+  return for_size<OlaGrid>(a.n_fft, [&](auto lh) { return ola_grid<decltype(lh)::value>(a); });
+}
+
+bool valid(const IfftOlaArgs& a) {
+  return valid_nfft(a.n_fft) && a.batch > 0 && a.n_frames > 0 && a.hop > 0 && a.out_len > 0;
 }
 
 }  // namespace
@@ -303,29 +634,30 @@ void frame_grid(int n_fft, int n_frames, int batch, int* fpc, int* grid_x, size_
 cudaError_t launch_fft_frames(const FftFramesArgs& a, cudaStream_t s) {
   if (!valid_nfft(a.n_fft) || a.batch <= 0 || a.n_frames <= 0) return cudaErrorInvalidValue;
   note_launch();
-  int fpc, gx;
-  size_t smem;
-  frame_grid(a.n_fft, a.n_frames, a.batch, &fpc, &gx, &smem);
-  fft_frames_kernel<<<dim3(gx, a.batch), 256, smem, s>>>(a, ilog2(a.n_fft / 2), fpc);
-  return cudaGetLastError();
+  return for_size<cudaError_t>(a.n_fft, [&](auto lh) {
+    return a.divide_envelope ? run_fft_frames<decltype(lh)::value, true>(a, s)
+                             : run_fft_frames<decltype(lh)::value, false>(a, s);
+  });
 }
 
-cudaError_t launch_ifft_frames(const IfftFramesArgs& a, cudaStream_t s) {
-  if (!valid_nfft(a.n_fft) || a.batch <= 0 || a.n_frames <= 0) return cudaErrorInvalidValue;
-  note_launch();
-  int fpc, gx;
-  size_t smem;
-  frame_grid(a.n_fft, a.n_frames, a.batch, &fpc, &gx, &smem);
-  ifft_frames_kernel<<<dim3(gx, a.batch), 256, smem, s>>>(a, ilog2(a.n_fft / 2), fpc);
-  return cudaGetLastError();
+int64_t ifft_ola_scratch(const IfftOlaArgs& a) {
+  if (!valid(a) || ola_grid_for(a).threads > 0) return 0;
+  return static_cast<int64_t>(a.batch) * a.n_frames * a.n_fft;
 }
 
-cudaError_t launch_ola_gather(const OlaArgs& a, cudaStream_t s) {
-  if (a.batch <= 0 || a.out_len <= 0) return cudaErrorInvalidValue;
-  note_launch();
-  int64_t blocks = (a.out_len + 255) / 256;
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  ola_gather_kernel<<<dim3(static_cast<unsigned>(blocks), a.batch), 256, 0, s>>>(a);
+cudaError_t launch_ifft_ola(const IfftOlaArgs& a, float* scratch, cudaStream_t s) {
+  if (!valid(a)) return cudaErrorInvalidValue;
+  const OlaGrid g = ola_grid_for(a);
+  if (g.threads > 0) {
+    note_launch();
+    return for_size<cudaError_t>(a.n_fft, [&](auto lh) { return run_ifft_ola<decltype(lh)::value>(a, g, s); });
+  }
+  note_launch(2);
+  cudaError_t e =
+      for_size<cudaError_t>(a.n_fft, [&](auto lh) { return run_ifft_frames<decltype(lh)::value>(a, scratch, s); });
+  if (e != cudaSuccess) return e;
+  const int64_t blocks = std::min<int64_t>((a.out_len + 255) / 256, kSms * 8);
+  ola_gather_kernel<<<dim3(static_cast<unsigned>(blocks), a.batch), 256, 0, s>>>(a, scratch);
   return cudaGetLastError();
 }
 

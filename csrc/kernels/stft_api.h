@@ -1,17 +1,15 @@
 // Launchers of the STFT / iSTFT kernels (plain C++ header).
 //
-// Two kernels cover forward and backward of both transforms:
-//   frames -> spectrum  (fft_frames):  one CTA per (batch, frame) loads n_fft
-//       samples (reflect padding or an envelope division fused into the load),
-//       multiplies by the window, runs a shared-memory radix-4 Stockham FFT and writes
-//       the n_fft/2+1 one-sided bins.
-//   spectrum -> frames  (ifft_frames): one CTA per (batch, frame) loads the
-//       one-sided bins (Hermitian-extended for an inverse real FFT, or
-//       zero-extended for the adjoint of the forward transform), runs the
-//       inverse FFT, multiplies by the window and writes a real frame; a gather
-//       kernel (ola_gather) then overlap-adds the frames without atomics and
-//       either folds the reflect padding back (STFT backward) or divides by the
-//       window envelope and trims (iSTFT forward).
+// Frames -> spectrum (fft_frames): a group of lanes per (batch, frame) loads n_fft samples (reflect
+//     padding or an envelope division fused into the load), multiplies by the window, transforms in
+//     registers and writes the n_fft/2+1 one-sided bins.
+// Spectrum -> signal (ifft_ola): a CTA owns a run of output samples, inverse-transforms every frame
+//     that covers it into shared memory and adds the overlapping frames up from there, in frame
+//     order: the frames never travel to global memory.  It either folds the reflect padding back
+//     (STFT backward) or divides by the window envelope and trims (iSTFT forward).
+// Where the overlapping frames of a sample do not fit shared memory (very small hops) or the signal
+// is so short that both folded edges meet, ifft_frames writes the windowed frames to a buffer and
+// ola_gather adds them up without atomics.
 #pragma once
 
 #include <cuda_runtime_api.h>
@@ -23,43 +21,43 @@ namespace kern {
 
 constexpr int kStftMaxNfft = 4096;
 
+// A window of `len` samples centred (from `left` on) in n_fft zeros.
+struct StftWindow {
+  const float* data;
+  int len, left;
+};
+
 struct FftFramesArgs {
   const float* signal;   // [batch, signal_len]
   int64_t signal_len;
-  const float* window;   // [n_fft] (already padded to n_fft)
+  StftWindow window;
   float* out;            // [batch, n_frames, n_fft/2+1] interleaved complex
   int batch, n_frames, n_fft, hop;
   int pad;               // frame f starts at f*hop - pad in signal coordinates
-  int reflect;           // 1: indices outside [0, signal_len) are reflected; 0: they read as zero
-  int divide_envelope;   // 1: each sample is divided by the window-square envelope first (iSTFT backward)
+  int reflect;           // 1: indices outside [0, signal_len) are reflected once; 0: they read as zero
+  int divide_envelope;   // 1 (iSTFT backward): each sample is divided by the window-square envelope first, and
+                         // bins 1..n_fft/2-1 are doubled, DC and Nyquist made real
   float scale;           // multiplied into every bin
-  int hermitian_weights; // 1: bins 1..n_fft/2-1 are additionally doubled (iSTFT backward)
 };
 
-struct IfftFramesArgs {
+struct IfftOlaArgs {
   const float* spec;     // complex, addressed with the strides below (in complex elements)
   int64_t stride_b, stride_f, stride_t;
-  const float* window;   // [n_fft]
-  float* frames;         // [batch, n_frames, n_fft] real
-  int batch, n_frames, n_fft;
+  StftWindow window;
+  float* out;            // [batch, out_len]
+  int64_t out_len;
+  int batch, n_frames, n_fft, hop;
   int hermitian;         // 1: inverse real FFT (mirror bins); 0: upper bins are zero (adjoint of forward)
   float scale;
-};
-
-struct OlaArgs {
-  const float* frames;   // [batch, n_frames, n_fft]
-  const float* window;   // [n_fft] (envelope mode)
-  float* out;            // [batch, out_len]
-  int batch, n_frames, n_fft, hop;
-  int64_t out_len;
   int pad;               // output sample t corresponds to padded position t + pad
   int fold_reflect;      // 1: add the mirrored padded regions back (adjoint of reflect padding)
   int normalize_envelope;// 1: divide by sum of window^2 over the covering frames
 };
 
 cudaError_t launch_fft_frames(const FftFramesArgs& a, cudaStream_t s);
-cudaError_t launch_ifft_frames(const IfftFramesArgs& a, cudaStream_t s);
-cudaError_t launch_ola_gather(const OlaArgs& a, cudaStream_t s);
+// Floats of scratch that launch_ifft_ola needs for this problem (0: it runs as one fused kernel).
+int64_t ifft_ola_scratch(const IfftOlaArgs& a);
+cudaError_t launch_ifft_ola(const IfftOlaArgs& a, float* scratch, cudaStream_t s);
 
 }  // namespace kern
 }  // namespace mccl

@@ -32,14 +32,13 @@ void check_common(int64_t n_fft, int64_t hop, int64_t win_length, const at::Tens
                     "the native STFT serves the CUDA backend (got '" << backend << "')");
 }
 
-// window of win_length centred inside n_fft zeros, fp32, on `like`'s device
-at::Tensor prepare_window(const at::Tensor& window, int64_t n_fft, const at::Tensor& like) {
-  at::Tensor w = window.to(like.device(), at::kFloat).contiguous();
-  if (w.numel() == n_fft) return w;
-  at::Tensor padded = at::zeros({n_fft}, w.options());
-  const int64_t left = (n_fft - w.numel()) / 2;
-  padded.narrow(0, left, w.numel()).copy_(w);
-  return padded;
+// fp32 and contiguous on `like`'s device; the kernels centre its win_length samples in n_fft zeros
+at::Tensor prepare_window(const at::Tensor& window, const at::Tensor& like) {
+  return window.to(like.device(), at::kFloat).contiguous();
+}
+kern::StftWindow centred(const at::Tensor& w, int64_t n_fft) {
+  const int64_t len = w.numel();
+  return {w.data_ptr<float>(), static_cast<int>(len), static_cast<int>((n_fft - len) / 2)};
 }
 
 at::Tensor as_batch(const at::Tensor& x) {
@@ -57,6 +56,14 @@ void spec_strides(const at::Tensor& spec, int64_t n_fft, int64_t& sb, int64_t& s
   sb = spec.stride(0);
   sf = spec.stride(1);
   st = spec.stride(2);
+}
+
+void run_ifft_ola(const kern::IfftOlaArgs& a, const at::Tensor& out) {
+  at::Tensor scratch;
+  const int64_t floats = kern::ifft_ola_scratch(a);
+  if (floats > 0) scratch = at::empty({floats}, out.options());
+  STFT_CK(kern::launch_ifft_ola(a, floats > 0 ? scratch.data_ptr<float>() : nullptr,
+                                at::cuda::getCurrentCUDAStream()));
 }
 
 }  // namespace
@@ -80,12 +87,12 @@ at::Tensor stft_forward(const at::Tensor& waveform, const at::Tensor& window, in
   MCCL_CHECK_TENSOR(!center || T > pad, "reflect padding needs a signal longer than n_fft/2");
   const int64_t frames = stft_num_frames(T, n_fft, hop, center);
   c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor w = prepare_window(window, n_fft, x);
+  at::Tensor w = prepare_window(window, x);
   at::Tensor out = at::empty({B, frames, n_fft / 2 + 1}, x.options().dtype(at::kComplexFloat));
   kern::FftFramesArgs a{};
   a.signal = x.data_ptr<float>();
   a.signal_len = T;
-  a.window = w.data_ptr<float>();
+  a.window = centred(w, n_fft);
   a.out = reinterpret_cast<float*>(out.data_ptr());
   a.batch = static_cast<int>(B);
   a.n_frames = static_cast<int>(frames);
@@ -95,7 +102,6 @@ at::Tensor stft_forward(const at::Tensor& waveform, const at::Tensor& window, in
   a.reflect = center ? 1 : 0;
   a.divide_envelope = 0;
   a.scale = normalized ? 1.0f / std::sqrt(static_cast<float>(n_fft)) : 1.0f;
-  a.hermitian_weights = 0;
   STFT_CK(kern::launch_fft_frames(a, at::cuda::getCurrentCUDAStream()));
   return out.transpose(1, 2);  // [batch, freq, frames]; frames-major storage keeps the kernel's writes coalesced
 }
@@ -108,36 +114,26 @@ at::Tensor stft_backward(const at::Tensor& grad_spec, const at::Tensor& window, 
   spec_strides(grad_spec, n_fft, sb, sf, st);
   const int64_t B = grad_spec.size(0), frames = grad_spec.size(2);
   c10::cuda::CUDAGuard guard(grad_spec.device());
-  at::Tensor w = prepare_window(window, n_fft, grad_spec);
-  at::Tensor buf = at::empty({B, frames, n_fft}, grad_spec.options().dtype(at::kFloat));
-  kern::IfftFramesArgs a{};
+  at::Tensor w = prepare_window(window, grad_spec);
+  at::Tensor out = at::empty({B, length}, grad_spec.options().dtype(at::kFloat));
+  kern::IfftOlaArgs a{};
   a.spec = reinterpret_cast<const float*>(grad_spec.data_ptr());
   a.stride_b = sb;
   a.stride_f = sf;
   a.stride_t = st;
-  a.window = w.data_ptr<float>();
-  a.frames = buf.data_ptr<float>();
+  a.window = centred(w, n_fft);
+  a.out = out.data_ptr<float>();
+  a.out_len = length;
   a.batch = static_cast<int>(B);
   a.n_frames = static_cast<int>(frames);
   a.n_fft = static_cast<int>(n_fft);
+  a.hop = static_cast<int>(hop);
   a.hermitian = 0;  // adjoint of the one-sided forward transform: upper bins contribute nothing
   a.scale = normalized ? 1.0f / std::sqrt(static_cast<float>(n_fft)) : 1.0f;
-  auto stream = at::cuda::getCurrentCUDAStream();
-  STFT_CK(kern::launch_ifft_frames(a, stream));
-  at::Tensor out = at::empty({B, length}, buf.options());
-  kern::OlaArgs o{};
-  o.frames = buf.data_ptr<float>();
-  o.window = w.data_ptr<float>();
-  o.out = out.data_ptr<float>();
-  o.batch = static_cast<int>(B);
-  o.n_frames = static_cast<int>(frames);
-  o.n_fft = static_cast<int>(n_fft);
-  o.hop = static_cast<int>(hop);
-  o.out_len = length;
-  o.pad = center ? static_cast<int>(n_fft / 2) : 0;
-  o.fold_reflect = center ? 1 : 0;
-  o.normalize_envelope = 0;
-  STFT_CK(kern::launch_ola_gather(o, stream));
+  a.pad = center ? static_cast<int>(n_fft / 2) : 0;
+  a.fold_reflect = center ? 1 : 0;
+  a.normalize_envelope = 0;
+  run_ifft_ola(a, out);
   return out;
 }
 
@@ -150,36 +146,26 @@ at::Tensor istft_forward(const at::Tensor& spec, const at::Tensor& window, int64
   const int64_t B = spec.size(0), frames = spec.size(2);
   MCCL_CHECK_TENSOR(length >= 1, "length must be >= 1");
   c10::cuda::CUDAGuard guard(spec.device());
-  at::Tensor w = prepare_window(window, n_fft, spec);
-  at::Tensor buf = at::empty({B, frames, n_fft}, spec.options().dtype(at::kFloat));
-  kern::IfftFramesArgs a{};
+  at::Tensor w = prepare_window(window, spec);
+  at::Tensor out = at::empty({B, length}, spec.options().dtype(at::kFloat));
+  kern::IfftOlaArgs a{};
   a.spec = reinterpret_cast<const float*>(spec.data_ptr());
   a.stride_b = sb;
   a.stride_f = sf;
   a.stride_t = st;
-  a.window = w.data_ptr<float>();
-  a.frames = buf.data_ptr<float>();
+  a.window = centred(w, n_fft);
+  a.out = out.data_ptr<float>();
+  a.out_len = length;
   a.batch = static_cast<int>(B);
   a.n_frames = static_cast<int>(frames);
   a.n_fft = static_cast<int>(n_fft);
+  a.hop = static_cast<int>(hop);
   a.hermitian = 1;
   a.scale = (normalized ? std::sqrt(static_cast<float>(n_fft)) : 1.0f) / static_cast<float>(n_fft);
-  auto stream = at::cuda::getCurrentCUDAStream();
-  STFT_CK(kern::launch_ifft_frames(a, stream));
-  at::Tensor out = at::empty({B, length}, buf.options());
-  kern::OlaArgs o{};
-  o.frames = buf.data_ptr<float>();
-  o.window = w.data_ptr<float>();
-  o.out = out.data_ptr<float>();
-  o.batch = static_cast<int>(B);
-  o.n_frames = static_cast<int>(frames);
-  o.n_fft = static_cast<int>(n_fft);
-  o.hop = static_cast<int>(hop);
-  o.out_len = length;
-  o.pad = center ? static_cast<int>(n_fft / 2) : 0;
-  o.fold_reflect = 0;
-  o.normalize_envelope = 1;
-  STFT_CK(kern::launch_ola_gather(o, stream));
+  a.pad = center ? static_cast<int>(n_fft / 2) : 0;
+  a.fold_reflect = 0;
+  a.normalize_envelope = 1;
+  run_ifft_ola(a, out);
   return out;
 }
 
@@ -190,12 +176,12 @@ at::Tensor istft_backward(const at::Tensor& grad_waveform, const at::Tensor& win
   at::Tensor g = as_batch(grad_waveform);
   const int64_t B = g.size(0), T = g.size(1);
   c10::cuda::CUDAGuard guard(g.device());
-  at::Tensor w = prepare_window(window, n_fft, g);
+  at::Tensor w = prepare_window(window, g);
   at::Tensor out = at::empty({B, n_frames, n_fft / 2 + 1}, g.options().dtype(at::kComplexFloat));
   kern::FftFramesArgs a{};
   a.signal = g.data_ptr<float>();
   a.signal_len = T;
-  a.window = w.data_ptr<float>();
+  a.window = centred(w, n_fft);
   a.out = reinterpret_cast<float*>(out.data_ptr());
   a.batch = static_cast<int>(B);
   a.n_frames = static_cast<int>(n_frames);
@@ -205,7 +191,6 @@ at::Tensor istft_backward(const at::Tensor& grad_waveform, const at::Tensor& win
   a.reflect = 0;
   a.divide_envelope = 1;
   a.scale = (normalized ? std::sqrt(static_cast<float>(n_fft)) : 1.0f) / static_cast<float>(n_fft);
-  a.hermitian_weights = 1;
   STFT_CK(kern::launch_fft_frames(a, at::cuda::getCurrentCUDAStream()));
   return out.transpose(1, 2);
 }

@@ -107,3 +107,68 @@ def test_rejects_unsupported_sizes(cuda_device):
     # "auto" falls back to ATen for sizes the kernels do not cover
     out = stft(x, n_fft=1000, hop_length=250, win_length=1000, window=torch.hann_window(1000, device=cuda_device))
     assert out.shape[1] == 501
+
+
+def _rel(got, ref):
+    got, ref = got.detach().cpu(), ref.detach()
+    return float((got - ref).norm() / ref.norm())
+
+
+# Every transform length, frames that fill a warp or leave lanes without one, one segment or many, odd lengths (rows off
+# an 8-byte boundary), hops that do not divide n_fft, hops so small that the inverse takes its two-kernel path, and
+# signals at and below the length from which the folded edges are disjoint (n_fft + 2).
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_fft,hop,samples,batch", [
+    (8, 2, 61, 3), (8, 4, 10, 1), (16, 4, 1001, 2), (16, 1, 77, 2), (32, 8, 4099, 1), (64, 20, 999, 3),
+    (128, 32, 30011, 2), (256, 80, 20001, 5), (512, 128, 16000, 1), (512, 512, 5000, 2), (1024, 256, 1025, 2),
+    (1024, 256, 1026, 2), (1024, 320, 120007, 3), (1024, 16, 9001, 1), (2048, 512, 1030, 2), (2048, 512, 300001, 4),
+    (4096, 1024, 4098, 1), (4096, 1024, 200003, 2), (4096, 1280, 50001, 2)])
+@pytest.mark.parametrize("frames_major", [True, False])
+def test_transforms_match_float64(cuda_device, n_fft, hop, samples, batch, frames_major):
+    gen = torch.Generator().manual_seed(n_fft + hop)
+    win_len = n_fft - n_fft // 8
+    w = 0.1 + torch.rand(win_len, generator=gen)  # asymmetric, no zeros inside
+    x = torch.randn(batch, samples, generator=gen)
+    kw = dict(n_fft=n_fft, hop_length=hop, win_length=win_len)
+    frames = 1 + samples // hop
+    g = torch.randn(batch, n_fft // 2 + 1, frames, dtype=torch.complex64, generator=gen)
+    spec = torch.randn(batch, n_fft // 2 + 1, frames, dtype=torch.complex64, generator=gen)
+    # relative to the norm of the whole result: log2(n_fft) + 1 <= 13 roundings of 6e-8 in the transform, a few more
+    # for the table entries, the window and the sum of the overlapping frames; they add up as a random walk
+    tol = 6e-8 * 16
+
+    def layout(t):  # same values; memory order frames-major (the framework's own) or bins-major (a network's output)
+        return t.transpose(1, 2).contiguous().transpose(1, 2) if frames_major else t.contiguous()
+
+    xd = x.double().requires_grad_(True)
+    ref = torch.stft(xd, window=w.double(), center=True, return_complex=True, **kw)
+    (ref_g,) = torch.autograd.grad(ref, xd, g.to(torch.complex128))
+    xc = x.to(cuda_device).requires_grad_(True)
+    out = stft(xc, window=w.to(cuda_device), backend="cuda", **kw)
+    (out_g,) = torch.autograd.grad(out, xc, layout(g.to(cuda_device)))
+    assert _rel(out, ref) < tol
+    assert _rel(out_g, ref_g) < tol
+
+    # the inverse over samples that some frame covers (win_len < n_fft leaves gaps when hop > win_len); its gradient
+    length = min(samples, (frames - 1) * hop)
+    if hop <= win_len and length > 0:
+        sd = spec.to(torch.complex128).requires_grad_(True)
+        inv = torch.istft(sd, window=w.double(), center=True, length=length, **kw)
+        (inv_g,) = torch.autograd.grad(inv, sd, x.double()[:, :length])
+        sc = layout(spec.to(cuda_device)).requires_grad_(True)
+        got = istft(sc, window=w.to(cuda_device), length=length, backend="cuda", **kw)
+        (got_g,) = torch.autograd.grad(got, sc, x.to(cuda_device)[:, :length])
+        assert _rel(got, inv) < tol
+        assert _rel(got_g, inv_g) < tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length", [3000, 20000])  # shorter and far longer than what the frames cover
+def test_istft_beyond_the_frames_is_zero(cuda_device, length):
+    spec = torch.randn(2, 129, 100, dtype=torch.complex64, device=cuda_device)
+    w = torch.ones(256, device=cuda_device)
+    full = istft(spec, n_fft=256, hop_length=64, win_length=256, window=w, length=64 * 99 + 128, backend="cuda")
+    got = istft(spec, n_fft=256, hop_length=64, win_length=256, window=w, length=length, backend="cuda")
+    keep = min(length, full.shape[1])
+    assert torch.equal(got[:, :keep], full[:, :keep])
+    assert not got[:, keep:].any()
