@@ -922,10 +922,11 @@ c10::intrusive_ptr<c10d::Work> ProcessGroupMCCL::allreduce_topk(at::Tensor& grad
     stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   }
   {
-    // scratch: radix histograms + counters; pairs: this rank's (idx,val) list of the largest segment
+    // scratch: candidate list + counters; pairs: this rank's (idx,val) list of the largest segment
     c10::cuda::CUDAStreamGuard sg(p2p ? cp->stream : c10::cuda::getCurrentCUDAStream(dev));
-    scratch = at::empty({static_cast<int64_t>(kern::topk_scratch_bytes())}, grad.options().dtype(at::kByte));
-    pairs = at::empty({k_for(std::min(seg, n)) * 2}, grad.options().dtype(at::kInt));
+    const int64_t most = std::min(seg, n);
+    scratch = at::empty({static_cast<int64_t>(kern::topk_scratch_bytes(most, k_for(most)))}, grad.options().dtype(at::kByte));
+    if (p2p) pairs = at::empty({k_for(most) * 2}, grad.options().dtype(at::kInt));
   }
   const size_t gsz = grad.element_size();
   uint64_t sent = 0;
@@ -939,10 +940,11 @@ c10::intrusive_ptr<c10d::Work> ProcessGroupMCCL::allreduce_topk(at::Tensor& grad
     a.n = cnt;
     a.k = k;
     a.scratch = scratch.data_ptr();
-    a.pairs = pairs.data_ptr();
+    a.scratch_bytes = scratch.nbytes();
+    a.pairs = p2p ? pairs.data_ptr() : nullptr;
     a.scale = scale;
-    if (!(cp && cp->skip)) MCCL_LAUNCH_CHECK(kern::launch_topk_select(a, stream));
     if (p2p) {
+      if (!cp->skip) MCCL_LAUNCH_CHECK(kern::launch_topk_select(a, stream));
       kern::CollParams p = cp->params();
       p.ctx[0].in = pairs.data_ptr();
       p.ctx[0].out = const_cast<void*>(a.grad);
@@ -951,7 +953,7 @@ c10::intrusive_ptr<c10d::Work> ProcessGroupMCCL::allreduce_topk(at::Tensor& grad
       if (!cp->skip) MCCL_LAUNCH_CHECK(kern::launch_topk_exchange_scatter(p, a, cp->cfg(static_cast<size_t>(k) * 8 * ws), stream));
       sent += static_cast<uint64_t>(k) * 8 * (ws - 1);
     } else {
-      MCCL_LAUNCH_CHECK(kern::launch_topk_local_scatter(a, stream));
+      MCCL_LAUNCH_CHECK(kern::launch_topk_dense(a, stream));
     }
   }
   if (p2p) {

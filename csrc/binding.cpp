@@ -281,7 +281,7 @@ class EmuGroup {
     std::vector<at::Tensor> pairs;
     kern::TopkArgs a0;
     for (int r = 0; r < ws_; ++r) {
-      at::Tensor scratch = at::empty({static_cast<int64_t>(kern::topk_scratch_bytes())}, grads[r].options().dtype(at::kByte));
+      at::Tensor scratch = at::empty({static_cast<int64_t>(kern::topk_scratch_bytes(n, k))}, grads[r].options().dtype(at::kByte));
       pairs.push_back(at::empty({k * 2}, grads[r].options().dtype(at::kInt)));
       kern::TopkArgs a;
       a.grad = grads[r].data_ptr();
@@ -290,6 +290,7 @@ class EmuGroup {
       a.n = n;
       a.k = k;
       a.scratch = scratch.data_ptr();
+      a.scratch_bytes = scratch.nbytes();
       a.pairs = pairs[r].data_ptr();
       a.scale = static_cast<float>(scale);
       CK(kern::launch_topk_select(a, stream));
@@ -328,7 +329,7 @@ at::Tensor topk_select(const at::Tensor& grad, at::Tensor residual, double ratio
   const int64_t n = grad.numel();
   int64_t k = std::max<int64_t>(1, static_cast<int64_t>(std::floor(static_cast<double>(n) * ratio)));
   k = std::min(k, n);
-  at::Tensor scratch = at::empty({static_cast<int64_t>(kern::topk_scratch_bytes())}, grad.options().dtype(at::kByte));
+  at::Tensor scratch = at::empty({static_cast<int64_t>(kern::topk_scratch_bytes(n, k))}, grad.options().dtype(at::kByte));
   at::Tensor pairs = at::empty({k, 2}, grad.options().dtype(at::kInt));
   kern::TopkArgs a;
   a.grad = grad.data_ptr();
@@ -337,6 +338,7 @@ at::Tensor topk_select(const at::Tensor& grad, at::Tensor residual, double ratio
   a.n = n;
   a.k = k;
   a.scratch = scratch.data_ptr();
+  a.scratch_bytes = scratch.nbytes();
   a.pairs = pairs.data_ptr();
   a.scale = 1.f;
   CK(kern::launch_topk_select(a, at::cuda::getCurrentCUDAStream()));

@@ -14,7 +14,7 @@
 
 namespace {
 
-constexpr size_t kScratchBytes = 64 * 1024;  // >= mccl::kern::topk_scratch_bytes(), checked at set-up
+constexpr size_t kScratchBytes = 64 * 1024;  // >= mccl::kern::topk_min_scratch_bytes(), checked at set-up
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_topk_scratch[kScratchBytes];
@@ -36,7 +36,7 @@ int scratch_for_current_device(void** out) {
   if (dev < 0 || dev >= kMaxDevices) return fail(1, "device index out of range");
   std::lock_guard<std::mutex> g(g_mu);
   if (g_scratch_addr[dev] == nullptr) {
-    if (mccl::kern::topk_scratch_bytes() > kScratchBytes) return fail(2, "built-in scratch array is too small");
+    if (mccl::kern::topk_min_scratch_bytes() > kScratchBytes) return fail(2, "built-in scratch array is too small");
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_noalloc_topk_scratch);
     if (e != cudaSuccess || p == nullptr) {
@@ -100,6 +100,7 @@ extern "C" __attribute__((visibility("default"))) int mccl_topk_select_noalloc(c
   a.n = n;
   a.k = k;
   a.scratch = scratch;  // the selection starts by clearing the histograms and state it uses
+  a.scratch_bytes = kScratchBytes;
   a.pairs = pairs_out;
   a.scale = 1.0f;
   cudaError_t e = mccl::kern::launch_topk_select(a, stream);

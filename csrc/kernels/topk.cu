@@ -1,5 +1,5 @@
 // Top-k gradient compression kernels (sm_100a): exact radix select with error
-// feedback, and the fused sparse exchange + deterministic scatter-add.
+// feedback in three passes and little scratch, and the fused sparse exchange + deterministic scatter-add.
 // See topk_api.h for the pipeline.  Semantics follow the host TopKCompressor
 // (csrc/compression/compressor.cpp), which is the oracle in the tests:
 // k = max(1, floor(n*ratio)), adjusted = g + residual, ties towards the lower
@@ -618,13 +618,6 @@ __global__ void __launch_bounds__(512) topk_exchange_scatter_kernel(const __grid
   scatter_lists<kBf16>(c.out, n, lists, c.ws, k, scale, cta, nctas);
 }
 
-template <bool kBf16>
-__global__ void __launch_bounds__(512) topk_local_scatter_kernel(void* dense, int64_t n, const uint2* pairs, int64_t k,
-                                                                 float scale) {
-  const uint2* lists[1] = {pairs};
-  scatter_lists<kBf16>(dense, n, lists, 1, k, scale, blockIdx.x, gridDim.x);
-}
-
 // Blocks of the collect and compaction passes.  Every block pays a fixed price (staging flush, block
 // reduction, histogram merge, ticket), so a block gets at least 32 Ki elements: with 8 Ki per block the
 // collect pass measured 54-67 us on 8 Mi elements, almost all of it that per-block overhead.
@@ -637,10 +630,19 @@ int select_blocks(int64_t n) {
 
 }  // namespace
 
-size_t topk_scratch_bytes() { return sizeof(TopkScratch); }
+size_t topk_min_scratch_bytes() { return sizeof(TopkScratch); }
+size_t topk_scratch_bytes(int64_t n, int64_t k) {
+  return std::max(sizeof(TopkScratch), topk_fits_cluster(n) ? size_t(0) : topk_list_scratch_bytes(n, k));
+}
+
+cudaError_t launch_topk_dense(const TopkArgs& a, cudaStream_t s) {
+  if (a.n <= 0 || a.k <= 0 || a.k > a.n || a.scratch_bytes < topk_scratch_bytes(a.n, a.k)) return cudaErrorInvalidValue;
+  return launch_topk_cluster(a, true, s);
+}
 
 cudaError_t launch_topk_select(const TopkArgs& a, cudaStream_t s) {
-  if (a.n <= 0 || a.k <= 0 || a.k > a.n) return cudaErrorInvalidValue;
+  if (a.n <= 0 || a.k <= 0 || a.k > a.n || a.scratch_bytes < sizeof(TopkScratch)) return cudaErrorInvalidValue;
+  if (a.scratch_bytes >= topk_scratch_bytes(a.n, a.k)) return launch_topk_cluster(a, false, s);
   TopkScratch* sc = static_cast<TopkScratch*>(a.scratch);
   const uint32_t k = static_cast<uint32_t>(a.k);
   note_launch(7);
@@ -687,19 +689,6 @@ cudaError_t launch_topk_exchange_scatter(const CollParams& p, const TopkArgs& a,
     topk_exchange_scatter_kernel<true><<<dim3(ctas, 1), 512, 0, s>>>(p, a.n, a.k, a.scale);
   else
     topk_exchange_scatter_kernel<false><<<dim3(ctas, 1), 512, 0, s>>>(p, a.n, a.k, a.scale);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_topk_local_scatter(const TopkArgs& a, cudaStream_t s) {
-  note_launch();
-  int ctas = static_cast<int>(std::min<int64_t>(148, (a.n + 4095) / 4096));
-  if (ctas < 1) ctas = 1;
-  if (a.grad_is_bf16)
-    topk_local_scatter_kernel<true><<<ctas, 512, 0, s>>>(const_cast<void*>(a.grad), a.n,
-                                                         static_cast<const uint2*>(a.pairs), a.k, a.scale);
-  else
-    topk_local_scatter_kernel<false><<<ctas, 512, 0, s>>>(const_cast<void*>(a.grad), a.n,
-                                                          static_cast<const uint2*>(a.pairs), a.k, a.scale);
   return cudaGetLastError();
 }
 

@@ -5,13 +5,15 @@
 //            radix select on the magnitude bits, ties to the lower index);
 //            emit them as (u32 index, f32 value) pairs sorted by index;
 //            e = a with the k selected entries zeroed          (topk_select)
-//            Three passes over the data: adjust + 13-bit histogram (12 B per
-//            fp32 element), collect (4 B: per-block counts of the elements
-//            above the chosen bin, the elements inside it go to a candidate
-//            list on which the remaining 18 bits are resolved), ordered
-//            compaction (4 B).  Only if the bin holds more than k elements
-//            (heavily tied data) two more full histogram passes and a count
-//            pass run instead of the candidate refinement.
+//            One pass over the data: the elements that reach a sampled
+//            magnitude are listed on the way and selected from afterwards.
+//            Without room for the list, three passes: adjust + 13-bit
+//            histogram (12 B per fp32 element), collect (4 B: per-block
+//            counts of the elements above the chosen bin, the elements inside
+//            it go to a candidate list on which the remaining 18 bits are
+//            resolved), ordered compaction (4 B); only if the bin holds more
+//            than k elements (heavily tied data) two more full histogram
+//            passes and a count pass instead of the candidate refinement.
 //   exchange every rank pushes its k pairs into slot[rank] of every peer's
 //            arena over NVLink, release flag                    (exchange)
 //   scatter  dense = scale * sum_r sparse_r, written into g: each CTA owns a
@@ -41,23 +43,34 @@ struct TopkArgs {
   float* residual;      // n fp32, in/out
   int64_t n;
   int64_t k;
-  void* scratch;        // topk_scratch_bytes() bytes of device memory (any contents)
-  void* pairs;          // k * 8 bytes: {u32 index, f32 value}
+  void* scratch;        // device memory (any contents)
+  size_t scratch_bytes; // of it; at least topk_min_scratch_bytes()
+  void* pairs;          // k * 8 bytes: {u32 index, f32 value}; unused by launch_topk_dense
   float scale;          // applied in scatter
 };
 
-// Scratch layout: 3 histograms, the selection state, per-block counts/offsets (about 53 KB).
-size_t topk_scratch_bytes();
+// What the fastest path for this problem wants.
+size_t topk_scratch_bytes(int64_t n, int64_t k);
+// What any problem can do with: 3 histograms, the selection state, per-block counts/offsets (about 53 KB).
+size_t topk_min_scratch_bytes();
 #ifdef __CUDACC__
 __host__ __device__
 #endif
 inline size_t topk_pad(size_t bytes) { return (bytes + 127) / 128 * 128; }
 
+// Three ways, with the same results: one cluster launch while the gradient fits a cluster's shared memory; sample,
+// adjust and select (topk_cluster.cu) above that; the three-pass radix select (topk.cu) where the caller's scratch
+// has no room for the candidate list.
 cudaError_t launch_topk_select(const TopkArgs& a, cudaStream_t s);
 // p: arena parameters (ctx[].in = pairs, ctx[].out = dense gradient); count = k.
 cudaError_t launch_topk_exchange_scatter(const CollParams& p, const TopkArgs& a, LaunchCfg cfg, cudaStream_t s);
-// World size 1: dense = scale * sparse.
-cudaError_t launch_topk_local_scatter(const TopkArgs& a, cudaStream_t s);
+// World size 1: select, and grad = scale * selection.  Needs topk_scratch_bytes(n, k) of scratch.
+cudaError_t launch_topk_dense(const TopkArgs& a, cudaStream_t s);
+
+// topk_cluster.cu
+size_t topk_list_scratch_bytes(int64_t n, int64_t k);
+bool topk_fits_cluster(int64_t n);  // on any device: one launch, no scratch
+cudaError_t launch_topk_cluster(const TopkArgs& a, bool dense, cudaStream_t s);
 
 }  // namespace kern
 }  // namespace mccl

@@ -52,6 +52,7 @@ CUDA_SOURCES = [
     "kernels/reduce_ws4.cu",
     "kernels/reduce_ws8.cu",
     "kernels/topk.cu",
+    "kernels/topk_cluster.cu",
     "kernels/stft.cu",
     "kernels/adamw.cu",
     "kernels/noalloc.cu",

@@ -104,3 +104,71 @@ def test_fused_topk_allreduce_is_consistent(native, cuda_device, ws, dtype):
             dense[idx] = (dense[idx].to(dtype).float() + torch.tensor(val) * scale).to(dtype).float()
         assert torch.equal(residuals[r].cpu(), comp.residual(0))
     assert torch.equal(grads[0].float().cpu(), dense.to(dtype).float())
+
+
+def _data(kind, n, dtype):
+    gen = torch.Generator().manual_seed(n)
+    g = 1e-3 * torch.randn(n, generator=gen)
+    r = 2e-3 * torch.randn(n, generator=gen)
+    if kind == "grid":            # 16-bit values and no residual yet: ties at every magnitude
+        g, r = g.bfloat16().float(), torch.zeros(n)
+    elif kind == "sparse":        # fewer non-zeros than entries to send: zeros are sent, lowest index first
+        g, r = torch.zeros(n), torch.zeros(n)
+        g[torch.randperm(n, generator=gen)[: max(1, n // 300)]] = 1.0
+    elif kind == "rows":          # an embedding's gradient: whole rows, the rest zero
+        g, r = g * (torch.rand(n // 1024 + 1, generator=gen) < 0.05).float().repeat_interleave(1024)[:n], torch.zeros(n)
+    elif kind == "levels":        # far more ties at the threshold than a candidate list holds
+        g, r = torch.randint(-3, 4, (n,), generator=gen).float(), torch.zeros(n)
+    elif kind == "wide":          # magnitudes over the whole range of the type, infinities among them
+        r = torch.zeros(n)
+        g = torch.ldexp(1 + torch.rand(n, generator=gen), torch.randint(-140, 127, (n,), generator=gen))
+        g[:: n // 3] = float("inf")
+    return g.to(dtype), r
+
+
+# One cluster launch up to 8 x 48 Ki elements, sample + adjust + select above; sizes around that limit, around the tile of
+# 1024 and the group of tiles, odd sizes, and every kind of data for which the sampled magnitude misses (fewer than k reach
+# it, or more than the list holds).  Integer selection rule: exact.
+@pytest.mark.parametrize("n,ratio", [(1, 1.0), (7, 0.5), (393_216, 0.01), (393_217, 0.01), (786_432, 0.1), (786_433, 0.01),
+                                     (1_048_577, 0.001), (3_000_001, 0.1), (9_437_184, 0.01), (2_000_000, 1.0)])
+@pytest.mark.parametrize("kind", ["normal", "grid", "sparse", "rows", "levels", "wide"])
+def test_select_and_dense_paths_match_host_oracle(native, cuda_device, one_rank, n, ratio, kind):
+    if n < 100 and kind != "normal":
+        pytest.skip("the kinds differ for many elements only")
+    dtype = torch.bfloat16 if n % 2 == 0 and kind != "wide" else torch.float32
+    g, r = _data(kind, n, dtype)
+    adjusted = g.float() + r
+    comp, idx, val = _oracle_pairs(native, adjusted, ratio)
+    idx, val = torch.tensor(idx), torch.tensor(val)
+    # pairs
+    res = r.to(cuda_device)
+    grad = g.to(cuda_device)
+    pairs = native._topk_select(grad, res, ratio).cpu()
+    assert torch.equal(pairs[:, 0].long(), idx)
+    assert torch.equal(pairs[:, 1].view(torch.float32), val)
+    assert torch.equal(res.cpu(), comp.residual(0))
+    assert torch.equal(grad.cpu(), g)
+    # dense, from arrays that are not 16-byte aligned
+    res = torch.zeros(n + 1, device=cuda_device)[1:]
+    grad = torch.zeros(n + 1, device=cuda_device, dtype=dtype)[1:]
+    res.copy_(r)
+    grad.copy_(g)
+    one_rank.allreduce_topk(grad, res, ratio, 0.25).wait()
+    want = torch.zeros(n)
+    want[idx] = val * 0.25
+    assert torch.equal(grad.cpu(), want.to(dtype))
+    assert torch.equal(res.cpu(), comp.residual(0))
+
+
+@pytest.fixture(scope="module")
+def one_rank(cuda_device):
+    import torch.distributed as dist
+
+    import mccl_b200
+
+    created = not dist.is_initialized()
+    if created:
+        dist.init_process_group("mccl", store=dist.HashStore(), rank=0, world_size=1)
+    yield mccl_b200.get_backend(device=cuda_device)
+    if created:
+        dist.destroy_process_group()
