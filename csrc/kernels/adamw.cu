@@ -54,15 +54,33 @@ __device__ __forceinline__ void adamw_chunk(const AdamWTable& tab, const AdamWHy
     const float4* g4 = reinterpret_cast<const float4*>(g + start);
     float4* m4 = reinterpret_cast<float4*>(m + start);
     float4* v4 = reinterpret_cast<float4*>(v + start);
-    for (int64_t i = threadIdx.x; i < nvec; i += blockDim.x) {
-      float4 pp = p4[i], gg = __ldcs(g4 + i), mm = m4[i], vv = v4[i];
-      update(pp.x, gg.x, mm.x, vv.x);
-      update(pp.y, gg.y, mm.y, vv.y);
-      update(pp.z, gg.z, mm.z, vv.z);
-      update(pp.w, gg.w, mm.w, vv.w);
-      p4[i] = pp;
-      m4[i] = mm;
-      v4[i] = vv;
+    // kDeep vectors of each of the four arrays are in flight before the first is used
+    constexpr int kDeep = 2;
+    for (int64_t i0 = threadIdx.x; i0 < nvec; i0 += kDeep * blockDim.x) {
+      float4 pp[kDeep], gg[kDeep], mm[kDeep], vv[kDeep];
+#pragma unroll
+      for (int u = 0; u < kDeep; ++u) {
+        const int64_t i = i0 + u * blockDim.x;
+        if (i < nvec) {
+          pp[u] = p4[i];
+          gg[u] = __ldcs(g4 + i);
+          mm[u] = m4[i];
+          vv[u] = v4[i];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kDeep; ++u) {
+        const int64_t i = i0 + u * blockDim.x;
+        if (i < nvec) {
+          update(pp[u].x, gg[u].x, mm[u].x, vv[u].x);
+          update(pp[u].y, gg[u].y, mm[u].y, vv[u].y);
+          update(pp[u].z, gg[u].z, mm[u].z, vv[u].z);
+          update(pp[u].w, gg[u].w, mm[u].w, vv[u].w);
+          p4[i] = pp[u];
+          m4[i] = mm[u];
+          v4[i] = vv[u];
+        }
+      }
     }
     for (int64_t i = start + nvec * 4 + threadIdx.x; i < end; i += blockDim.x) update(p[i], g[i], m[i], v[i]);
   } else {

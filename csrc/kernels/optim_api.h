@@ -9,7 +9,10 @@
 namespace mccl {
 namespace kern {
 
-constexpr int kAdamWChunk = 16384;  // elements handled by one CTA (multiple of 4)
+// Elements handled by one CTA: 256 threads, four 16-byte vectors of each array, two of them in flight together.
+// (Chunks of 16384 with one vector in flight: 85 M parameters 385 us, 6.17 TB/s; so: 362 us, 6.56 TB/s, and a
+// small model spreads over four times as many SMs.)
+constexpr int kAdamWChunk = 4096;
 
 // All pointers are device pointers; arrays are indexed by tensor id.
 struct AdamWTable {
