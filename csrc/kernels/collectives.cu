@@ -307,18 +307,18 @@ size_t twoshot_arena_bytes(size_t nbytes_wire, int ws, bool push_gather) {
 
 cudaError_t launch_allreduce_oneshot(const CollParams& p, DType dtype, DType wire, LaunchCfg cfg,
                                      cudaStream_t s) {
-  int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * dtype_size(wire) * (p.ctx[0].ws - 1), p.ctx[0].ws, 0), cfg);
+  int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * dtype_size(wire) * (p.ctx[0].ws - 1), p.ctx[0].ws, 0));
   return launch_reduce(kOneShot, p, dtype, wire, ctas, cfg, s);
 }
 cudaError_t launch_allreduce_twoshot(const CollParams& p, DType dtype, DType wire, LaunchCfg cfg,
                                      cudaStream_t s) {
-  int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * dtype_size(wire), p.ctx[0].ws, 0), cfg);
+  int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * dtype_size(wire), p.ctx[0].ws, 0));
   return launch_reduce(kTwoShot, p, dtype, wire, ctas, cfg, s);
 }
 cudaError_t launch_reduce_scatter(const CollParams& p, DType dtype, DType wire, LaunchCfg cfg,
                                   cudaStream_t s) {
   int ctas = clamp_ctas(
-      cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * dtype_size(wire) * p.ctx[0].ws, p.ctx[0].ws, 0), cfg);
+      cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * dtype_size(wire) * p.ctx[0].ws, p.ctx[0].ws, 0));
   return launch_reduce(kReduceScatter, p, dtype, wire, ctas, cfg, s);
 }
 size_t allgather_stage_bytes(size_t nbytes_per_rank, int ws) {
@@ -327,7 +327,7 @@ size_t allgather_stage_bytes(size_t nbytes_per_rank, int ws) {
 size_t broadcast_stage_bytes(size_t nbytes) { return round_up(nbytes, 16); }
 
 cudaError_t launch_allgather(const CollParams& p, LaunchCfg cfg, cudaStream_t s) {
-  int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * p.ctx[0].ws, p.ctx[0].ws, 0), cfg);
+  int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * p.ctx[0].ws, p.ctx[0].ws, 0));
   if (p.use_nvls) {
     if (cfg.emulate_ranks > 0 || p.ctx[0].nvls_mc == nullptr) return cudaErrorInvalidValue;
     return do_launch(allgather_kernel<true>, p, ctas, cfg.threads, 0, s);
@@ -335,7 +335,7 @@ cudaError_t launch_allgather(const CollParams& p, LaunchCfg cfg, cudaStream_t s)
   return do_launch(allgather_kernel<false>, p, ctas, cfg.threads, cfg.emulate_ranks, s);
 }
 cudaError_t launch_broadcast(const CollParams& p, LaunchCfg cfg, cudaStream_t s) {
-  int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count, p.ctx[0].ws, 0), cfg);
+  int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count, p.ctx[0].ws, 0));
   if (p.use_nvls) {
     if (cfg.emulate_ranks > 0 || p.ctx[0].nvls_mc == nullptr) return cudaErrorInvalidValue;
     return do_launch(broadcast_kernel<true>, p, ctas, cfg.threads, 0, s);

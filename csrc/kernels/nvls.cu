@@ -422,7 +422,7 @@ cudaError_t launch_allreduce_nvls_inplace(const CollParams& p, DType dtype, Laun
   if ((p.count * dtype_size(dtype)) % 16 != 0 || (p.nvls_offset % 16) != 0) return cudaErrorInvalidValue;
   // each rank only moves its own chunk: size the grid for count / ws
   const size_t own_bytes = p.count * dtype_size(dtype) / p.ctx[0].ws;
-  const int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(own_bytes, p.ctx[0].ws, 0), cfg);
+  const int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(own_bytes, p.ctx[0].ws, 0));
   if (dtype == F32) return do_launch(nvls_inplace_kernel<float>, p, ctas, link_threads(), 0, s);
   if (dtype == F16) return do_launch(nvls_inplace_kernel<__half>, p, ctas, link_threads(), 0, s);
   return do_launch(nvls_inplace_kernel<__nv_bfloat16>, p, ctas, link_threads(), 0, s);
@@ -432,7 +432,7 @@ cudaError_t launch_allreduce_nvls(const CollParams& p, DType dtype, DType wire, 
                                   bool split) {
   if (!nvls_allreduce_supported(dtype, wire, p.op) || cfg.emulate_ranks > 0 || p.ctx[0].nvls_mc == nullptr)
     return cudaErrorNotSupported;
-  const int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * dtype_size(wire), p.ctx[0].ws, 0), cfg);
+  const int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * dtype_size(wire), p.ctx[0].ws, 0));
   if (split) {
     if (dtype == F32 && wire == F32) return go_split<float, float>(p, ctas, cfg, s);
     if (dtype == F32 && wire == BF16) return go_split<float, __nv_bfloat16>(p, ctas, cfg, s);
