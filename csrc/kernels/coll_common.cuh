@@ -24,6 +24,18 @@ constexpr int64_t kBroadcastDirectBytes = 256 << 10;
 __device__ __forceinline__ uint4 ldg16(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ void stg16(void* p, uint4 v) { __stcg(reinterpret_cast<uint4*>(p), v); }
 
+// Bytes s .. s + 15 of the 32 bytes {lo, hi}, 0 <= s < 16.
+__device__ __forceinline__ uint4 shift_bytes(uint4 lo, uint4 hi, uint32_t s) {
+  uint32_t w0 = lo.x, w1 = lo.y, w2 = lo.z, w3 = lo.w, w4 = hi.x;
+  if (s & 8) { w0 = lo.z; w1 = lo.w; w2 = hi.x; w3 = hi.y; w4 = hi.z; }
+  if (s & 4) {
+    w0 = w1; w1 = w2; w2 = w3; w3 = w4;
+    w4 = s & 8 ? hi.w : hi.y;
+  }
+  const uint32_t r = (s & 3) * 8;
+  return make_uint4(__funnelshift_r(w0, w1, r), __funnelshift_r(w1, w2, r), __funnelshift_r(w2, w3, r),
+                    __funnelshift_r(w3, w4, r));
+}
 __host__ __device__ inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // One 16-byte wire unit = N elements of W; the same N elements of T span

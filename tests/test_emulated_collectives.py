@@ -428,3 +428,36 @@ def test_debug_checks_pass_on_the_small_case_matrix_and_catch_a_short_buffer(nat
     g.allgather(outs, ins)
     torch.cuda.synchronize()
     assert torch.equal(outs[0], torch.cat(ins))
+
+
+@pytest.mark.parametrize("rest", range(16))
+def test_gather_and_scatter_of_ragged_blocks_stay_in_their_range(native, cuda_device, rest):
+    # Blocks of every length modulo 16, from and into views at every alignment, with guards around them: shorter than one
+    # vector, a few vectors, more than one tile per CTA.
+    ws = 3
+    g = native.EmuGroup(ws, 16 << 20)
+    for n in (rest + 1, 160 + rest, 700_000 + rest):
+        room = n * ws + 64
+        ins = [torch.randint(0, 250, (n + 32,), dtype=torch.uint8, device=cuda_device) for _ in range(ws)]
+        outs = [torch.full((room,), 255, dtype=torch.uint8, device=cuda_device) for _ in range(ws)]
+        at = [(5 * r + rest) % 16 for r in range(ws)]
+        src = [ins[r][r:r + n] for r in range(ws)]
+        g.allgather([outs[r][16 + at[r]:16 + at[r] + n * ws] for r in range(ws)], src)
+        torch.cuda.synchronize()
+        want = torch.cat(src)
+        for r in range(ws):
+            lo, hi = 16 + at[r], 16 + at[r] + n * ws
+            assert torch.equal(outs[r][lo:hi], want)
+            assert (outs[r][:lo] == 255).all() and (outs[r][hi:] == 255).all()
+        # guards that would show in a sum
+        full = [torch.full((room,), float("nan"), device=cuda_device) for _ in range(ws)]
+        for r in range(ws):
+            full[r][r + 1:r + 1 + n * ws] = torch.randint(-8, 8, (n * ws,), device=cuda_device).float()
+        res = [torch.full((n + 8,), 99.0, device=cuda_device) for _ in range(ws)]
+        views = [full[r][r + 1:r + 1 + n * ws] for r in range(ws)]
+        g.reduce_scatter([res[r][r:r + n] for r in range(ws)], views, "sum")
+        torch.cuda.synchronize()
+        total = sum(v.double() for v in views)
+        for r in range(ws):
+            assert torch.equal(res[r][r:r + n].double(), total[r * n:(r + 1) * n])
+            assert (res[r][:r] == 99.0).all() and (res[r][r + n:] == 99.0).all()
