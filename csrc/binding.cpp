@@ -345,6 +345,37 @@ at::Tensor topk_select(const at::Tensor& grad, at::Tensor residual, double ratio
   return pairs;
 }
 
+// One optimizer step of a parameter group, checks included, if `plan` covers exactly `params` and everything is as
+// the kernel wants it; false, with nothing done, otherwise (the caller then goes through the parameters one by one).
+// `steps`: the parameters' step counters, host tensors; the first says which step this is, all are advanced to it.
+bool adamw_step_group(AdamWPlan& plan, const py::list& params, const py::list& steps, double lr, double beta1,
+                      double beta2, double eps, double weight_decay, double grad_scale) {
+  auto plain = [](const py::handle& h) { return THPVariable_CheckExact(h.ptr()); };
+  const std::vector<at::Tensor>& own = plan.params();
+  if (params.size() != own.size() || steps.size() != own.size()) return false;
+  std::vector<at::Tensor> grads, counters;
+  grads.reserve(own.size());
+  counters.reserve(own.size());
+  for (size_t i = 0; i < own.size(); ++i) {
+    if (!plain(params[i]) || !plain(steps[i])) return false;
+    const at::Tensor& p = THPVariable_Unpack(py::handle(params[i]).ptr());
+    const at::Tensor& c = THPVariable_Unpack(py::handle(steps[i]).ptr());
+    auto dense_floats = [&](const at::Tensor& t) {
+      return t.defined() && t.is_cuda() && t.layout() == at::kStrided && t.scalar_type() == at::kFloat &&
+             t.is_contiguous() && t.numel() == own[i].numel();
+    };
+    if (!dense_floats(p) || p.data_ptr() != own[i].data_ptr() || !dense_floats(p.grad())) return false;
+    if (!c.defined() || !c.is_cpu() || c.layout() != at::kStrided || c.scalar_type() != at::kFloat || c.numel() != 1)
+      return false;
+    grads.push_back(p.grad());
+    counters.push_back(c);
+  }
+  const int64_t step = static_cast<int64_t>(*counters[0].data_ptr<float>()) + 1;
+  plan.step(grads, lr, beta1, beta2, eps, weight_decay, step, grad_scale);
+  for (at::Tensor& c : counters) c.fill_(static_cast<double>(step));
+  return true;
+}
+
 py::bytes pack_header(int op, uint32_t seq, uint32_t tid, uint32_t chunk_index, uint32_t payload_bytes,
                       int flags, uint32_t crc) {
   MessageHeader h = make_header(static_cast<mccl::OpType>(op), seq, tid, chunk_index, payload_bytes,
@@ -633,6 +664,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            py::arg("exp_avg"), py::arg("exp_avg_sq"))
       .def("step", &AdamWPlan::step, py::arg("grads"), py::arg("lr"), py::arg("beta1"), py::arg("beta2"),
            py::arg("eps"), py::arg("weight_decay"), py::arg("step"), py::arg("grad_scale") = 1.0)
+      .def("step_group", &adamw_step_group, py::arg("params"), py::arg("steps"), py::arg("lr"), py::arg("beta1"),
+           py::arg("beta2"), py::arg("eps"), py::arg("weight_decay"), py::arg("grad_scale"))
       .def_property_readonly("num_chunks", &AdamWPlan::num_chunks);
   // ---- native DDP hook: allreduce + AdamW per bucket, registered on the C++ reducer ----
   py::class_<BucketOptimizerState, std::shared_ptr<BucketOptimizerState>>(m, "BucketOptimizerState")

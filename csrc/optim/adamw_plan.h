@@ -119,6 +119,7 @@ class AdamWPlan {
     MCCL_PLAN_CK(kern::launch_adamw_multi(tab, h, stream, max_ctas));
   }
   int num_chunks() const { return num_chunks_; }
+  const std::vector<at::Tensor>& params() const { return params_; }
 
  private:
   std::vector<at::Tensor> params_, m_, v_;

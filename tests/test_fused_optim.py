@@ -1,4 +1,6 @@
 """Fused AdamW kernel vs torch.optim.AdamW, and per-bucket stepping inside backward (one GPU)."""
+import copy
+
 import pytest
 import torch
 
@@ -25,6 +27,53 @@ def test_fused_adamw_matches_torch(cuda_device):
     # interchangeable state
     o2.load_state_dict(o1.state_dict())
     o1.load_state_dict(o2.state_dict())
+
+
+def test_step_follows_what_changes_between_steps(cuda_device):
+    # Everything that takes a step off the one-call path and back: a missing gradient, a moved or non-contiguous one, a
+    # replaced parameter, counters loaded from a checkpoint, changed hyper-parameters.
+    from mccl_b200.optim import FusedAdamW
+    torch.manual_seed(1)
+    shapes = [(64, 32), (32,), (5000,)]
+    p1 = [torch.nn.Parameter(torch.randn(s, device=cuda_device)) for s in shapes]
+    p2 = [torch.nn.Parameter(p.detach().clone()) for p in p1]
+    o1, o2 = FusedAdamW(p1, lr=1e-2), torch.optim.AdamW(p2, lr=1e-2)
+
+    def step(change=None):
+        for i, (a, b) in enumerate(zip(p1, p2)):
+            g = torch.randn_like(a)
+            a.grad, b.grad = g.clone(), g.clone()
+            if change == "missing" and i == 1:
+                a.grad = b.grad = None
+            if change == "strided" and i == 0:
+                a.grad = g.t().contiguous().t()
+        o1.step()
+        o2.step()
+        for a, b in zip(p1, p2):
+            assert torch.allclose(a, b, rtol=1e-5, atol=1e-6), change
+            sa, sb = o1.state[a], o2.state[b]
+            assert float(sa["step"]) == float(sb["step"]) and torch.allclose(sa["exp_avg"], sb["exp_avg"], atol=1e-6)
+
+    step()
+    step()
+    step("strided")
+    step()
+    for o in (o1, o2):
+        o.param_groups[0]["lr"] = 3e-3
+        o.param_groups[0]["weight_decay"] = 0.1
+    step()
+    o1.load_state_dict(copy.deepcopy(o2.state_dict()))  # (without the copy the two would share their moments)
+    step()
+    with torch.no_grad():
+        p1[0].data = p1[0].detach().clone()  # another address
+    step()
+    for a, b in zip(p1, p2):
+        a.grad = b.grad = None
+    before = [p.detach().clone() for p in p1]
+    o1.step()
+    assert all(torch.equal(p, q) for p, q in zip(p1, before))
+    assert o1.state[p1[0]]["step"] == o2.state[p2[0]]["step"]
+    step("missing")
 
 
 def _oib_single(rank, ws):
