@@ -263,12 +263,13 @@ __device__ __forceinline__ void store_folded(const IfftOlaArgs& a, float* out, i
   }
 }
 
-// One row of finished samples, by one warp, two samples per lane (hop is even).  pass: 0 away from folded edges.
-template <bool kNorm>
+// One row of finished samples, by one warp, two samples per lane (hop is even), N pairs of each lane at a time (a
+// short hop has fewer: with N = 4 throughout and larger CTAs, n_fft 256 and hop 64 took 226 us instead of 174).
+// pass: 0 away from folded edges.
+template <int N, bool kNorm>
 __device__ __forceinline__ void emit_row_pairs(const IfftOlaArgs& a, const float2* slots, int slot_floats,
                                                const float* win, int ring, int s, int i_hi, int i_lo, int64_t q0,
                                                float* out, int lane, int pass) {
-  constexpr int N = 4;
   const bool paired = pass == 0 && q0 >= 0 && q0 + a.hop <= a.out_len && (reinterpret_cast<uintptr_t>(out + q0) & 7) == 0;
   for (int c = 0; c < a.hop; c += 64 * N) {
     const int j = c + 2 * lane;
@@ -383,10 +384,14 @@ __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const
         int s = i_lo < pl.reach ? slot0 + static_cast<int>(row - f0) : 0;  // slot of frame `row`
         if (s >= pl.ring) s -= pl.ring;
         if ((a.hop & 1) == 0) {
-          if (a.normalize_envelope)
-            emit_row_pairs<true>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, 0);
-          else
-            emit_row_pairs<false>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, folds ? pass : 0);
+          const int p = folds ? pass : 0;
+          if (a.normalize_envelope) {
+            if (LH <= 8 && a.hop <= 64) emit_row_pairs<1, true>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p);
+            else emit_row_pairs<LH <= 8 ? 2 : 4, true>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p);
+          } else {
+            if (LH <= 8 && a.hop <= 64) emit_row_pairs<1, false>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p);
+            else emit_row_pairs<LH <= 8 ? 2 : 4, false>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p);
+          }
           continue;
         }
         for (int j = lane; j < a.hop; j += 32) {
@@ -570,8 +575,10 @@ OlaGrid ola_grid(const IfftOlaArgs& a) {
   pl.row_base = fold ? 0 : a.pad / a.hop;
   pl.rows = (end + a.hop - 1) / a.hop - pl.row_base;
   pl.reach = static_cast<int>(reach);
-  // two CTAs of 8 warps per SM before one of 16, that before whatever fits
-  static const int kChoices[][2] = {{8, 2}, {16, 1}, {8, 1}, {4, 1}};
+  // {warps, CTAs per SM}.  Several small CTAs before one of 16 warps, that before whatever fits: the phases of one
+  // overlap with another's.  Frames of up to 512 samples (several per warp) do best with four of 4 warps; for 1024
+  // three of 5 repeat too many frames at the segments' ends (160 us against 137 us for 16 x 1 Mi samples).
+  static const int kChoices[][2] = {{LH <= 8 ? 4 : 8, LH <= 8 ? 4 : 2}, {8, 2}, {16, 1}, {8, 1}, {4, 1}};
   for (const auto& choice : kChoices) {
     const int warps = choice[0];
     int resident = choice[1];
