@@ -141,8 +141,8 @@ def bench_topk_exchange(native, n, iters, ws=4):
         grp.topk_allreduce(gs, rs, 0.01, 1.0 / ws, 16)
     ms = timeit(run, iters)
     k = max(1, int(n * 0.01))
-    # select (20 B/elem) + pairs pushed to ws ranks + dense zero-fill and sparse adds
-    return ms, (n * 20 + k * 8 * (1 + ws) + n * 4 + k * 8 * ws) * ws, f"emulated {ws} ranks: select + sparse exchange + scatter"
+    # select (12 B/elem) + pairs pushed to ws ranks + dense zero-fill and sparse adds
+    return ms, (n * 12 + k * 8 * (1 + ws) + n * 4 + k * 8 * ws) * ws, f"emulated {ws} ranks: select + sparse exchange + scatter"
 
 
 def bench_topk(native, n, iters):
@@ -151,7 +151,7 @@ def bench_topk(native, n, iters):
 
     def run():
         native._topk_select(g, r, 0.01)
-    return timeit(run, iters), n * 20, "adjust + histogram (12 B) + collect (4 B) + ordered compaction (4 B) per element"
+    return timeit(run, iters), n * 12, "gradient and residual read, residual written: 12 B per element"
 
 
 def bench_stft(native, n, iters, n_fft=2048):
