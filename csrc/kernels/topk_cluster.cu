@@ -9,10 +9,13 @@
 //            octave per bin, from which the last block takes the bin of the k-th element
 //   select   candidates above the bin are selected, those inside it are gathered, and the last block finds the
 //            exact threshold (and the index limit among ties) on them
-// followed, for pairs sorted by index, by a count per run of tiles and the ordered output (two launches).
+// followed by a count per run of tiles and the ordered output (two launches), which put out pairs sorted by index, or
+// leave at once if the result is dense and already there.
 //
-// The sample decides speed, never results: if fewer than k elements reach its magnitude, or more than the list
-// holds, or the k-th is two octaves above it, one cluster selects from the whole adjusted vector instead.
+// The sample decides speed, never results.  Heavily tied data (more elements than the list holds, or a crowded bin):
+// the select launch takes the exact threshold from the whole adjusted vector and the last two rank the ties in index
+// order.  Fewer non-zeros than k: the same two take all of them and the first zeros.  What is left, a sample that missed
+// by five standard deviations or a k-th element two octaves above it, one cluster selects from the whole vector.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -60,27 +63,38 @@ __device__ __forceinline__ float scaled(float v, float scale) { return fmaf(v, s
 __device__ __forceinline__ int64_t at_most(int64_t a, int64_t b) { return a < b ? a : b; }
 
 constexpr int kBinShift = 13;            // keys per histogram bin: 1/1024 octave
+constexpr int kSubBins = 1 << kBinShift;
 constexpr int kRun = 4;                  // tiles whose pairs one warp puts out
+// Entries of the k-th element's bin that one block resolves; more (ties) are left to the whole grid.  51.5 M bf16
+// elements, dense result: 255 levels at 1 %, about 50 thousand entries, 222 us with one block and 441 us with the grid;
+// 40 levels at 1 %, 190 thousand, 480 and 450 us; 40 levels at 10 %, over a million, 1709 and 509 us.
+constexpr uint32_t kOneBlock = 128 * 1024;
+// kList: from the candidates.  kWhole: by one cluster from the vector.  kTies: the bin is known, threshold and ties
+// come from the vector.  kZeros: all non-zeros and the first zeros.
+enum Mode : uint32_t { kList, kWhole, kTies, kZeros };
 
-// the select kernel's exact rule: an entry is sent if key > threshold, or key == threshold and index <= last_index
+// The exact rule: an element is sent if key > threshold, or key == threshold and index <= last_index (kList) or it is
+// one of the first `need` (kTies, kZeros).
 struct ListState {
   uint32_t hist[kBins];  // candidates by (key - base) >> kBinShift, the last bin open-ended
   uint32_t base;         // smallest magnitude key that is a candidate
   uint32_t count;        // entries in the list
   uint32_t overflow;     // the list did not hold them all
-  uint32_t slow;         // the candidates do not decide: select from the whole vector
+  uint32_t mode;         // how the selection is decided: Mode
   uint32_t bin, need;    // the k-th element's bin, and how many of that bin are selected
   uint32_t in_bin;       // entries gathered from the bin
   uint32_t threshold, last_index;
-  uint32_t ticket[3];    // blocks done: adjust, select, pair counts
+  uint32_t ticket[3];    // blocks done: adjust, select, counts
+  uint32_t sub[kSubBins];  // kTies: elements of the bin by key
 };
-// scratch: ListState, {start, count} per tile, the list of {index, value}, its entries inside the bin, pairs per run
+static_assert(sizeof(ListState) % sizeof(uint4) == 0, "8-byte entries follow it in the scratch");
+// scratch: ListState, {start, count} per tile, the list of {index, value}, its entries inside the bin, counts per run
 struct ListView {
   ListState* state;
   uint2* tiles;
   uint2* list;
   uint2* bin_list;
-  uint32_t* runs;
+  uint2* runs;
   uint32_t cap;
 };
 
@@ -104,7 +118,7 @@ inline ListView list_view(void* scratch, int64_t n, int64_t k) {
   v.list = v.tiles + tile_count(n);
   v.cap = static_cast<uint32_t>(list_capacity(n, k));
   v.bin_list = v.list + v.cap;
-  v.runs = reinterpret_cast<uint32_t*>(v.bin_list + v.cap);
+  v.runs = v.bin_list + v.cap;
   return v;
 }
 
@@ -359,7 +373,7 @@ __device__ __forceinline__ uint32_t bin_of(uint32_t key_above_base) {
 // a = g + e, e = a, candidates to the list.  A warp owns `group` consecutive tiles at a time and appends their
 // candidates in index order: one global atomic per group, entries of a group contiguous.
 // Bound by HBM: 12 bytes per bf16 element with a dense result.
-// 50257 x 1024 bf16 elements (618 MB): 106 us, 5.8 TB/s.  The whole selection: 404 us in four passes, 177 us so.
+// 50257 x 1024 bf16 elements (618 MB): 106 us, 5.8 TB/s.  The whole selection: 404 us in four passes, 185 us so.
 template <bool kBf16, bool kVec, bool kDense>
 __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a, int group) {
   extern __shared__ __align__(16) uint2 staging[];
@@ -391,12 +405,12 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
     auto flush = [&]() {
       uint32_t start;
       __syncwarp();
-      if (reserve(first, staged, &start))
-        for (uint32_t i = lane; i < staged; i += 32) {
-          const uint2 e = stage[i];
-          list.list[start + i] = e;
-          atomicAdd(&hist[bin_of((e.y & 0x7FFFFFFFu) - base)], 1u);
-        }
+      const bool fits = reserve(first, staged, &start);
+      for (uint32_t i = lane; i < staged; i += 32) {
+        const uint2 e = stage[i];
+        if (fits) list.list[start + i] = e;
+        atomicAdd(&hist[bin_of((e.y & 0x7FFFFFFFu) - base)], 1u);
+      }
       __syncwarp();
       staged = 0;
     };
@@ -477,7 +491,7 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
         list.tiles[tile] = make_uint2(0u, 0u);  // found under `first`
       }
       uint2* to = here > kStage ? list.list + direct : stage + staged;
-      if (here && fits) {
+      if (here) {
         uint32_t put = 0;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {  // 128 consecutive elements, four per lane
@@ -493,8 +507,9 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             if ((nib >> j) & 1u) {
-              to[put + before + __popc(nib & ((1u << j) - 1u))] =
-                  make_uint2(static_cast<uint32_t>(t0 + 128 * q + j), __float_as_uint(v[q][j]));
+              if (fits)
+                to[put + before + __popc(nib & ((1u << j) - 1u))] =
+                    make_uint2(static_cast<uint32_t>(t0 + 128 * q + j), __float_as_uint(v[q][j]));
               if (here > kStage) atomicAdd(&hist[bin_of(key_of(v[q][j]) - base)], 1u);
             }
           put += all;
@@ -525,11 +540,17 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
     if (above < a.k && above + c[i] >= a.k) {
       list.state->bin = static_cast<uint32_t>(top - i);
       list.state->need = a.k - above;
-      if (top - i == kBins - 1) list.state->slow = 1u;  // open-ended
+      const bool crowded = __ldcg(&list.state->overflow) != 0u || c[i] > kOneBlock;
+      list.state->mode = top - i == kBins - 1 ? kWhole : crowded ? kTies : kList;  // the last bin is open-ended
     }
     above += c[i];
   }
-  if (threadIdx.x == 0 && (__ldcg(&list.state->overflow) != 0u || __ldcg(&list.state->count) < a.k)) list.state->slow = 1u;
+  const uint32_t count = __ldcg(&list.state->count);
+  if (threadIdx.x == 0 && count < a.k) {
+    list.state->mode = base == 1u ? kZeros : kWhole;  // every non-zero is a candidate, or the sample missed
+    list.state->threshold = 0u;
+    list.state->need = a.k - count;
+  }
 }
 
 // The need-th largest (kDown) or smallest of the m entries' words of `bits` bits, found by one block 11 bits at a
@@ -577,15 +598,67 @@ __device__ uint32_t block_nth(uint32_t* hist, uint32_t* wsum, uint32_t* s_pick, 
   return prefix;
 }
 
-// Selection among the candidates, a grid of whole clusters; if they do not decide it, the first cluster selects from
-// the whole adjusted vector and the others leave.  e and (kDense) g hold the values of elements that are not selected.
+// Selection among the candidates, a grid of whole clusters; for kTies only the threshold, from the whole vector; for
+// kWhole the first cluster selects from the whole vector and the others leave.  e and (kDense) g hold the values of elements that are not selected.
 template <bool kBf16, bool kDense>
 __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectArgs a) {
   __shared__ ClusterShared sh;
   __shared__ uint32_t s_count, s_base, s_pick[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   ListState* st = a.list.state;
-  if (st->slow == 0u) {
+  const uint32_t mode = st->mode;
+  if (mode == kZeros) return;
+  if (mode == kTies) {
+    extern __shared__ __align__(16) uint32_t sub[];
+    const uint32_t floor_key = st->base + (st->bin << kBinShift);
+    for (int i = tid; i < kSubBins; i += kThreads) sub[i] = 0;
+    __syncthreads();
+    auto add = [&](float v, bool valid) {  // equal keys of a warp are counted together: most are ties
+      const uint32_t d = key_of(v) - floor_key;
+      const bool in = valid && d < kSubBins;
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
+      if (!in) return;
+      const uint32_t same = __match_any_sync(m, d);
+      if (lane == __ffs(same) - 1) atomicAdd(&sub[d], static_cast<uint32_t>(__popc(same)));
+    };
+    constexpr int kAhead = 8;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads * kAhead;
+    for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * kThreads * kAhead; i0 < a.n; i0 += step) {
+      float v[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int64_t i = i0 + u * kThreads + tid;
+        v[u] = i < a.n ? __ldcs(a.residual + i) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) add(v[u], i0 + u * kThreads + tid < a.n);
+    }
+    __syncthreads();
+    for (int i = tid; i < kSubBins; i += kThreads)
+      if (sub[i]) atomicAdd(&st->sub[i], sub[i]);
+    if (!last_block_done(&st->ticket[1])) return;
+    constexpr int kPer = kSubBins / kThreads;
+    const int top = kSubBins - 1 - kPer * tid;
+    const uint32_t need = st->need;
+    uint32_t c[kPer], run = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      c[i] = __ldcg(&st->sub[top - i]);
+      run += c[i];
+    }
+    uint32_t above = block_excl_scan(run, sh.wsum);
+    __syncthreads();  // every thread has read `need`
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      if (above < need && above + c[i] >= need) {
+        st->threshold = floor_key + static_cast<uint32_t>(top - i);
+        st->need = need - above;
+      }
+      above += c[i];
+    }
+    return;
+  }
+  if (mode == kList) {
     const uint32_t count = st->count, base = st->base, bin = st->bin;
     uint2* bin_list = a.list.bin_list;
     constexpr int kAhead = 4;
@@ -683,32 +756,61 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
                });
 }
 
-// The pairs, sorted by index.  A warp owns a run of tiles; kCount: how many of its candidates are selected, and the
-// last block turns the counts into offsets; otherwise they are put out, in order.
-template <bool kCount>
-__global__ void __launch_bounds__(kThreads, 1) topk_pairs_kernel(const SelectArgs a) {
+// What is left to put out, in index order.  A warp owns a run of tiles; kCount: how many of its elements lie above the
+// threshold and at it, and the last block turns the counts into offsets; otherwise they are put out.  kList: pairs
+// from the candidates (a dense result is complete already).  kTies, kZeros: from the vector.
+template <bool kCount, bool kBf16, bool kDense>
+__global__ void __launch_bounds__(kThreads, 1) topk_output_kernel(const SelectArgs a) {
   const int lane = threadIdx.x & 31;
   ListState* st = a.list.state;
-  if (st->slow != 0u) return;
-  const uint32_t threshold = st->threshold, last_index = st->last_index;
+  const uint32_t mode = st->mode;
+  if (mode == kWhole || (mode == kList && kDense)) return;
+  const uint32_t threshold = st->threshold, last_index = st->last_index, need = st->need;
+  const uint32_t lower = (1u << lane) - 1u;
   const int64_t tiles = tile_count(a.n), runs = run_count(a.n);
   for (int64_t run = static_cast<int64_t>(blockIdx.x) * kWarps + (threadIdx.x >> 5); run < runs; run += gridDim.x * kWarps) {
     const int64_t t0 = run * kRun;
-    const uint2 place = lane < kRun && t0 + lane < tiles ? a.list.tiles[t0 + lane] : make_uint2(0u, 0u);
-    uint32_t done = kCount ? 0u : a.list.runs[run];
-    for (int l = 0; l < kRun; ++l) {
-      const uint32_t start = __shfl_sync(0xFFFFFFFFu, place.x, l), cnt = __shfl_sync(0xFFFFFFFFu, place.y, l);
+    uint2 done = kCount ? make_uint2(0u, 0u) : a.list.runs[run];
+    if (mode == kList) {
+      const uint2 place = lane < kRun && t0 + lane < tiles ? a.list.tiles[t0 + lane] : make_uint2(0u, 0u);
+      for (int l = 0; l < kRun; ++l) {
+        const uint32_t start = __shfl_sync(0xFFFFFFFFu, place.x, l), cnt = __shfl_sync(0xFFFFFFFFu, place.y, l);
 #pragma unroll 4
-      for (uint32_t i = 0; i < cnt; i += 32) {
-        const uint2 e = i + lane < cnt ? a.list.list[start + i + lane] : make_uint2(0u, 0u);
-        const uint32_t key = e.y & 0x7FFFFFFFu;
-        const bool sent = i + lane < cnt && (key > threshold || (key == threshold && e.x <= last_index));
-        const uint32_t m = __ballot_sync(0xFFFFFFFFu, sent);
-        if (!kCount && sent) {
-          a.pairs[done + __popc(m & ((1u << lane) - 1u))] = e;
-          a.residual[e.x] = 0.f;  // nothing left to feed back
+        for (uint32_t i = 0; i < cnt; i += 32) {
+          const uint2 e = i + lane < cnt ? a.list.list[start + i + lane] : make_uint2(0u, 0u);
+          const uint32_t key = e.y & 0x7FFFFFFFu;
+          const bool sent = i + lane < cnt && (key > threshold || (key == threshold && e.x <= last_index));
+          const uint32_t m = __ballot_sync(0xFFFFFFFFu, sent);
+          if (!kCount && sent) {
+            a.pairs[done.x + __popc(m & lower)] = e;
+            a.residual[e.x] = 0.f;  // nothing left to feed back
+          }
+          done.x += __popc(m);
         }
-        done += __popc(m);
+      }
+    } else {
+      const int64_t lo = t0 * kTile, hi = at_most(a.n, lo + kRun * kTile);
+      constexpr int kAhead = 8;
+      for (int64_t i0 = lo; i0 < hi; i0 += 32 * kAhead) {
+        float v[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) v[u] = i0 + 32 * u + lane < hi ? __ldcg(a.residual + i0 + 32 * u + lane) : 0.f;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const int64_t i = i0 + 32 * u + lane;
+          const uint32_t key = key_of(v[u]);
+          const bool gt = i < hi && key > threshold, eq = i < hi && key == threshold;
+          const uint32_t m_gt = __ballot_sync(0xFFFFFFFFu, gt), m_eq = __ballot_sync(0xFFFFFFFFu, eq);
+          if (!kCount) {
+            const uint32_t r_gt = done.x + __popc(m_gt & lower), r_eq = done.y + __popc(m_eq & lower);
+            if (gt || (eq && r_eq < need)) {
+              send<kBf16, kDense>(a, static_cast<uint32_t>(i), v[u]);
+              if (!kDense) a.pairs[r_gt + (r_eq < need ? r_eq : need)] = make_uint2(static_cast<uint32_t>(i), __float_as_uint(v[u]));
+            }
+          }
+          done.x += __popc(m_gt);
+          done.y += __popc(m_eq);
+        }
       }
     }
     if (kCount && lane == 0) a.list.runs[run] = done;
@@ -717,13 +819,21 @@ __global__ void __launch_bounds__(kThreads, 1) topk_pairs_kernel(const SelectArg
   __shared__ uint32_t wsum[33];
   const int64_t per = (runs + kThreads - 1) / kThreads;
   const int64_t r0 = at_most(runs, threadIdx.x * per), r1 = at_most(runs, r0 + per);
-  uint32_t sum = 0;
-  for (int64_t r = r0; r < r1; ++r) sum += __ldcg(&a.list.runs[r]);
-  uint32_t before = block_excl_scan(sum, wsum);
+  uint2 sum = make_uint2(0u, 0u);
   for (int64_t r = r0; r < r1; ++r) {
-    const uint32_t c = __ldcg(&a.list.runs[r]);
+    const uint2 c = __ldcg(&a.list.runs[r]);
+    sum.x += c.x;
+    sum.y += c.y;
+  }
+  uint2 before;
+  before.x = block_excl_scan(sum.x, wsum);
+  __syncthreads();
+  before.y = block_excl_scan(sum.y, wsum);
+  for (int64_t r = r0; r < r1; ++r) {
+    const uint2 c = __ldcg(&a.list.runs[r]);
     a.list.runs[r] = before;
-    before += c;
+    before.x += c.x;
+    before.y += c.y;
   }
 }
 
@@ -795,7 +905,7 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
   e = cluster_size(reinterpret_cast<const void*>(sample), sample_size, 0, &ctas);
   if (e != cudaSuccess) return e;
   const uint32_t rank = sample_rank(a.n, a.k);
-  note_launch(3);
+  note_launch(5);
   e = launch_cluster(sample, 1, ctas, 0, s, a, rank);
   if (e != cudaSuccess) return e;
 
@@ -817,15 +927,14 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
 
   auto select = topk_select_kernel<kBf16, kDense>;
-  e = cluster_size(reinterpret_cast<const void*>(select), select_size, 0, &ctas);
+  e = cluster_size(reinterpret_cast<const void*>(select), select_size, kSubBins * sizeof(uint32_t), &ctas);
   if (e != cudaSuccess) return e;
-  const int clusters = static_cast<int>(std::min<int64_t>(128 / ctas, (a.list.cap + 16383) / 16384));
-  e = launch_cluster(select, clusters, ctas, 0, s, a);
-  if (e != cudaSuccess || kDense) return e;
-  note_launch(2);
+  const int clusters = static_cast<int>(std::min<int64_t>(128 / ctas, (a.n + (1 << 20) - 1) >> 20));
+  e = launch_cluster(select, clusters, ctas, kSubBins * sizeof(uint32_t), s, a);
+  if (e != cudaSuccess) return e;
   const unsigned pgrid = static_cast<unsigned>(std::min<int64_t>(148, (run_count(a.n) + kWarps - 1) / kWarps));
-  topk_pairs_kernel<true><<<pgrid, kThreads, 0, s>>>(a);
-  topk_pairs_kernel<false><<<pgrid, kThreads, 0, s>>>(a);
+  topk_output_kernel<true, kBf16, kDense><<<pgrid, kThreads, 0, s>>>(a);
+  topk_output_kernel<false, kBf16, kDense><<<pgrid, kThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -833,7 +942,7 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
 
 size_t topk_list_scratch_bytes(int64_t n, int64_t k) {
   return sizeof(ListState) + static_cast<size_t>(tile_count(n) + 2 * list_capacity(n, k)) * sizeof(uint2) +
-         static_cast<size_t>(run_count(n)) * sizeof(uint32_t);
+         static_cast<size_t>(run_count(n)) * sizeof(uint2);
 }
 
 cudaError_t launch_topk_cluster(const TopkArgs& t, bool dense, cudaStream_t s) {

@@ -119,6 +119,8 @@ def _data(kind, n, dtype):
         g, r = g * (torch.rand(n // 1024 + 1, generator=gen) < 0.05).float().repeat_interleave(1024)[:n], torch.zeros(n)
     elif kind == "levels":        # far more ties at the threshold than a candidate list holds
         g, r = torch.randint(-3, 4, (n,), generator=gen).float(), torch.zeros(n)
+    elif kind == "steps":         # a crowded bin, within what the list holds or not
+        g, r = (8 * torch.randn(n, generator=gen)).round(), torch.zeros(n)
     elif kind == "wide":          # magnitudes over the whole range of the type, infinities among them
         r = torch.zeros(n)
         g = torch.ldexp(1 + torch.rand(n, generator=gen), torch.randint(-140, 127, (n,), generator=gen))
@@ -131,7 +133,7 @@ def _data(kind, n, dtype):
 # it, or more than the list holds).  Integer selection rule: exact.
 @pytest.mark.parametrize("n,ratio", [(1, 1.0), (7, 0.5), (393_216, 0.01), (393_217, 0.01), (786_432, 0.1), (786_433, 0.01),
                                      (1_048_577, 0.001), (3_000_001, 0.1), (9_437_184, 0.01), (2_000_000, 1.0)])
-@pytest.mark.parametrize("kind", ["normal", "grid", "sparse", "rows", "levels", "wide"])
+@pytest.mark.parametrize("kind", ["normal", "grid", "sparse", "rows", "levels", "steps", "wide"])
 def test_select_and_dense_paths_match_host_oracle(native, cuda_device, one_rank, n, ratio, kind):
     if n < 100 and kind != "normal":
         pytest.skip("the kinds differ for many elements only")
