@@ -59,7 +59,7 @@ __host__ __device__
 inline size_t topk_pad(size_t bytes) { return (bytes + 127) / 128 * 128; }
 
 // Three ways, with the same results: one cluster launch while the gradient fits a cluster's shared memory; sample,
-// adjust and select (topk_cluster.cu) above that; the three-pass radix select (topk.cu) where the caller's scratch
+// adjust, select and output (topk_cluster.cu) above that; the three-pass radix select (topk.cu) where the caller's scratch
 // has no room for the candidate list.
 cudaError_t launch_topk_select(const TopkArgs& a, cudaStream_t s);
 // p: arena parameters (ctx[].in = pairs, ctx[].out = dense gradient); count = k.

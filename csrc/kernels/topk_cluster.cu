@@ -1,7 +1,7 @@
 // Top-k selection with a single pass over the data (sm_100a).
 //
 // A gradient that fits the shared memory of one thread-block cluster is selected from there by one launch: exact
-// radix select, ordered output or dense result, one read and one write of every element.  A larger one takes three:
+// radix select, ordered output or dense result, one read and one write of every element.  A larger one takes five:
 //   sample   a cluster reads 64 Ki evenly spread elements of g + e and takes, from their exact selection, a
 //            magnitude that clearly more than k elements reach
 //   adjust   all SMs: a = g + e, e = a (and g = 0 where the result is dense); the few elements that reach the
@@ -9,8 +9,8 @@
 //            octave per bin, from which the last block takes the bin of the k-th element
 //   select   candidates above the bin are selected, those inside it are gathered, and the last block finds the
 //            exact threshold (and the index limit among ties) on them
-// followed by a count per run of tiles and the ordered output (two launches), which put out pairs sorted by index, or
-// leave at once if the result is dense and already there.
+//   output   a count per run of tiles, then the ordered output: pairs sorted by index; a dense result is there already
+//            (both launches leave at once)
 //
 // The sample decides speed, never results.  Heavily tied data (more elements than the list holds, or a crowded bin):
 // the select launch takes the exact threshold from the whole adjusted vector and the last two rank the ties in index
@@ -281,7 +281,7 @@ struct SelectArgs {
 // The whole selection of a gradient that fits the cluster's shared memory: read once, written once.
 // Bound by latency: two cluster barriers per radix level, three levels, two for the rest.
 // 262144 fp32 elements, 1 %, dense result: 65 us in eight launches of all SMs, 23 us so; from about twice that size
-// on the three launches below take over (700000 elements: 38 us from one cluster).
+// on the launches below take over (700000 elements: 38 us from one cluster).
 template <bool kBf16, bool kDense>
 __global__ void __launch_bounds__(kThreads, 1) topk_cluster_kernel(const SelectArgs a, int per) {
   extern __shared__ __align__(16) float items[];

@@ -128,7 +128,7 @@ def _data(kind, n, dtype):
     return g.to(dtype), r
 
 
-# One cluster launch up to 8 x 48 Ki elements, sample + adjust + select above; sizes around that limit, around the tile of
+# One cluster launch up to 8 x 48 Ki elements, sample + adjust + select + output above; sizes around that limit, around the tile of
 # 1024 and the group of tiles, odd sizes, and every kind of data for which the sampled magnitude misses (fewer than k reach
 # it, or more than the list holds).  Integer selection rule: exact.
 @pytest.mark.parametrize("n,ratio", [(1, 1.0), (7, 0.5), (393_216, 0.01), (393_217, 0.01), (786_432, 0.1), (786_433, 0.01),
