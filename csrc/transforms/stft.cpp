@@ -32,17 +32,22 @@ void check_common(int64_t n_fft, int64_t hop, int64_t win_length, const at::Tens
                     "the native STFT serves the CUDA backend (got '" << backend << "')");
 }
 
+// The kernels read memory: a lazy conjugation or negation (`spec.conj()`, the gradient that autograd hands back
+// through it) is carried out before they run.
+at::Tensor plain(const at::Tensor& t) { return t.resolve_conj().resolve_neg(); }
+
 // fp32 and contiguous on `like`'s device; the kernels centre its win_length samples in n_fft zeros
 at::Tensor prepare_window(const at::Tensor& window, const at::Tensor& like) {
-  return window.to(like.device(), at::kFloat).contiguous();
+  return plain(window.to(like.device(), at::kFloat).contiguous());
 }
 kern::StftWindow centred(const at::Tensor& w, int64_t n_fft) {
   const int64_t len = w.numel();
   return {w.data_ptr<float>(), static_cast<int>(len), static_cast<int>((n_fft - len) / 2)};
 }
 
-at::Tensor as_batch(const at::Tensor& x) {
-  MCCL_CHECK_TENSOR(x.is_cuda() && x.scalar_type() == at::kFloat, "expected a float32 CUDA tensor");
+at::Tensor as_batch(const at::Tensor& t) {
+  MCCL_CHECK_TENSOR(t.is_cuda() && t.scalar_type() == at::kFloat, "expected a float32 CUDA tensor");
+  const at::Tensor x = plain(t);
   if (x.dim() == 1) return x.unsqueeze(0).contiguous();
   if (x.dim() == 3 && x.size(1) == 1) return x.squeeze(1).contiguous();
   MCCL_CHECK_TENSOR(x.dim() == 2, "expected [time], [batch, time] or [batch, 1, time]");
@@ -106,10 +111,11 @@ at::Tensor stft_forward(const at::Tensor& waveform, const at::Tensor& window, in
   return out.transpose(1, 2);  // [batch, freq, frames]; frames-major storage keeps the kernel's writes coalesced
 }
 
-at::Tensor stft_backward(const at::Tensor& grad_spec, const at::Tensor& window, int64_t n_fft, int64_t hop,
+at::Tensor stft_backward(const at::Tensor& grad_spec_in, const at::Tensor& window, int64_t n_fft, int64_t hop,
                          int64_t win_length, bool center, bool normalized, int64_t length,
                          const std::string& backend) {
   check_common(n_fft, hop, win_length, window, backend);
+  const at::Tensor grad_spec = plain(grad_spec_in);
   int64_t sb, sf, st;
   spec_strides(grad_spec, n_fft, sb, sf, st);
   const int64_t B = grad_spec.size(0), frames = grad_spec.size(2);
@@ -137,10 +143,11 @@ at::Tensor stft_backward(const at::Tensor& grad_spec, const at::Tensor& window, 
   return out;
 }
 
-at::Tensor istft_forward(const at::Tensor& spec, const at::Tensor& window, int64_t n_fft, int64_t hop,
+at::Tensor istft_forward(const at::Tensor& spec_in, const at::Tensor& window, int64_t n_fft, int64_t hop,
                          int64_t win_length, bool center, bool normalized, int64_t length,
                          const std::string& backend) {
   check_common(n_fft, hop, win_length, window, backend);
+  const at::Tensor spec = plain(spec_in);
   int64_t sb, sf, st;
   spec_strides(spec, n_fft, sb, sf, st);
   const int64_t B = spec.size(0), frames = spec.size(2);

@@ -172,3 +172,48 @@ def test_istft_beyond_the_frames_is_zero(cuda_device, length):
     keep = min(length, full.shape[1])
     assert torch.equal(got[:, :keep], full[:, :keep])
     assert not got[:, keep:].any()
+
+
+# Lazy views: `.conj()` only sets a bit, and autograd hands such tensors to backward as well; `.conj().imag` sets the
+# negative bit.  The transforms have to see the values, in both memory orders.
+@pytest.mark.gpu
+@pytest.mark.parametrize("frames_major", [True, False])
+def test_lazily_conjugated_and_negated_inputs(cuda_device, frames_major):
+    n_fft, hop, samples = 256, 64, 4001
+    gen = torch.Generator().manual_seed(9)
+    w = torch.hann_window(n_fft)
+    kw = dict(n_fft=n_fft, hop_length=hop, win_length=n_fft)
+    z = torch.randn(2, samples, dtype=torch.complex64, generator=gen)
+    spec = torch.randn(2, n_fft // 2 + 1, 1 + samples // hop, dtype=torch.complex64, generator=gen)
+    dev_spec = spec.to(cuda_device)
+    if frames_major:
+        dev_spec = dev_spec.transpose(1, 2).contiguous().transpose(1, 2)
+    tol = 6e-8 * 16
+
+    def reference(fn):  # fn on float64 host tensors, with torch's own transforms
+        return fn(lambda t: torch.stft(t, window=w.double(), return_complex=True, **kw),
+                  lambda s, n: torch.istft(s, window=w.double(), length=n, **kw), z.to(torch.complex128), spec.to(torch.complex128))
+
+    def ours(fn):
+        wd = w.to(cuda_device)
+        return fn(lambda t: stft(t, window=wd, backend="cuda", **kw),
+                  lambda s, n: istft(s, window=wd, length=n, backend="cuda", **kw), z.to(cuda_device), dev_spec)
+
+    length = (spec.shape[2] - 1) * hop
+
+    def inverse(fwd, inv, z, s):
+        return inv(s.conj(), length)
+
+    def negated_waveform(fwd, inv, z, s):
+        return fwd(z.conj().imag)
+
+    def gradient_through_conj(fwd, inv, z, s):
+        x = z.real.clone().requires_grad_(True)
+        return torch.autograd.grad(fwd(x).conj(), x, s)[0]
+
+    def gradient_of_inverse_through_conj(fwd, inv, z, s):
+        s = s.detach().clone().requires_grad_(True)
+        return torch.autograd.grad(inv(s.conj(), length), s, z.conj().imag[:, :length])[0]
+
+    for fn in (inverse, negated_waveform, gradient_through_conj, gradient_of_inverse_through_conj):
+        assert _rel(ours(fn), reference(fn)) < tol, fn.__name__
