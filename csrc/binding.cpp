@@ -347,7 +347,7 @@ at::Tensor topk_select(const at::Tensor& grad, at::Tensor residual, double ratio
 
 // One optimizer step of a parameter group, checks included, if `plan` covers exactly `params` and everything is as
 // the kernel wants it; false, with nothing done, otherwise (the caller then goes through the parameters one by one).
-// `steps`: the parameters' step counters, host tensors; the first says which step this is, all are advanced to it.
+// `steps`: the parameters' step counters, host tensors that agree; all are advanced.
 bool adamw_step_group(AdamWPlan& plan, const py::list& params, const py::list& steps, double lr, double beta1,
                       double beta2, double eps, double weight_decay, double grad_scale) {
   auto plain = [](const py::handle& h) { return THPVariable_CheckExact(h.ptr()); };
@@ -367,6 +367,7 @@ bool adamw_step_group(AdamWPlan& plan, const py::list& params, const py::list& s
     if (!dense_floats(p) || p.data_ptr() != own[i].data_ptr() || !dense_floats(p.grad())) return false;
     if (!c.defined() || !c.is_cpu() || c.layout() != at::kStrided || c.scalar_type() != at::kFloat || c.numel() != 1)
       return false;
+    if (i > 0 && *c.data_ptr<float>() != *counters[0].data_ptr<float>()) return false;  // each has its own bias correction
     grads.push_back(p.grad());
     counters.push_back(c);
   }

@@ -36,7 +36,7 @@ struct BucketOptimizerState {
   };
   struct ParamEntry {
     at::Tensor p, m, v;
-    int group = 0;
+    int group = 0;  // negative: its update is left to optimizer.step()
   };
   struct BucketPlan {
     std::vector<int64_t> signature;                      // addresses of the bucket's parameters
@@ -99,7 +99,7 @@ class BucketOptimizerHook : public c10d::CommHookInterface {
       for (size_t i = 0; i < params.size(); ++i) {
         auto it = st.params.find(sig[i]);
         MCCL_CHECK(it != st.params.end(), "a DDP bucket holds a parameter the optimizer was not given");
-        by_group[it->second.group].push_back(i);
+        if (it->second.group >= 0) by_group[it->second.group].push_back(i);
       }
       for (auto& kv : by_group) {
         std::vector<at::Tensor> ps, ms, vs;
@@ -126,7 +126,8 @@ class BucketOptimizerHook : public c10d::CommHookInterface {
       MCCL_CHECK(bp.groups[k] < static_cast<int>(st.hyper.size()), "hyper-parameters of param group " << bp.groups[k] << " were never set");
       launches.push_back({bp.plans[k].get(), st.hyper[bp.groups[k]]});
     }
-    for (int64_t a : sig) st.stepped.push_back(a);
+    for (const auto& positions : bp.positions)
+      for (size_t i : positions) st.stepped.push_back(sig[i]);
     const int64_t step = st.step;
     const float scale = static_cast<float>(st.scale);
     lk.unlock();

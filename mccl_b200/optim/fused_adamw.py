@@ -42,6 +42,25 @@ class FusedAdamW(torch.optim.Optimizer):
             self._index_params()
             self._bw_cache.clear()
 
+    def _state_of(self, p):
+        st = self.state[p]
+        if "exp_avg" not in st:
+            st["step"] = torch.tensor(0.0)
+            st["exp_avg"] = torch.zeros_like(p, memory_format=torch.preserve_format)
+            st["exp_avg_sq"] = torch.zeros_like(p, memory_format=torch.preserve_format)
+        return st
+
+    def _by_step(self, params):
+        """``{step number of the coming update: its parameters}``; one entry unless some parameter missed a step."""
+        counters = [self._state_of(p)["step"] for p in params]
+        if all(isinstance(c, torch.Tensor) and c.is_cuda for c in counters):
+            # (torch's own fused AdamW keeps them on the device: one copy for all instead of one for each)
+            counters = torch.stack([c.reshape(()) for c in counters]).tolist()
+        out = {}
+        for p, c in zip(params, counters):
+            out.setdefault(int(c) + 1, []).append(p)
+        return out
+
     def _plan_for(self, gi, params):
         key = (gi, tuple(p.data_ptr() for p in params))
         plan = self._plans.get(gi)
@@ -49,11 +68,7 @@ class FusedAdamW(torch.optim.Optimizer):
             native = require_native()
             ms, vs = [], []
             for p in params:
-                st = self.state[p]
-                if "exp_avg" not in st:
-                    st["step"] = torch.tensor(0.0)
-                    st["exp_avg"] = torch.zeros_like(p, memory_format=torch.preserve_format)
-                    st["exp_avg_sq"] = torch.zeros_like(p, memory_format=torch.preserve_format)
+                st = self._state_of(p)
                 ms.append(st["exp_avg"])
                 vs.append(st["exp_avg_sq"])
             plan = (key, native.AdamWPlan([p.data for p in params], ms, vs))
@@ -94,35 +109,42 @@ class FusedAdamW(torch.optim.Optimizer):
             if not all(p.is_cuda and p.dtype == torch.float32 and p.is_contiguous() for p in params):
                 raise RuntimeError("FusedAdamW handles contiguous float32 CUDA parameters "
                                    "(see mccl_b200.params.ensure_contiguous_parameters)")
-            plan = self._plan_for(gi, params)
-            st0 = self.state[params[0]]
-            step = int(st0["step"].item()) + 1 if isinstance(st0["step"], torch.Tensor) else int(st0["step"]) + 1
-            grads = [p.grad if p.grad.is_contiguous() else p.grad.contiguous() for p in params]
             b1, b2 = group["betas"]
-            plan.step(grads, group["lr"], b1, b2, group["eps"], group["weight_decay"], step, grad_scale)
-            for p in params:
-                s = self.state[p]["step"]
-                if isinstance(s, torch.Tensor):
-                    s.fill_(float(step))  # host tensor, as torch.optim.AdamW keeps it by default
-                else:
-                    self.state[p]["step"] = step
+            # the bias corrections are those of a parameter's own counter: one launch for each value among them
+            for part, (step, own) in enumerate(self._by_step(params).items()):
+                plan = self._plan_for(gi if part == 0 else (gi, part), own)
+                grads = [p.grad if p.grad.is_contiguous() else p.grad.contiguous() for p in own]
+                plan.step(grads, group["lr"], b1, b2, group["eps"], group["weight_decay"], step, grad_scale)
+                for p in own:
+                    s = self.state[p]["step"]
+                    if isinstance(s, torch.Tensor):
+                        s.fill_(float(step))  # host tensor, as torch.optim.AdamW keeps it by default
+                    else:
+                        self.state[p]["step"] = step
         self._bw_done = set()
         return loss
 
     # ---- per-bucket stepping (optimizer inside backward) -----------------------
+    # One step number, that of the first trainable parameter, serves all that is updated inside backward.  Parameters
+    # whose counters differ from it (as a checkpoint can hold them) are left to `step()`, which knows each one's own.
+    def _next_step(self) -> int:
+        params = [p for g in self.param_groups for p in g["params"]]
+        st = self.state[next((p for p in params if p.requires_grad), params[0])]
+        return int(st["step"]) + 1 if "step" in st else 1
+
+    def _on_shared_step(self, params) -> set:
+        return {id(p) for p in self._by_step(params).get(self._next_step(), ())}
+
     def begin_step_in_backward(self) -> int:
         """Advances the shared step counter once per iteration; returns the new step."""
-        self._bw_step = getattr(self, "_bw_step", None)
-        any_p = next(p for g in self.param_groups for p in g["params"])
-        st = self.state[any_p]
-        cur = int(st["step"].item()) if "step" in st else 0
-        self._bw_step = cur + 1
+        self._bw_step = self._next_step()
         self._bw_done = set()
         self._bw_touched = []
         return self._bw_step
 
     def bucket_plans(self, key, params):
-        """Launch plans of one DDP bucket: a list of ``(plan, group, own_params, positions)``.
+        """Launch plans of one DDP bucket: a list of ``(plan, group, own_params, positions)``, without the parameters
+        that ``step()`` will update.
 
         A bucket may hold parameters of several param groups (for example weights with weight decay
         and biases without); each group gets its own plan so that every parameter is updated with its
@@ -134,11 +156,14 @@ class FusedAdamW(torch.optim.Optimizer):
         ent = self._bw_cache.get(key)
         if ent is None or ent[0] != sig:
             by_group = {}
-            for pos, p in enumerate(params):
-                try:
-                    own, gi = self._by_ptr[p.data_ptr()]
-                except KeyError:
-                    raise KeyError("a DDP bucket holds a parameter this optimizer was not given") from None
+            try:
+                found = [self._by_ptr[p.data_ptr()] for p in params]
+            except KeyError:
+                raise KeyError("a DDP bucket holds a parameter this optimizer was not given") from None
+            here = self._on_shared_step([own for own, _ in found])
+            for pos, (own, gi) in enumerate(found):
+                if id(own) not in here:
+                    continue
                 by_group.setdefault(gi, ([], []))
                 by_group[gi][0].append(own)
                 by_group[gi][1].append(pos)
@@ -155,21 +180,18 @@ class FusedAdamW(torch.optim.Optimizer):
         """Creates the AdamW state of every parameter (so that a native hook can be given the tensors)."""
         for group in self.param_groups:
             for p in group["params"]:
-                st = self.state[p]
-                if "exp_avg" not in st:
-                    st["step"] = torch.tensor(0.0)
-                    st["exp_avg"] = torch.zeros_like(p, memory_format=torch.preserve_format)
-                    st["exp_avg_sq"] = torch.zeros_like(p, memory_format=torch.preserve_format)
+                self._state_of(p)
 
     def attach_native_hook(self, hook_state) -> None:
         """Hands parameters, state tensors and group indices to a ``BucketOptimizerState``."""
         self.ensure_state()
+        here = self._on_shared_step([p for g in self.param_groups for p in g["params"]])
         for gi, group in enumerate(self.param_groups):
             for p in group["params"]:
                 if not (p.is_cuda and p.dtype == torch.float32 and p.is_contiguous()):
                     raise RuntimeError("FusedAdamW handles contiguous float32 CUDA parameters")
                 st = self.state[p]
-                hook_state.add_param(p.data, st["exp_avg"], st["exp_avg_sq"], gi)
+                hook_state.add_param(p.data, st["exp_avg"], st["exp_avg_sq"], gi if id(p) in here else -1)
         self._native_hook = hook_state
         self.sync_native_hook()
 
@@ -184,10 +206,7 @@ class FusedAdamW(torch.optim.Optimizer):
         for gi, group in enumerate(self.param_groups):
             b1, b2 = group["betas"]
             self._native_hook.set_hyper(gi, group["lr"], b1, b2, group["eps"], group["weight_decay"])
-        any_p = next(p for g in self.param_groups for p in g["params"])
-        st = self.state[any_p]
-        cur = int(st["step"].item()) if "step" in st else 0
-        self._native_hook.set_step(cur + 1)
+        self._native_hook.set_step(self._next_step())
 
     def mark_bucket_stepped(self, own) -> None:
         self._bw_touched.append(own)
