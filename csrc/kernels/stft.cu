@@ -111,12 +111,13 @@ __global__ void __launch_bounds__(256, LH <= 6 ? 4 : LH <= 8 ? 3 : LH <= 10 ? 2 
   F::fill_tables(tw, split);
   for (int j = threadIdx.x; j < F::n; j += blockDim.x) win[j] = window_at(a.window, j);
   __syncthreads();
-  const int reach = (F::n + a.hop - 1) / a.hop;  // frames that cover a sample
+  const int hop = min(a.hop, F::n);              // no sums beyond the int range with a hop near its end
+  const int reach = (F::n + hop - 1) / hop;      // frames that cover a sample
   if (kEnvelope) {
-    for (int j = threadIdx.x; j < a.hop && j < F::n; j += blockDim.x) {
+    for (int j = threadIdx.x; j < hop; j += blockDim.x) {
       float e = 0.f;
-      for (int i = j + (F::n - 1 - j) / a.hop * a.hop; i >= 0; i -= a.hop) e += win[i] * win[i];  // in frame order
-      for (int i = j; i < F::n; i += a.hop) win_env[i] = e > 1e-11f ? win[i] / e : 0.f;
+      for (int i = j + (F::n - 1 - j) / hop * hop; i >= 0; i -= hop) e += win[i] * win[i];  // in frame order
+      for (int i = j; i < F::n; i += hop) win_env[i] = e > 1e-11f ? win[i] / e : 0.f;
     }
     __syncthreads();
   }

@@ -3,7 +3,9 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <algorithm>
 #include <cmath>
+#include <limits>
 
 #include "common/errors.h"
 #include "kernels/stft_api.h"
@@ -63,6 +65,14 @@ void spec_strides(const at::Tensor& spec, int64_t n_fft, int64_t& sb, int64_t& s
   st = spec.stride(2);
 }
 
+// The kernels take an int.  Where frame 1 starts behind all samples of the padded signal every frame but the first is
+// empty, and any longer hop does the same.
+int kernel_hop(int64_t hop, int64_t samples, int64_t n_fft) {
+  hop = std::min(hop, samples + 2 * n_fft);
+  MCCL_CHECK_TENSOR(hop <= std::numeric_limits<int>::max(), "hop_length is out of range");
+  return static_cast<int>(hop);
+}
+
 void run_ifft_ola(const kern::IfftOlaArgs& a, const at::Tensor& out) {
   at::Tensor scratch;
   const int64_t floats = kern::ifft_ola_scratch(a);
@@ -102,7 +112,7 @@ at::Tensor stft_forward(const at::Tensor& waveform, const at::Tensor& window, in
   a.batch = static_cast<int>(B);
   a.n_frames = static_cast<int>(frames);
   a.n_fft = static_cast<int>(n_fft);
-  a.hop = static_cast<int>(hop);
+  a.hop = kernel_hop(hop, T, n_fft);
   a.pad = static_cast<int>(pad);
   a.reflect = center ? 1 : 0;
   a.divide_envelope = 0;
@@ -133,7 +143,7 @@ at::Tensor stft_backward(const at::Tensor& grad_spec_in, const at::Tensor& windo
   a.batch = static_cast<int>(B);
   a.n_frames = static_cast<int>(frames);
   a.n_fft = static_cast<int>(n_fft);
-  a.hop = static_cast<int>(hop);
+  a.hop = kernel_hop(hop, length, n_fft);
   a.hermitian = 0;  // adjoint of the one-sided forward transform: upper bins contribute nothing
   a.scale = normalized ? 1.0f / std::sqrt(static_cast<float>(n_fft)) : 1.0f;
   a.pad = center ? static_cast<int>(n_fft / 2) : 0;
@@ -166,7 +176,7 @@ at::Tensor istft_forward(const at::Tensor& spec_in, const at::Tensor& window, in
   a.batch = static_cast<int>(B);
   a.n_frames = static_cast<int>(frames);
   a.n_fft = static_cast<int>(n_fft);
-  a.hop = static_cast<int>(hop);
+  a.hop = kernel_hop(hop, length, n_fft);
   a.hermitian = 1;
   a.scale = (normalized ? std::sqrt(static_cast<float>(n_fft)) : 1.0f) / static_cast<float>(n_fft);
   a.pad = center ? static_cast<int>(n_fft / 2) : 0;
@@ -193,7 +203,7 @@ at::Tensor istft_backward(const at::Tensor& grad_waveform, const at::Tensor& win
   a.batch = static_cast<int>(B);
   a.n_frames = static_cast<int>(n_frames);
   a.n_fft = static_cast<int>(n_fft);
-  a.hop = static_cast<int>(hop);
+  a.hop = kernel_hop(hop, T, n_fft);
   a.pad = center ? static_cast<int>(n_fft / 2) : 0;
   a.reflect = 0;
   a.divide_envelope = 1;

@@ -217,3 +217,24 @@ def test_lazily_conjugated_and_negated_inputs(cuda_device, frames_major):
 
     for fn in (inverse, negated_waveform, gradient_through_conj, gradient_of_inverse_through_conj):
         assert _rel(ours(fn), reference(fn)) < tol, fn.__name__
+
+
+# A hop far beyond the signal, up to and beyond the range of an int: one frame, whatever the hop.
+@pytest.mark.gpu
+@pytest.mark.parametrize("hop", [1_000_000, 2**30 + 1, 2**31 - 4000, 2**31 - 1, 2**31, 2**32, 2**33 + 7])
+@pytest.mark.parametrize("n_fft", [8, 1024, 4096])
+def test_hops_beyond_the_signal(cuda_device, n_fft, hop):
+    samples, length = 3 * n_fft, n_fft // 2
+    gen = torch.Generator(device=cuda_device).manual_seed(5)
+    w = 0.1 + torch.rand(n_fft, generator=gen, device=cuda_device)
+    x = torch.randn(2, samples, generator=gen, device=cuda_device, requires_grad=True)
+    spec = torch.randn(2, n_fft // 2 + 1, 1, dtype=torch.complex64, generator=gen, device=cuda_device, requires_grad=True)
+
+    def all_four(h):
+        kw = dict(n_fft=n_fft, hop_length=h, win_length=n_fft, window=w, backend="cuda")
+        out, back = stft(x, **kw), istft(spec, length=length, **kw)
+        return (out, torch.autograd.grad(out, x, spec.detach())[0], back,
+                torch.autograd.grad(back, spec, x.detach()[:, :length])[0])
+
+    for got, want in zip(all_four(hop), all_four(samples + 1)):
+        assert torch.equal(got, want)
