@@ -14,8 +14,10 @@
 //
 // The sample decides speed, never results.  Heavily tied data (more elements than the list holds, or a crowded bin):
 // the select launch takes the exact threshold from the whole adjusted vector and the last two rank the ties in index
-// order.  Fewer non-zeros than k: the same two take all of them and the first zeros.  What is left, a sample that missed
-// by five standard deviations or a k-th element two octaves above it, one cluster selects from the whole vector.
+// order.  Fewer non-zeros than k, or all elements sent: the same two take all of them and the first zeros.  A k-th element
+// below the sampled magnitude (by five standard deviations, or a ratio above 0.98, at which nothing is listed) or two octaves
+// and more above it (hardly more non-zeros than k; layers of very different scale in one bucket; small ratios of heavy-tailed data): the select launch
+// first finds its bin, from the whole vector or from the list, its blocks meeting between two counts, and goes on from there.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -64,19 +66,22 @@ __device__ __forceinline__ int64_t at_most(int64_t a, int64_t b) { return a < b 
 
 constexpr int kBinShift = 13;            // keys per histogram bin: 1/1024 octave
 constexpr int kSubBins = 1 << kBinShift;
+constexpr int kCoarseShift = 20;         // kWide, kWhole: 11 bits, then 7; 13 are left
+constexpr int kFineBins = 1 << (kCoarseShift - kBinShift);
 constexpr int kRun = 4;                  // tiles whose pairs one warp puts out
 // Entries of the k-th element's bin that one block resolves; more (ties) are left to the whole grid.  51.5 M bf16
 // elements, dense result: 255 levels at 1 %, about 50 thousand entries, 222 us with one block and 441 us with the grid;
 // 40 levels at 1 %, 190 thousand, 480 and 450 us; 40 levels at 10 %, over a million, 1709 and 509 us.
 constexpr uint32_t kOneBlock = 128 * 1024;
-// kList: from the candidates.  kWhole: by one cluster from the vector.  kTies: the bin is known, threshold and ties
-// come from the vector.  kZeros: all non-zeros and the first zeros.
-enum Mode : uint32_t { kList, kWhole, kTies, kZeros };
+// kList: from the candidates.  kWide: from the candidates, among those of the open-ended last bin.  kTies: the bin is known,
+// threshold and ties come from the vector.  kWhole: the bin comes from the vector as well.  kZeros: all non-zeros and the
+// first zeros.
+enum Mode : uint32_t { kList, kWide, kWhole, kTies, kZeros };
 
 // The exact rule: an element is sent if key > threshold, or key == threshold and index <= last_index (kList) or it is
 // one of the first `need` (kTies, kZeros).
 struct ListState {
-  uint32_t hist[kBins];  // candidates by (key - base) >> kBinShift, the last bin open-ended
+  uint32_t hist[kBins];  // candidates by (key - base) >> kBinShift, the last bin open-ended; then by key >> kCoarseShift
   uint32_t base;         // smallest magnitude key that is a candidate
   uint32_t count;        // entries in the list
   uint32_t overflow;     // the list did not hold them all
@@ -86,6 +91,8 @@ struct ListState {
   uint32_t threshold, last_index;
   uint32_t ticket[3];    // blocks done: adjust, select, counts
   uint32_t sub[kSubBins];  // kTies: elements of the bin by key
+  uint32_t fine[kFineBins];  // kWide, kWhole: elements of the chosen coarse bin
+  uint32_t gate[4][2];   // kWide, kWhole: blocks that came to a meeting, and how it ended
 };
 static_assert(sizeof(ListState) % sizeof(uint4) == 0, "8-byte entries follow it in the scratch");
 // scratch: ListState, {start, count} per tile, the list of {index, value}, its entries inside the bin, counts per run
@@ -107,7 +114,10 @@ inline uint32_t sample_rank(int64_t n, int64_t k) {
   return static_cast<uint32_t>(std::min<double>(kSample, hits + 5.0 * std::sqrt(hits) + 8.0));
 }
 // Room for the elements that reach it: six standard deviations above their expected number, and some for ties.
+// None where the whole sample would be needed, at ratios above 0.98: its smallest element bounds nothing, and the list would
+// hold twice the vector's bytes (6.5 M fp32 elements, ratio 0.99: 359 us dense, 372 us pairs with it, 144 and 146 us without).
 inline int64_t list_capacity(int64_t n, int64_t k) {
+  if (sample_rank(n, k) == kSample) return 0;
   const double rank = sample_rank(n, k), expected = rank / kSample * static_cast<double>(n);
   return std::min<int64_t>(n, static_cast<int64_t>(expected * (1.06 + 6.0 / std::sqrt(rank))) + 4096);
 }
@@ -354,7 +364,8 @@ __global__ void __launch_bounds__(kThreads, 1) topk_sample_kernel(const SelectAr
     uint32_t* words = reinterpret_cast<uint32_t*>(a.list.state);
     for (int i = threadIdx.x; i < static_cast<int>(sizeof(ListState) / 4); i += kThreads) words[i] = 0u;
     __syncthreads();
-    if (threadIdx.x == 0) a.list.state->base = threshold > 0 ? threshold : 1u;  // zeros are never worth listing
+    if (threadIdx.x == 0)
+      a.list.state->base = rank == kSample ? 0xFFFFFFFFu : threshold > 0 ? threshold : 1u;  // zeros are never worth listing
   }
 }
 
@@ -540,16 +551,19 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
     if (above < a.k && above + c[i] >= a.k) {
       list.state->bin = static_cast<uint32_t>(top - i);
       list.state->need = a.k - above;
-      const bool crowded = __ldcg(&list.state->overflow) != 0u || c[i] > kOneBlock;
-      list.state->mode = top - i == kBins - 1 ? kWhole : crowded ? kTies : kList;  // the last bin is open-ended
+      const bool missing = __ldcg(&list.state->overflow) != 0u;
+      if (top - i == kBins - 1) list.state->mode = missing ? kWhole : kWide;
+      else list.state->mode = missing || c[i] > kOneBlock ? kTies : kList;
     }
     above += c[i];
+    list.state->hist[top - i] = 0u;
   }
   const uint32_t count = __ldcg(&list.state->count);
   if (threadIdx.x == 0 && count < a.k) {
-    list.state->mode = base == 1u ? kZeros : kWhole;  // every non-zero is a candidate, or the sample missed
+    // every non-zero is a candidate, everything is sent, or the sample missed (or none was taken)
+    list.state->mode = base == 1u || a.k == a.n ? kZeros : kWhole;
     list.state->threshold = 0u;
-    list.state->need = a.k - count;
+    list.state->need = a.k == a.n ? a.k : a.k - count;
   }
 }
 
@@ -598,48 +612,143 @@ __device__ uint32_t block_nth(uint32_t* hist, uint32_t* wsum, uint32_t* s_pick, 
   return prefix;
 }
 
-// Selection among the candidates, a grid of whole clusters; for kTies only the threshold, from the whole vector; for
-// kWhole the first cluster selects from the whole vector and the others leave.  e and (kDense) g hold the values of elements that are not selected.
+// Adds n keys to this block's counts by digit(key); those whose digit is `bins` or more are left out.  What comes here is
+// mostly tied: the digits of two lanes of a warp are counted for all that share them, and only the rest one by one.
+template <typename Key, typename Digit>
+__device__ __forceinline__ void count_digits(uint32_t* counts, uint32_t bins, int64_t n, Key&& key, Digit&& digit) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int i = tid; i < static_cast<int>(bins); i += kThreads) counts[i] = 0;
+  __syncthreads();
+  constexpr int kAhead = 8;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads * kAhead;
+  for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * kThreads * kAhead; i0 < n; i0 += step) {
+    uint32_t d[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int64_t i = i0 + u * kThreads + tid;
+      d[u] = i < n ? key(i) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      d[u] = digit(d[u]);
+      bool in = i0 + u * kThreads + tid < n && d[u] < bins;
+#pragma unroll
+      for (int round = 0; round < 2; ++round) {
+        const uint32_t left = __ballot_sync(0xFFFFFFFFu, in);
+        if (left == 0u) break;
+        const int leader = __ffs(left) - 1;
+        const uint32_t first = __shfl_sync(0xFFFFFFFFu, d[u], leader);  // by all lanes, whether counted or not
+        const bool same = in && d[u] == first;
+        const uint32_t all = __ballot_sync(0xFFFFFFFFu, same);
+        if (lane == leader) atomicAdd(&counts[first], static_cast<uint32_t>(__popc(all)));
+        in = in && !same;
+      }
+      if (in) atomicAdd(&counts[d[u]], 1u);
+    }
+  }
+  __syncthreads();
+}
+
+// Waits for all blocks of the grid, with a limit: true in every block (what the others wrote before is then visible) or,
+// if one did not come in time because another grid holds its SM, false in every block.  One word decides.
+__device__ __forceinline__ bool grid_meets(uint32_t* gate, int tries) {
+  constexpr uint32_t kMet = 1u, kMissed = 2u;
+  __shared__ uint32_t s_end;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t end = 0u;
+    const bool last = atomicAdd(&gate[0], 1u) == gridDim.x - 1;
+    for (int i = 0; !last && end == 0u && i < tries; ++i) {
+      __nanosleep(100);
+      end = *reinterpret_cast<volatile uint32_t*>(&gate[1]);
+    }
+    if (end == 0u) {
+      const uint32_t mine = last ? kMet : kMissed, was = atomicCAS(&gate[1], 0u, mine);
+      end = was == 0u ? mine : was;
+    }
+    __threadfence();
+    s_end = end;
+  }
+  __syncthreads();
+  return s_end == kMet;
+}
+
+// The kBinShift-wide bin that holds the need-th largest of n keys, from two counts by the whole grid; *need becomes how many
+// of its entries are selected, *entries how many it has.  False if the grid could not meet.
+template <typename Key>
+__device__ __forceinline__ bool find_bin(ListState* st, uint32_t* counts, uint32_t* wsum, uint32_t* s_pick, int64_t n, Key&& key,
+                                         uint32_t* floor_key, uint32_t* need, uint32_t* entries) {
+  const int tid = threadIdx.x;
+  uint32_t prefix = 0;
+  // All blocks start as soon as the launch before is done; once they have met they only wait for the slowest count.
+  if (!grid_meets(st->gate[0], 500)) return false;
+#pragma unroll 1
+  for (int level = 0; level < 2; ++level) {
+    const int bins = level == 0 ? kBins : kFineBins;
+    uint32_t* total = level == 0 ? st->hist : st->fine;
+    count_digits(counts, bins, n, key, [&](uint32_t k) {
+      if (level == 0) return k >> kCoarseShift;
+      return k >> kCoarseShift == prefix ? (k >> kBinShift) & (kFineBins - 1u) : 0xFFFFFFFFu;
+    });
+    for (int i = tid; i < bins; i += kThreads)
+      if (counts[i]) atomicAdd(&total[i], counts[i]);
+    if (!grid_meets(st->gate[level + 1], 1000000)) return false;
+    const int top = bins - 1 - 2 * tid;  // from the top bin down, two per thread
+    const uint32_t c0 = top > 0 ? __ldcg(&total[top]) : 0u, c1 = top > 0 ? __ldcg(&total[top - 1]) : 0u;
+    const uint32_t above = block_excl_scan(c0 + c1, wsum), left = *need;
+    if (above < left && above + c0 >= left) {
+      s_pick[0] = top;
+      s_pick[1] = above;
+      s_pick[2] = c0;
+    } else if (above + c0 < left && above + c0 + c1 >= left) {
+      s_pick[0] = top - 1;
+      s_pick[1] = above + c0;
+      s_pick[2] = c1;
+    }
+    __syncthreads();
+    *need = left - s_pick[1];
+    *entries = s_pick[2];
+    prefix = level == 0 ? s_pick[0] : prefix * kFineBins + s_pick[0];
+    __syncthreads();
+  }
+  *floor_key = prefix << kBinShift;
+  return true;
+}
+
+// Selection among the candidates, a grid of whole clusters; for kTies and kWhole only the threshold, from the whole vector.
+// e and (kDense) g hold the values of elements that are not selected.
+// 51.5 M fp32 elements, k = 0.1 % of two populations, the larger 1.1 k (kWide), pairs: the three passes of topk.cu 345 us, one
+// cluster over the vector 2287 us, so 181 us.  All of them sent (ratio 1, kZeros): 519, 2755 and 366 us.
 template <bool kBf16, bool kDense>
 __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectArgs a) {
   __shared__ ClusterShared sh;
-  __shared__ uint32_t s_count, s_base, s_pick[2];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ uint32_t s_count, s_base, s_pick[3];
+  extern __shared__ __align__(16) uint32_t sub[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   ListState* st = a.list.state;
-  const uint32_t mode = st->mode;
+  uint32_t mode = st->mode;
   if (mode == kZeros) return;
+  uint32_t floor_key = st->base + (st->bin << kBinShift), need = st->need;  // the k-th element's bin
+  auto vector_key = [&](int64_t i) { return key_of(__ldcs(a.residual + i)); };
+  if (mode == kWide) {
+    need = a.k;
+    uint32_t entries = 0;
+    if (find_bin(st, sub, sh.wsum, s_pick, st->count, [&](int64_t i) { return a.list.list[i].y & 0x7FFFFFFFu; }, &floor_key,
+                 &need, &entries))
+      mode = entries > kOneBlock ? kTies : kList;
+  } else if (mode == kWhole) {
+    need = a.k;
+    uint32_t entries = 0;
+    if (find_bin(st, sub, sh.wsum, s_pick, a.n, vector_key, &floor_key, &need, &entries)) mode = kTies;
+  }
   if (mode == kTies) {
-    extern __shared__ __align__(16) uint32_t sub[];
-    const uint32_t floor_key = st->base + (st->bin << kBinShift);
-    for (int i = tid; i < kSubBins; i += kThreads) sub[i] = 0;
-    __syncthreads();
-    auto add = [&](float v, bool valid) {  // equal keys of a warp are counted together: most are ties
-      const uint32_t d = key_of(v) - floor_key;
-      const bool in = valid && d < kSubBins;
-      const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
-      if (!in) return;
-      const uint32_t same = __match_any_sync(m, d);
-      if (lane == __ffs(same) - 1) atomicAdd(&sub[d], static_cast<uint32_t>(__popc(same)));
-    };
-    constexpr int kAhead = 8;
-    const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads * kAhead;
-    for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * kThreads * kAhead; i0 < a.n; i0 += step) {
-      float v[kAhead];
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int64_t i = i0 + u * kThreads + tid;
-        v[u] = i < a.n ? __ldcs(a.residual + i) : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) add(v[u], i0 + u * kThreads + tid < a.n);
-    }
-    __syncthreads();
+    count_digits(sub, kSubBins, a.n, vector_key, [&](uint32_t key) { return key - floor_key; });
     for (int i = tid; i < kSubBins; i += kThreads)
       if (sub[i]) atomicAdd(&st->sub[i], sub[i]);
     if (!last_block_done(&st->ticket[1])) return;
     constexpr int kPer = kSubBins / kThreads;
     const int top = kSubBins - 1 - kPer * tid;
-    const uint32_t need = st->need;
     uint32_t c[kPer], run = 0;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
@@ -647,7 +756,6 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
       run += c[i];
     }
     uint32_t above = block_excl_scan(run, sh.wsum);
-    __syncthreads();  // every thread has read `need`
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       if (above < need && above + c[i] >= need) {
@@ -656,10 +764,11 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
       }
       above += c[i];
     }
+    if (tid == 0) st->mode = kTies;
     return;
   }
   if (mode == kList) {
-    const uint32_t count = st->count, base = st->base, bin = st->bin;
+    const uint32_t count = st->count;
     uint2* bin_list = a.list.bin_list;
     constexpr int kAhead = 4;
     const uint32_t step = gridDim.x * kThreads * kAhead;
@@ -677,9 +786,9 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
       for (int u = 0; u < kAhead; ++u) {
         const bool valid = i0 + u * kThreads + tid < count;
         const float v = __uint_as_float(e[u].y);
-        const uint32_t b = valid ? bin_of(key_of(v) - base) : 0u;
-        if (kDense && valid && b > bin) send<kBf16, kDense>(a, e[u].x, v);
-        const bool inside = valid && b == bin;
+        const uint32_t key = key_of(v), from_floor = key - floor_key;  // wraps below the bin
+        if (kDense && valid && key >= floor_key && from_floor >= kSubBins) send<kBf16, kDense>(a, e[u].x, v);
+        const bool inside = valid && from_floor < kSubBins;
         at[u] = inside ? atomicAdd(&s_count, 1u) : 0xFFFFFFFFu;
       }
       __syncthreads();
@@ -692,8 +801,9 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
     }
     if (!last_block_done(&st->ticket[1])) return;
     // the bin's entries: the exact key, then the index limit among the entries that share it
-    const uint32_t m = __ldcg(&st->in_bin), floor_key = base + (bin << kBinShift);
-    uint32_t need = st->need, equal = 0;
+    const uint32_t m = __ldcg(&st->in_bin);
+    uint32_t equal = 0;
+    if (tid == 0) st->mode = kList;
     const uint32_t low = block_nth<true>(sh.hist, sh.wsum, s_pick, m, &need, &equal, kBinShift, [&](uint32_t i) {
       return static_cast<uint64_t>((__ldcg(&bin_list[i].y) & 0x7FFFFFFFu) - floor_key);
     });
@@ -716,6 +826,7 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
     }
     return;
   }
+  // the grid is not resident as a whole: the first cluster selects from the vector, the others leave
   cg::cluster_group cluster = cg::this_cluster();
   const int ctas = static_cast<int>(cluster.num_blocks()), me = static_cast<int>(cluster.block_rank());
   if (static_cast<int>(blockIdx.x) >= ctas) return;
@@ -764,7 +875,7 @@ __global__ void __launch_bounds__(kThreads, 1) topk_output_kernel(const SelectAr
   const int lane = threadIdx.x & 31;
   ListState* st = a.list.state;
   const uint32_t mode = st->mode;
-  if (mode == kWhole || (mode == kList && kDense)) return;
+  if (mode == kWhole || mode == kWide || (mode == kList && kDense)) return;
   const uint32_t threshold = st->threshold, last_index = st->last_index, need = st->need;
   const uint32_t lower = (1u << lane) - 1u;
   const int64_t tiles = tile_count(a.n), runs = run_count(a.n);
@@ -838,11 +949,11 @@ __global__ void __launch_bounds__(kThreads, 1) topk_output_kernel(const SelectAr
 }
 
 // Sixteen CTAs where a cluster of that size can be resident (it needs a GPC with as many free SMs), else the
-// portable eight.  Asked once per kernel and device.
+// portable eight; `resident`: how many such clusters the device holds at once.  Asked once per kernel and device.
 struct ClusterSize {
-  std::atomic<int> of[64] = {};
+  std::atomic<int> of[64] = {};  // size + 64 * resident
 };
-cudaError_t cluster_size(const void* kernel, ClusterSize& cache, size_t most_smem, int* out) {
+cudaError_t cluster_size(const void* kernel, ClusterSize& cache, size_t most_smem, int* out, int* resident = nullptr) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -863,11 +974,17 @@ cudaError_t cluster_size(const void* kernel, ClusterSize& cache, size_t most_sme
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    size = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0 ? kMaxCluster : 8;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters <= 0) {
+      attr.val.clusterDim.x = 8;
+      cfg.gridDim = dim3(8);
+      if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters <= 0) clusters = 1;
+    }
     cudaGetLastError();  // a failed query only means the portable size
+    size = static_cast<int>(cfg.gridDim.x) + 64 * clusters;
     if (dev < 64) cache.of[dev].store(size, std::memory_order_release);
   }
-  *out = size;
+  *out = size % 64;
+  if (resident != nullptr) *resident = size / 64;
   return cudaSuccess;
 }
 
@@ -927,9 +1044,11 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
 
   auto select = topk_select_kernel<kBf16, kDense>;
-  e = cluster_size(reinterpret_cast<const void*>(select), select_size, kSubBins * sizeof(uint32_t), &ctas);
+  int resident_clusters = 0;
+  e = cluster_size(reinterpret_cast<const void*>(select), select_size, kSubBins * sizeof(uint32_t), &ctas, &resident_clusters);
   if (e != cudaSuccess) return e;
-  const int clusters = static_cast<int>(std::min<int64_t>(128 / ctas, (a.n + (1 << 20) - 1) >> 20));
+  // no more than can meet (kWhole)
+  const int clusters = static_cast<int>(std::min<int64_t>({128 / ctas, resident_clusters, (a.n + (1 << 20) - 1) >> 20}));
   e = launch_cluster(select, clusters, ctas, kSubBins * sizeof(uint32_t), s, a);
   if (e != cudaSuccess) return e;
   const unsigned pgrid = static_cast<unsigned>(std::min<int64_t>(148, (run_count(a.n) + kWarps - 1) / kWarps));

@@ -162,6 +162,87 @@ def test_select_and_dense_paths_match_host_oracle(native, cuda_device, one_rank,
     assert torch.equal(res.cpu(), comp.residual(0))
 
 
+def _missing(kind, n, ratio):
+    """Data for which the k-th element lies outside what the sampled magnitude bounds."""
+    gen = torch.Generator().manual_seed(n)
+    g = torch.randn(n, generator=gen)
+    if kind == "nonzeros":        # somewhat more non-zeros than entries to send: the bound is the smallest non-zero
+        g = g * (torch.rand(n, generator=gen) < 1.1 * ratio)
+    elif kind == "two_scales":    # the larger population ends between rank k and the sampled rank
+        g = torch.where(torch.rand(n, generator=gen) < 1.1 * ratio, g.sign() * (100 + g.abs()), 0.1 * g)
+    elif kind == "two_levels":    # the same with ties on both sides
+        g = torch.where(torch.rand(n, generator=gen) < 1.1 * ratio, 64 * g.sign(), 0.25 * g.sign())
+    elif kind == "heavy":         # magnitudes over hundreds of octaves
+        g = g * torch.exp2(20 * torch.randn(n, generator=gen))
+    return g
+
+
+# k below and above the sampled rank, close to n, and all of n; tiles and groups cut short.  Exact.
+@pytest.mark.parametrize("n,ratio", [(393_217, 0.01), (1_048_577, 0.001), (3_000_001, 0.1), (5_000_000, 1e-5), (700_001, 0.99),
+                                     (2_000_001, 1.0)])
+@pytest.mark.parametrize("kind", ["nonzeros", "two_scales", "two_levels", "heavy", "normal"])
+def test_select_where_the_sampled_bound_misses(native, cuda_device, one_rank, n, ratio, kind):
+    g = _missing(kind, n, ratio)
+    comp, idx, val = _oracle_pairs(native, g, ratio)
+    idx, val = torch.tensor(idx), torch.tensor(val)
+    res = torch.zeros(n, device=cuda_device)
+    pairs = native._topk_select(g.to(cuda_device), res, ratio).cpu()
+    assert torch.equal(pairs[:, 0].long(), idx)
+    assert torch.equal(pairs[:, 1].view(torch.float32), val)
+    assert torch.equal(res.cpu(), comp.residual(0))
+    grad, res = g.to(cuda_device), torch.zeros(n, device=cuda_device)
+    one_rank.allreduce_topk(grad, res, ratio, 0.5).wait()
+    want = torch.zeros(n)
+    want[idx] = val * 0.5
+    assert torch.equal(grad.cpu(), want)
+    assert torch.equal(res.cpu(), comp.residual(0))
+
+
+def _time_us(fn, reset, runs=5):
+    best = float("inf")
+    for _ in range(runs):
+        reset()
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(200_000)  # the launches are all queued when the first one runs
+        a.record()
+        fn()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b) * 1e3)
+    return best
+
+
+@pytest.mark.parametrize("kind,ratio", [("two_scales", 0.01), ("nonzeros", 0.01), ("normal", 1.0)])
+def test_a_missed_bound_costs_passes_not_a_single_cluster(native, cuda_device, kind, ratio):
+    # Eight passes of the whole GPU at the very most against three; one cluster over the vector takes more than tenfold.
+    n = 32_000_000
+    res = torch.zeros(n, device=cuda_device)
+
+    def cost(g, ratio):
+        return _time_us(lambda: native._topk_select(g, res, ratio), res.zero_)
+
+    plain = cost(_missing("normal", n, 0.01).to(cuda_device), 0.01)
+    assert cost(_missing(kind, n, ratio).to(cuda_device), ratio) < 5 * plain
+
+
+def test_a_missed_bound_on_two_streams_at_once(native, cuda_device):
+    # Two grids that each want most of the device: whichever is not resident as a whole falls back and stays exact.
+    n, ratio = 4_000_001, 0.01
+    gs = [_missing("two_scales", n - i, ratio).to(cuda_device) for i in range(2)]
+    want = [native._topk_select(g, torch.zeros_like(g), ratio).clone() for g in gs]
+    streams = [torch.cuda.Stream() for _ in gs]
+    torch.cuda.synchronize()
+    for _ in range(10):
+        got = []
+        for g, s in zip(gs, streams):
+            with torch.cuda.stream(s):
+                got.append((native._topk_select(g, torch.zeros_like(g), ratio)))
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+
+
 @pytest.fixture(scope="module")
 def one_rank(cuda_device):
     import torch.distributed as dist
