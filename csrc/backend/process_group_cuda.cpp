@@ -19,6 +19,7 @@
 
 #include "backend/process_group.h"
 #include "backend/tensor_checks.h"
+#include "backend/topk_scratch.h"
 #include "common/log.h"
 #include "kernels/topk_api.h"
 #include "runtime/nvls.h"
@@ -925,8 +926,8 @@ c10::intrusive_ptr<c10d::Work> ProcessGroupMCCL::allreduce_topk(at::Tensor& grad
     // scratch: candidate list + counters; pairs: this rank's (idx,val) list of the largest segment
     c10::cuda::CUDAStreamGuard sg(p2p ? cp->stream : c10::cuda::getCurrentCUDAStream(dev));
     const int64_t most = std::min(seg, n);
-    scratch = at::empty({static_cast<int64_t>(kern::topk_scratch_bytes(most, k_for(most)))}, grad.options().dtype(at::kByte));
     if (p2p) pairs = at::empty({k_for(most) * 2}, grad.options().dtype(at::kInt));
+    scratch = topk_scratch(most, k_for(most), !p2p, grad.options());
   }
   const size_t gsz = grad.element_size();
   uint64_t sent = 0;

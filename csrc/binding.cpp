@@ -24,6 +24,7 @@
 #include "backend/options.h"
 #include "backend/process_group.h"
 #include "backend/tensor_checks.h"
+#include "backend/topk_scratch.h"
 #include "common/version.h"
 #include "compression/compressor.h"
 #include "cpu/reduce.h"
@@ -281,8 +282,8 @@ class EmuGroup {
     std::vector<at::Tensor> pairs;
     kern::TopkArgs a0;
     for (int r = 0; r < ws_; ++r) {
-      at::Tensor scratch = at::empty({static_cast<int64_t>(kern::topk_scratch_bytes(n, k))}, grads[r].options().dtype(at::kByte));
       pairs.push_back(at::empty({k * 2}, grads[r].options().dtype(at::kInt)));
+      at::Tensor scratch = topk_scratch(n, k, false, grads[r].options());
       kern::TopkArgs a;
       a.grad = grads[r].data_ptr();
       a.grad_is_bf16 = grads[r].scalar_type() == at::kBFloat16;
@@ -329,8 +330,8 @@ at::Tensor topk_select(const at::Tensor& grad, at::Tensor residual, double ratio
   const int64_t n = grad.numel();
   int64_t k = std::max<int64_t>(1, static_cast<int64_t>(std::floor(static_cast<double>(n) * ratio)));
   k = std::min(k, n);
-  at::Tensor scratch = at::empty({static_cast<int64_t>(kern::topk_scratch_bytes(n, k))}, grad.options().dtype(at::kByte));
   at::Tensor pairs = at::empty({k, 2}, grad.options().dtype(at::kInt));
+  at::Tensor scratch = topk_scratch(n, k, false, grad.options());
   kern::TopkArgs a;
   a.grad = grad.data_ptr();
   a.grad_is_bf16 = grad.scalar_type() == at::kBFloat16;

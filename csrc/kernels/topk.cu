@@ -635,8 +635,10 @@ size_t topk_scratch_bytes(int64_t n, int64_t k) {
   return std::max(sizeof(TopkScratch), topk_fits_cluster(n) ? size_t(0) : topk_list_scratch_bytes(n, k));
 }
 
+size_t topk_dense_min_scratch_bytes(int64_t n) { return topk_fits_cluster(n) ? 0 : topk_list_min_scratch_bytes(n); }
+
 cudaError_t launch_topk_dense(const TopkArgs& a, cudaStream_t s) {
-  if (a.n <= 0 || a.k <= 0 || a.k > a.n || a.scratch_bytes < topk_scratch_bytes(a.n, a.k)) return cudaErrorInvalidValue;
+  if (a.n <= 0 || a.k <= 0 || a.k > a.n || a.scratch_bytes < topk_dense_min_scratch_bytes(a.n)) return cudaErrorInvalidValue;
   return launch_topk_cluster(a, true, s);
 }
 

@@ -44,15 +44,18 @@ struct TopkArgs {
   int64_t n;
   int64_t k;
   void* scratch;        // device memory (any contents)
-  size_t scratch_bytes; // of it; at least topk_min_scratch_bytes()
+  size_t scratch_bytes; // of it; at least topk_min_scratch_bytes() or topk_dense_min_scratch_bytes(n)
   void* pairs;          // k * 8 bytes: {u32 index, f32 value}; unused by launch_topk_dense
   float scale;          // applied in scatter
 };
 
-// What the fastest path for this problem wants.
+// What the fastest path for this problem wants: above 384 Ki elements 8 bytes for each of somewhat more than k listed
+// elements (1.2 k + 4096 at 1 % of 51.5 M; none above a ratio of 0.98), 1 MB at most for those of one bin, 10 bytes per 1024 elements.
 size_t topk_scratch_bytes(int64_t n, int64_t k);
-// What any problem can do with: 3 histograms, the selection state, per-block counts/offsets (about 53 KB).
+// What any problem can do with: 3 histograms, the selection state, per-block counts/offsets (about 53 KB) for
+// launch_topk_select, and 10 bytes per 1024 elements and 60 KB for launch_topk_dense, whose list then overflows.
 size_t topk_min_scratch_bytes();
+size_t topk_dense_min_scratch_bytes(int64_t n);
 #ifdef __CUDACC__
 __host__ __device__
 #endif
@@ -64,11 +67,12 @@ inline size_t topk_pad(size_t bytes) { return (bytes + 127) / 128 * 128; }
 cudaError_t launch_topk_select(const TopkArgs& a, cudaStream_t s);
 // p: arena parameters (ctx[].in = pairs, ctx[].out = dense gradient); count = k.
 cudaError_t launch_topk_exchange_scatter(const CollParams& p, const TopkArgs& a, LaunchCfg cfg, cudaStream_t s);
-// World size 1: select, and grad = scale * selection.  Needs topk_scratch_bytes(n, k) of scratch.
+// World size 1: select, and grad = scale * selection.
 cudaError_t launch_topk_dense(const TopkArgs& a, cudaStream_t s);
 
 // topk_cluster.cu
 size_t topk_list_scratch_bytes(int64_t n, int64_t k);
+size_t topk_list_min_scratch_bytes(int64_t n);
 bool topk_fits_cluster(int64_t n);  // on any device: one launch, no scratch
 cudaError_t launch_topk_cluster(const TopkArgs& a, bool dense, cudaStream_t s);
 

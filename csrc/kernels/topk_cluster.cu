@@ -95,13 +95,13 @@ struct ListState {
   uint32_t gate[4][2];   // kWide, kWhole: blocks that came to a meeting, and how it ended
 };
 static_assert(sizeof(ListState) % sizeof(uint4) == 0, "8-byte entries follow it in the scratch");
-// scratch: ListState, {start, count} per tile, the list of {index, value}, its entries inside the bin, counts per run
+// scratch: ListState, {start, count} per tile, counts per run, the list of {index, value}, its entries inside the bin
 struct ListView {
   ListState* state;
   uint2* tiles;
+  uint2* runs;
   uint2* list;
   uint2* bin_list;
-  uint2* runs;
   uint32_t cap;
 };
 
@@ -121,14 +121,21 @@ inline int64_t list_capacity(int64_t n, int64_t k) {
   const double rank = sample_rank(n, k), expected = rank / kSample * static_cast<double>(n);
   return std::min<int64_t>(n, static_cast<int64_t>(expected * (1.06 + 6.0 / std::sqrt(rank))) + 4096);
 }
-inline ListView list_view(void* scratch, int64_t n, int64_t k) {
+inline int64_t table_bytes(int64_t n) {
+  return static_cast<int64_t>(sizeof(ListState)) + (tile_count(n) + run_count(n)) * static_cast<int64_t>(sizeof(uint2));
+}
+// The entries of one bin: at most as many as the list has, or one block resolves.
+inline int64_t bin_capacity(int64_t cap) { return std::min<int64_t>(cap, kOneBlock); }
+// The list takes what there is room for; one that is too short overflows, which is as good as heavily tied data.
+inline ListView list_view(void* scratch, size_t bytes, int64_t n, int64_t k) {
+  const int64_t room = (static_cast<int64_t>(bytes) - table_bytes(n)) / static_cast<int64_t>(sizeof(uint2));
   ListView v;
   v.state = static_cast<ListState*>(scratch);
   v.tiles = reinterpret_cast<uint2*>(v.state + 1);
-  v.list = v.tiles + tile_count(n);
-  v.cap = static_cast<uint32_t>(list_capacity(n, k));
+  v.runs = v.tiles + tile_count(n);
+  v.list = v.runs + run_count(n);
+  v.cap = static_cast<uint32_t>(std::min(list_capacity(n, k), std::max(room / 2, room - static_cast<int64_t>(kOneBlock))));
   v.bin_list = v.list + v.cap;
-  v.runs = v.bin_list + v.cap;
   return v;
 }
 
@@ -796,7 +803,7 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
       __syncthreads();
 #pragma unroll
       for (int u = 0; u < kAhead; ++u)
-        if (at[u] != 0xFFFFFFFFu) bin_list[s_base + at[u]] = e[u];  // at most as many as the list has
+        if (at[u] != 0xFFFFFFFFu) bin_list[s_base + at[u]] = e[u];  // kList: no more than bin_capacity()
       __syncthreads();
     }
     if (!last_block_done(&st->ticket[1])) return;
@@ -1059,20 +1066,22 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
 
 }  // namespace
 
+size_t topk_list_min_scratch_bytes(int64_t n) { return static_cast<size_t>(table_bytes(n)) + 2 * kTile * sizeof(uint2); }
 size_t topk_list_scratch_bytes(int64_t n, int64_t k) {
-  return sizeof(ListState) + static_cast<size_t>(tile_count(n) + 2 * list_capacity(n, k)) * sizeof(uint2) +
-         static_cast<size_t>(run_count(n)) * sizeof(uint2);
+  const int64_t cap = list_capacity(n, k);
+  return std::max(topk_list_min_scratch_bytes(n),
+                  static_cast<size_t>(table_bytes(n) + (cap + bin_capacity(cap)) * static_cast<int64_t>(sizeof(uint2))));
 }
 
 cudaError_t launch_topk_cluster(const TopkArgs& t, bool dense, cudaStream_t s) {
-  SelectArgs a;
+  SelectArgs a{};
   a.grad = const_cast<void*>(t.grad);
   a.residual = t.residual;
   a.pairs = static_cast<uint2*>(t.pairs);
   a.n = t.n;
   a.k = static_cast<uint32_t>(t.k);
   a.scale = t.scale;
-  a.list = list_view(t.scratch, t.n, t.k);
+  if (!topk_fits_cluster(t.n)) a.list = list_view(t.scratch, t.scratch_bytes, t.n, t.k);
   if (t.grad_is_bf16) return dense ? run<true, true>(t, a, s) : run<true, false>(t, a, s);
   return dense ? run<false, true>(t, a, s) : run<false, false>(t, a, s);
 }

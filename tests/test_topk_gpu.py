@@ -243,6 +243,32 @@ def test_a_missed_bound_on_two_streams_at_once(native, cuda_device):
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("megabytes", [28, 8])
+def test_selection_without_room_for_the_list(native, cuda_device, one_rank, megabytes):
+    # Above the list's size a device has: what the pairs alone would need, and less.  The same results either way.
+    n, ratio = 20_000_001, 0.1
+    for kind in ("normal", "two_levels"):
+        g = _missing(kind, n, ratio).to(cuda_device)
+        want_grad, want_res, res = g.clone(), torch.zeros_like(g), torch.zeros_like(g)
+        one_rank.allreduce_topk(want_grad, want_res, ratio, 0.5).wait()
+        want_pairs = native._topk_select(g, res, ratio)
+        got_grad, got_res = g.clone(), torch.zeros_like(g)
+        res2 = torch.zeros_like(g)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        total = torch.cuda.get_device_properties(cuda_device).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (megabytes << 20)) / total)
+        try:
+            one_rank.allreduce_topk(got_grad, got_res, ratio, 0.5).wait()
+            pairs = native._topk_select(g, res2, ratio) if megabytes > 16 else None
+            torch.cuda.synchronize()
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        assert torch.equal(got_grad, want_grad) and torch.equal(got_res, want_res)
+        if pairs is not None:
+            assert torch.equal(pairs, want_pairs) and torch.equal(res2, res)
+
+
 @pytest.fixture(scope="module")
 def one_rank(cuda_device):
     import torch.distributed as dist
