@@ -1017,16 +1017,16 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
   static ClusterSize small_size, sample_size, select_size;
   constexpr size_t kItemBytes = kItemCap * sizeof(float);
   int ctas = 0;
-  auto small = topk_cluster_kernel<kBf16, kDense>;
-  cudaError_t e = cluster_size(reinterpret_cast<const void*>(small), small_size, kItemBytes, &ctas);
-  if (e != cudaSuccess) return e;
   if (topk_fits_cluster(a.n)) {
+    auto small = topk_cluster_kernel<kBf16, kDense>;
+    cudaError_t e = cluster_size(reinterpret_cast<const void*>(small), small_size, kItemBytes, &ctas);
+    if (e != cudaSuccess) return e;
     const int per = static_cast<int>(((a.n + ctas - 1) / ctas + 7) / 8 * 8);
     note_launch();
     return launch_cluster(small, 1, ctas, per * sizeof(float), s, a, per);
   }
   auto sample = topk_sample_kernel<kBf16>;
-  e = cluster_size(reinterpret_cast<const void*>(sample), sample_size, 0, &ctas);
+  cudaError_t e = cluster_size(reinterpret_cast<const void*>(sample), sample_size, 0, &ctas);
   if (e != cudaSuccess) return e;
   const uint32_t rank = sample_rank(a.n, a.k);
   note_launch(5);
@@ -1040,12 +1040,10 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
   const int group = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({8, by_ratio, tiles / resident})));
   const int64_t blocks = (tiles + 8 * group - 1) / (8 * group);
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(148 * 3, blocks));
-  const size_t smem = 8 * kStage * sizeof(uint2);
+  constexpr size_t smem = 8 * kStage * sizeof(uint2);
+  static_assert(smem + (kBins + 64) * sizeof(uint32_t) <= 48 << 10, "more would have to be asked for");
   const bool vec = ((reinterpret_cast<uintptr_t>(t.grad) | reinterpret_cast<uintptr_t>(t.residual)) & 15) == 0;
   auto adjust = vec ? topk_adjust_kernel<kBf16, true, kDense> : topk_adjust_kernel<kBf16, false, kDense>;
-  e = cudaFuncSetAttribute(reinterpret_cast<const void*>(adjust), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem));
-  if (e != cudaSuccess) return e;
   adjust<<<grid, 256, smem, s>>>(a, group);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
