@@ -116,9 +116,10 @@ __device__ __noinline__ void copy_bytes_out(char* dst, const char* src, int64_t 
 }
 
 // dst[u*16 ...] = staged units [u0, u1); `src` is unit-indexed from 0, dst holds nbytes bytes.
+template <bool kAligned = false>
 __device__ __forceinline__ void copy_units_out(const CtaCtx& k, char* dst, const char* src, int64_t u0, int64_t u1,
                                                int64_t nbytes, int64_t readable) {
-  if (!is_aligned16(dst)) {
+  if (!kAligned && !is_aligned16(dst)) {
     copy_bytes_out(dst, src, u0, u1, nbytes, readable);
     return;
   }
@@ -137,8 +138,9 @@ __device__ __forceinline__ void copy_units_out(const CtaCtx& k, char* dst, const
   }
 }
 
-// allgather: staging slot r of every rank receives rank r's block.
-template <bool kMC>
+// allgather: staging slot r of every rank receives rank r's block.  kAligned: all blocks of this rank's output begin on
+// 16-byte boundaries; a kernel of its own, because the call to copy_bytes_out costs the shared one 24 to 32 bytes of spills.
+template <bool kMC, bool kAligned>
 __global__ void __launch_bounds__(512) allgather_kernel(const __grid_constant__ CollParams p) {
   CtaCtx k = make_ctx(p);
   const RankCtx& c = *k.c;
@@ -156,7 +158,7 @@ __global__ void __launch_bounds__(512) allgather_kernel(const __grid_constant__ 
   const bool in_al = is_aligned16(in);
   char* own_out = out + static_cast<int64_t>(c.rank) * pitch;
   const bool own_copy = own_out != in;  // in-place allgather: the own block is already there
-  const bool own_al = is_aligned16(own_out);
+  const bool own_al = kAligned || is_aligned16(own_out);
   const uint32_t peers = ((1u << c.ws) - 1u) & ~(1u << c.rank);
   for (int64_t it = 0; it <= my_tiles; ++it) {
     if (it < my_tiles) {  // push tile `it` of my block
@@ -173,11 +175,11 @@ __global__ void __launch_bounds__(512) allgather_kernel(const __grid_constant__ 
           const int64_t u = ub + k.tid + static_cast<int64_t>(i) * k.nthreads;
           if (u < u1) {
             push16<kMC>(k, c.rank * slot_bytes + static_cast<size_t>(u) * 16, v[i], peers);
-            if (own_copy && (own_al || !in_al)) st_vec_guarded<uint8_t>(reinterpret_cast<uint8_t*>(own_out), u, nbytes, own_al, v[i]);
+            if (own_copy && (kAligned || own_al || !in_al)) st_vec_guarded<uint8_t>(reinterpret_cast<uint8_t*>(own_out), u, nbytes, own_al, v[i]);
           }
         }
       }
-      if (own_copy && in_al && !own_al) copy_bytes_out(own_out, in, u0, u1, nbytes, nbytes);
+      if (!kAligned && own_copy && in_al && !own_al) copy_bytes_out(own_out, in, u0, u1, nbytes, nbytes);
       signal_all(k, 0, static_cast<uint32_t>(it + 1));
     }
     if (it >= 1) {  // copy tile it-1 of every peer's block out of my staging buffer
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(512) allgather_kernel(const __grid_constant__ 
       for (int d = 1; d < c.ws; ++d) {
         int q = c.rank + d;
         if (q >= c.ws) q -= c.ws;
-        copy_units_out(k, out + static_cast<int64_t>(q) * pitch, stage + q * slot_bytes, u0, u1, nbytes, slot_bytes);
+        copy_units_out<kAligned>(k, out + static_cast<int64_t>(q) * pitch, stage + q * slot_bytes, u0, u1, nbytes, slot_bytes);
       }
     }
   }
@@ -367,11 +369,16 @@ size_t broadcast_stage_bytes(size_t nbytes) { return round_up(nbytes, 16); }
 
 cudaError_t launch_allgather(const CollParams& p, LaunchCfg cfg, cudaStream_t s) {
   int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count * p.ctx[0].ws, p.ctx[0].ws, 0));
+  // Each rank picks for its own output: the exchange is the same either way.
+  uint64_t places = static_cast<uint64_t>(p.out_pitch > 0 ? p.out_pitch : p.count);
+  for (int r = 0; r < std::max(1, cfg.emulate_ranks); ++r) places |= reinterpret_cast<uintptr_t>(p.ctx[r].out);
+  const bool aligned = places % 16 == 0;
   if (p.use_nvls) {
     if (cfg.emulate_ranks > 0 || p.ctx[0].nvls_mc == nullptr) return cudaErrorInvalidValue;
-    return do_launch(allgather_kernel<true>, p, ctas, cfg.threads, 0, s);
+    return do_launch(aligned ? allgather_kernel<true, true> : allgather_kernel<true, false>, p, ctas, cfg.threads, 0, s);
   }
-  return do_launch(allgather_kernel<false>, p, ctas, cfg.threads, cfg.emulate_ranks, s);
+  return do_launch(aligned ? allgather_kernel<false, true> : allgather_kernel<false, false>, p, ctas, cfg.threads,
+                   cfg.emulate_ranks, s);
 }
 cudaError_t launch_broadcast(const CollParams& p, LaunchCfg cfg, cudaStream_t s) {
   int ctas = clamp_ctas(cfg.ctas > 0 ? cfg.ctas : pick_ctas(p.count, p.ctx[0].ws, 0));
