@@ -31,6 +31,7 @@
 #include "kernels/api.h"
 #include "kernels/launch_count.h"
 #include "kernels/optim_api.h"
+#include "kernels/stft_api.h"
 #include "kernels/topk_api.h"
 #include "optim/adamw_plan.h"
 #include "optim/bucket_hook.h"
@@ -689,6 +690,21 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       },
       py::arg("reducer"), py::arg("state"),
       "Installs the native allreduce+AdamW bucket hook on a DistributedDataParallel reducer (ddp.reducer).");
+
+#ifdef MCCL_WITH_STFT
+  m.def("_test_stft_inverse_shape", [](int n_fft, int hop, int64_t length, int n_frames, int batch, bool fold) {
+    kern::IfftOlaArgs a{};
+    a.n_fft = n_fft;
+    a.hop = hop;
+    a.out_len = length;
+    a.n_frames = n_frames;
+    a.batch = batch;
+    a.pad = n_fft / 2;
+    a.fold_reflect = fold ? 1 : 0;
+    const kern::OlaShape s = kern::ifft_ola_shape(a);
+    return py::make_tuple(s.reach, s.batch, s.most, s.begins);
+  });
+#endif
 
   // Drives the pool's range allocator with a script of (+bytes | -index) steps: +n allocates n bytes,
   // -i releases the block returned by step i.  Returns (offsets, bytes in use, free blocks).

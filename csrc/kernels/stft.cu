@@ -54,12 +54,11 @@ __device__ __forceinline__ void copy_async(void* smem, const void* gmem) {
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Samples of a frame that reaches over the signal's ends (or, when dividing by the envelope, of one that lacks
-// neighbours), in `buf`.  Every lane prepares the pairs that it will read back; the copies are
-// asynchronous, so that a small call waits for memory once and not once per pair.
-template <int LH, bool kEnvelope>
-__device__ __forceinline__ void load_edge_frame(const FftFramesArgs& a, const float* sig, const float* win, float2* buf,
-                                                int f, int t, int reach) {
+// Samples, times the window, of a frame that reaches over the signal's ends, in `buf`.  Every lane prepares the pairs that it
+// will read back; the copies are asynchronous, so that a small call waits for memory once and not once per pair.
+template <int LH>
+__device__ __forceinline__ void load_edge_frame(const FftFramesArgs& a, const float* sig, const float* win, float2* buf, int f,
+                                                int t, float2 (&v)[WarpFft<LH>::V]) {
   using F = WarpFft<LH>;
   const int64_t start = static_cast<int64_t>(f) * a.hop - a.pad;
   for (int r = 0; r < 2 * F::V; ++r) {
@@ -74,22 +73,73 @@ __device__ __forceinline__ void load_edge_frame(const FftFramesArgs& a, const fl
     else *dst = 0.f;
   }
   copy_async_wait();
-  if (kEnvelope) {
-    const int before = min(reach - 1, f), after = min(reach - 1, a.n_frames - 1 - f);
-#pragma unroll 2
-    for (int r = 0; r < F::V; ++r) {
-      const int m = r * F::L + t;
-      float2 e = make_float2(0.f, 0.f);
-      for (int i = before; i >= -after; --i) {  // frame f - i, in frame order
-        const int o = 2 * m + i * a.hop;
-        if (o >= 0 && o < F::n) e.x += win[o] * win[o];
-        if (o + 1 >= 0 && o + 1 < F::n) e.y += win[o + 1] * win[o + 1];
+#pragma unroll
+  for (int r = 0; r < F::V; ++r) {
+    const float2 w = reinterpret_cast<const float2*>(win)[r * F::L + t];
+    v[r] = buf[r * F::L + t];
+    v[r].x *= w.x;
+    v[r].y *= w.y;
+  }
+}
+
+// Samples, times window / envelope, of a frame that lacks neighbours or reaches over the signal's ends.  Only rows of `hop`
+// samples that lack a frame get an envelope of their own, eight pairs of every lane at a time so that their loads overlap;
+// the others take it from the table.  Every lane prepares the weights that it will read back, in `buf`.
+// (2 x 48000 samples, n_fft 2048, the inverse's backward: 19.5 us with an envelope for every sample one by one, 14.9 us so.)
+template <int LH>
+__device__ __forceinline__ void load_edge_frame_over_envelope(const FftFramesArgs& a, const float* sig, const float* win,
+                                                              const float* win_env, float2* buf, int f, int t, int hop,
+                                                              int reach, float2 (&v)[WarpFft<LH>::V]) {
+  using F = WarpFft<LH>;
+  const int64_t start = static_cast<int64_t>(f) * a.hop - a.pad, left = a.signal_len - start;
+  const float* src = sig + start;
+  const int lo = start < 0 ? static_cast<int>(-start) : 0;  // samples [lo, hi) lie in the signal
+  const int hi = left >= F::n ? F::n : left > 0 ? static_cast<int>(left) : 0;
+#pragma unroll
+  for (int r = 0; r < F::V; ++r) {
+    const int j = 2 * (r * F::L + t);
+    v[r] = make_float2(j >= lo && j < hi ? src[j] : 0.f, j + 1 >= lo && j + 1 < hi ? src[j + 1] : 0.f);
+  }
+  // Frames f - before .. f + after reach into this one.  A row of the padded signal has a full set of them from row
+  // reach - 1 to row n_frames - 1: samples [full_lo, full_hi) of this frame.
+  const int before = min(reach - 1, f), after = min(reach - 1, a.n_frames - 1 - f);
+  const int full_lo = (reach - 1 - before) * hop, full_hi = after == reach - 1 ? F::n : (after + 1) * hop;
+  auto place = [&](int r) { return 2 * ((r / 2) * F::L + t) + (r & 1); };
+  float* weights = reinterpret_cast<float*>(buf);
+#pragma unroll 4
+  for (int r = 0; r < 2 * F::V; ++r) {
+    const int j = place(r);
+    weights[j] = j >= full_lo && j < full_hi ? win_env[j] : 0.f;
+  }
+  constexpr int kAhead = 2 * F::V < 16 ? 2 * F::V : 16, kSpan = kAhead * F::L;
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const int j0 = max(side == 0 ? 0 : max(full_lo, full_hi), lo), j1 = min(side == 0 ? full_lo : F::n, hi);
+#pragma unroll 1
+    for (int base = j0 / kSpan * kSpan; base < j1; base += kSpan) {
+      const int i_hi = min(before, (F::n - 1 - base) / hop), i_lo = -min(after, (base + kSpan - 1) / hop);
+      float e[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) e[u] = 0.f;
+#pragma unroll 1
+      for (int i = i_hi; i >= i_lo; --i) {  // frame f - i, in frame order
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const int o = base + place(u) + i * hop;
+          if (o >= 0 && o < F::n) e[u] += win[o] * win[o];
+        }
       }
-      float2 v = buf[m];
-      v.x = e.x > 1e-11f ? v.x / e.x : 0.f;
-      v.y = e.y > 1e-11f ? v.y / e.y : 0.f;
-      buf[m] = v;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int j = base + place(u);
+        if (j >= j0 && j < j1) weights[j] = e[u] > 1e-11f ? win[j] / e[u] : 0.f;
+      }
     }
+  }
+#pragma unroll
+  for (int r = 0; r < F::V; ++r) {  // (a sample that no frame covers takes no part, whatever it is)
+    const float2 w = buf[r * F::L + t];
+    v[r] = make_float2(w.x != 0.f ? v[r].x * w.x : 0.f, w.y != 0.f ? v[r].y * w.y : 0.f);
   }
 }
 
@@ -153,14 +203,8 @@ __global__ void __launch_bounds__(256, LH <= 6 ? 4 : LH <= 8 ? 3 : LH <= 10 ? 2 
         v[r].y *= w.y;
       }
     } else {
-      load_edge_frame<LH, kEnvelope>(a, sig, win, buf, f, t, reach);
-#pragma unroll
-      for (int r = 0; r < F::V; ++r) {
-        const float2 w = reinterpret_cast<const float2*>(win)[r * F::L + t];
-        v[r] = buf[r * F::L + t];
-        v[r].x *= w.x;
-        v[r].y *= w.y;
-      }
+      if constexpr (kEnvelope) load_edge_frame_over_envelope<LH>(a, sig, win, win_env, buf, f, t, hop, reach, v);
+      else load_edge_frame<LH>(a, sig, win, buf, f, t, v);
     }
     __syncwarp();
     F::transform(v, tw, buf, t);
@@ -216,6 +260,12 @@ struct OlaPlan {
   int reach;          // frames that cover a sample
   int64_t row_base;   // row r of the padded signal is [r * hop, (r + 1) * hop)
   int64_t rows;       // rows to emit, from row_base on
+  int64_t edge;       // rows of the first and of the last segment; 0: as many as the others have
+  // first row of segment s, from row_base on
+  __host__ __device__ int64_t begin(int64_t s) const {
+    if (edge == 0) return rows * s / segments;
+    return s == 0 ? 0 : s == segments ? rows : edge + (rows - 2 * edge) * (s - 1) / (segments - 2);
+  }
 };
 
 // The sum over the frames that cover them of N pairs of samples, 64 apart, of row `row`: pair u of a lane is
@@ -270,9 +320,9 @@ __device__ __forceinline__ void store_folded(const IfftOlaArgs& a, float* out, i
 template <int N, bool kNorm>
 __device__ __forceinline__ void emit_row_pairs(const IfftOlaArgs& a, const float2* slots, int slot_floats,
                                                const float* win, int ring, int s, int i_hi, int i_lo, int64_t q0,
-                                               float* out, int lane, int pass) {
+                                               float* out, int lane, int pass, int part, int parts) {
   const bool paired = pass == 0 && q0 >= 0 && q0 + a.hop <= a.out_len && (reinterpret_cast<uintptr_t>(out + q0) & 7) == 0;
-  for (int c = 0; c < a.hop; c += 64 * N) {
+  for (int c = 64 * N * part; c < a.hop; c += 64 * N * parts) {
     const int j = c + 2 * lane;
     float2 v[N], e[N];
     if (c + 64 * N <= a.hop && (i_hi + 1) * a.hop <= a.n_fft)
@@ -322,8 +372,7 @@ __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const
   __syncthreads();
 
   const int b = blockIdx.x / pl.segments, seg = blockIdx.x % pl.segments;
-  const int64_t row0 = pl.row_base + pl.rows * seg / pl.segments;
-  const int64_t row1 = pl.row_base + pl.rows * (seg + 1) / pl.segments;
+  const int64_t row0 = pl.row_base + pl.begin(seg), row1 = pl.row_base + pl.begin(seg + 1);
   const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane / F::L, t = lane % F::L;
   const int batch = warps * F::kPerWarp;             // frames transformed together
@@ -370,10 +419,16 @@ __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const
     const bool last = f0 + batch >= f_end;
     const int64_t e1 = last ? row1 : f0 + batch;
 
-    for (int pass = at_edge ? 1 : 2; pass <= 2; ++pass) {
-      for (int64_t row = e0 + warp; row < e1; row += warps) {
+    const bool folding = at_edge && (e0 * a.hop - a.pad <= a.pad || e1 * a.hop - a.pad >= T - a.pad);
+    for (int pass = folding ? 1 : 2; pass <= 2; ++pass) {
+      // A warp per row, or, where the passes of a folded edge have few long rows each, per part of a row (2 x 48000 samples,
+      // n_fft 4096, backward: 20.8 us with whole rows, 17.3 us so; n_fft 512, hop 128: 0.6 us slower).
+      const int log_parts = LH < 10 || !folding || a.hop < 512 ? 0 : a.hop < 1024 ? 1 : 2, parts = 1 << log_parts;
+      for (int64_t item = (e0 << log_parts) + warp; item < e1 << log_parts; item += warps) {
+        const int64_t row = item >> log_parts;
+        const int part = static_cast<int>(item) & (parts - 1);
         const int64_t q0 = row * a.hop - a.pad, q1 = q0 + a.hop;  // its output samples
-        const bool folds = at_edge && (q0 <= a.pad || q1 >= T - a.pad);
+        const bool folds = folding && (q0 <= a.pad || q1 >= T - a.pad);
         if (pass == 1) {  // rows that hold samples to store for later
           if (q0 >= 0 && (q1 < T - a.pad || q0 > T - 2)) continue;
         } else if (folds && (q1 <= 0 || (q0 >= T - 1 - a.pad && q1 < T))) {
@@ -387,15 +442,15 @@ __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const
         if ((a.hop & 1) == 0) {
           const int p = folds ? pass : 0;
           if (a.normalize_envelope) {
-            if (LH <= 8 && a.hop <= 64) emit_row_pairs<1, true>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p);
-            else emit_row_pairs<LH <= 8 ? 2 : 4, true>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p);
+            if (LH <= 8 && a.hop <= 64) emit_row_pairs<1, true>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p, part, parts);
+            else emit_row_pairs<LH <= 8 ? 2 : 4, true>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p, part, parts);
           } else {
-            if (LH <= 8 && a.hop <= 64) emit_row_pairs<1, false>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p);
-            else emit_row_pairs<LH <= 8 ? 2 : 4, false>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p);
+            if (LH <= 8 && a.hop <= 64) emit_row_pairs<1, false>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p, part, parts);
+            else emit_row_pairs<LH <= 8 ? 2 : 4, false>(a, slots, 2 * F::kSlot, win, pl.ring, s, i_hi, i_lo, q0, out, lane, p, part, parts);
           }
           continue;
         }
-        for (int j = lane; j < a.hop; j += 32) {
+        for (int j = 32 * part + lane; j < a.hop; j += 32 * parts) {
           float v = 0.f, e = 0.f;
           for (int i = i_hi; i >= i_lo; --i) {       // frame row - i, in frame order
             const int si = s - i < 0 ? s - i + pl.ring : s - i, o = j + i * a.hop;
@@ -555,12 +610,14 @@ cudaError_t run_ifft_frames(const IfftOlaArgs& a, float* frames, cudaStream_t s)
   return cudaGetLastError();
 }
 
-// Geometry of the fused inverse: the most warps whose frames, with the reach - 1 frames before them, fit
-// shared memory; fewer if that leaves SMs without a CTA.  threads == 0: this problem takes the two-kernel path,
+// Geometry of the fused inverse: the first choice whose frames, with the reach - 1 frames before them, fit
+// shared memory.  threads == 0: this problem takes the two-kernel path,
 // because a batch would be shorter than the overlap (tiny hops: neighbours would mostly repeat each other's
 // frames) or because the signal is so short that the two folded edges meet.
 struct OlaGrid {
   OlaPlan plan;
+  int batch = 0;      // frames transformed together
+  int64_t most = 0;   // segments of one batch entry that are resident together
   int threads = 0;
   size_t smem = 0;
 };
@@ -588,11 +645,25 @@ OlaGrid ola_grid(const IfftOlaArgs& a) {
     const int64_t ring = batch + reach - 1;
     const size_t smem = table_bytes<LH>() + static_cast<size_t>(ring) * F::kSlot * sizeof(float2);
     if (batch < reach || resident * (smem + 1024) > kSmemPerSm) continue;
-    // a folded edge lies within one segment: reach + 1 rows are enough for either
-    const int64_t min_rows = std::max<int64_t>(fold ? reach + 1 : 1, batch - (reach - 1));
-    int64_t segments = std::max<int64_t>(1, pl.rows / min_rows);
-    segments = std::max<int64_t>(1, std::min<int64_t>(segments, static_cast<int64_t>(kSms) * resident / a.batch));
+    // As many segments as are resident together; where one batch of frames is enough for each, no more than it takes, but none
+    // with a second batch for a row or two too many.  (2 x 48000 samples, n_fft 2048: 18 segments of 5 and 6 rows, the longer
+    // ones in two batches: backward 12.3, inverse 13.3 us; none above 5 rows: 10.9 and 8.8 us.  With more rounds the last,
+    // short one costs less than segments of full batches would: 8 x 200000 samples, n_fft 1024: 18.5 and 20.6 us.)
+    const int64_t most = std::max<int64_t>(1, static_cast<int64_t>(kSms) * resident / a.batch);
+    const int64_t rounds = (((pl.rows + most - 1) / most) + (reach - 1) + batch - 1) / batch;
+    const int64_t longest = rounds * batch - (reach - 1);
+    int64_t segments = rounds == 1 ? (pl.rows + longest - 1) / longest : most;
+    // a folded edge lies within one segment: reach + 1 rows are enough for either, and the first and the last segment have
+    // no frames before or behind them to repeat
+    const int64_t edge = reach + 1;
+    pl.edge = 0;
+    if (fold && segments > 1 && pl.rows / segments < edge) {
+      if (pl.rows > 2 * edge) pl.edge = edge;
+      segments = pl.edge > 0 ? 2 + (pl.rows - 2 * edge + longest - 1) / longest : 1;
+    }
     if (segments * a.batch > 0x7FFFFFFF) continue;
+    g.batch = static_cast<int>(batch);
+    g.most = most;
     pl.segments = static_cast<int>(segments);
     pl.ring = static_cast<int>(ring);
     g.threads = 32 * warps;
@@ -646,6 +717,18 @@ cudaError_t launch_fft_frames(const FftFramesArgs& a, cudaStream_t s) {
     return a.divide_envelope ? run_fft_frames<decltype(lh)::value, true>(a, s)
                              : run_fft_frames<decltype(lh)::value, false>(a, s);
   });
+}
+
+OlaShape ifft_ola_shape(const IfftOlaArgs& a) {
+  OlaShape shape{};
+  if (!valid(a)) return shape;
+  const OlaGrid g = ola_grid_for(a);
+  if (g.threads == 0) return shape;
+  shape.reach = g.plan.reach;
+  shape.batch = g.batch;
+  shape.most = g.most;
+  for (int s = 0; s <= g.plan.segments; ++s) shape.begins.push_back(g.plan.row_base + g.plan.begin(s));
+  return shape;
 }
 
 int64_t ifft_ola_scratch(const IfftOlaArgs& a) {

@@ -15,6 +15,7 @@
 #include <cuda_runtime_api.h>
 
 #include <cstdint>
+#include <vector>
 
 namespace mccl {
 namespace kern {
@@ -57,6 +58,13 @@ struct IfftOlaArgs {
 cudaError_t launch_fft_frames(const FftFramesArgs& a, cudaStream_t s);
 // Floats of scratch that launch_ifft_ola needs for this problem (0: it runs as one fused kernel).
 int64_t ifft_ola_scratch(const IfftOlaArgs& a);
+// How the fused kernel cuts one batch entry into rows of `hop` samples (host arithmetic only; for the tests).
+struct OlaShape {
+  int reach, batch;             // frames that cover a sample; frames that a CTA transforms together
+  int64_t most;                 // segments that are resident together
+  std::vector<int64_t> begins;  // first row of every segment, and the end; empty where it cannot run
+};
+OlaShape ifft_ola_shape(const IfftOlaArgs& a);
 cudaError_t launch_ifft_ola(const IfftOlaArgs& a, float* scratch, cudaStream_t s);
 
 }  // namespace kern

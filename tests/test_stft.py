@@ -238,3 +238,36 @@ def test_hops_beyond_the_signal(cuda_device, n_fft, hop):
 
     for got, want in zip(all_four(hop), all_four(samples + 1)):
         assert torch.equal(got, want)
+
+
+# The fused inverse cuts the output into segments of rows, one per CTA.  Every row once and in order; a folded edge within one
+# segment; and no segment with more batches of frames than the longest of an even cut would need (a row or two too many
+# cost calls of few frames a second batch).
+@pytest.mark.parametrize("n_fft,hop", [(8, 2), (64, 20), (256, 64), (512, 128), (1024, 256), (1024, 320), (2048, 512), (2048, 1024),
+                                       (2048, 2048), (1024, 128), (4096, 1024), (4096, 1280), (4096, 3000)])
+@pytest.mark.parametrize("fold", [True, False])
+def test_inverse_segments(native, n_fft, hop, fold):
+    for batch in (1, 2, 5, 16, 400):
+        for frames in list(range(1, 40)) + [64, 94, 95, 188, 313, 1000, 2049, 20001]:
+            length = max(1, (frames - 1) * hop + (hop * 3) // 7)
+            reach, together, most, begins = native._test_stft_inverse_shape(n_fft, hop, length, frames, batch, fold)
+            if not begins:
+                assert fold and length < n_fft + 2
+                continue
+            first = 0 if fold else (n_fft // 2) // hop
+            end = -(-(length + (n_fft if fold else n_fft // 2)) // hop)
+            assert begins[0] == first and begins[-1] == end
+            sizes = [b - a for a, b in zip(begins, begins[1:])]
+            assert min(sizes) >= 1
+            if fold and len(sizes) > 1:
+                assert min(sizes[0], sizes[-1]) >= reach + 1
+            assert len(sizes) <= most + 2
+
+            def batches(lo, hi):
+                return -(-max(0, min(hi, frames) - max(0, lo - reach + 1)) // together)
+
+            even = -(-(end - first) // most)          # rows
+            bound = -(-(even + reach - 1) // together)
+            # a segment that has to hold a folded edge may need one more
+            edges = -(-(reach + 1) // together) if fold else 0
+            assert max(batches(a, b) for a, b in zip(begins, begins[1:])) <= max(bound, edges) or len(sizes) == 1
