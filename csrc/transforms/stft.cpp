@@ -36,7 +36,7 @@ void check_common(int64_t n_fft, int64_t hop, int64_t win_length, const at::Tens
 
 // The kernels read memory: a lazy conjugation or negation (`spec.conj()`, the gradient that autograd hands back
 // through it) is carried out before they run.
-at::Tensor plain(const at::Tensor& t) { return t.resolve_conj().resolve_neg(); }
+at::Tensor plain(const at::Tensor& t) { return t.is_conj() || t.is_neg() ? t.resolve_conj().resolve_neg() : t; }
 
 // fp32 and contiguous on `like`'s device; the kernels centre its win_length samples in n_fft zeros
 at::Tensor prepare_window(const at::Tensor& window, const at::Tensor& like) {
