@@ -81,7 +81,7 @@ enum Mode : uint32_t { kList, kWide, kWhole, kTies, kZeros };
 // The exact rule: an element is sent if key > threshold, or key == threshold and index <= last_index (kList) or it is
 // one of the first `need` (kTies, kZeros).
 struct ListState {
-  uint32_t hist[kBins];  // candidates by (key - base) >> kBinShift, the last bin open-ended; then by key >> kCoarseShift
+  uint32_t hist[kBins];  // candidates by (key - base) >> kBinShift, the last bin open-ended
   uint32_t base;         // smallest magnitude key that is a candidate
   uint32_t count;        // entries in the list
   uint32_t overflow;     // the list did not hold them all
@@ -91,7 +91,8 @@ struct ListState {
   uint32_t threshold, last_index;
   uint32_t ticket[3];    // blocks done: adjust, select, counts
   uint32_t sub[kSubBins];  // kTies: elements of the bin by key
-  uint32_t fine[kFineBins];  // kWide, kWhole: elements of the chosen coarse bin
+  uint32_t coarse[kBins];    // kWide, kWhole: keys by key >> kCoarseShift
+  uint32_t fine[kFineBins];  // and of the chosen coarse bin
   uint32_t gate[4][2];   // kWide, kWhole: blocks that came to a meeting, and how it ended
 };
 static_assert(sizeof(ListState) % sizeof(uint4) == 0, "8-byte entries follow it in the scratch");
@@ -546,6 +547,7 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
   __shared__ uint32_t wsum[33];
   constexpr int kPer = kBins / 256;
   const int top = kBins - 1 - kPer * static_cast<int>(threadIdx.x);
+  const uint32_t count = __ldcg(&list.state->count), missing = __ldcg(&list.state->overflow);
   uint32_t c[kPer], run = 0;
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
@@ -558,14 +560,11 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
     if (above < a.k && above + c[i] >= a.k) {
       list.state->bin = static_cast<uint32_t>(top - i);
       list.state->need = a.k - above;
-      const bool missing = __ldcg(&list.state->overflow) != 0u;
       if (top - i == kBins - 1) list.state->mode = missing ? kWhole : kWide;
       else list.state->mode = missing || c[i] > kOneBlock ? kTies : kList;
     }
     above += c[i];
-    list.state->hist[top - i] = 0u;
   }
-  const uint32_t count = __ldcg(&list.state->count);
   if (threadIdx.x == 0 && count < a.k) {
     // every non-zero is a candidate, everything is sent, or the sample missed (or none was taken)
     list.state->mode = base == 1u || a.k == a.n ? kZeros : kWhole;
@@ -681,11 +680,12 @@ __device__ __forceinline__ bool grid_meets(uint32_t* gate, int tries) {
   return s_end == kMet;
 }
 
-// The kBinShift-wide bin that holds the need-th largest of n keys, from two counts by the whole grid; *need becomes how many
-// of its entries are selected, *entries how many it has.  False if the grid could not meet.
-template <typename Key>
-__device__ __forceinline__ bool find_bin(ListState* st, uint32_t* counts, uint32_t* wsum, uint32_t* s_pick, int64_t n, Key&& key,
-                                         uint32_t* floor_key, uint32_t* need, uint32_t* entries) {
+// The kBinShift-wide bin that holds the need-th largest of n keys (the list's or, where that is null, the vector's), from two
+// counts by the whole grid; *need becomes how many of its entries are selected, *entries how many it has.  False if the grid
+// could not meet.  Not inlined: the ordinary selection does not come here.
+__device__ __noinline__ bool find_bin(ListState* st, uint32_t* counts, uint32_t* wsum, uint32_t* s_pick, int64_t n,
+                                      const uint2* list, const float* vector, uint32_t* floor_key, uint32_t* need,
+                                      uint32_t* entries) {
   const int tid = threadIdx.x;
   uint32_t prefix = 0;
   // All blocks start as soon as the launch before is done; once they have met they only wait for the slowest count.
@@ -693,7 +693,8 @@ __device__ __forceinline__ bool find_bin(ListState* st, uint32_t* counts, uint32
 #pragma unroll 1
   for (int level = 0; level < 2; ++level) {
     const int bins = level == 0 ? kBins : kFineBins;
-    uint32_t* total = level == 0 ? st->hist : st->fine;
+    uint32_t* total = level == 0 ? st->coarse : st->fine;
+    auto key = [&](int64_t i) { return list != nullptr ? list[i].y & 0x7FFFFFFFu : key_of(__ldcs(vector + i)); };
     count_digits(counts, bins, n, key, [&](uint32_t k) {
       if (level == 0) return k >> kCoarseShift;
       return k >> kCoarseShift == prefix ? (k >> kBinShift) & (kFineBins - 1u) : 0xFFFFFFFFu;
@@ -737,20 +738,19 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
   uint32_t mode = st->mode;
   if (mode == kZeros) return;
   uint32_t floor_key = st->base + (st->bin << kBinShift), need = st->need;  // the k-th element's bin
-  auto vector_key = [&](int64_t i) { return key_of(__ldcs(a.residual + i)); };
-  if (mode == kWide) {
-    need = a.k;
-    uint32_t entries = 0;
-    if (find_bin(st, sub, sh.wsum, s_pick, st->count, [&](int64_t i) { return a.list.list[i].y & 0x7FFFFFFFu; }, &floor_key,
-                 &need, &entries))
-      mode = entries > kOneBlock ? kTies : kList;
-  } else if (mode == kWhole) {
-    need = a.k;
-    uint32_t entries = 0;
-    if (find_bin(st, sub, sh.wsum, s_pick, a.n, vector_key, &floor_key, &need, &entries)) mode = kTies;
+  if (mode == kWide || mode == kWhole) {
+    const bool listed = mode == kWide;
+    uint32_t floor_found, need_found = a.k, entries;
+    if (find_bin(st, sub, sh.wsum, s_pick, listed ? st->count : a.n, listed ? a.list.list : nullptr, a.residual, &floor_found,
+                 &need_found, &entries)) {
+      floor_key = floor_found;
+      need = need_found;
+      mode = listed && entries <= kOneBlock ? kList : kTies;
+    }
   }
   if (mode == kTies) {
-    count_digits(sub, kSubBins, a.n, vector_key, [&](uint32_t key) { return key - floor_key; });
+    count_digits(sub, kSubBins, a.n, [&](int64_t i) { return key_of(__ldcs(a.residual + i)); },
+                 [&](uint32_t key) { return key - floor_key; });
     for (int i = tid; i < kSubBins; i += kThreads)
       if (sub[i]) atomicAdd(&st->sub[i], sub[i]);
     if (!last_block_done(&st->ticket[1])) return;
