@@ -56,14 +56,15 @@ class DevicePrefetcher:
     ``batches`` is any iterable of tuples of pinned CPU tensors.  ``next()`` returns the device copy
     of the next batch (the compute stream is made to wait for the copy) and at once enqueues the
     host->device copy of the batch after it on a side stream, so that copy overlaps the step that
-    is about to be launched.  The reference's examples copy each batch synchronously at the top of
+    is about to be launched.  ``stream``: the side stream (default: one of its own); feeds that follow one
+    another on the same one reuse its device memory.  The reference's examples copy each batch synchronously at the top of
     the step (reference examples/ddp_dummy_train.py:196-204).
     """
 
-    def __init__(self, batches, device):
+    def __init__(self, batches, device, stream=None):
         self._it = iter(batches)
         self._dev = torch.device(device)
-        self._stream = torch.cuda.Stream(self._dev)
+        self._stream = torch.cuda.Stream(self._dev) if stream is None else stream
         self._ready = None  # (tensors, event) of the batch whose copy is in flight
         self._enqueue()
 

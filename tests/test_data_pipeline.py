@@ -20,6 +20,19 @@ def test_prefetcher_yields_every_batch_once_in_order(cuda_device):
         feed.next()
 
 
+def test_prefetchers_on_one_stream_reuse_its_memory(cuda_device):
+    from mccl_b200.utils.data import DevicePrefetcher
+    stream = torch.cuda.Stream(cuda_device)
+    host = [(torch.full((1 << 22,), float(i)).pin_memory(),) for i in range(6)]
+    reserved = []
+    for _ in range(3):
+        for i, (x,) in enumerate(DevicePrefetcher(iter(host), cuda_device, stream=stream)):
+            assert float(x[0]) == float(i) and float(x[-1]) == float(i)
+        torch.cuda.synchronize()
+        reserved.append(torch.cuda.memory_reserved(cuda_device))
+    assert reserved[1:] == reserved[:1] * 2
+
+
 def test_async_scalar_reader_returns_values_in_push_order(cuda_device):
     from mccl_b200.utils.data import AsyncScalarReader
     r = AsyncScalarReader(cuda_device, depth=3)
