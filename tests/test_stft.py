@@ -219,6 +219,32 @@ def test_lazily_conjugated_and_negated_inputs(cuda_device, frames_major):
         assert _rel(ours(fn), reference(fn)) < tol, fn.__name__
 
 
+# A spectrum (or its gradient) with any strides: expanded over the batch, sliced in every dimension, one frame or bin
+# repeated by a zero stride.  The same values give the same bits whatever the strides.
+@pytest.mark.gpu
+def test_transforms_follow_the_spectrum_strides(cuda_device):
+    n_fft, hop, samples = 512, 128, 9001
+    frames, bins = 1 + samples // hop, n_fft // 2 + 1
+    gen = torch.Generator(device=cuda_device).manual_seed(3)
+    w = torch.hann_window(n_fft, device=cuda_device)
+    kw = dict(n_fft=n_fft, hop_length=hop, win_length=n_fft, window=w, backend="cuda")
+
+    def rand(*shape):
+        return torch.randn(*shape, dtype=torch.complex64, generator=gen, device=cuda_device)
+
+    views = [rand(1, bins, frames).expand(3, -1, -1), rand(3, 1, frames).expand(-1, bins, -1),
+             rand(3, bins, 1).expand(-1, -1, frames), rand(6, 2 * bins, 3 * frames)[::2, 1::2, 2::3],
+             rand(frames, bins, 3).permute(2, 1, 0), rand(3, frames, bins + 5)[:, :, 3:-2].transpose(1, 2),
+             rand(1, 1, 1).expand(3, bins, frames)]
+    x = torch.randn(3, samples, generator=gen, device=cuda_device, requires_grad=True)
+    for v in views:
+        assert v.shape == (3, bins, frames)
+        for plain in (v.contiguous(), v.transpose(1, 2).contiguous().transpose(1, 2)):
+            assert torch.equal(istft(v, length=samples, **kw), istft(plain, length=samples, **kw))
+            got, want = (torch.autograd.grad(stft(x, **kw), x, g)[0] for g in (v, plain))
+            assert torch.equal(got, want)
+
+
 # A hop far beyond the signal, up to and beyond the range of an int: one frame, whatever the hop.
 @pytest.mark.gpu
 @pytest.mark.parametrize("hop", [1_000_000, 2**30 + 1, 2**31 - 4000, 2**31 - 1, 2**31, 2**32, 2**33 + 7])

@@ -40,9 +40,8 @@ def test_select_ties_take_lower_index(native, cuda_device):
 
 @pytest.mark.parametrize("kind", ["few_magnitudes", "mostly_zero", "all_equal", "bf16_grid"])
 def test_select_on_heavily_tied_data_matches_host_oracle(native, cuda_device, kind):
-    # The chosen top-digit bin holds far more than k elements here, so the candidate list of the
-    # collect pass overflows and the full-vector refinement passes decide the threshold; the ties at
-    # the threshold must still go to the lowest indices, exactly like the host implementation.
+    # Many elements share the k-th magnitude (or it is zero): threshold and ties come from the whole
+    # vector, and the ties must still go to the lowest indices, exactly like the host implementation.
     n, ratio = 400_003, 0.02
     gen = torch.Generator().manual_seed(11)
     if kind == "few_magnitudes":

@@ -60,6 +60,37 @@ def test_noalloc_matches_regular_entry_point_twice(native, cuda_device):
         assert torch.equal(res.cpu(), host.residual(0)), f"call {call}: residual differs from the host compressor"
 
 
+# Above 384 Ki elements this entry point is the only caller of the three-pass radix select: the fixed scratch has no room
+# for the list of the one-pass selection.  Aligned arrays and others, and data whose chosen bin holds more than k elements, so
+# that the candidate list of the collect pass overflows and full-vector passes decide.  The host implementation is the oracle; the
+# second call meets the residual and the scratch that the first one left.
+@pytest.mark.parametrize("n,ratio", [(393_217, 0.01), (1_048_576, 0.1), (3_000_001, 0.001), (600_000, 1.0)])
+@pytest.mark.parametrize("kind", ["normal", "few_magnitudes", "mostly_zero", "all_equal"])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_noalloc_three_pass_select_matches_host(native, cuda_device, n, ratio, kind, offset):
+    import numpy as np
+    lib = _lib(native)
+    stream = torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator().manual_seed(n + offset)
+    g = {"normal": lambda: torch.randn(n, generator=gen),
+         "few_magnitudes": lambda: torch.randint(-3, 4, (n,), generator=gen).float(),
+         "mostly_zero": lambda: torch.randn(n, generator=gen) * (torch.rand(n, generator=gen) < 0.0005),
+         "all_equal": lambda: torch.full((n,), -0.75)}[kind]()
+    k = _k(n, ratio)
+    grad = torch.zeros(n + offset, device=cuda_device)[offset:]
+    grad.copy_(g)
+    res = torch.zeros(n + offset, device=cuda_device)[offset:]
+    host = native.TopKCompressor(ratio)
+    for call in range(2):
+        pairs = torch.empty(k, 2, dtype=torch.int32, device=cuda_device)
+        rc = lib.mccl_topk_select_noalloc(grad.data_ptr(), res.data_ptr(), n, k, pairs.data_ptr(), stream)
+        assert rc == 0, lib.mccl_noalloc_last_error()
+        wire = host.compress(g, 0)
+        rec = np.frombuffer(wire[4:4 + k * 8], dtype=np.uint32).reshape(k, 2)
+        assert np.array_equal(pairs.cpu().numpy().view(np.uint32), rec), f"call {call}"
+        assert torch.equal(res.cpu(), host.residual(0)), f"call {call}"
+
+
 def test_noalloc_rejects_bad_sizes(native, cuda_device):
     lib = _lib(native)
     x = torch.zeros(16, device=cuda_device)
