@@ -83,9 +83,9 @@ __device__ __forceinline__ void load_edge_frame(const FftFramesArgs& a, const fl
 }
 
 // Samples, times window / envelope, of a frame that lacks neighbours or reaches over the signal's ends.  Only rows of `hop`
-// samples that lack a frame get an envelope of their own, eight pairs of every lane at a time so that their loads overlap;
+// samples that lack a frame get an envelope of their own, several pairs of every lane at a time so that their loads overlap;
 // the others take it from the table.  Every lane prepares the weights that it will read back, in `buf`.
-// (2 x 48000 samples, n_fft 2048, the inverse's backward: 19.5 us with an envelope for every sample one by one, 14.9 us so.)
+// (2 x 48000 samples, n_fft 2048, the inverse's backward: 19.6 us with an envelope for every sample one by one, 12.6 us so.)
 template <int LH>
 __device__ __forceinline__ void load_edge_frame_over_envelope(const FftFramesArgs& a, const float* sig, const float* win,
                                                               const float* win_env, float2* buf, int f, int t, int hop,
@@ -111,7 +111,8 @@ __device__ __forceinline__ void load_edge_frame_over_envelope(const FftFramesArg
     const int j = place(r);
     weights[j] = j >= full_lo && j < full_hi ? win_env[j] : 0.f;
   }
-  constexpr int kAhead = 2 * F::V < 16 ? 2 * F::V : 16, kSpan = kAhead * F::L;
+  constexpr int kMost = LH <= 6 ? 4 : LH <= 8 ? 8 : 16;  // (short frames have 64 or 80 registers: more would spill)
+  constexpr int kAhead = 2 * F::V < kMost ? 2 * F::V : kMost, kSpan = kAhead * F::L;
 #pragma unroll 1
   for (int side = 0; side < 2; ++side) {
     const int j0 = max(side == 0 ? 0 : max(full_lo, full_hi), lo), j1 = min(side == 0 ? full_lo : F::n, hi);
@@ -357,7 +358,7 @@ __device__ __forceinline__ void emit_row_pairs(const IfftOlaArgs& a, const float
 // 16 warps per SM that the ring leaves room for; two CTAs of 8 overlap one's transforms with the other's
 // barriers and loads.
 // 16 x 1 Mi samples, n_fft 2048, hop 512 (336 MB): 591 us with the frames written to memory and gathered
-// by a second kernel, 148 us so.
+// by a second kernel, 144 us so.
 // 16 x 240007 samples, n_fft 1024, hop 256, bins-major spectrum (77 MB): 247 us, 55 us so.
 template <int LH>
 __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const IfftOlaArgs a, const OlaPlan pl) {
