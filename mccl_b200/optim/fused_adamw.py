@@ -128,8 +128,8 @@ class FusedAdamW(torch.optim.Optimizer):
     # One step number, that of the first trainable parameter, serves all that is updated inside backward.  Parameters
     # whose counters differ from it (as a checkpoint can hold them) are left to `step()`, which knows each one's own.
     def _next_step(self) -> int:
-        params = [p for g in self.param_groups for p in g["params"]]
-        st = self.state[next((p for p in params if p.requires_grad), params[0])]
+        trainable = (p for g in self.param_groups for p in g["params"] if p.requires_grad)
+        st = self.state[next(trainable, self.param_groups[0]["params"][0])]
         return int(st["step"]) + 1 if "step" in st else 1
 
     def _on_shared_step(self, params) -> set:
