@@ -50,10 +50,10 @@ struct TopkArgs {
 };
 
 // What the fastest path for this problem wants: above 384 Ki elements 8 bytes for each of somewhat more than k listed
-// elements (1.2 k + 4096 at 1 % of 51.5 M; none above a ratio of 0.98), 1 MB at most for those of one bin, 10 bytes per 1024 elements.
+// elements (1.5 k + 4096 at 1 % of 51.5 M; none above a ratio of 0.98), 1 MB at most for those of one bin, 10 bytes per 1024 elements.
 size_t topk_scratch_bytes(int64_t n, int64_t k);
 // What any problem can do with: 3 histograms, the selection state, per-block counts/offsets (about 53 KB) for
-// launch_topk_select, and 10 bytes per 1024 elements and 60 KB for launch_topk_dense, whose list then overflows.
+// launch_topk_select, and 10 bytes per 1024 elements and 66 KB for launch_topk_dense, whose list then overflows.
 size_t topk_min_scratch_bytes();
 size_t topk_dense_min_scratch_bytes(int64_t n);
 #ifdef __CUDACC__

@@ -163,7 +163,7 @@ def bench_stft(native, n, iters, n_fft=2048):
     def run():
         stft(x, n_fft=n_fft, hop_length=hop, win_length=n_fft, window=w)
     frames = 1 + (n // 16) // hop
-    return timeit(run, iters), 16 * frames * (n_fft * 4 + (n_fft // 2 + 1) * 8), "frame loads (L2-resident overlap) + spectrum written"
+    return timeit(run, iters), n * 4 + 16 * frames * (n_fft // 2 + 1) * 8, "signal read once + spectrum written"
 
 
 def stft_vs_torch(native, n, iters):
