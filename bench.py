@@ -180,6 +180,8 @@ def main():
                            optimizer_in_backward=opt if in_bw else None)
         else:
             from torch.nn.parallel import DistributedDataParallel
+            for layer in model.net:  # torch's own products, like the rest of this arm
+                layer.stock = True
             ddp = DistributedDataParallel(model, device_ids=[local_rank], bucket_cap_mb=args.bucket_mb,
                                           gradient_as_bucket_view=True, process_group=group)
             opt = torch.optim.AdamW(ddp.parameters(), lr=1e-3, fused=True)

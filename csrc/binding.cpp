@@ -33,6 +33,7 @@
 #include "kernels/optim_api.h"
 #include "kernels/stft_api.h"
 #include "kernels/topk_api.h"
+#include "ops/linear.h"
 #include "optim/adamw_plan.h"
 #include "optim/bucket_hook.h"
 #include "runtime/arena.h"
@@ -834,4 +835,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("hop_length"), py::arg("win_length"), py::arg("center") = true, py::arg("normalized") = false,
         py::arg("n_frames"), py::arg("backend") = "auto");
 #endif
+
+  // ---- fp32 linear layer on the tensor cores ----------------------------------------------------------
+  m.def("_linear", &linear, py::arg("input"), py::arg("weight"), py::arg("bias") = py::none());
+  m.def("_linear_native", &linear_native, py::arg("input"), py::arg("weight"), py::arg("bias") = py::none());
 }

@@ -1,0 +1,235 @@
+#include "ops/linear.h"
+
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/custom_function.h>
+
+#include <algorithm>
+#include <mutex>
+
+#include "common/errors.h"
+#include "kernels/gemm_api.h"
+
+namespace mccl {
+
+namespace {
+
+#define LINEAR_CK(expr)                                                      \
+  do {                                                                       \
+    cudaError_t _e = (expr);                                                 \
+    if (_e != cudaSuccess) {                                                 \
+      cudaGetLastError();                                                    \
+      throw DeviceError(std::string(#expr) + ": " + cudaGetErrorString(_e)); \
+    }                                                                        \
+  } while (0)
+
+// A word of mapped host memory in which a kernel notes that one of its bounded waits ran out.
+uint32_t* wait_status() {
+  static uint32_t* word = [] {
+    void* p = nullptr;
+    auto mode = cudaStreamCaptureModeRelaxed;  // the first call may be under capture
+    LINEAR_CK(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaHostAlloc(&p, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable);
+    LINEAR_CK(cudaThreadExchangeStreamCaptureMode(&mode));
+    LINEAR_CK(e);
+    *static_cast<uint32_t*>(p) = 0;
+    return static_cast<uint32_t*>(p);
+  }();
+  return word;
+}
+void check_waits() {
+  if (*static_cast<volatile uint32_t*>(wait_status()) != 0)
+    throw DeviceError("a wait inside a matrix product kernel ran out; results since then are undefined");
+}
+
+// A tensor as the kernels read it: memory on the device, nothing lazy, no wrapper (vmap, functorch, subclasses), no tangent.
+bool ordinary(const at::Tensor& t) {
+  using c10::DispatchKey;
+  constexpr auto allowed = c10::DispatchKeySet({DispatchKey::CUDA, DispatchKey::AutogradCUDA, DispatchKey::ADInplaceOrView,
+                                                DispatchKey::AutocastCUDA});
+  return t.defined() && allowed.isSupersetOf(t.key_set()) && t.scalar_type() == at::kFloat && !t._fw_grad(0).defined();
+}
+// No mode that wants to see the operators (Python modes, functorch transforms, functionalization).
+bool no_modes() {
+  const auto included = c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set;
+  return included.empty();
+}
+bool rows_ok(const at::Tensor& t) {
+  return t.dim() == 2 && t.numel() > 0 && t.stride(1) == 1 && (t.size(0) == 1 || t.stride(0) >= t.size(1));
+}
+bool blackwell(int device) {
+  const auto* p = at::cuda::getDeviceProperties(static_cast<c10::DeviceIndex>(device));
+  return p->major == 10 && p->minor == 0;
+}
+
+kern::MatrixF32 matrix(const at::Tensor& t) {
+  return {t.const_data_ptr<float>(), t.size(0) == 1 ? std::max(t.stride(0), t.size(1)) : t.stride(0), t.size(0), t.size(1)};
+}
+
+int64_t align(int64_t bytes) { return (bytes + 255) / 256 * 256; }
+
+// Scratch of one or two products that run one behind the other: tickets, partial sums (shared), images.
+struct Scratch {
+  at::Tensor buffer;
+  char* at = nullptr;
+  char* take(int64_t bytes) {
+    char* p = at;
+    at += align(bytes);
+    return p;
+  }
+};
+Scratch scratch_for(std::initializer_list<const kern::GemmPlan*> plans, const at::TensorOptions& like) {
+  int64_t bytes = 0, partial = 0;
+  for (const auto* p : plans) {
+    bytes += align(p->tickets * 4) + align(p->a_image) + align(p->b_image);
+    partial = std::max(partial, p->partial);
+  }
+  Scratch s;
+  s.buffer = at::empty({bytes + align(partial)}, like.dtype(at::kByte));
+  s.at = static_cast<char*>(s.buffer.data_ptr());
+  return s;
+}
+
+at::Tensor forward_product(const at::Tensor& x, const at::Tensor& w, const at::Tensor& bias) {
+  check_waits();
+  c10::cuda::CUDAGuard guard(x.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  const kern::GemmPlan plan = kern::gemm_plan(kern::Product::kForward, x.size(0), w.size(1), w.size(0));
+  at::Tensor y = at::empty({x.size(0), w.size(0)}, x.options());
+  Scratch s = scratch_for({&plan}, x.options());
+  auto* tickets = reinterpret_cast<uint32_t*>(s.take(plan.tickets * 4));
+  char* image = s.take(plan.b_image);
+  auto* partial = reinterpret_cast<float*>(s.take(plan.partial));
+  const kern::SplitJob job{matrix(x), image, plan.cols, nullptr};
+  LINEAR_CK(kern::launch_split_f32(&job, 1, nullptr, tickets, plan.tickets, stream));
+  const kern::MatrixF32 wm = matrix(w);
+  kern::GemmArgs g{};
+  g.product = kern::Product::kForward;
+  g.plan = plan;
+  g.weight = wm.data;
+  g.ldw = wm.ld;
+  g.b_image = image;
+  g.bias = bias.defined() ? bias.const_data_ptr<float>() : nullptr;
+  g.c = y.data_ptr<float>();
+  g.ldc = w.size(0);
+  g.partial = partial;
+  g.tickets = tickets;
+  g.failed = wait_status();
+  LINEAR_CK(kern::launch_gemm_f32(g, stream));
+  return y;
+}
+
+struct Gradients {
+  at::Tensor x, w, bias;
+};
+Gradients backward_products(const at::Tensor& grad, const at::Tensor& x, const at::Tensor& w, bool need_x, bool need_w,
+                            bool need_bias) {
+  check_waits();
+  const int64_t batch = x.size(0), in = w.size(1), out = w.size(0);
+  c10::cuda::CUDAGuard guard(x.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  Gradients r;
+  const bool own_x = need_x && kern::gemm_pays(kern::Product::kInput, batch, in, out);
+  const bool own_w = need_w && kern::gemm_pays(kern::Product::kWeight, batch, in, out);
+  if (need_x && !own_x) r.x = grad.mm(w);
+  if (need_w && !own_w) r.w = grad.t().mm(x);
+  if (!own_x && !own_w) {
+    if (need_bias) r.bias = grad.sum(0);
+    return r;
+  }
+  kern::GemmPlan px{}, pw{};
+  if (own_x) px = kern::gemm_plan(kern::Product::kInput, batch, in, out);
+  if (own_w) pw = kern::gemm_plan(kern::Product::kWeight, batch, in, out);
+  Scratch s = scratch_for({&px, &pw}, x.options());
+  auto* tickets = reinterpret_cast<uint32_t*>(s.take((px.tickets + pw.tickets) * 4));
+  char *gx = s.take(px.b_image), *gw = s.take(pw.b_image), *xw = s.take(pw.a_image);
+  auto* partial = reinterpret_cast<float*>(s.take(std::max(px.partial, pw.partial)));
+  if (need_bias) r.bias = at::empty({out}, x.options());
+  const kern::SplitJob jobs[2] = {{matrix(grad), own_x ? gx : nullptr, px.cols, own_w ? gw : nullptr},
+                                  {matrix(x), nullptr, 0, xw}};
+  LINEAR_CK(kern::launch_split_f32(jobs, own_w ? 2 : 1, need_bias ? r.bias.data_ptr<float>() : nullptr, tickets,
+                                   px.tickets + pw.tickets, stream));
+  if (own_x) {
+    r.x = at::empty({batch, in}, x.options());
+    const kern::MatrixF32 wm = matrix(w);
+    kern::GemmArgs g{};
+    g.product = kern::Product::kInput;
+    g.plan = px;
+    g.weight = wm.data;
+    g.ldw = wm.ld;
+    g.b_image = gx;
+    g.c = r.x.data_ptr<float>();
+    g.ldc = in;
+    g.partial = partial;
+    g.tickets = tickets;
+    g.failed = wait_status();
+    LINEAR_CK(kern::launch_gemm_f32(g, stream));
+  }
+  if (own_w) {
+    r.w = at::empty({out, in}, x.options());
+    kern::GemmArgs g{};
+    g.product = kern::Product::kWeight;
+    g.plan = pw;
+    g.a_image = xw;
+    g.b_image = gw;
+    g.c = r.w.data_ptr<float>();
+    g.ldc = in;
+    g.partial = partial;
+    g.tickets = tickets + px.tickets;
+    g.failed = wait_status();
+    LINEAR_CK(kern::launch_gemm_f32(g, stream));
+  }
+  return r;
+}
+
+struct LinearFn : torch::autograd::Function<LinearFn> {
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& x, const at::Tensor& w,
+                            const c10::optional<at::Tensor>& bias) {
+    ctx->save_for_backward({x, w});
+    ctx->saved_data["bias"] = bias.has_value();
+    return forward_product(x, w, bias ? *bias : at::Tensor());
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    at::Tensor grad = grads[0];
+    if (!grad.defined()) return {at::Tensor(), at::Tensor(), at::Tensor()};
+    const auto saved = ctx->get_saved_variables();
+    const at::Tensor &x = saved[0], &w = saved[1];
+    const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1), 
+               need_bias = ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2);
+    // a second derivative, or tensors that are no longer what forward saw (a hook, vmap over the backward pass): operators
+    // that autograd knows
+    if (at::GradMode::is_enabled() || !no_modes() || !ordinary(grad) || !ordinary(x) || !ordinary(w) || !rows_ok(x) ||
+        !rows_ok(w) || x.device() != grad.device() || w.device() != grad.device())
+      return {need_x ? grad.mm(w) : at::Tensor(), need_w ? grad.t().mm(x) : at::Tensor(),
+              need_bias ? grad.sum(0) : at::Tensor()};
+    if (!rows_ok(grad)) grad = grad.contiguous();
+    Gradients r = backward_products(grad, x, w, need_x, need_w, need_bias);
+    return {r.x, r.w, r.bias};
+  }
+};
+
+}  // namespace
+
+bool linear_native(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias) {
+  if (!no_modes() || !ordinary(x) || !ordinary(w) || !rows_ok(x) || !rows_ok(w) || x.size(1) != w.size(1) ||
+      x.device() != w.device())
+    return false;
+  if (bias && bias->defined() &&
+      (!ordinary(*bias) || bias->dim() != 1 || bias->size(0) != w.size(0) || bias->stride(0) != 1 || bias->device() != x.device()))
+    return false;
+  // a program that lets torch round its fp32 products has asked for something else
+  if (at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA)) return false;
+  return blackwell(x.get_device()) && kern::gemm_pays(kern::Product::kForward, x.size(0), w.size(1), w.size(0));
+}
+
+at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias) {
+  if (!linear_native(x, w, bias)) return at::linear(x, w, bias);
+  const bool has_bias = bias && bias->defined();
+  if (!at::GradMode::is_enabled() || !(x.requires_grad() || w.requires_grad() || (has_bias && bias->requires_grad())))
+    return forward_product(x, w, has_bias ? *bias : at::Tensor());
+  return LinearFn::apply(x, w, has_bias ? bias : c10::nullopt);
+}
+
+}  // namespace mccl

@@ -42,6 +42,7 @@ CPP_SOURCES = [
     "compression/compressor.cpp",
     "cpu/reduce.cpp",
     "transforms/stft.cpp",
+    "ops/linear.cpp",
     "p2p/nccl_p2p.cpp",
 ]
 CUDA_SOURCES = [
@@ -55,6 +56,7 @@ CUDA_SOURCES = [
     "kernels/topk_cluster.cu",
     "kernels/stft.cu",
     "kernels/adamw.cu",
+    "kernels/gemm_f32.cu",
     "kernels/noalloc.cu",
 ]
 

@@ -4,6 +4,8 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from ..ops.linear import Linear
+
 
 class MLP94M(nn.Module):
     """The ~94 M parameter fp32 MLP of the headline DDP benchmark.
@@ -16,10 +18,10 @@ class MLP94M(nn.Module):
 
     def __init__(self, in_features: int = 2048, hidden: int = 3072, depth: int = 9, classes: int = 1000):
         super().__init__()
-        layers = [nn.Linear(in_features, hidden), nn.GELU()]
+        layers = [Linear(in_features, hidden), nn.GELU()]
         for _ in range(depth):
-            layers += [nn.Linear(hidden, hidden), nn.GELU()]
-        layers.append(nn.Linear(hidden, classes))
+            layers += [Linear(hidden, hidden), nn.GELU()]
+        layers.append(Linear(hidden, classes))
         self.net = nn.Sequential(*layers)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:

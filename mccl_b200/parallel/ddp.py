@@ -21,6 +21,8 @@ import torch
 import torch.distributed as dist
 from torch.nn.parallel import DistributedDataParallel
 
+from ..ops.linear import Linear
+
 
 def _backend_for(process_group, device):
     pg = process_group if process_group is not None else dist.distributed_c10d._get_default_group()
@@ -216,6 +218,11 @@ def wrap_ddp(module: torch.nn.Module, *, device_ids=None, bucket_cap_mb: Optiona
     ddp_kwargs.setdefault("gradient_as_bucket_view", True)
     on_cuda = next(module.parameters()).is_cuda
     mode = compression if compression is not None else os.environ.get("MCCL_COMPRESSION", "none")
+    if on_cuda and mode == "topk":
+        # which entries are sent is decided by comparing fp32 gradients, where the last bit can count: they stay torch's
+        for m in module.modules():
+            if isinstance(m, Linear):
+                m.stock = True
     pool = None
     if on_cuda and mode != "topk" and nvls_buckets is not False and dist.is_initialized():
         pool = _nvls_bucket_pool(module, process_group)

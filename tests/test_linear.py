@@ -1,0 +1,156 @@
+"""The fp32 linear layer on the tensor cores against the same products in 64 bits."""
+import copy
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+import mccl_b200
+from mccl_b200.models import MLP94M
+from mccl_b200.ops.linear import Linear, linear
+
+
+def _bound(absolute, depth):
+    """What may separate a product from its value: three parts leave 2^-24 of every factor out, the tensor cores cut off
+    (2^-23 of the running sum) each of the at most 8 sums of 16 products between two rounded additions, and the additions
+    of the depth / 64 parts round by 2^-24 each.  `absolute`: the product of the absolute values."""
+    return absolute * (2.0 ** -20 + (depth / 64 + 2) * 2.0 ** -24)
+
+
+# rows around the tiles of 32, 64 and 128; features that are no multiple of anything; split and unsplit reductions
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,n_in,n_out", [
+    (8, 3072, 3072), (32, 1027, 1001), (33, 1001, 1027), (64, 1500, 1500), (65, 1237, 1300), (100, 1100, 1000),
+    (127, 3071, 1000), (128, 1024, 1024), (129, 1023, 1025), (255, 2048, 3000), (256, 3072, 3072), (700, 1000, 2100),
+])
+def test_linear_matches_64_bits(batch, n_in, n_out):
+    native = mccl_b200.require_native()
+    torch.manual_seed(batch)
+    x = torch.randn(batch, n_in, device="cuda", requires_grad=True)
+    w = torch.randn(n_out, n_in, device="cuda", requires_grad=True)
+    b = torch.randn(n_out, device="cuda", requires_grad=True)
+    g = torch.randn(batch, n_out, device="cuda")
+    assert native._linear_native(x, w, b)
+    y = linear(x, w, b)
+    got = [y, *torch.autograd.grad(y, (x, w, b), g)]
+    x, w, b, g = (t.detach().double() for t in (x, w, b, g))
+    want = [x @ w.T + b, g @ w, g.T @ x, g.sum(0)]
+    size = [x.abs() @ w.abs().T + b.abs(), g.abs() @ w.abs(), g.abs().T @ x.abs(), g.abs().sum(0)]
+    for name, a, r, s, depth in zip("y x w b".split(), got, want, size, (n_in, n_out, batch, batch)):
+        assert ((a.detach().double() - r).abs() <= _bound(s, depth)).all(), name
+
+
+# views: rows of a wider matrix, a start that is off 16 bytes, a gradient that is a transposed or expanded view
+@pytest.mark.gpu
+@pytest.mark.parametrize("shift,pad", [(0, 0), (0, 4), (1, 3), (3, 1), (0, 5)])
+def test_linear_of_views(shift, pad):
+    torch.manual_seed(0)
+    batch, n_in, n_out = 130, 1004, 1100
+
+    def view(rows, cols):
+        return torch.randn(rows, cols + shift + pad, device="cuda")[:, shift:shift + cols]
+
+    x, w = view(batch, n_in).requires_grad_(), view(n_out, n_in).requires_grad_()
+    assert mccl_b200.require_native()._linear_native(x, w, None)
+    for g in (view(batch, n_out), view(n_out, batch).T, torch.randn(1, n_out, device="cuda").expand(batch, n_out)):
+        y = linear(x, w)
+        got = [y, *torch.autograd.grad(y, (x, w), g)]
+        xd, wd, gd = (t.detach().double() for t in (x, w, g))
+        for a, r, s, depth in ((got[0], xd @ wd.T, xd.abs() @ wd.abs().T, n_in),
+                               (got[1], gd @ wd, gd.abs() @ wd.abs(), n_out),
+                               (got[2], gd.T @ xd, gd.abs().T @ xd.abs(), batch)):
+            assert ((a.detach().double() - r).abs() <= _bound(s, depth)).all()
+
+
+@pytest.mark.gpu
+def test_linear_special_values():
+    """Infinities, NaN and the largest and smallest normal numbers go through as in a multiplication."""
+    torch.manual_seed(0)
+    x, w = torch.randn(64, 1024, device="cuda"), torch.randn(1024, 1024, device="cuda")
+    x[0, 5], x[1, 6], x[2, 7], w[3, 9], w[4, 10] = float("inf"), float("nan"), -float("inf"), float("inf"), float("nan")
+    x[5, 20], w[6, 21] = 3.4028234e38, -3.4028234e38
+    w[:, 5] = torch.where(w[:, 5].abs() < 0.1, 0.0, w[:, 5])  # inf * 0
+    x[7], w[:, 20] = x[7] * 1e-37, w[:, 20] * 1e-3
+    x[8, 6] = torch.tensor(0x7F800001, dtype=torch.int32).view(torch.float32).item()  # a NaN in its last bit alone
+    got, want = linear(x, w), F.linear(x, w)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    exact = x.double() @ w.double().T
+    ok = want.isfinite()
+    bound = _bound(x.double().abs() @ w.double().abs().T, 1024)
+    assert ((got.double() - exact).abs()[ok] <= bound[ok]).all()
+
+
+@pytest.mark.gpu
+def test_linear_keeps_what_autograd_offers():
+    torch.manual_seed(0)
+    x = torch.randn(64, 1024, device="cuda", requires_grad=True)
+    layer = Linear(1024, 1024).cuda()
+    w, b = layer.weight, layer.bias
+
+    def both(fn):
+        torch.testing.assert_close(fn(linear), fn(F.linear), rtol=1e-4, atol=1e-3)
+
+    def second(f):
+        (g,) = torch.autograd.grad(f(x, w, b).square().sum(), x, create_graph=True)
+        return torch.autograd.grad(g.square().sum(), w)[0] * 1e-4
+
+    both(second)
+    both(lambda f: torch.func.jvp(lambda t: f(t, w, b), (x,), (x,))[1])
+    both(lambda f: torch.func.vmap(lambda t: f(t, w, b))(x.expand(2, 64, 1024)))
+    both(lambda f: torch.func.grad(lambda t: f(x, t, b).square().sum())(w) * 1e-3)
+    both(lambda f: torch.autograd.grad(f(x, w, b), x, torch.ones(3, 64, 1024, device="cuda"), is_grads_batched=True)[0])
+    both(lambda f: torch.autograd.grad(f(x, w, b).sum(), b)[0])
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t, lambda t: t):
+        linear(x, w, b).sum().backward()
+    assert packed == [x.shape, w.shape] and layer.weight.grad is not None
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert layer(x).dtype == torch.bfloat16
+    y = layer(x).sum()
+    with torch.no_grad():
+        w.add_(1.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward()
+    stock = copy.deepcopy(layer)
+    stock.stock = True
+    assert torch.equal(stock(x), F.linear(x, w, b))
+
+
+@pytest.mark.gpu
+def test_linear_under_capture_and_streams():
+    x, w = torch.randn(64, 2048, device="cuda"), torch.randn(1000, 2048, device="cuda")
+    want = linear(x, w)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        other = linear(x, w)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = linear(x, w)
+    for _ in range(2):
+        y.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and torch.equal(other, want)
+
+
+def test_linear_elsewhere_is_torch():
+    """What the kernels do not take is torch's own call: other devices, types and orders, scripting and tracing."""
+    native = mccl_b200.require_native()
+    torch.manual_seed(0)
+    for dtype in (torch.float32, torch.float64, torch.bfloat16):
+        x, w, b = (torch.randn(*s).to(dtype) for s in ((4, 64, 48), (32, 48), (32,)))
+        for xi in (x, x[0], x[0, 0], x[0, :, ::2].expand(64, 24)):
+            wi = w[:, :xi.shape[-1]]
+            assert not native._linear_native(xi, wi, b)
+            assert torch.equal(native._linear(xi, wi, b), F.linear(xi, wi, b))
+            assert torch.equal(linear(xi, wi), F.linear(xi, wi))
+    model = MLP94M(64, 48, 1, 5)
+    x = torch.randn(3, 64)
+    assert torch.equal(torch.jit.script(model)(x), model(x)) and torch.equal(torch.jit.trace(model, x)(x), model(x))
+    assert torch.equal(torch.fx.symbolic_trace(model)(x), model(x))
+    assert all(isinstance(m, torch.nn.Linear) for m in model.net[::2])
+    assert list(model.state_dict())[:2] == ["net.0.weight", "net.0.bias"]
+    with pytest.raises(RuntimeError):
+        linear(torch.randn(3, 5), torch.randn(4, 6))
