@@ -248,7 +248,7 @@ template <int NT>
 struct Shape {
   static constexpr int part_b = NT * kDepth * 2;
   static constexpr int stage = 3 * (kPartA + part_b);  // bytes
-  static constexpr int stages = NT == 128 ? 4 : NT == 64 ? 6 : 7;
+  static constexpr int stages = 4;
   static constexpr int smem = stages * stage + 1024;
   static constexpr int columns = NT == 128 ? 512 : NT == 64 ? 256 : 128;  // of tensor memory: 3 NT, a power of two
 };
@@ -264,10 +264,14 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
 
 // One tile of 128 by NT per CTA and, where the tiles do not fill the device, a share of its reduction; tiles in turn where
 // there are more than SMs.  One warp issues all products, eight take acc0 out while the other products of a stage run,
-// the rest cut the weights (once per tile: no pass over them before) or copy images in, four to seven stages ahead.
+// the rest cut the weights (once per tile: no pass over them before) or copy images in, four stages ahead (six or seven for
+// the narrow tiles: 20.0 against 19.3 us, 32 x 3072 x 3072 forward; what the stages leave is the weights' cache).
 // Bound by shared memory: a stage of NT = 128 moves 128 KB through it, 1024 cycles, where its products take 768; measured
-// 1350.  256 x 3072 x 3072 (B200, with the images' launch): forward 128.8 us with cuBLAS's fp32 kernel, 36.8 so; input
-// gradient 121.7 and 34.0; weight gradient 98.9 and 30.0: 130 to 160 TFLOP/s of fp32 products, 0.8 to 1 PFLOP/s of bf16.
+// 870 without the weights' share, 1300 with it.  256 x 3072 x 3072 with weights that come from memory, us, with the images'
+// launch (B200): forward 128.8 with cuBLAS's fp32 kernel, 36.9 so; input gradient 121.7 and 36.2; weight gradient, whose
+// images take the second-level cache 9 TB/s, 98.9 and 30.1: 130 to 160 TFLOP/s of fp32 products, 0.8 to 1 PFLOP/s of bf16.
+// Tried and left: pairs of CTAs on one tile (92 KB per stage, but each turn waits for both: 47.5 us), weights cut straight
+// into tensor memory (72 KB; a lane's 32 loads per stage cost what that saves: 36.0 and 48.4 us).
 template <int NT, int kSource>
 __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Work w) {
   constexpr bool kAInner = kSource == kWeightRows, kBInner = kSource != kImage;
@@ -498,40 +502,50 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
   __syncthreads();
   fence_after();
   if (w.splits > 1) {
-    // The CTA that is the last of its tile adds up all parts, in order.  Four numbers per thread and load, all loads in
-    // flight together.
+    // The CTA that is the last of its tile adds up all parts, in order.  Eight loads of four numbers per thread in flight:
+    // with one part after the other, and the bias only then, the three parts of a forward product took 2 us longer.
     const int tile = first_tile;
     if (tid == 0) last_here = atomicAdd(w.tickets + tile, 1u) == static_cast<uint32_t>(w.splits - 1);
     __syncthreads();
     if (last_here) {
       __threadfence();
-      constexpr int kStride = kThreads<kSource>, kVecs = NT * kRows / 4, kEach = (kVecs + kStride - 1) / kStride;
+      constexpr int kStride = kThreads<kSource>, kVecs = NT * kRows / 4;
       const float4* from = reinterpret_cast<const float4*>(w.partial) + static_cast<int64_t>(tile) * w.splits * kVecs;
-      float4 sum[kEach];
+      const int64_t i = static_cast<int64_t>(tile % w.tiles_i) * kRows + tid % (kRows / 4) * 4;
+      static_assert(kStride % (kRows / 4) == 0, "all numbers of a thread belong to the same four i");
+      float add[4];
 #pragma unroll
-      for (int e = 0; e < kEach; ++e)
-        if (tid + e * kStride < kVecs) sum[e] = __ldcg(from + tid + e * kStride);
-      for (int r = 1; r < w.splits; ++r) {
-        from += kVecs;
-        float4 x[kEach];
+      for (int n = 0; n < 4; ++n) add[n] = w.bias && i + n < w.rows_i ? w.bias[i + n] : 0.f;
+      constexpr int kBatch = 4;
+      for (int v0 = tid; v0 < kVecs; v0 += kBatch * kStride) {
+        float4 sum[kBatch];
+        for (int r = 0; r < w.splits; r += 2) {  // two parts of four vectors in flight
+          float4 x[2][kBatch];
 #pragma unroll
-        for (int e = 0; e < kEach; ++e)
-          if (tid + e * kStride < kVecs) x[e] = __ldcg(from + tid + e * kStride);
+          for (int p = 0; p < 2; ++p)
 #pragma unroll
-        for (int e = 0; e < kEach; ++e) {
-          sum[e].x += x[e].x; sum[e].y += x[e].y; sum[e].z += x[e].z; sum[e].w += x[e].w;
+            for (int e = 0; e < kBatch; ++e)
+              x[p][e] = r + p < w.splits && v0 + e * kStride < kVecs ? __ldcg(from + (r + p) * kVecs + v0 + e * kStride)
+                                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int e = 0; e < kBatch; ++e) {
+            if (r == 0) sum[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+              sum[e].x += x[p][e].x; sum[e].y += x[p][e].y; sum[e].z += x[p][e].z; sum[e].w += x[p][e].w;
+            }
+          }
         }
-      }
 #pragma unroll
-      for (int e = 0; e < kEach; ++e) {
-        const int v = tid + e * kStride;
-        const int64_t i = static_cast<int64_t>(tile % w.tiles_i) * kRows + v % (kRows / 4) * 4;
-        const int64_t j = static_cast<int64_t>(tile / w.tiles_i) * NT + v / (kRows / 4);
-        if (v >= kVecs || j >= w.rows_j) continue;
-        float out[4] = {sum[e].x, sum[e].y, sum[e].z, sum[e].w};
+        for (int e = 0; e < kBatch; ++e) {
+          const int v = v0 + e * kStride;
+          const int64_t j = static_cast<int64_t>(tile / w.tiles_i) * NT + v / (kRows / 4);
+          if (v >= kVecs || j >= w.rows_j) continue;
+          const float out[4] = {sum[e].x, sum[e].y, sum[e].z, sum[e].w};
 #pragma unroll
-        for (int n = 0; n < 4; ++n)
-          if (i + n < w.rows_i) w.c[j * w.ldc + i + n] = w.bias ? out[n] + w.bias[i + n] : out[n];
+          for (int n = 0; n < 4; ++n)
+            if (i + n < w.rows_i) w.c[j * w.ldc + i + n] = w.bias ? out[n] + add[n] : out[n];
+        }
       }
     }
   }
