@@ -3,14 +3,16 @@
 // A gradient that fits the shared memory of one thread-block cluster is selected from there by one launch: exact
 // radix select, ordered output or dense result, one read and one write of every element.  A larger one takes five:
 //   sample   a cluster reads 64 Ki evenly spread elements of g + e and takes, from their exact selection, a
-//            magnitude that clearly more than k elements reach
+//            magnitude that clearly more than k elements reach and one that clearly fewer do
 //   adjust   all SMs: a = g + e, e = a (and g = 0 where the result is dense); the few elements that reach the
 //            sampled magnitude go to a candidate list, tile by tile in index order, and into a histogram of 1/1024
-//            octave per bin, from which the last block takes the bin of the k-th element
+//            octave per bin, from which the last block takes the bin of the k-th element; where the result is dense,
+//            those above the second magnitude are sent at once
 //   select   candidates above the bin are selected, those inside it are gathered, and the last block finds the
-//            exact threshold (and the index limit among ties) on them
-//   output   a count per run of tiles, then the ordered output: pairs sorted by index; a dense result is there already
-//            (both launches leave at once)
+//            exact threshold (and the index limit among ties) on them; what was sent too early is taken back
+//   output   a count per run of tiles, then the ordered output: pairs sorted by index; a dense result only gets the
+//            entries of the k-th element's bin
+// Each comes up while the one before ends (a dependent launch: 8 of 44 us at 700 000 elements).
 //
 // The sample decides speed, never results.  Heavily tied data (more elements than the list holds, or a crowded bin):
 // the select launch takes the exact threshold from the whole adjusted vector and the last two rank the ties in index
@@ -71,18 +73,20 @@ constexpr int kFineBins = 1 << (kCoarseShift - kBinShift);
 constexpr int kRun = 4;                  // tiles whose pairs one warp puts out
 // Entries of the k-th element's bin that one block resolves; more (ties) are left to the whole grid.  51.5 M bf16
 // elements, dense result: 255 levels at 1 %, about 50 thousand entries, 222 us with one block and 441 us with the grid;
-// 40 levels at 1 %, 190 thousand, 480 and 450 us; 40 levels at 10 %, over a million, 1709 and 509 us.
+// 40 levels at 1 %, 190 thousand, 480 and 450 us; 40 levels at 10 %, over a million, 1709 and 509 us (that block then also
+// sent them).
 constexpr uint32_t kOneBlock = 128 * 1024;
 // kList: from the candidates.  kWide: from the candidates, among those of the open-ended last bin.  kTies: the bin is known,
 // threshold and ties come from the vector.  kWhole: the bin comes from the vector as well.  kZeros: all non-zeros and the
-// first zeros.
-enum Mode : uint32_t { kList, kWide, kWhole, kTies, kZeros };
+// first zeros.  kAll: all non-zeros are listed, and a dense result needs no more.
+enum Mode : uint32_t { kList, kWide, kWhole, kTies, kZeros, kAll };
 
 // The exact rule: an element is sent if key > threshold, or key == threshold and index <= last_index (kList) or it is
 // one of the first `need` (kTies, kZeros).
 struct ListState {
   uint32_t hist[kBins];  // candidates by (key - base) >> kBinShift, the last bin open-ended
   uint32_t base;         // smallest magnitude key that is a candidate
+  uint32_t sure;         // dense result: candidates above it were sent by the adjust launch
   uint32_t count;        // entries in the list
   uint32_t overflow;     // the list did not hold them all
   uint32_t mode;         // how the selection is decided: Mode
@@ -93,6 +97,7 @@ struct ListState {
   uint32_t sub[kSubBins];  // kTies: elements of the bin by key
   uint32_t coarse[kBins];    // kWide, kWhole: keys by key >> kCoarseShift
   uint32_t fine[kFineBins];  // and of the chosen coarse bin
+  uint32_t pad[3];
   uint32_t gate[4][2];   // kWide, kWhole: blocks that came to a meeting, and how it ended
 };
 static_assert(sizeof(ListState) % sizeof(uint4) == 0, "8-byte entries follow it in the scratch");
@@ -113,6 +118,12 @@ __host__ __device__ inline int64_t run_count(int64_t n) { return (tile_count(n) 
 inline uint32_t sample_rank(int64_t n, int64_t k) {
   const double hits = static_cast<double>(kSample) * static_cast<double>(k) / static_cast<double>(n);
   return static_cast<uint32_t>(std::min<double>(kSample, hits + 5.0 * std::sqrt(hits) + 8.0));
+}
+// The other bound: so few sampled elements lie above the magnitude of this rank that fewer than k of all do (five standard
+// deviations again).  0: the selection is too small for one.
+inline uint32_t sure_rank(int64_t n, int64_t k) {
+  const double hits = static_cast<double>(kSample) * static_cast<double>(k) / static_cast<double>(n);
+  return sample_rank(n, k) == kSample ? 0u : static_cast<uint32_t>(std::max(0.0, hits - 5.0 * std::sqrt(hits) - 8.0));
 }
 // Room for the elements that reach it: six standard deviations above their expected number, and some for ties.
 // None where the whole sample would be needed, at ratios above 0.98: its smallest element bounds nothing, and the list would
@@ -140,6 +151,11 @@ inline ListView list_view(void* scratch, size_t bytes, int64_t n, int64_t k) {
   return v;
 }
 
+// ---- launches that follow one another ----------------------------------------------------------------------
+// The next launch's blocks may come up now; they wait, before they touch anything, until this one is complete.
+__device__ __forceinline__ void start_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- selection by a cluster ---------------------------------------------------------------------------------
 // True in exactly one block of the grid: the one that finishes last.  What the others wrote before their call is
 // visible to it.
@@ -153,13 +169,16 @@ __device__ __forceinline__ bool last_block_done(uint32_t* ticket) {
   return s_last;
 }
 
-struct ClusterShared {
-  uint32_t hist[kBins];    // this CTA's counts
-  uint32_t total[kBins];   // the cluster's
+template <int kRanks>
+struct Counts {
+  uint32_t hist[kRanks * kBins];   // this CTA's counts
+  uint32_t total[kRanks * kBins];  // the cluster's
   uint32_t wsum[33];
+  uint32_t digit[kRanks], above[kRanks];
+};
+struct ClusterShared : Counts<1> {
   uint2 counts_of[kMaxCluster];
   uint2 warp_counts[kWarps];
-  uint32_t digit, above;
 };
 
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_sums) {
@@ -184,35 +203,38 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_s
   return warp_sums[warp] + inc - v;
 }
 
-// The key of the need-th largest item of the cluster and how many items equal to it belong to the selection.
+// The keys of the need[r]-th largest items of the cluster and how many items equal to each belong to the selection.
 // each(f) calls f(key) for every item of the calling thread; every thread of the cluster calls this together, and
 // there are at least `need` items.  With two levels instead of three the lowest 9 of the 31 bits stay open (zero).
 // No CTA's shared memory is touched by another after the return.
-template <int kLevels, typename Each>
-__device__ void cluster_threshold(ClusterShared& sh, uint32_t need, Each&& each, uint32_t* threshold,
-                                  uint32_t* need_eq) {
+template <int kLevels, int kRanks, typename Each>
+__device__ void cluster_thresholds(Counts<kRanks>& sh, uint32_t (&need)[kRanks], Each&& each, uint32_t (&threshold)[kRanks]) {
   cg::cluster_group cluster = cg::this_cluster();
   const int ctas = static_cast<int>(cluster.num_blocks()), me = static_cast<int>(cluster.block_rank());
   const int tid = threadIdx.x, lane = tid & 31;
   int width = 11, shift = 20;  // 31 bits of magnitude
-  uint32_t prefix = 0;
+  uint32_t prefix[kRanks] = {};
   for (int level = 0;; ++level) {
-    for (int i = tid; i < kBins; i += kThreads) sh.hist[i] = 0;
+    const int ranks = level == 0 ? 1 : kRanks;  // the first level's counts serve all
+    for (int i = tid; i < ranks * kBins; i += kThreads) sh.hist[i] = 0;
     __syncthreads();
     uint32_t lowest = 0;  // the lowest bin's items (zeros, where there are many) are counted in a register
     const uint32_t mask = (1u << width) - 1u;
     each([&](uint32_t key) {
-      if ((key >> shift) >> width != prefix) return;
-      const uint32_t d = (key >> shift) & mask;
-      if (d == 0) ++lowest;
-      else atomicAdd(&sh.hist[d], 1u);
+#pragma unroll
+      for (int r = 0; r < kRanks; ++r) {
+        if (r >= ranks || (key >> shift) >> width != prefix[r]) continue;
+        const uint32_t d = (key >> shift) & mask;
+        if (r == 0 && d == 0) ++lowest;
+        else atomicAdd(&sh.hist[r * kBins + d], 1u);
+      }
     });
     lowest = __reduce_add_sync(0xFFFFFFFFu, lowest);
     if (lane == 0 && lowest) atomicAdd(&sh.hist[0], lowest);
     cluster.sync();
     // Every CTA adds up its share of the bins over the cluster and hands the sums to all.  A thread per bin, its
     // loads independent (spreading a bin over several threads, or warps over CTAs, measured 15 to 30 % slower).
-    const int share = kBins / ctas;
+    const int share = ranks * kBins / ctas;
     if (tid < share) {
       uint32_t sum = 0;
 #pragma unroll
@@ -225,24 +247,35 @@ __device__ void cluster_threshold(ClusterShared& sh, uint32_t need, Each&& each,
     cluster.sync();
     // from the top bin down: the bin at which the running count reaches `need`
     const int top = kBins - 1 - 2 * tid;
-    const uint32_t c0 = sh.total[top], c1 = sh.total[top - 1];
-    const uint32_t above = block_excl_scan(c0 + c1, sh.wsum);
-    if (above < need && above + c0 >= need) {
-      sh.digit = top;
-      sh.above = above;
-    } else if (above + c0 < need && above + c0 + c1 >= need) {
-      sh.digit = top - 1;
-      sh.above = above + c0;
+#pragma unroll
+    for (int r = 0; r < kRanks; ++r) {
+      const uint32_t* total = sh.total + (level == 0 ? 0 : r * kBins);
+      const uint32_t c0 = total[top], c1 = total[top - 1];
+      const uint32_t above = block_excl_scan(c0 + c1, sh.wsum);
+      if (above < need[r] && above + c0 >= need[r]) {
+        sh.digit[r] = top;
+        sh.above[r] = above;
+      } else if (above + c0 < need[r] && above + c0 + c1 >= need[r]) {
+        sh.digit[r] = top - 1;
+        sh.above[r] = above + c0;
+      }
+      __syncthreads();
+      need[r] -= sh.above[r];
+      prefix[r] = (prefix[r] << width) | sh.digit[r];
     }
-    __syncthreads();
-    need -= sh.above;
-    prefix = (prefix << width) | sh.digit;
     if (level == kLevels - 1) break;
     width = shift < 11 ? shift : 11;
     shift -= width;
   }
-  *threshold = prefix << shift;
-  *need_eq = need;
+#pragma unroll
+  for (int r = 0; r < kRanks; ++r) threshold[r] = prefix[r] << shift;
+}
+template <int kLevels, typename Each>
+__device__ void cluster_threshold(Counts<1>& sh, uint32_t need, Each&& each, uint32_t* threshold, uint32_t* need_eq) {
+  uint32_t left[1] = {need}, found[1];
+  cluster_thresholds<kLevels, 1>(sh, left, each, found);
+  *threshold = found[0];
+  *need_eq = left[0];
 }
 
 // Emits the selection in index order.  walk(f) calls f(index, value, valid) with all lanes of the calling warp, for
@@ -345,11 +378,13 @@ __global__ void __launch_bounds__(kThreads, 1) topk_cluster_kernel(const SelectA
                });
 }
 
-// The magnitude that `rank` of the kSample sampled elements reach, as the list's smallest key.
+// The magnitude that `rank` of the kSample sampled elements reach, as the list's smallest key, and the one that `sure` of
+// them reach, rounded up (0: none).
 template <bool kBf16>
-__global__ void __launch_bounds__(kThreads, 1) topk_sample_kernel(const SelectArgs a, uint32_t rank) {
+__global__ void __launch_bounds__(kThreads, 1) topk_sample_kernel(const SelectArgs a, uint32_t rank, uint32_t sure) {
   constexpr int kMost = kSample / 8 / kThreads;  // per thread, in a cluster of eight CTAs
-  __shared__ ClusterShared sh;
+  __shared__ Counts<2> sh;
+  start_dependents();
   cg::cluster_group cluster = cg::this_cluster();
   const int per = kSample / static_cast<int>(cluster.num_blocks()), mine = per / kThreads;
   const int64_t stride = a.n / kSample;
@@ -362,18 +397,20 @@ __global__ void __launch_bounds__(kThreads, 1) topk_sample_kernel(const SelectAr
     const int64_t i = s * stride + (static_cast<uint64_t>((s * 2654435761u) >> 8) * stride >> 24);
     key[j] = key_of(load_grad<kBf16>(a.grad, i) + a.residual[i]);
   }
-  uint32_t threshold, unused;
-  cluster_threshold<2>(sh, rank, [&](auto&& f) {
+  uint32_t need[2] = {rank, sure > 0 ? sure : 1u}, found[2];
+  cluster_thresholds<2, 2>(sh, need, [&](auto&& f) {
 #pragma unroll
     for (int j = 0; j < kMost; ++j)
       if (j < mine) f(key[j]);
-  }, &threshold, &unused);
+  }, found);
   if (cluster.block_rank() == 0) {
     uint32_t* words = reinterpret_cast<uint32_t*>(a.list.state);
     for (int i = threadIdx.x; i < static_cast<int>(sizeof(ListState) / 4); i += kThreads) words[i] = 0u;
     __syncthreads();
-    if (threadIdx.x == 0)
-      a.list.state->base = rank == kSample ? 0xFFFFFFFFu : threshold > 0 ? threshold : 1u;  // zeros are never worth listing
+    if (threadIdx.x == 0) {
+      a.list.state->base = rank == kSample ? 0xFFFFFFFFu : found[0] > 0 ? found[0] : 1u;  // zeros are never worth listing
+      a.list.state->sure = sure > 0 ? found[1] | 0x1FFu : 0xFFFFFFFFu;
+    }
   }
 }
 
@@ -383,6 +420,12 @@ __device__ __forceinline__ void send(const SelectArgs& a, uint32_t i, float v) {
   a.residual[i] = 0.f;
   if (kDense) store_dense<kBf16>(a.grad, i, scaled(v, a.scale));
 }
+// Takes one back that was sent.
+template <bool kBf16, bool kDense>
+__device__ __forceinline__ void unsend(const SelectArgs& a, uint32_t i, float v) {
+  a.residual[i] = v;
+  if (kDense) store_dense<kBf16>(a.grad, i, 0.f);
+}
 
 __device__ __forceinline__ uint32_t bin_of(uint32_t key_above_base) {
   const uint32_t b = key_above_base >> kBinShift;
@@ -391,8 +434,12 @@ __device__ __forceinline__ uint32_t bin_of(uint32_t key_above_base) {
 
 // a = g + e, e = a, candidates to the list.  A warp owns `group` consecutive tiles at a time and appends their
 // candidates in index order: one global atomic per group, entries of a group contiguous.
+// A dense result gets its surely selected entries here, while the lines just written are in the cache: sent by the next
+// launch, half a million scattered pairs of stores fetched and wrote a sector each (select 64 us, all 211 us a pass among
+// others; so 165); kept back until a warp's stage was full they did no better (207), and worked into the vector stores they
+// cost registers (218).
 // Bound by HBM: 12 bytes per bf16 element with a dense result.
-// 50257 x 1024 bf16 elements (618 MB): 106 us, 5.8 TB/s.  The whole selection: 404 us in four passes, 185 us so.
+// 50257 x 1024 bf16 elements (618 MB): 122 us among others, 5.1 TB/s, 112 without the entries.
 template <bool kBf16, bool kVec, bool kDense>
 __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a, int group) {
   extern __shared__ __align__(16) uint2 staging[];
@@ -402,7 +449,9 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint2* stage = staging + warp * kStage;
   const ListView list = a.list;
-  const uint32_t base = list.state->base;
+  start_dependents();
+  wait_for_previous();
+  const uint32_t base = list.state->base, sure = kDense ? list.state->sure : 0xFFFFFFFFu;
   const int64_t tiles = tile_count(a.n);
   const uint32_t lower = (1u << lane) - 1u;
   const int64_t step = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32) * group;
@@ -416,10 +465,12 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
       if (lane == 0) {
         if (cnt) start = atomicAdd(&list.state->count, cnt);
         list.tiles[t] = make_uint2(start, cnt);
-        if (start > list.cap || cnt > list.cap - start) list.state->overflow = 1u;
       }
       *at = start = __shfl_sync(0xFFFFFFFFu, start, 0);
-      return start <= list.cap && cnt <= list.cap - start;
+      if (start <= list.cap && cnt <= list.cap - start) return true;
+      if (lane == 0) list.state->overflow = 1u;
+      for (uint32_t i = start + lane; i < list.cap; i += 32) list.list[i] = make_uint2(0u, 0u);  // the list's end: no entries
+      return false;
     };
     auto flush = [&]() {
       uint32_t start;
@@ -427,8 +478,10 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
       const bool fits = reserve(first, staged, &start);
       for (uint32_t i = lane; i < staged; i += 32) {
         const uint2 e = stage[i];
+        const uint32_t key = e.y & 0x7FFFFFFFu;
         if (fits) list.list[start + i] = e;
-        atomicAdd(&hist[bin_of((e.y & 0x7FFFFFFFu) - base)], 1u);
+        else if (key > sure) unsend<kBf16, kDense>(a, e.x, __uint_as_float(e.y));  // what is sent is listed
+        atomicAdd(&hist[bin_of(key - base)], 1u);
       }
       __syncwarp();
       staged = 0;
@@ -526,9 +579,12 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             if ((nib >> j) & 1u) {
-              if (fits)
+              if (fits) {
                 to[put + before + __popc(nib & ((1u << j) - 1u))] =
                     make_uint2(static_cast<uint32_t>(t0 + 128 * q + j), __float_as_uint(v[q][j]));
+                // while the lines just written are in the cache
+                if (key_of(v[q][j]) > sure) send<kBf16, kDense>(a, static_cast<uint32_t>(t0 + 128 * q + j), v[q][j]);
+              }
               if (here > kStage) atomicAdd(&hist[bin_of(key_of(v[q][j]) - base)], 1u);
             }
           put += all;
@@ -567,7 +623,7 @@ __global__ void __launch_bounds__(256, 3) topk_adjust_kernel(const SelectArgs a,
   }
   if (threadIdx.x == 0 && count < a.k) {
     // every non-zero is a candidate, everything is sent, or the sample missed (or none was taken)
-    list.state->mode = base == 1u || a.k == a.n ? kZeros : kWhole;
+    list.state->mode = kDense && base == 1u && missing == 0u ? kAll : base == 1u || a.k == a.n ? kZeros : kWhole;
     list.state->threshold = 0u;
     list.state->need = a.k == a.n ? a.k : a.k - count;
   }
@@ -619,12 +675,12 @@ __device__ uint32_t block_nth(uint32_t* hist, uint32_t* wsum, uint32_t* s_pick, 
 }
 
 // Adds n keys to this block's counts by digit(key); those whose digit is `bins` or more are left out.  What comes here is
-// mostly tied: the digits of two lanes of a warp are counted for all that share them, and only the rest one by one.
+// mostly tied: the digits of two lanes of a warp are counted for all that share them, and only the rest one by one.  One
+// source of keys at a time: a choice between two within `key` keeps the loads from going out together (51.5 M equal bf16
+// elements: 527 and 670 us).
 template <typename Key, typename Digit>
 __device__ __forceinline__ void count_digits(uint32_t* counts, uint32_t bins, int64_t n, Key&& key, Digit&& digit) {
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < static_cast<int>(bins); i += kThreads) counts[i] = 0;
-  __syncthreads();
   constexpr int kAhead = 8;
   const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads * kAhead;
   for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * kThreads * kAhead; i0 < n; i0 += step) {
@@ -655,6 +711,11 @@ __device__ __forceinline__ void count_digits(uint32_t* counts, uint32_t bins, in
   __syncthreads();
 }
 
+__device__ __forceinline__ void clear_counts(uint32_t* counts, int bins) {
+  for (int i = threadIdx.x; i < bins; i += kThreads) counts[i] = 0;
+  __syncthreads();
+}
+
 // Waits for all blocks of the grid, with a limit: true in every block (what the others wrote before is then visible) or,
 // if one did not come in time because another grid holds its SM, false in every block.  One word decides.
 __device__ __forceinline__ bool grid_meets(uint32_t* gate, int tries) {
@@ -680,12 +741,18 @@ __device__ __forceinline__ bool grid_meets(uint32_t* gate, int tries) {
   return s_end == kMet;
 }
 
-// The kBinShift-wide bin that holds the need-th largest of n keys (the list's or, where that is null, the vector's), from two
+// A listed key above the given one; another is no key at all.
+__device__ __forceinline__ uint32_t listed_key(const uint2* list, int64_t i, uint32_t above) {
+  const uint32_t key = list[i].y & 0x7FFFFFFFu;
+  return key > above ? key : 0xFFFFFFFFu;
+}
+
+// The kBinShift-wide bin that holds the need-th largest of the vector's n keys and the listed ones above `above_key`, from two
 // counts by the whole grid; *need becomes how many of its entries are selected, *entries how many it has.  False if the grid
 // could not meet.  Not inlined: the ordinary selection does not come here.
 __device__ __noinline__ bool find_bin(ListState* st, uint32_t* counts, uint32_t* wsum, uint32_t* s_pick, int64_t n,
-                                      const uint2* list, const float* vector, uint32_t* floor_key, uint32_t* need,
-                                      uint32_t* entries) {
+                                      int64_t listed, const uint2* list, uint32_t above_key, const float* vector,
+                                      uint32_t* floor_key, uint32_t* need, uint32_t* entries) {
   const int tid = threadIdx.x;
   uint32_t prefix = 0;
   // All blocks start as soon as the launch before is done; once they have met they only wait for the slowest count.
@@ -694,11 +761,13 @@ __device__ __noinline__ bool find_bin(ListState* st, uint32_t* counts, uint32_t*
   for (int level = 0; level < 2; ++level) {
     const int bins = level == 0 ? kBins : kFineBins;
     uint32_t* total = level == 0 ? st->coarse : st->fine;
-    auto key = [&](int64_t i) { return list != nullptr ? list[i].y & 0x7FFFFFFFu : key_of(__ldcs(vector + i)); };
-    count_digits(counts, bins, n, key, [&](uint32_t k) {
+    auto digit = [&](uint32_t k) {
       if (level == 0) return k >> kCoarseShift;
       return k >> kCoarseShift == prefix ? (k >> kBinShift) & (kFineBins - 1u) : 0xFFFFFFFFu;
-    });
+    };
+    clear_counts(counts, bins);
+    count_digits(counts, bins, n, [&](int64_t i) { return key_of(__ldcs(vector + i)); }, digit);
+    count_digits(counts, bins, listed, [&](int64_t i) { return listed_key(list, i, above_key); }, digit);
     for (int i = tid; i < bins; i += kThreads)
       if (counts[i]) atomicAdd(&total[i], counts[i]);
     if (!grid_meets(st->gate[level + 1], 1000000)) return false;
@@ -735,22 +804,38 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
   extern __shared__ __align__(16) uint32_t sub[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   ListState* st = a.list.state;
+  start_dependents();
+  wait_for_previous();
   uint32_t mode = st->mode;
   if (mode == kZeros) return;
+  // What the adjust launch has sent is zero in the vector and is counted from the list.  All of it belongs to the selection;
+  // where the sample was wrong about that, it is taken back.
+  const uint32_t sure = kDense ? st->sure : 0xFFFFFFFFu;
+  const int64_t listed = st->count < a.list.cap ? st->count : a.list.cap;
+  auto sent_early = [&](int64_t i) { return kDense && (a.list.list[i].y & 0x7FFFFFFFu) > sure; };
+  if (mode == kAll) {
+    for (int64_t i = blockIdx.x * kThreads + tid; i < listed; i += gridDim.x * kThreads) {
+      const uint2 e = a.list.list[i];
+      if (!sent_early(i)) send<kBf16, kDense>(a, e.x, __uint_as_float(e.y));
+    }
+    return;
+  }
   uint32_t floor_key = st->base + (st->bin << kBinShift), need = st->need;  // the k-th element's bin
   if (mode == kWide || mode == kWhole) {
-    const bool listed = mode == kWide;
+    const bool wide = mode == kWide;
     uint32_t floor_found, need_found = a.k, entries;
-    if (find_bin(st, sub, sh.wsum, s_pick, listed ? st->count : a.n, listed ? a.list.list : nullptr, a.residual, &floor_found,
-                 &need_found, &entries)) {
+    if (find_bin(st, sub, sh.wsum, s_pick, wide ? 0 : a.n, wide || kDense ? listed : 0, a.list.list, wide ? 0u : sure, a.residual,
+                 &floor_found, &need_found, &entries)) {
       floor_key = floor_found;
       need = need_found;
-      mode = listed && entries <= kOneBlock ? kList : kTies;
+      mode = wide && entries <= kOneBlock ? kList : kTies;
     }
   }
   if (mode == kTies) {
-    count_digits(sub, kSubBins, a.n, [&](int64_t i) { return key_of(__ldcs(a.residual + i)); },
-                 [&](uint32_t key) { return key - floor_key; });
+    auto digit = [&](uint32_t key) { return key - floor_key; };
+    clear_counts(sub, kSubBins);
+    count_digits(sub, kSubBins, a.n, [&](int64_t i) { return key_of(__ldcs(a.residual + i)); }, digit);
+    if (kDense) count_digits(sub, kSubBins, listed, [&](int64_t i) { return listed_key(a.list.list, i, sure); }, digit);
     for (int i = tid; i < kSubBins; i += kThreads)
       if (sub[i]) atomicAdd(&st->sub[i], sub[i]);
     if (!last_block_done(&st->ticket[1])) return;
@@ -766,18 +851,24 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       if (above < need && above + c[i] >= need) {
-        st->threshold = floor_key + static_cast<uint32_t>(top - i);
+        st->threshold = s_base = floor_key + static_cast<uint32_t>(top - i);
         st->need = need - above;
       }
       above += c[i];
     }
     if (tid == 0) st->mode = kTies;
+    __syncthreads();
+    if (kDense && s_base > sure)
+      for (int64_t i = tid; i < listed; i += kThreads) {
+        const uint2 e = a.list.list[i];
+        if (sent_early(i) && (e.y & 0x7FFFFFFFu) <= s_base) unsend<kBf16, kDense>(a, e.x, __uint_as_float(e.y));
+      }
     return;
   }
   if (mode == kList) {
     const uint32_t count = st->count;
     uint2* bin_list = a.list.bin_list;
-    constexpr int kAhead = 4;
+    constexpr int kAhead = 8;
     const uint32_t step = gridDim.x * kThreads * kAhead;
     for (uint32_t i0 = blockIdx.x * kThreads * kAhead; i0 < count; i0 += step) {
       uint2 e[kAhead];
@@ -794,7 +885,8 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
         const bool valid = i0 + u * kThreads + tid < count;
         const float v = __uint_as_float(e[u].y);
         const uint32_t key = key_of(v), from_floor = key - floor_key;  // wraps below the bin
-        if (kDense && valid && key >= floor_key && from_floor >= kSubBins) send<kBf16, kDense>(a, e[u].x, v);
+        if (kDense && valid && key >= floor_key && from_floor >= kSubBins && key <= sure) send<kBf16, kDense>(a, e[u].x, v);
+        if (kDense && valid && key < floor_key && key > sure) unsend<kBf16, kDense>(a, e[u].x, v);
         const bool inside = valid && from_floor < kSubBins;
         at[u] = inside ? atomicAdd(&s_count, 1u) : 0xFFFFFFFFu;
       }
@@ -821,13 +913,7 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
         const uint2 e = __ldcg(&bin_list[i]);
         return (e.y & 0x7FFFFFFFu) == threshold ? static_cast<uint64_t>(e.x) : kNone;
       });
-    if (kDense) {
-      for (uint32_t i = tid; i < m; i += kThreads) {
-        const uint2 e = __ldcg(&bin_list[i]);
-        const uint32_t key = e.y & 0x7FFFFFFFu;
-        if (key > threshold || (key == threshold && e.x <= last_index)) send<kBf16, kDense>(a, e.x, __uint_as_float(e.y));
-      }
-    } else if (tid == 0) {
+    if (tid == 0) {
       st->threshold = threshold;
       st->last_index = last_index;
     }
@@ -850,7 +936,17 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
       for (int u = 0; u < kAhead; ++u)
         if (i + u * kThreads < hi) f(key_of(v[u]));
     }
+    for (int64_t i = me * kThreads + tid; kDense && i < listed; i += ctas * kThreads)
+      if (sent_early(i)) f(a.list.list[i].y & 0x7FFFFFFFu);
   }, &threshold, &need_eq);
+  if (kDense && threshold > sure) {
+    for (int64_t i = me * kThreads + tid; i < listed; i += ctas * kThreads) {
+      const uint2 e = a.list.list[i];
+      if (sent_early(i) && (e.y & 0x7FFFFFFFu) <= threshold) unsend<kBf16, kDense>(a, e.x, __uint_as_float(e.y));
+    }
+    __threadfence();
+    cluster.sync();
+  }
   const int64_t per_warp = (hi - lo + kWarps - 1) / kWarps;
   const int64_t w0 = at_most(hi, lo + per_warp * warp), w1 = at_most(hi, w0 + per_warp);
   cluster_emit(sh, threshold, need_eq,
@@ -868,7 +964,7 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const SelectAr
                  }
                },
                [&](uint32_t i, float v, uint32_t pos, bool selected) {
-                 if (!selected) return;
+                 if (!selected || (kDense && key_of(v) == 0u)) return;  // a zero, or sent already
                  send<kBf16, kDense>(a, i, v);
                  if (!kDense) a.pairs[pos] = make_uint2(i, __float_as_uint(v));
                });
@@ -881,9 +977,25 @@ template <bool kCount, bool kBf16, bool kDense>
 __global__ void __launch_bounds__(kThreads, 1) topk_output_kernel(const SelectArgs a) {
   const int lane = threadIdx.x & 31;
   ListState* st = a.list.state;
+  start_dependents();
+  wait_for_previous();
   const uint32_t mode = st->mode;
-  if (mode == kWhole || mode == kWide || (mode == kList && kDense)) return;
+  if (mode == kWhole || mode == kWide || mode == kAll) return;
   const uint32_t threshold = st->threshold, last_index = st->last_index, need = st->need;
+  const bool early = kDense && st->sure != 0xFFFFFFFFu;
+  if (mode == kList && kDense) {
+    // the entries of the k-th element's bin: by one block, where they were gathered, 14 thousand took 24 us
+    if (!kCount) return;
+    const uint32_t sure = st->sure, m = st->in_bin;
+    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < m; i += gridDim.x * kThreads) {
+      const uint2 e = __ldcg(&a.list.bin_list[i]);
+      const uint32_t key = e.y & 0x7FFFFFFFu;
+      const bool selected = key > threshold || (key == threshold && e.x <= last_index);
+      if (selected && key <= sure) send<kBf16, kDense>(a, e.x, __uint_as_float(e.y));
+      if (!selected && key > sure) unsend<kBf16, kDense>(a, e.x, __uint_as_float(e.y));
+    }
+    return;
+  }
   const uint32_t lower = (1u << lane) - 1u;
   const int64_t tiles = tile_count(a.n), runs = run_count(a.n);
   for (int64_t run = static_cast<int64_t>(blockIdx.x) * kWarps + (threadIdx.x >> 5); run < runs; run += gridDim.x * kWarps) {
@@ -921,7 +1033,7 @@ __global__ void __launch_bounds__(kThreads, 1) topk_output_kernel(const SelectAr
           const uint32_t m_gt = __ballot_sync(0xFFFFFFFFu, gt), m_eq = __ballot_sync(0xFFFFFFFFu, eq);
           if (!kCount) {
             const uint32_t r_gt = done.x + __popc(m_gt & lower), r_eq = done.y + __popc(m_eq & lower);
-            if (gt || (eq && r_eq < need)) {
+            if (gt || (eq && r_eq < need && !(early && key == 0u))) {  // a zero may be one that was sent, and sends nothing
               send<kBf16, kDense>(a, static_cast<uint32_t>(i), v[u]);
               if (!kDense) a.pairs[r_gt + (r_eq < need ? r_eq : need)] = make_uint2(static_cast<uint32_t>(i), __float_as_uint(v[u]));
             }
@@ -995,20 +1107,28 @@ cudaError_t cluster_size(const void* kernel, ClusterSize& cache, size_t most_sme
   return cudaSuccess;
 }
 
+// `ctas`: of a cluster; `follows`: the blocks come up while the launch before ends, and wait for it.
 template <typename... Params, typename... Args>
-cudaError_t launch_cluster(void (*kernel)(Params...), int clusters, int ctas, size_t smem, cudaStream_t s,
-                           Args... args) {
+cudaError_t launch(void (*kernel)(Params...), unsigned grid, int threads, int ctas, size_t smem, bool follows, cudaStream_t s,
+                   Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = ctas;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.gridDim = dim3(clusters * ctas);
-  cfg.blockDim = dim3(kThreads);
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  if (ctas > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = ctas;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (follows) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
@@ -1023,14 +1143,14 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const int per = static_cast<int>(((a.n + ctas - 1) / ctas + 7) / 8 * 8);
     note_launch();
-    return launch_cluster(small, 1, ctas, per * sizeof(float), s, a, per);
+    return launch(small, ctas, kThreads, ctas, per * sizeof(float), false, s, a, per);
   }
   auto sample = topk_sample_kernel<kBf16>;
   cudaError_t e = cluster_size(reinterpret_cast<const void*>(sample), sample_size, 0, &ctas);
   if (e != cudaSuccess) return e;
   const uint32_t rank = sample_rank(a.n, a.k);
   note_launch(5);
-  e = launch_cluster(sample, 1, ctas, 0, s, a, rank);
+  e = launch(sample, ctas, kThreads, ctas, 0, false, s, a, rank, sure_rank(a.n, a.k));
   if (e != cudaSuccess) return e;
 
   // tiles per group: about half a stage of candidates, and every warp of the grid busy
@@ -1044,8 +1164,7 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
   static_assert(smem + (kBins + 64) * sizeof(uint32_t) <= 48 << 10, "more would have to be asked for");
   const bool vec = ((reinterpret_cast<uintptr_t>(t.grad) | reinterpret_cast<uintptr_t>(t.residual)) & 15) == 0;
   auto adjust = vec ? topk_adjust_kernel<kBf16, true, kDense> : topk_adjust_kernel<kBf16, false, kDense>;
-  adjust<<<grid, 256, smem, s>>>(a, group);
-  e = cudaGetLastError();
+  e = launch(adjust, grid, 256, 1, smem, true, s, a, group);
   if (e != cudaSuccess) return e;
 
   auto select = topk_select_kernel<kBf16, kDense>;
@@ -1054,12 +1173,12 @@ cudaError_t run(const TopkArgs& t, const SelectArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   // no more than can meet (kWhole)
   const int clusters = static_cast<int>(std::min<int64_t>({128 / ctas, resident_clusters, (a.n + (1 << 20) - 1) >> 20}));
-  e = launch_cluster(select, clusters, ctas, kSubBins * sizeof(uint32_t), s, a);
+  e = launch(select, clusters * ctas, kThreads, ctas, kSubBins * sizeof(uint32_t), true, s, a);
   if (e != cudaSuccess) return e;
   const unsigned pgrid = static_cast<unsigned>(std::min<int64_t>(148, (run_count(a.n) + kWarps - 1) / kWarps));
-  topk_output_kernel<true, kBf16, kDense><<<pgrid, kThreads, 0, s>>>(a);
-  topk_output_kernel<false, kBf16, kDense><<<pgrid, kThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  e = launch(topk_output_kernel<true, kBf16, kDense>, pgrid, kThreads, 1, 0, true, s, a);
+  if (e != cudaSuccess) return e;
+  return launch(topk_output_kernel<false, kBf16, kDense>, pgrid, kThreads, 1, 0, true, s, a);
 }
 
 }  // namespace

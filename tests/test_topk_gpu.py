@@ -197,6 +197,75 @@ def test_select_where_the_sampled_bound_misses(native, cuda_device, one_rank, n,
     assert torch.equal(res.cpu(), comp.residual(0))
 
 
+def _misled(kind, n, ratio):
+    """Data whose sampled elements are smaller than the rest: more than k elements lie above the magnitude up to which the
+    first launch of a dense selection sends on its own."""
+    gen = torch.Generator().manual_seed(n)
+    if kind == "narrow":          # that magnitude and the k-th element's in one crowded bin; the sample is right
+        return 1 + 1e-6 * torch.randn(n, generator=gen)
+    s = torch.arange(65536, dtype=torch.int64)
+    stride = n // 65536
+    sampled = s * stride + ((((s * 2654435761) % 2 ** 32) >> 8) * stride >> 24)
+    k = int(n * ratio)
+    rest = torch.ones(n, dtype=torch.bool)
+    rest[sampled] = False
+    rest = rest.nonzero()[:, 0]
+    large = rest[torch.randperm(rest.numel(), generator=gen)[: int(1.15 * k)]]
+    g = 0.01 * torch.rand(n, generator=gen)
+    g[sampled] = 0.001 * torch.rand(65536, generator=gen)
+    some = sampled[torch.randperm(65536, generator=gen)[: int(1.5 * 65536 * ratio)]]
+    g[some] = 0.6 + 0.3 * torch.rand(some.numel(), generator=gen)
+    if kind == "octave":          # the k-th element within the histogram, its bin above that magnitude
+        g[large] = 1 + 0.3 * torch.rand(large.numel(), generator=gen)
+    elif kind == "far":           # beyond it
+        g[large] = 64 + torch.rand(large.numel(), generator=gen)
+    elif kind == "ties":
+        g[large] = 1.0
+    elif kind == "crowded":       # one bin, more entries than one block resolves
+        g[large] = 1 + 2.0 ** -23 * torch.randint(0, 5, (large.numel(),), generator=gen)
+    elif kind == "overflow":      # more than the list holds
+        g[rest] = 1 + torch.rand(rest.numel(), generator=gen)
+    return torch.where(torch.rand(n, generator=gen) < 0.5, -g, g)
+
+
+# What was sent too early is taken back: from the list, at the threshold's ties, where the list overflows.  Exact.
+@pytest.mark.parametrize("kind,n,ratio", [("octave", 1_000_003, 0.01), ("octave", 524_288, 0.1), ("far", 1_000_003, 0.01),
+                                          ("far", 3_000_000, 0.003), ("ties", 1_000_003, 0.01), ("crowded", 20_000_003, 0.01),
+                                          ("overflow", 1_000_003, 0.01), ("overflow", 700_001, 0.1),
+                                          ("narrow", 20_000_003, 0.01)])
+def test_dense_selection_where_the_upper_bound_misses(native, cuda_device, one_rank, kind, n, ratio):
+    g = _misled(kind, n, ratio)
+    comp, idx, val = _oracle_pairs(native, g, ratio)
+    want = torch.zeros(n)
+    want[torch.tensor(idx)] = torch.tensor(val) * 0.5
+    grad, res = g.to(cuda_device), torch.zeros(n, device=cuda_device)
+    one_rank.allreduce_topk(grad, res, ratio, 0.5).wait()
+    assert torch.equal(grad.cpu(), want)
+    assert torch.equal(res.cpu(), comp.residual(0))
+
+
+def test_dense_selections_side_by_side(cuda_device, one_rank):
+    # Both lanes at once: a grid that is not resident as a whole selects by one cluster, with what was sent early in the list.
+    n, ratio = 4_000_001, 0.01
+    gs = [_missing("two_scales", n, ratio).to(cuda_device), _misled("far", n, ratio).to(cuda_device)]
+
+    def run(wait_each):
+        grads, res = [g.clone() for g in gs], [torch.zeros_like(g) for g in gs]
+        works = []
+        for g, r in zip(grads, res):
+            works.append(one_rank.allreduce_topk(g, r, ratio, 1.0))
+            if wait_each:
+                works[-1].wait()
+        for w in works:
+            w.wait()
+        torch.cuda.synchronize()
+        return grads + res
+
+    want = run(True)
+    for _ in range(10):
+        assert all(torch.equal(a, b) for a, b in zip(run(False), want))
+
+
 def _time_us(fn, reset, runs=5):
     best = float("inf")
     for _ in range(runs):
