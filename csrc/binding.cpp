@@ -822,6 +822,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 
 #ifdef MCCL_WITH_STFT
   // ---- STFT / iSTFT ---------------------------------------------------------------------------------
+  m.def("_stft_direct", &stft_direct);
+  m.def("_istft_direct", &istft_direct);
   m.def("_stft_forward", &stft_forward, py::arg("waveform"), py::arg("window"), py::arg("n_fft"),
         py::arg("hop_length"), py::arg("win_length"), py::arg("center") = true, py::arg("normalized") = false,
         py::arg("backend") = "auto");

@@ -10,6 +10,7 @@
 
 #include "common/errors.h"
 #include "kernels/gemm_api.h"
+#include "ops/ordinary.h"
 
 namespace mccl {
 
@@ -43,20 +44,8 @@ void check_waits() {
     throw DeviceError("a wait inside a matrix product kernel ran out; results since then are undefined");
 }
 
-// A tensor as the kernels read it: memory on the device, nothing lazy, no wrapper (vmap, functorch, subclasses), no tangent.
-bool ordinary(const at::Tensor& t) {
-  using c10::DispatchKey;
-  constexpr auto allowed = c10::DispatchKeySet({DispatchKey::CUDA, DispatchKey::AutogradCUDA, DispatchKey::ADInplaceOrView,
-                                                DispatchKey::AutocastCUDA});
-  return t.defined() && allowed.isSupersetOf(t.key_set()) && t.scalar_type() == at::kFloat && !t._fw_grad(0).defined();
-}
-// No mode that wants to see the operators (Python modes, functorch transforms, functionalization).
-bool no_modes() {
-  const auto included = c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set;
-  return included.empty();
-}
 bool rows_ok(const at::Tensor& t) {
-  return t.dim() == 2 && t.numel() > 0 && t.stride(1) == 1 && (t.size(0) == 1 || t.stride(0) >= t.size(1));
+  return t.scalar_type() == at::kFloat && t.dim() == 2 && t.numel() > 0 && t.stride(1) == 1 && (t.size(0) == 1 || t.stride(0) >= t.size(1));
 }
 bool blackwell(int device) {
   const auto* p = at::cuda::getDeviceProperties(static_cast<c10::DeviceIndex>(device));
@@ -200,7 +189,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
                need_bias = ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2);
     // a second derivative, or tensors that are no longer what forward saw (a hook, vmap over the backward pass): operators
     // that autograd knows
-    if (at::GradMode::is_enabled() || !no_modes() || !ordinary(grad) || !ordinary(x) || !ordinary(w) || !rows_ok(x) ||
+    if (at::GradMode::is_enabled() || !no_modes() || !ordinary(grad) || grad.scalar_type() != at::kFloat || !ordinary(x) || !ordinary(w) || !rows_ok(x) ||
         !rows_ok(w) || x.device() != grad.device() || w.device() != grad.device())
       return {need_x ? grad.mm(w) : at::Tensor(), need_w ? grad.t().mm(x) : at::Tensor(),
               need_bias ? grad.sum(0) : at::Tensor()};
@@ -217,7 +206,7 @@ bool linear_native(const at::Tensor& x, const at::Tensor& w, const c10::optional
       x.device() != w.device())
     return false;
   if (bias && bias->defined() &&
-      (!ordinary(*bias) || bias->dim() != 1 || bias->size(0) != w.size(0) || bias->stride(0) != 1 || bias->device() != x.device()))
+      (!ordinary(*bias) || bias->scalar_type() != at::kFloat || bias->dim() != 1 || bias->size(0) != w.size(0) || bias->stride(0) != 1 || bias->device() != x.device()))
     return false;
   // a program that lets torch round its fp32 products has asked for something else
   if (at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA)) return false;

@@ -2,6 +2,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/custom_function.h>
 
 #include <algorithm>
 #include <cmath>
@@ -9,6 +10,7 @@
 
 #include "common/errors.h"
 #include "kernels/stft_api.h"
+#include "ops/ordinary.h"
 
 namespace mccl {
 
@@ -210,6 +212,72 @@ at::Tensor istft_backward(const at::Tensor& grad_waveform, const at::Tensor& win
   a.scale = (normalized ? std::sqrt(static_cast<float>(n_fft)) : 1.0f) / static_cast<float>(n_fft);
   STFT_CK(kern::launch_fft_frames(a, at::cuda::getCurrentCUDAStream()));
   return out.transpose(1, 2);
+}
+
+namespace {
+
+// n_fft, hop, win_length, center, normalized, and what the gradient's shape needs
+using Config = std::vector<int64_t>;
+
+at::Tensor forward_of(const at::Tensor& waveform, const at::Tensor& window, const Config& c) {
+  const at::Tensor x = waveform.dim() == 3 && waveform.size(1) == 1 ? waveform.squeeze(1) : waveform;
+  return stft_forward(x.contiguous().to(at::kFloat), window, c[0], c[1], c[2], c[3] != 0, c[4] != 0, "cuda");
+}
+at::Tensor inverse_of(const at::Tensor& spec, const at::Tensor& window, const Config& c) {
+  return istft_forward(spec, window, c[0], c[1], c[2], c[3] != 0, c[4] != 0, c[5], "cuda");
+}
+
+struct StftFn : torch::autograd::Function<StftFn> {
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& waveform, const at::Tensor& window,
+                            const Config& c) {
+    ctx->save_for_backward({window});
+    ctx->saved_data["config"] = c;
+    ctx->saved_data["shape"] = waveform.sizes().vec();
+    return forward_of(waveform, window, c);
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    const Config c = ctx->saved_data["config"].toIntVector(), shape = ctx->saved_data["shape"].toIntVector();
+    const at::Tensor g = stft_backward(grads[0], ctx->get_saved_variables()[0], c[0], c[1], c[2], c[3] != 0, c[4] != 0,
+                                       shape.back(), "cuda");
+    return {g.reshape(shape), at::Tensor(), at::Tensor()};
+  }
+};
+
+struct IstftFn : torch::autograd::Function<IstftFn> {
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& spec, const at::Tensor& window,
+                            const Config& c) {
+    ctx->save_for_backward({window});
+    ctx->saved_data["config"] = c;
+    ctx->saved_data["frames"] = spec.dim() > 0 ? spec.size(-1) : int64_t(0);
+    return inverse_of(spec, window, c);
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    const Config c = ctx->saved_data["config"].toIntVector();
+    const at::Tensor g = istft_backward(grads[0].contiguous(), ctx->get_saved_variables()[0], c[0], c[1], c[2], c[3] != 0,
+                                        c[4] != 0, ctx->saved_data["frames"].toInt(), "cuda");
+    return {g, at::Tensor(), at::Tensor()};
+  }
+};
+
+template <typename Fn, typename Run>
+c10::optional<at::Tensor> direct(const at::Tensor& t, const at::Tensor& window, const Config& c, Run&& run) {
+  if (!no_modes() || !ordinary(t) || !ordinary(window)) return c10::nullopt;
+  if (!at::GradMode::is_enabled() || !(t.requires_grad() || window.requires_grad())) return run(t, window, c);
+  return Fn::apply(t, window, c);
+}
+
+}  // namespace
+
+c10::optional<at::Tensor> stft_direct(const at::Tensor& waveform, const at::Tensor& window, int64_t n_fft, int64_t hop,
+                                      int64_t win_length, bool center, bool normalized) {
+  return direct<StftFn>(waveform, window, {n_fft, hop, win_length, center, normalized}, forward_of);
+}
+
+c10::optional<at::Tensor> istft_direct(const at::Tensor& spec, const at::Tensor& window, int64_t n_fft, int64_t hop,
+                                       int64_t win_length, int64_t length, bool center, bool normalized) {
+  return direct<IstftFn>(spec, window, {n_fft, hop, win_length, center, normalized, length}, inverse_of);
 }
 
 }  // namespace mccl

@@ -29,4 +29,11 @@ at::Tensor istft_backward(const at::Tensor& grad_waveform, const at::Tensor& win
                           int64_t hop_length, int64_t win_length, bool center, bool normalized, int64_t n_frames,
                           const std::string& backend);
 
+// The differentiable transforms.  None where autograd, tracing or a transform has more to see than a native function shows
+// (see ops/ordinary.h): the caller then takes the form that it knows.
+c10::optional<at::Tensor> stft_direct(const at::Tensor& waveform, const at::Tensor& window, int64_t n_fft, int64_t hop_length,
+                                      int64_t win_length, bool center, bool normalized);
+c10::optional<at::Tensor> istft_direct(const at::Tensor& spec, const at::Tensor& window, int64_t n_fft, int64_t hop_length,
+                                       int64_t win_length, int64_t length, bool center, bool normalized);
+
 }  // namespace mccl

@@ -15,6 +15,8 @@ from typing import Optional
 
 import torch
 
+from .. import require_native
+
 _ALIASES = {"metal": "cuda", "vdsp": "cpu"}
 _BACKENDS = frozenset({"cuda", "cpu", "auto"})
 
@@ -42,10 +44,17 @@ def _use_native(t: torch.Tensor, n_fft: int, backend: str) -> bool:
     return _native_ok(t, n_fft)
 
 
+# Without anything that has to see the call (tracing, compilation, a mode), autograd and the kernels are one native call: of
+# a pass of two seconds of stereo, forward and backward, these functions took 17 of 79 us, of one second of speech 6 of 14.
+# The classes below serve the rest.
+def _direct_ok(t: torch.Tensor) -> bool:
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and torch._C._get_tracing_state() is None
+            and not torch.compiler.is_compiling() and not torch._C._is_torch_function_mode_enabled())
+
+
 class _StftFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, waveform, window, n_fft, hop_length, win_length, center, normalized):
-        from .. import require_native
         native = require_native()
         ctx.in_shape = tuple(waveform.shape)
         x = waveform.squeeze(1) if waveform.dim() == 3 and waveform.size(1) == 1 else waveform
@@ -57,7 +66,6 @@ class _StftFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_spec):
-        from .. import require_native
         (window,) = ctx.saved_tensors
         n_fft, hop, win, center, normalized, length = ctx.cfg
         g = require_native()._stft_backward(grad_spec, window, n_fft, hop, win, center, normalized, length, "cuda")
@@ -67,7 +75,6 @@ class _StftFn(torch.autograd.Function):
 class _IstftFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, spec, window, n_fft, hop_length, win_length, length, center, normalized):
-        from .. import require_native
         ctx.save_for_backward(window)
         ctx.cfg = (int(n_fft), int(hop_length), int(win_length), bool(center), bool(normalized), int(spec.shape[-1]))
         return require_native()._istft_forward(spec, window, int(n_fft), int(hop_length), int(win_length),
@@ -75,7 +82,6 @@ class _IstftFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_waveform):
-        from .. import require_native
         (window,) = ctx.saved_tensors
         n_fft, hop, win, center, normalized, frames = ctx.cfg
         g = require_native()._istft_backward(grad_waveform.contiguous(), window, n_fft, hop, win, center,
@@ -87,6 +93,11 @@ def stft(waveform: torch.Tensor, *, n_fft: int, hop_length: int, win_length: int
          center: bool = True, normalized: bool = False, backend: str = "auto") -> torch.Tensor:
     """Complex one-sided STFT ``[batch, n_fft/2+1, frames]`` (torch.stft semantics, reflect padding)."""
     if _use_native(waveform, n_fft, backend):
+        if _direct_ok(waveform) and type(window) is torch.Tensor:
+            out = require_native()._stft_direct(waveform, window, int(n_fft), int(hop_length), int(win_length),
+                                                bool(center), bool(normalized))
+            if out is not None:
+                return out
         return _StftFn.apply(waveform, window, n_fft, hop_length, win_length, center, normalized)
     x = waveform.squeeze(1) if waveform.dim() == 3 and waveform.size(1) == 1 else waveform
     dev = x.device
@@ -101,6 +112,11 @@ def istft(spec: torch.Tensor, *, n_fft: int, hop_length: int, win_length: int, w
           center: bool = True, normalized: bool = False, backend: str = "auto") -> torch.Tensor:
     """Inverse STFT returning ``[batch, length]`` (torch.istft semantics)."""
     if _use_native(spec, n_fft, backend):
+        if _direct_ok(spec) and type(window) is torch.Tensor:
+            out = require_native()._istft_direct(spec, window, int(n_fft), int(hop_length), int(win_length), int(length),
+                                                 bool(center), bool(normalized))
+            if out is not None:
+                return out
         return _IstftFn.apply(spec, window, n_fft, hop_length, win_length, length, center, normalized)
     dev = spec.device
     s = spec.cpu() if resolve_backend(backend) == "cpu" else spec

@@ -297,3 +297,40 @@ def test_inverse_segments(native, n_fft, hop, fold):
             # a segment that has to hold a folded edge may need one more
             edges = -(-(reach + 1) // together) if fold else 0
             assert max(batches(a, b) for a, b in zip(begins, begins[1:])) <= max(bound, edges) or len(sizes) == 1
+
+
+# the one native call against the Python functions that it stands in for: bit for bit, over the forms that both take
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,dtype,window_grad", [((4000,), torch.float32, False), ((2, 4001), torch.float32, False),
+                                                     ((2, 1, 4001), torch.float32, True), ((3, 4000), torch.bfloat16, False)])
+def test_direct_calls_match_the_functions(shape, dtype, window_grad):
+    from mccl_b200.transforms import stft as module_fn  # noqa: F401  (the package exports the functions)
+    import importlib
+    mod = importlib.import_module("mccl_b200.transforms.stft")
+    torch.manual_seed(0)
+    x = torch.randn(*shape, device="cuda").to(dtype).requires_grad_()
+    win = torch.hann_window(400, device="cuda").requires_grad_(window_grad)
+    kw = dict(n_fft=512, hop_length=128, win_length=400, window=win)
+    native = mod.require_native()
+    got = mod.stft(x, **kw)
+    want = mod._StftFn.apply(x, win, 512, 128, 400, True, False)
+    g = torch.randn_like(want)
+    assert torch.equal(got, want) and got.requires_grad and got.stride() == want.stride()
+    assert torch.equal(torch.autograd.grad(got, x, g)[0], torch.autograd.grad(want, x, g)[0])
+    spec = want.detach().requires_grad_()
+    got = mod.istft(spec, length=4000, **kw)
+    want = mod._IstftFn.apply(spec, win, 512, 128, 400, 4000, True, False)
+    g = torch.randn_like(want)
+    assert torch.equal(got, want)
+    assert torch.equal(torch.autograd.grad(got, spec, g)[0], torch.autograd.grad(want, spec, g)[0])
+    with torch.no_grad():
+        assert torch.equal(mod.stft(x, **kw), mod.stft(x.detach(), **kw)) and not mod.stft(x, **kw).requires_grad
+    # what has more to see goes the other way: lazy views, tangents, transforms, a window on the host
+    conj = spec.detach().conj()
+    assert native._istft_direct(conj, win, 512, 128, 400, 4000, True, False) is None
+    assert native._stft_direct(x, win.detach().cpu(), 512, 128, 400, True, False) is None
+    assert torch.equal(mod.stft(x, **{**kw, "window": win.detach().cpu()}), mod.stft(x, **kw))
+    with pytest.raises(Exception):
+        torch.func.jvp(lambda t: mod.stft(t, **kw), (x,), (torch.ones_like(x),))
+    with pytest.raises(Exception):
+        torch.func.vmap(lambda t: mod.stft(t, **kw))(x.detach().expand(2, *shape))
