@@ -90,6 +90,19 @@ __host__ __device__ constexpr int bit_reverse(int v, int n) {
   return r;
 }
 
+// Sums and differences of complex numbers.  kPacked: both parts in one instruction, which rounds as two do and takes one issue
+// slot, but wants its numbers in pairs of registers.  Forward, 16 x 1 Mi samples, hop n_fft / 4, n_fft 512 .. 4096: 81, 88, 89,
+// 133 us without, 76, 82, 82, 118 with it; for the window, the split and the scale as well: 78, 84, 88, 119.
+template <bool kPacked>
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  if constexpr (kPacked) return __fadd2_rn(a, b);
+  else return make_float2(a.x + b.x, a.y + b.y);
+}
+template <bool kPacked>
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  if constexpr (kPacked) return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+  else return make_float2(a.x - b.x, a.y - b.y);
+}
 // d * exp(-2 pi i K / R)
 template <int K, int R>
 __device__ __forceinline__ float2 mul_root(float2 d) {
@@ -104,32 +117,34 @@ __device__ __forceinline__ float2 mul_root(float2 d) {
 // Forward FFT of v[O .. O + R), in place, decimation in frequency: X[k] ends up in v[O + bit_reverse(k, R)].
 // Radix 4 (a value meets one twiddle where two radix-2 stages would have two: fewer roundings and fewer
 // instructions), with a last radix-2 stage for odd powers of two.
-template <int R, int O, int N>
+template <bool kPacked, int R, int O, int N>
 __device__ __forceinline__ void fft_registers(float2 (&v)[N]) {
   if constexpr (R == 2) {
     const float2 p = v[O], q = v[O + 1];
-    v[O] = make_float2(p.x + q.x, p.y + q.y);
-    v[O + 1] = make_float2(p.x - q.x, p.y - q.y);
+    v[O] = add2<kPacked>(p, q);
+    v[O + 1] = sub2<kPacked>(p, q);
   } else if constexpr (R >= 4) {
     constexpr int Q = R / 4;
     static_for<0, Q>([&](auto jc) {
       constexpr int j = decltype(jc)::value;
       const float2 v0 = v[O + j], v1 = v[O + j + Q], v2 = v[O + j + 2 * Q], v3 = v[O + j + 3 * Q];
-      const float2 a0 = make_float2(v0.x + v2.x, v0.y + v2.y), a1 = make_float2(v0.x - v2.x, v0.y - v2.y);
-      const float2 a2 = make_float2(v1.x + v3.x, v1.y + v3.y), a3 = make_float2(v1.x - v3.x, v1.y - v3.y);
-      v[O + j] = make_float2(a0.x + a2.x, a0.y + a2.y);
-      v[O + j + Q] = mul_root<2 * j, R>(make_float2(a0.x - a2.x, a0.y - a2.y));
+      const float2 a0 = add2<kPacked>(v0, v2), a1 = sub2<kPacked>(v0, v2);
+      const float2 a2 = add2<kPacked>(v1, v3), a3 = sub2<kPacked>(v1, v3);
+      v[O + j] = add2<kPacked>(a0, a2);
+      v[O + j + Q] = mul_root<2 * j, R>(sub2<kPacked>(a0, a2));
       v[O + j + 2 * Q] = mul_root<j, R>(make_float2(a1.x + a3.y, a1.y - a3.x));
       v[O + j + 3 * Q] = mul_root<3 * j, R>(make_float2(a1.x - a3.y, a1.y + a3.x));
     });
-    fft_registers<Q, O>(v);
-    fft_registers<Q, O + Q>(v);
-    fft_registers<Q, O + 2 * Q>(v);
-    fft_registers<Q, O + 3 * Q>(v);
+    fft_registers<kPacked, Q, O>(v);
+    fft_registers<kPacked, Q, O + Q>(v);
+    fft_registers<kPacked, Q, O + 2 * Q>(v);
+    fft_registers<kPacked, Q, O + 3 * Q>(v);
   }
 }
 
-template <int LH>
+// kPacked: forward transforms; the kernel that shares its registers with an overlap-add
+// by the whole CTA loses more to the pairs than it gains (16 x 1 Mi samples, n_fft 2048, bins-major: 229 and 238 us).
+template <int LH, bool kPacked = true>
 struct WarpFft {
   static constexpr int h = 1 << LH, n = 2 * h;
   static constexpr int V = 1 << ((LH + 1) / 2);  // values per lane
@@ -152,7 +167,7 @@ struct WarpFft {
   // In: v[r] = z[r * L + t].  Out: Z[t + L * g + V * k] in v[at(g, k)].  `buf`: the frame's slot.
   __host__ __device__ static constexpr int at(int g, int k) { return g * L + bit_reverse(k, L); }
   static __device__ __forceinline__ void transform(float2 (&v)[V], const float2* tw, float2* buf, int t) {
-    fft_registers<V, 0>(v);
+    fft_registers<kPacked, V, 0>(v);
     static_for<0, V>([&](auto rc) {
       constexpr int r = decltype(rc)::value;
       float2 z = v[bit_reverse(r, V)];
@@ -168,8 +183,8 @@ struct WarpFft {
       v[i] = buf[(t + L * (i / L)) * (L + 1) + i % L];
     });
     __syncwarp();
-    fft_registers<L, 0>(v);
-    if constexpr (G == 2) fft_registers<L, L>(v);
+    fft_registers<kPacked, L, 0>(v);
+    if constexpr (G == 2) fft_registers<kPacked, L, L>(v);
   }
 
   static __device__ __forceinline__ float2 from_mirror_lane(float2 v, int t) {

@@ -228,7 +228,7 @@ template <int LH>
 __device__ __forceinline__ void inverse_frame(const IfftOlaArgs& a, const float2* spec, int64_t stride_f,
                                               const float2* tw, const float2* split, const float2* win2, float2* slot,
                                               int t) {
-  using F = WarpFft<LH>;
+  using F = WarpFft<LH, false>;
   // hermitian: inverse real FFT of the one-sided bins.  Otherwise the adjoint of the forward
   // transform, Re(sum_{k<=h} X[k] e^{+2 pi i k n / N}), which equals half the inverse real FFT of the
   // same bins with the real parts of DC and Nyquist doubled.
@@ -362,7 +362,7 @@ __device__ __forceinline__ void emit_row_pairs(const IfftOlaArgs& a, const float
 // 16 x 240007 samples, n_fft 1024, hop 256, bins-major spectrum (77 MB): 247 us, 55 us so.
 template <int LH>
 __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const IfftOlaArgs a, const OlaPlan pl) {
-  using F = WarpFft<LH>;
+  using F = WarpFft<LH, false>;
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* split = tw + F::h;
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const
 template <int LH>
 __global__ void __launch_bounds__(256, LH <= 8 ? 3 : LH <= 10 ? 2 : 1)
     ifft_frames_kernel(const IfftOlaArgs a, float* frames, int64_t total) {
-  using F = WarpFft<LH>;
+  using F = WarpFft<LH, false>;
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* split = tw + F::h;
