@@ -142,7 +142,7 @@ __device__ __forceinline__ void fft_registers(float2 (&v)[N]) {
   }
 }
 
-// kPacked: forward transforms; the kernel that shares its registers with an overlap-add
+// kPacked: forward transforms and the stream kernel (see stft.cu); the kernel that shares its registers with an overlap-add
 // by the whole CTA loses more to the pairs than it gains (16 x 1 Mi samples, n_fft 2048, bins-major: 229 and 238 us).
 template <int LH, bool kPacked = true>
 struct WarpFft {
@@ -181,6 +181,34 @@ struct WarpFft {
     static_for<0, V>([&](auto ic) {
       constexpr int i = decltype(ic)::value;
       v[i] = buf[(t + L * (i / L)) * (L + 1) + i % L];
+    });
+    __syncwarp();
+    fft_registers<kPacked, L, 0>(v);
+    if constexpr (G == 2) fft_registers<kPacked, L, L>(v);
+  }
+
+  // The same with half the shared memory: real parts first, then imaginary ones, in a slot of kHalfSlot floats.  (Where several
+  // frames share a warp their slots start on different banks.)
+  static constexpr int kHalfSlot = V * (L + 1) + (L == 16 && V == 32 ? 16 : L == 8 && V == 16 ? 8 : 0);
+  static __device__ __forceinline__ void transform_halves(float2 (&v)[V], const float2* tw, float* buf, int t) {
+    fft_registers<kPacked, V, 0>(v);
+    static_for<1, V>([&](auto rc) {
+      constexpr int r = decltype(rc)::value, at = bit_reverse(r, V);
+      const float2 z = v[at], w = tw[r * L + t];
+      v[at] = make_float2(z.x * w.x - z.y * w.y, z.x * w.y + z.y * w.x);
+    });
+    static_for<0, V>([&](auto rc) { buf[decltype(rc)::value * (L + 1) + t] = v[bit_reverse(decltype(rc)::value, V)].x; });
+    __syncwarp();
+    static_for<0, V>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      v[i].x = buf[(t + L * (i / L)) * (L + 1) + i % L];
+    });
+    __syncwarp();
+    static_for<0, V>([&](auto rc) { buf[decltype(rc)::value * (L + 1) + t] = v[bit_reverse(decltype(rc)::value, V)].y; });
+    __syncwarp();
+    static_for<0, V>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      v[i].y = buf[(t + L * (i / L)) * (L + 1) + i % L];
     });
     __syncwarp();
     fft_registers<kPacked, L, 0>(v);

@@ -361,19 +361,9 @@ __device__ __forceinline__ void emit_row_pairs(const IfftOlaArgs& a, const float
 // by a second kernel, 144 us so.
 // 16 x 240007 samples, n_fft 1024, hop 256, bins-major spectrum (77 MB): 247 us, 55 us so.
 template <int LH>
-__global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const IfftOlaArgs a, const OlaPlan pl) {
+__device__ __forceinline__ void ola_rows(const IfftOlaArgs& a, const OlaPlan& pl, const float2* tw, const float2* split, const float* win,
+                                         float2* slots, int b, int64_t row0, int64_t row1, bool at_edge) {
   using F = WarpFft<LH, false>;
-  extern __shared__ float2 smem[];
-  float2* tw = smem;
-  float2* split = tw + F::h;
-  float* win = reinterpret_cast<float*>(split + F::h / 2);
-  float2* slots = reinterpret_cast<float2*>(win + F::n);
-  F::fill_tables(tw, split);
-  for (int j = threadIdx.x; j < F::n; j += blockDim.x) win[j] = window_at(a.window, j);
-  __syncthreads();
-
-  const int b = blockIdx.x / pl.segments, seg = blockIdx.x % pl.segments;
-  const int64_t row0 = pl.row_base + pl.begin(seg), row1 = pl.row_base + pl.begin(seg + 1);
   const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane / F::L, t = lane % F::L;
   const int batch = warps * F::kPerWarp;             // frames transformed together
@@ -382,7 +372,6 @@ __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const
   const float2* spec = reinterpret_cast<const float2*>(a.spec) + b * a.stride_b;
   float* out = a.out + b * a.out_len;
   const int64_t T = a.out_len;
-  const bool at_edge = a.fold_reflect && (seg == 0 || seg == pl.segments - 1);
   const bool direct = a.stride_f == 1;
 
   int64_t f0 = f_begin, e0 = row0;
@@ -476,11 +465,181 @@ __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const
   }
 }
 
+template <int LH>
+__global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const IfftOlaArgs a, const OlaPlan pl) {
+  using F = WarpFft<LH>;
+  extern __shared__ float2 smem[];
+  float2* tw = smem;
+  float2* split = tw + F::h;
+  float* win = reinterpret_cast<float*>(split + F::h / 2);
+  float2* slots = reinterpret_cast<float2*>(win + F::n);
+  F::fill_tables(tw, split);
+  for (int j = threadIdx.x; j < F::n; j += blockDim.x) win[j] = window_at(a.window, j);
+  __syncthreads();
+  const int b = blockIdx.x / pl.segments, seg = blockIdx.x % pl.segments;
+  ola_rows<LH>(a, pl, tw, split, win, slots, b, pl.row_base + pl.begin(seg), pl.row_base + pl.begin(seg + 1),
+               a.fold_reflect && (seg == 0 || seg == pl.segments - 1));
+}
+
+// sum of window^2 over the frames that cover sample j of row `row`
+__device__ __forceinline__ float row_envelope(const float* win, int n_fft, int hop, int n_frames, int64_t row, int j) {
+  float e = 0.f;
+  const int i_hi = row * hop + j < n_fft ? static_cast<int>(row) : (n_fft - 1 - j) / hop;
+  for (int i = i_hi; i >= 0; --i)  // frame row - i, in frame order
+    if (row - i < n_frames) e += win[j + i * hop] * win[j + i * hop];
+  return e;
+}
+
+// Spectrum -> signal, frames-major spectra of long signals.  A lane's samples of one frame are its own samples of the next
+// frame as well, hop / 2L registers further down (hop is a multiple of 2L).  So a lane group walks a run of frames by itself:
+// what later frames will add to stays in its lanes' own places in shared memory, every frame finishes one row, and nothing
+// waits for another warp until the end, when each group adds what it has left to the rows that the next one opened.  Only
+// the first group of a CTA repeats the reach - 1 frames before its rows.
+// pl.edge rows at a folded end are left to ola_rows in the first and the last CTA of a batch entry.
+template <int LH, bool kNorm>
+__global__ void __launch_bounds__(512, 1) ifft_stream_kernel(IfftOlaArgs a, const OlaPlan pl) {
+  using F = WarpFft<LH>;
+  extern __shared__ float2 smem[];
+  float2* tw = smem;
+  float2* split = tw + F::h;
+  float* win = reinterpret_cast<float*>(split + F::h / 2);
+  float* env = win + F::n;  // of a row that a full set of frames covers
+  float2* slots = reinterpret_cast<float2*>(env + (kNorm ? a.hop : 0));
+  F::fill_tables(tw, split);
+  for (int j = threadIdx.x; j < F::n; j += blockDim.x) win[j] = window_at(a.window, j);
+  __syncthreads();
+  const float edge = a.hermitian ? 1.0f : 2.0f, post = a.hermitian ? a.scale : 0.5f * a.scale;
+  if (!kNorm) {  // the window serves nothing else: it takes the scale
+    for (int j = threadIdx.x; j < F::n; j += blockDim.x) win[j] *= post;
+    a.scale = a.hermitian ? 1.0f : 2.0f;
+    __syncthreads();
+  }
+  if (kNorm) {
+    for (int j = threadIdx.x; j < a.hop; j += blockDim.x)
+      env[j] = row_envelope(win, F::n, a.hop, a.n_frames, pl.reach - 1, j);
+    __syncthreads();
+  }
+  const int b = blockIdx.x / pl.segments, seg = blockIdx.x % pl.segments;
+  int64_t r0 = pl.row_base + pl.rows * seg / pl.segments, r1 = pl.row_base + pl.rows * (seg + 1) / pl.segments;
+  if (pl.edge > 0 && seg == 0) {
+    ola_rows<LH>(a, pl, tw, split, win, slots, b, r0, r0 + pl.edge, true);
+    r0 += pl.edge;
+    __syncthreads();
+  }
+  if (pl.edge > 0 && seg == pl.segments - 1) r1 -= pl.edge;
+
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+  const int t = lane % F::L, group = warp * F::kPerWarp + lane / F::L, groups = warps * F::kPerWarp;
+  const int done = a.hop / (2 * F::L), kept = F::V - done;  // registers of a lane that a frame finishes, and leaves open
+  float* buf = reinterpret_cast<float*>(slots) + group * F::kHalfSlot;
+  float2* open = reinterpret_cast<float2*>(reinterpret_cast<float*>(slots) + groups * F::kHalfSlot) + group * kept * F::L + t;
+  const int warm = r0 < pl.reach - 1 ? static_cast<int>(r0) : pl.reach - 1;
+  const int steps = static_cast<int>(r1 - r0) + warm, each = (steps + groups - 1) / groups;
+  const int64_t first = r0 - warm + static_cast<int64_t>(group) * each;
+  const int count = max(0, min(each, steps - group * each));
+  const float2* spec = reinterpret_cast<const float2*>(a.spec) + b * a.stride_b;
+  float* out = a.out + b * a.out_len;
+  const float2* win2 = reinterpret_cast<const float2*>(win) + t;
+  // One pair of finished samples; `raw`: another group has more to add.
+  auto put = [&](int64_t row, int64_t q0, int j, float2 v, bool raw) {
+    if (kNorm && !raw) {
+      const bool full = row >= pl.reach - 1 && row < a.n_frames;
+      const float2 e = full ? *reinterpret_cast<const float2*>(env + j)
+                            : make_float2(row_envelope(win, F::n, a.hop, a.n_frames, row, j),
+                                          row_envelope(win, F::n, a.hop, a.n_frames, row, j + 1));
+      v.x = e.x > 1e-11f ? v.x / e.x : 0.f;
+      v.y = e.y > 1e-11f ? v.y / e.y : 0.f;
+    }
+    const int64_t q = q0 + j;
+    if (q >= 0 && q + 1 < a.out_len && (reinterpret_cast<uintptr_t>(out + q) & 7) == 0) {
+      *reinterpret_cast<float2*>(out + q) = v;
+    } else {
+      if (q >= 0 && q < a.out_len) out[q] = v.x;
+      if (q + 1 >= 0 && q + 1 < a.out_len) out[q + 1] = v.y;
+    }
+  };
+  for (int r = 0; r < kept; ++r) open[r * F::L] = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int i = 0; i < each; ++i) {
+    const int64_t row = first + i;
+    const bool live = i < count, framed = live && row < a.n_frames;
+    float2 x[F::V];
+    if (__any_sync(0xFFFFFFFFu, framed)) {
+      const float2* from = spec + (framed ? row : a.n_frames - 1) * a.stride_t;
+#pragma unroll
+      for (int r = 0; r < F::V; ++r) x[r] = from[r * F::L + t];
+      const float2 nyquist = from[F::h];
+      if (LH >= 10 && i + 1 < count && row + 1 < a.n_frames)
+        for (int k = 16 * t; k <= F::h; k += 16 * F::L) prefetch_l2(from + a.stride_t + k);
+      F::merge_bins(x, nyquist, split, t, edge);
+      F::transform_halves(x, tw, buf, t);
+    }
+    const int64_t q0 = row * a.hop - a.pad;
+    const bool emits = live && row >= r0;
+    // a whole row of aligned pairs with nothing more to come and (kNorm) a full set of frames; others go through `put`
+    const bool plain = emits && q0 >= 0 && q0 + a.hop <= a.out_len && (reinterpret_cast<uintptr_t>(out + q0) & 7) == 0 &&
+                       (group == 0 || i * done >= kept) && (!kNorm || (row >= pl.reach - 1 && row < a.n_frames));
+    float2* to = reinterpret_cast<float2*>(out + q0) + t;
+    float2* later = reinterpret_cast<float2*>(buf) + t;
+    const float2* before = open;
+    if (!framed) {
+#pragma unroll
+      for (int r = 0; r < F::V; ++r) x[r] = make_float2(0.f, 0.f);
+    }
+    static_for<0, F::V>([&](auto rc) {
+      constexpr int r = decltype(rc)::value, g = r % F::G, k2 = r / F::G;
+      const float2 z = x[F::at(g, k2)], w = win2[r * F::L];
+      float2 y = kNorm ? make_float2(z.y * post * w.x, z.x * post * w.y) : make_float2(z.y * w.x, z.x * w.y);
+      if (r < F::V / 2 || r < kept) {  // at the first frame the open places hold zeros
+        const float2 sum = before[r * F::L];
+        y = add2<true>(sum, y);
+      }
+      if (r < F::V / 2 && r < done) {
+        if (plain) {
+          if (kNorm) {
+            const float2 e = reinterpret_cast<const float2*>(env)[r * F::L + t];
+            y = make_float2(e.x > 1e-11f ? y.x / e.x : 0.f, e.y > 1e-11f ? y.y / e.y : 0.f);
+          }
+          to[r * F::L] = y;
+        } else {
+          later[r * F::L] = y;
+        }
+      } else if (live) {
+        open[(r - done) * F::L] = y;
+      }
+    });
+    if (emits && !plain)
+#pragma unroll 1
+      for (int r = 0; r < done; ++r) put(row, q0, 2 * (r * F::L + t), later[r * F::L], group > 0 && i * done + r < kept);
+  }
+  __syncthreads();
+  // what this group's frames add to the rows that the next group has opened
+  if (count == each && first + each < r1) {
+    int64_t row = first + each;
+    int at = 0;
+#pragma unroll 1
+    for (int r = 0; r < kept && row < r1; ++r) {
+      const int64_t q0 = row * a.hop - a.pad;
+      const int j = 2 * (at * F::L + t);
+      const int64_t q = q0 + j;
+      float2 v = open[r * F::L];
+      if (q >= 0 && q < a.out_len) v.x += out[q];
+      if (q + 1 >= 0 && q + 1 < a.out_len) v.y += out[q + 1];
+      put(row, q0, j, v, false);
+      if (++at == done) at = 0, ++row;
+    }
+  }
+  if (pl.edge > 0 && seg == pl.segments - 1) {
+    __syncthreads();
+    ola_rows<LH>(a, pl, tw, split, win, slots, b, r1, r1 + pl.edge, true);
+  }
+}
+
 // Spectrum -> windowed frames in global memory (only where ifft_ola_kernel cannot run).
 template <int LH>
 __global__ void __launch_bounds__(256, LH <= 8 ? 3 : LH <= 10 ? 2 : 1)
     ifft_frames_kernel(const IfftOlaArgs a, float* frames, int64_t total) {
-  using F = WarpFft<LH, false>;
+  using F = WarpFft<LH>;
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* split = tw + F::h;
@@ -674,6 +833,49 @@ OlaGrid ola_grid(const IfftOlaArgs& a) {
   return g;
 }
 
+// The stream kernel's geometry; threads == 0: not for this problem.  It wants runs of frames that are long against what two
+// neighbours share.
+template <int LH>
+OlaGrid stream_grid(const IfftOlaArgs& a) {
+  using F = WarpFft<LH>;
+  OlaGrid g;
+  if (LH < 6 || a.stride_f != 1 || a.hop % (2 * F::L) != 0 || a.hop > F::n / 2) return g;
+  const OlaGrid rows = ola_grid<LH>(a);
+  if (rows.threads == 0) return g;
+  const bool fold = a.fold_reflect != 0;
+  // 16 x 1 Mi samples, hop n_fft / 4, backward, batches and streams: n_fft 256 166 and 121 us, 512 131 and 110, 2048 144 and
+  // 140 (inverse 156 and 146); but 1024 133 and 145, 4096 185 and 218: two frames per warp in 128 registers, and half the warps
+  if (LH == 9 || LH == 11) return g;
+  constexpr int warps = 16, groups = warps * F::kPerWarp;
+  g.plan = rows.plan;
+  OlaPlan& pl = g.plan;
+  pl.edge = fold ? pl.reach + 1 : 0;
+  pl.ring = groups + pl.reach - 1;
+  const int64_t most = std::max<int64_t>(1, kSms / a.batch);
+  const int64_t least = 3ll * (pl.reach - 1) * groups + 2 * pl.edge;  // rows of a CTA
+  pl.segments = static_cast<int>(std::min<int64_t>(most, pl.rows / std::max<int64_t>(1, least)));
+  if (pl.segments < 1 || (pl.segments < most && static_cast<int64_t>(pl.segments) * a.batch < kSms * 3 / 4)) return g;
+  const size_t kept = F::V - a.hop / (2 * F::L);
+  const size_t stream = groups * (F::kHalfSlot * sizeof(float) + kept * F::L * sizeof(float2)) +
+                        (a.normalize_envelope ? a.hop * sizeof(float) : 0);
+  const size_t edges = fold ? static_cast<size_t>(pl.ring) * F::kSlot * sizeof(float2) : 0;
+  g.smem = table_bytes<LH>() + std::max(stream, edges);
+  if (g.smem > kMaxSmem) return g;
+  g.threads = 32 * warps;
+  return g;
+}
+
+template <int LH>
+cudaError_t run_ifft_stream(const IfftOlaArgs& a, const OlaGrid& g, cudaStream_t s) {
+  static std::atomic<uint64_t> smem_set[2] = {};
+  const int norm = a.normalize_envelope ? 1 : 0;
+  const auto kernel = norm ? ifft_stream_kernel<LH, true> : ifft_stream_kernel<LH, false>;
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem_set[norm]);
+  if (e != cudaSuccess) return e;
+  kernel<<<static_cast<unsigned>(g.plan.segments) * a.batch, g.threads, g.smem, s>>>(a, g.plan);
+  return cudaGetLastError();
+}
+
 template <int LH>
 cudaError_t run_ifft_ola(const IfftOlaArgs& a, const OlaGrid& g, cudaStream_t s) {
   static std::atomic<uint64_t> smem_set{0};
@@ -739,6 +941,14 @@ int64_t ifft_ola_scratch(const IfftOlaArgs& a) {
 
 cudaError_t launch_ifft_ola(const IfftOlaArgs& a, float* scratch, cudaStream_t s) {
   if (!valid(a)) return cudaErrorInvalidValue;
+  const OlaGrid stream = for_size<OlaGrid>(a.n_fft, [&](auto lh) { return stream_grid<decltype(lh)::value>(a); });
+  if (stream.threads > 0) {
+    note_launch();
+    return for_size<cudaError_t>(a.n_fft, [&](auto lh) -> cudaError_t {
+      if constexpr (decltype(lh)::value >= 6 && decltype(lh)::value != 9 && decltype(lh)::value != 11) return run_ifft_stream<decltype(lh)::value>(a, stream, s);
+      return cudaErrorInvalidValue;
+    });
+  }
   const OlaGrid g = ola_grid_for(a);
   if (g.threads > 0) {
     note_launch();

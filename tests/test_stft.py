@@ -334,3 +334,40 @@ def test_direct_calls_match_the_functions(shape, dtype, window_grad):
         torch.func.jvp(lambda t: mod.stft(t, **kw), (x,), (torch.ones_like(x),))
     with pytest.raises(Exception):
         torch.func.vmap(lambda t: mod.stft(t, **kw))(x.detach().expand(2, *shape))
+
+
+# Long frames-major signals walk their frames in streams: every frame size that does, hops of a half, a quarter and five
+# sixteenths, rows off 8 bytes (odd lengths), edges that fold, missing neighbours, more and fewer samples than the frames cover.
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_fft,hop,batch,samples,center", [
+    (128, 32, 16, 300_001, True), (256, 64, 16, 400_003, True), (256, 80, 5, 1_048_575, False), (512, 128, 16, 400_000, True),
+    (512, 256, 3, 2_000_001, True), (2048, 512, 16, 1_000_001, True), (2048, 640, 2, 9_000_000, False),
+    (2048, 1024, 8, 2_000_003, True),
+])
+def test_streamed_inverse_matches_64_bits(n_fft, hop, batch, samples, center):
+    torch.manual_seed(0)
+    win = torch.hann_window(n_fft - n_fft // 8, device="cuda")
+    x = torch.randn(batch, samples, device="cuda", requires_grad=True)
+    kw = dict(n_fft=n_fft, hop_length=hop, win_length=win.numel(), window=win, center=center)
+    spec = stft(x, **kw)
+    g = torch.randn(spec.shape[0], spec.shape[2], spec.shape[1], dtype=torch.complex64, device="cuda").transpose(1, 2)
+    (grad,) = torch.autograd.grad(spec, x, g)
+    padded = torch.nn.functional.pad(win.double(), (n_fft // 16, n_fft // 16))
+    kw64 = dict(n_fft=n_fft, hop_length=hop, window=padded, center=center)
+    x64 = x.detach().double().requires_grad_()
+    spec64 = torch.stft(x64, pad_mode="reflect", return_complex=True, **kw64)
+    (grad64,) = torch.autograd.grad(spec64, x64, g.to(torch.complex128))
+
+    def close(got, want):  # a few roundings of 2^-24 per radix and per frame, against the result's size
+        assert (got.double() - want).norm() <= 4e-7 * want.norm() and (got.double() - want).abs().max() <= 4e-6 * want.abs().max()
+
+    close(grad, grad64)
+    if not center:
+        return
+    for length in (samples, samples + 3 * n_fft + 1, samples - 5 * hop - 3):
+        got = istft(g, length=length, **kw)
+        cover = istft(torch.ones_like(g), length=length, **kw)  # torch refuses what no frame covers
+        want = torch.istft(g.to(torch.complex128), length=min(length, samples), **kw64)
+        close(got[:, :want.shape[1] - n_fft], want[:, :want.shape[1] - n_fft])
+        end = (g.shape[2] - 1) * hop + n_fft // 2
+        assert torch.isfinite(got).all() and (length <= end or not got[:, end:].any()) and cover.shape == got.shape
