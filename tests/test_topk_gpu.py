@@ -161,6 +161,29 @@ def test_select_and_dense_paths_match_host_oracle(native, cuda_device, one_rank,
     assert torch.equal(res.cpu(), comp.residual(0))
 
 
+# k at the end of a run of equal magnitudes, where the radix select stops early, one before and one behind; the runs differ in
+# the first, the second and the third digit, and the last one is zeros.  Exact.
+@pytest.mark.parametrize("k", [99, 100, 101, 250, 299, 300, 301, 600, 601, 999, 1000])
+@pytest.mark.parametrize("n", [1000, 20_000])
+def test_selection_at_the_end_of_a_run(native, cuda_device, one_rank, n, k):
+    gen = torch.Generator().manual_seed(k)
+    g = torch.zeros(n)
+    g[:1000] = torch.tensor([8.0] * 100 + [1.0 + 2.0 ** -11] * 200 + [1.0 + 2.0 ** -22] * 300 + [0.0] * 400)
+    g = torch.where(torch.rand(n, generator=gen) < 0.5, -g, g)[torch.randperm(n, generator=gen)]
+    ratio = k / n
+    comp, idx, val = _oracle_pairs(native, g, ratio)
+    assert len(idx) == k
+    res = torch.zeros(n, device=cuda_device)
+    pairs = native._topk_select(g.to(cuda_device), res, ratio).cpu()
+    assert torch.equal(pairs[:, 0].long(), torch.tensor(idx))
+    assert torch.equal(res.cpu(), comp.residual(0))
+    grad, res = g.to(cuda_device), torch.zeros(n, device=cuda_device)
+    one_rank.allreduce_topk(grad, res, ratio, 0.5).wait()
+    want = torch.zeros(n)
+    want[torch.tensor(idx)] = torch.tensor(val) * 0.5
+    assert torch.equal(grad.cpu(), want) and torch.equal(res.cpu(), comp.residual(0))
+
+
 def _missing(kind, n, ratio):
     """Data for which the k-th element lies outside what the sampled magnitude bounds."""
     gen = torch.Generator().manual_seed(n)
