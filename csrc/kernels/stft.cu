@@ -362,7 +362,7 @@ __device__ __forceinline__ void emit_row_pairs(const IfftOlaArgs& a, const float
 // 16 x 240007 samples, n_fft 1024, hop 256, bins-major spectrum (77 MB): 247 us, 55 us so.
 template <int LH>
 __device__ __forceinline__ void ola_rows(const IfftOlaArgs& a, const OlaPlan& pl, const float2* tw, const float2* split, const float* win,
-                                         float2* slots, int b, int64_t row0, int64_t row1, bool at_edge) {
+                                         float2* slots, int b, int64_t row0, int64_t row1, int seg) {
   using F = WarpFft<LH, false>;
   const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane / F::L, t = lane % F::L;
@@ -372,6 +372,7 @@ __device__ __forceinline__ void ola_rows(const IfftOlaArgs& a, const OlaPlan& pl
   const float2* spec = reinterpret_cast<const float2*>(a.spec) + b * a.stride_b;
   float* out = a.out + b * a.out_len;
   const int64_t T = a.out_len;
+  const bool at_edge = a.fold_reflect && (seg == 0 || seg == pl.segments - 1);
   const bool direct = a.stride_f == 1;
 
   int64_t f0 = f_begin, e0 = row0;
@@ -477,8 +478,7 @@ __global__ void __launch_bounds__(LH >= 11 ? 256 : 512, 1) ifft_ola_kernel(const
   for (int j = threadIdx.x; j < F::n; j += blockDim.x) win[j] = window_at(a.window, j);
   __syncthreads();
   const int b = blockIdx.x / pl.segments, seg = blockIdx.x % pl.segments;
-  ola_rows<LH>(a, pl, tw, split, win, slots, b, pl.row_base + pl.begin(seg), pl.row_base + pl.begin(seg + 1),
-               a.fold_reflect && (seg == 0 || seg == pl.segments - 1));
+  ola_rows<LH>(a, pl, tw, split, win, slots, b, pl.row_base + pl.begin(seg), pl.row_base + pl.begin(seg + 1), seg);
 }
 
 // sum of window^2 over the frames that cover sample j of row `row`
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(512, 1) ifft_stream_kernel(IfftOlaArgs a, cons
   const int b = blockIdx.x / pl.segments, seg = blockIdx.x % pl.segments;
   int64_t r0 = pl.row_base + pl.rows * seg / pl.segments, r1 = pl.row_base + pl.rows * (seg + 1) / pl.segments;
   if (pl.edge > 0 && seg == 0) {
-    ola_rows<LH>(a, pl, tw, split, win, slots, b, r0, r0 + pl.edge, true);
+    ola_rows<LH>(a, pl, tw, split, win, slots, b, r0, r0 + pl.edge, seg);
     r0 += pl.edge;
     __syncthreads();
   }
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(512, 1) ifft_stream_kernel(IfftOlaArgs a, cons
   }
   if (pl.edge > 0 && seg == pl.segments - 1) {
     __syncthreads();
-    ola_rows<LH>(a, pl, tw, split, win, slots, b, r1, r1 + pl.edge, true);
+    ola_rows<LH>(a, pl, tw, split, win, slots, b, r1, r1 + pl.edge, seg);
   }
 }
 
@@ -844,7 +844,7 @@ OlaGrid stream_grid(const IfftOlaArgs& a) {
   if (rows.threads == 0) return g;
   const bool fold = a.fold_reflect != 0;
   // 16 x 1 Mi samples, hop n_fft / 4, backward, batches and streams: n_fft 256 166 and 121 us, 512 131 and 110, 2048 144 and
-  // 140 (inverse 156 and 146); but 1024 133 and 145, 4096 185 and 218: two frames per warp in 128 registers, and half the warps
+  // 136 (inverse 156 and 152); but 1024 133 and 145, 4096 185 and 218: two frames per warp in 128 registers, and half the warps
   if (LH == 9 || LH == 11) return g;
   constexpr int warps = 16, groups = warps * F::kPerWarp;
   g.plan = rows.plan;
