@@ -43,7 +43,8 @@ struct SplitJob {
   int tile;
   void* by_rows;
 };
-// Up to two matrices in one launch; column sums of the first to `sums` unless null; `zeroed` 32-bit words set to zero.
+// Up to two matrices in one launch: the first is the products' `b` (cut at half its value), the second an `a`; column sums of
+// the first to `sums` unless null; `zeroed` 32-bit words set to zero.
 cudaError_t launch_split_f32(const SplitJob* jobs, int n, float* sums, uint32_t* zero, int64_t zeroed, cudaStream_t s);
 
 // `weight`: fp32, of kForward and kInput; kWeight reads a_image in its place.  `c`: rows of ldc numbers.

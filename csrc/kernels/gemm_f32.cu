@@ -1,13 +1,16 @@
 // fp32 matrix products on the fifth-generation tensor cores (sm_100a).
 //
-// A float is the sum of three bf16 numbers: hi its upper 8 significant bits (cut off), mid the next 8 (rounded), lo what
-// is left, exactly.  A product of two floats is six bf16 products (hi hi; hi mid + mid hi; hi lo + mid mid + lo hi), what
-// is left out being below 2^-24 of it.  mid and lo are stored 2^7 and 2^14 times as large, so that they keep all their bits
-// wherever the float is normal, and every order of magnitude has an accumulator of its own in tensor memory:
-//     c = acc0 + 2^-7 (acc1 + 2^-7 acc2)
+// A float is the sum of three bf16 numbers: hi its upper 8 significant bits (rounded to nearest, or cut off where that would
+// overflow), mid the next 8 (rounded), lo what is left, exactly.  A product of two floats is six bf16 products (hi hi; hi mid +
+// mid hi; hi lo + mid mid + lo hi); what is left out is below 2^-24 of it.  mid and lo are stored 2^7 and 2^14 times as large, so
+// that they keep all their bits from 2^-123 on, and every order of magnitude has an accumulator of its own in tensor memory:
+//     c = 2 (acc0 + 2^-7 (acc1 + 2^-7 acc2))
 // The tensor cores cut off their sums, which a long chain shows: acc0 is taken out and added in registers, rounded to
 // nearest, every kGroup stages of the reduction.  Infinities and NaN come out of acc0 as they would out of a
-// multiplication; where it holds one the other two, which may hold inf - inf, are left out.
+// multiplication; where it holds one the other two, which may hold inf - inf, are left out.  Finite results never overflow on
+// the way: `b` takes part with half its value, so that hi hi, which may be 2^-7 above its product, has room, and mid as
+// stored is at most half of hi, so the terms of acc1 are no larger than those of acc0.
+// (With hi cut off everywhere mid was up to all of hi: what was left out came to 2^-22, and acc1 overflowed at half of FLT_MAX.)
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -31,6 +34,7 @@ constexpr int kAhead = 3;                 // stages of `a` that a producer holds
 constexpr int kAdders = 256, kIssuer = kAdders / 32, kProducer0 = kAdders + 32;
 constexpr int kProducers = 256;           // where `a` is read as it is; one warp otherwise
 constexpr float kUnscale = 1.0f / 128.0f;
+constexpr float kMostBf16 = 0x1.FEp127f;
 constexpr int kPartA = kRows * kDepth * 2;
 
 // ---- PTX ----------------------------------------------------------------------------------------------------
@@ -107,11 +111,14 @@ __device__ __forceinline__ bool elect() {
   return one != 0;
 }
 
-// Two floats into three bf16 pairs.
-__device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(x1), "f"(x0));
-  const float r0 = (x0 - __uint_as_float(hi << 16)) * 128.0f;
-  const float r1 = (x1 - __uint_as_float(hi & 0xFFFF0000u)) * 128.0f;
+// Two floats' leading bf16 parts, those of y rounded to nearest, and what they leave of x, 2^7 times as large.
+__device__ __forceinline__ void lead2(float y0, float y1, float x0, float x1, uint32_t& hi, float& r0, float& r1) {
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(y1), "f"(y0));
+  r0 = (x0 - __uint_as_float(hi << 16)) * 128.0f;
+  r1 = (x1 - __uint_as_float(hi & 0xFFFF0000u)) * 128.0f;
+}
+// The rest as two bf16 pairs.
+__device__ __forceinline__ void rest2(float r0, float r1, uint32_t& mid, uint32_t& lo) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(r1), "f"(r0));
   const float s0 = (r0 - __uint_as_float(mid << 16)) * 128.0f;
   const float s1 = (r1 - __uint_as_float(mid & 0xFFFF0000u)) * 128.0f;
@@ -141,12 +148,28 @@ __device__ __forceinline__ void load8(const float* data, int64_t ld, int64_t row
 struct Split8 {
   uint4 part[3];
 };
+__device__ __forceinline__ void lead8(const float (&y)[8], const float (&x)[8], uint4& hi, float (&r)[8]) {
+  lead2(y[0], y[1], x[0], x[1], hi.x, r[0], r[1]);
+  lead2(y[2], y[3], x[2], x[3], hi.y, r[2], r[3]);
+  lead2(y[4], y[5], x[4], x[5], hi.z, r[4], r[5]);
+  lead2(y[6], y[7], x[6], x[7], hi.w, r[6], r[7]);
+}
 __device__ __forceinline__ Split8 split8(const float (&v)[8]) {
   Split8 s;
-  split2(v[0], v[1], s.part[0].x, s.part[1].x, s.part[2].x);
-  split2(v[2], v[3], s.part[0].y, s.part[1].y, s.part[2].y);
-  split2(v[4], v[5], s.part[0].z, s.part[1].z, s.part[2].z);
-  split2(v[6], v[7], s.part[0].w, s.part[1].w, s.part[2].w);
+  float r[8], most = 0.f;
+  lead8(v, v, s.part[0], r);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) most = fmaxf(most, fabsf(r[i]));  // passes over NaN, which an infinity or a NaN leaves
+  if (most == INFINITY) {
+    float cut[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) cut[i] = fabsf(r[i]) == INFINITY ? copysignf(kMostBf16, v[i]) : v[i];
+    lead8(cut, v, s.part[0], r);
+  }
+  rest2(r[0], r[1], s.part[1].x, s.part[2].x);
+  rest2(r[2], r[3], s.part[1].y, s.part[2].y);
+  rest2(r[4], r[5], s.part[1].z, s.part[2].z);
+  rest2(r[6], r[7], s.part[1].w, s.part[2].w);
   return s;
 }
 __device__ __forceinline__ void store8(char* to, int part, const Split8& s) {
@@ -209,6 +232,9 @@ __global__ void __launch_bounds__(256) split_f32_kernel(const SplitAll w) {
     const int64_t row = unit % m.blocks_r * 8 + (lane >> 2), col = unit / m.blocks_r * 32 + (lane & 3) * 8;
     float v[8];
     load8(m.data, m.ld, m.rows, m.cols, m.vec, row, col, v);
+    if (u < w.job[0].warps)  // `b`
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] *= 0.5f;
     const Split8 s = split8(v);
     if (m.by_cols && row < m.rows_cols && col < m.col_stages * kDepth) {
       const int part = m.tile * kDepth * 2;
@@ -493,7 +519,7 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
         const int cols = static_cast<int>(min(static_cast<int64_t>(kCols), w.rows_j - j0));
 #pragma unroll
         for (int e = 0; e < kCols; ++e)
-          if (e < cols) out[e * w.ldc] = w.bias ? sum[e] + add : sum[e];
+          if (e < cols) out[e * w.ldc] = w.bias ? fmaf(2.f, sum[e], add) : 2.f * sum[e];
       }
     }
   }
@@ -544,7 +570,7 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
           const float out[4] = {sum[e].x, sum[e].y, sum[e].z, sum[e].w};
 #pragma unroll
           for (int n = 0; n < 4; ++n)
-            if (i + n < w.rows_i) w.c[j * w.ldc + i + n] = w.bias ? out[n] + add[n] : out[n];
+            if (i + n < w.rows_i) w.c[j * w.ldc + i + n] = w.bias ? fmaf(2.f, out[n], add[n]) : 2.f * out[n];
         }
       }
     }

@@ -81,6 +81,42 @@ def test_linear_special_values():
     assert ((got.double() - exact).abs()[ok] <= bound[ok]).all()
 
 
+def _floats(gen, rows, cols, exponent):
+    """Positive floats of one power of two whose lower 16 bits, what the leading bf16 part leaves, are of every size."""
+    upper = torch.randint(0, 128, (rows, cols), generator=gen) << 16
+    lower = torch.where(torch.rand(rows, cols, generator=gen) < 0.5, torch.randint(0, 65536, (rows, cols), generator=gen),
+                        torch.randint(0x7F00, 0x8100, (rows, cols), generator=gen) ^ 0x8000)
+    return (((exponent + 127) << 23) | upper | lower).int().view(torch.float32)
+
+
+# One non-zero per row of the input: every result is one product, in the left-over terms and the range of which nothing hides.
+# Left out: mid lo + lo mid + lo lo with |mid| <= 2^-8 and |lo| <= 2^-17 of the power of two of its number: 2^-24 (1 + 2^-10) of
+# the product.  Joining the accumulators rounds twice, 2^-24 of the result and 2^-24 of its part below 2^-7; 2^-29 for sums cut off.
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,exponents", [(32, (0, 0)), (64, (3, -60)), (128, (0, 127)), (64, (63, 63)), (32, (127, 0)),
+                                             (64, (64, 63))])
+def test_linear_of_single_products(batch, exponents):
+    gen = torch.Generator().manual_seed(batch)
+    x = torch.zeros(batch, 1024)
+    at = torch.arange(batch)
+    x[at, 7 * at] = _floats(gen, batch, 1, exponents[0])[:, 0] * torch.where(at % 2 == 0, 1.0, -1.0)
+    w = _floats(gen, 1024, 1024, exponents[1])
+    w[0] = (2 - 2.0 ** -23) * 2.0 ** exponents[1]  # for an exponent of 127 the largest number there is
+    assert mccl_b200.require_native()._linear_native(x.cuda(), w.cuda(), None)
+    got = linear(x.cuda(), w.cuda()).cpu().double()
+    want = x[at, 7 * at].double()[:, None] * w.T[7 * at].double()
+    most = torch.finfo(torch.float32).max
+    fits = want.abs() <= most * (1 - 2.0 ** -23)
+    bound = want.abs() * 2.0 ** -24 * (2 + 2.0 ** -5)
+    assert ((got - want).abs() <= bound)[fits].all(), ((got - want).abs() / bound)[fits].max()
+    over = want.abs() >= most * (1 + 2.0 ** -23)
+    assert got[over].isinf().all() and torch.equal(got[over].sign(), want[over].sign())
+    if sum(exponents) < 126:
+        assert fits.all()
+    elif sum(exponents) < 127:
+        assert fits.any()
+
+
 @pytest.mark.gpu
 def test_linear_keeps_what_autograd_offers():
     torch.manual_seed(0)
