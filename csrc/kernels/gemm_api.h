@@ -59,7 +59,8 @@ struct GemmArgs {
   int64_t ldc;
   float* partial;
   uint32_t* tickets;
-  uint32_t* failed;  // set to 1 where a wait runs out; or null
+  uint32_t* failed;     // set to 1 where a wait runs out, whose tiles then are NaN; or null
+  int64_t wait_limit;   // cycles of a wait; negative: about a second
 };
 cudaError_t launch_gemm_f32(const GemmArgs& g, cudaStream_t s);
 

@@ -56,13 +56,27 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-// Waits for the phase of that parity, for about a second at most.
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-  if (bar_try(bar, parity)) return true;
-  const long long begin = clock64();
-  while (!bar_try(bar, parity))
-    if (clock64() - begin > 2000000000ll) return false;
-  return true;
+__device__ __forceinline__ bool bar_test(uint32_t bar, uint32_t parity) {  // a look that never sleeps
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// Waits for the phase of that parity, for `limit` cycles at most.  A long time between two looks (another process has the
+// device, a debugger stopped it) counts as kGap: nothing that this wait is for went on either.
+constexpr long long kWaitLimit = 2000000000ll, kGap = 2000000ll;  // about a second and a millisecond
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, long long limit) {
+  if (bar_test(bar, parity)) return true;
+  for (long long last = clock64(); limit > 0;) {
+    if (bar_try(bar, parity)) return true;
+    const long long now = clock64();
+    limit -= min(now - last, kGap);
+    last = now;
+  }
+  return false;
 }
 // Shared-memory matrix descriptors.  k innermost: rows of 64 bytes (32 k), 64-byte swizzle, 512 bytes per eight rows.
 // Own index innermost: rows of 128 bytes (64 rows of the operand, one k), 128-byte swizzle, 1024 bytes per eight k, 4096
@@ -266,6 +280,7 @@ struct Work {
   float* partial;
   uint32_t* tickets;
   uint32_t* failed;
+  long long limit;                  // of each wait
 };
 
 template <int kSource>
@@ -304,8 +319,9 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
   constexpr int kStages = Shape<NT>::stages, kStage = Shape<NT>::stage, kPartB = Shape<NT>::part_b;
   static_assert(kBInner || NT == 128, "an operand with its own index innermost comes in runs of 64 rows");
   extern __shared__ char raw[];
-  __shared__ alignas(8) uint64_t bars[2 * kStages + 4];
+  __shared__ alignas(8) uint64_t bars[2 * kStages + 5];
   __shared__ uint32_t tmem_base, last_here;
+  __shared__ int issued, given[kProducers / 32];  // stages that images were asked for, and that each producer warp has filled
   char* smem = raw + ((1024u - (smem_addr(raw) & 1023u)) & 1023u);
   const uint32_t smem0 = smem_addr(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -313,7 +329,7 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
   auto full = [&](int s) { return bar0 + 8u * s; };
   auto empty = [&](int s) { return bar0 + 8u * (kStages + s); };
   const uint32_t acc0_full = bar0 + 8u * (2 * kStages), acc0_free = acc0_full + 8, all_full = acc0_full + 16,
-                 all_free = acc0_full + 24;
+                 all_free = acc0_full + 24, drained = acc0_full + 32;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -324,6 +340,7 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
     bar_init(acc0_free, kAdders / 32);
     bar_init(all_full, 1);
     bar_init(all_free, kAdders / 32);
+    bar_init(drained, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kIssuer) {
@@ -339,7 +356,8 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
   const int rank = static_cast<int>(blockIdx.x) % w.splits;
   const int first_tile = static_cast<int>(blockIdx.x) / w.splits, tile_step = static_cast<int>(gridDim.x) / w.splits;
   const int c0 = rank * w.per_split, c1 = min(w.stages, c0 + w.per_split);  // host: c0 < stages
-  bool ok = true;
+  bool ok = true;  // alike in a warp's lanes, but for the lanes that load images and issue products on their own
+  bool issues = false;
 
   if (warp > kIssuer) {
     const int ptid = tid - kProducer0;
@@ -357,10 +375,12 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
         asm volatile("griddepcontrol.wait;" ::: "memory");
         for (int tile = first_tile; ok && tile < w.tiles; tile += tile_step)
           for (int c = c0; ok && c < c1; ++c) {
-            ok = bar_wait(empty(s), (turn & 1) ^ 1);
-            if (ok) load_images(tile, c, s);
+            ok = bar_wait(empty(s), (turn & 1) ^ 1, w.limit);
+            if (!ok) break;
+            load_images(tile, c, s);
             if (++s == kStages) s = 0, ++turn;
           }
+        issued = turn * kStages + s;
       }
       __syncwarp();
     } else {
@@ -411,8 +431,9 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
 #pragma unroll
         for (int b = 0; b < kAhead; ++b) {
           if (!ok || tile >= w.tiles) break;
-          ok = bar_wait(empty(s), (turn & 1) ^ 1);
-          if (ok && loads) load_images(tile, c, s);
+          ok = __all_sync(0xFFFFFFFFu, bar_wait(empty(s), (turn & 1) ^ 1, w.limit));
+          if (!ok) break;
+          if (loads) load_images(tile, c, s);
           char* to = mine + s * kStage;
 #pragma unroll
           for (int j = 0; j < 2; ++j) store8(to + j * 4096, kPartA, split8(v[b][j]));
@@ -424,20 +445,23 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
           if (++c == c1) c = c0, tile += tile_step;
         }
       }
+      if (lane == 0) given[warp - kIssuer - 1] = turn * kStages + s;
+      if (loads) issued = turn * kStages + s;
     }
   } else if (warp == kIssuer) {
-    if (elect()) {
+    issues = elect();
+    if (issues) {
       constexpr uint32_t one = make_idesc(kAInner, kBInner, NT), two = make_idesc(kAInner, kBInner, 2 * NT);
       constexpr uint32_t step_a = kStep<kAInner>, step_b = kStep<kBInner>;
       const uint32_t acc0 = tmem, acc1 = tmem + NT, acc2 = tmem + 2 * NT;
       const uint64_t a0 = make_desc<kAInner>(smem0), b0 = make_desc<kBInner>(smem0 + 3 * kPartA);
       int groups = 0, done = 0, s = 0, turn = 0;
       for (int tile = first_tile; ok && tile < w.tiles; tile += tile_step, ++done) {
-        if (done > 0) ok = bar_wait(all_free, (done - 1) & 1);
+        if (done > 0) ok = bar_wait(all_free, (done - 1) & 1, w.limit);
         for (int c = c0; ok && c < c1; ++c) {
           const bool opens = (c - c0) % kGroup == 0, closes = (c - c0) % kGroup == kGroup - 1 || c == c1 - 1;
-          if (opens && groups > 0) ok = bar_wait(acc0_free, (groups - 1) & 1);
-          ok = ok && bar_wait(full(s), turn & 1);
+          if (opens && groups > 0) ok = bar_wait(acc0_free, (groups - 1) & 1, w.limit);
+          ok = ok && bar_wait(full(s), turn & 1, w.limit);
           if (!ok) break;
           fence_after();
           const uint64_t ah = a0 + s * (kStage >> 4), am = ah + (kPartA >> 4), al = am + (kPartA >> 4);
@@ -460,7 +484,6 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
         }
         mma_commit(all_full);
       }
-      if (!ok) bar_wait(all_full, (done - 1) & 1);  // what is in flight ends before tensor memory is given back
     }
     __syncwarp();
   } else {
@@ -475,7 +498,8 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
       for (int i = 0; i < kCols; ++i) sum[i] = 0.f;
       for (int c = c0; ok && c < c1; c += kGroup) {
         // the other five products of the group's last stage run while acc0 is taken out
-        ok = bar_wait(acc0_full, groups++ & 1);
+        ok = __all_sync(0xFFFFFFFFu, bar_wait(acc0_full, groups++ & 1, w.limit));
+        if (!ok) break;
         fence_after();
 #pragma unroll
         for (int i = 0; i < kCols; i += 16) {
@@ -489,7 +513,8 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
         __syncwarp();
         if (lane == 0) bar_arrive(acc0_free);
       }
-      ok = ok && bar_wait(all_full, done & 1);
+      ok = ok && __all_sync(0xFFFFFFFFu, bar_wait(all_full, done & 1, w.limit));
+      if (!ok) break;
       fence_after();
 #pragma unroll
       for (int i = 0; i < kCols; i += 16) {
@@ -523,10 +548,38 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
       }
     }
   }
-  if (!ok && w.failed) *w.failed = 1u;
   fence_before();
-  __syncthreads();
+  const bool failed = __syncthreads_or(!ok);
   fence_after();
+  if (failed) {
+    if (tid == 0) {
+      if (w.failed) *w.failed = 1u;
+      // The copies in flight end before this CTA's shared memory is another's.  A stage is full when they and all producer
+      // warps have come: for warps that left early this thread does.
+      for (int n = max(issued - kStages, 0); n < issued; ++n) {
+        if (kSource != kImage)
+          for (int p = 0; p < kProducers / 32; ++p)
+            if (given[p] <= n) bar_arrive(full(n % kStages));
+        bar_wait(full(n % kStages), (n / kStages) & 1, kWaitLimit);
+      }
+    }
+    if (issues) {  // and the products, before tensor memory is
+      mma_commit(drained);
+      bar_wait(drained, 0, kWaitLimit);
+    }
+    __syncwarp();
+    // no number that looks like a result
+    for (int tile = first_tile; tile < w.tiles; tile += tile_step) {
+      const int64_t i0 = static_cast<int64_t>(tile % w.tiles_i) * kRows, j0 = static_cast<int64_t>(tile / w.tiles_i) * NT;
+      for (int v = tid; v < NT * kRows; v += kThreads<kSource>) {
+        const int64_t i = i0 + v % kRows, j = j0 + v / kRows;
+        if (w.splits > 1) __stcg(w.partial + (static_cast<int64_t>(tile) * w.splits + rank) * (NT * kRows) + v, NAN);
+        else if (i < w.rows_i && j < w.rows_j) w.c[j * w.ldc + i] = NAN;
+      }
+    }
+    __threadfence();
+    __syncthreads();
+  }
   if (w.splits > 1) {
     // The CTA that is the last of its tile adds up all parts, in order.  Eight loads of four numbers per thread in flight:
     // with one part after the other, and the bias only then, the three parts of a forward product took 2 us longer.
@@ -702,6 +755,7 @@ cudaError_t launch_gemm_f32(const GemmArgs& g, cudaStream_t s) {
   w.partial = g.partial;
   w.tickets = g.tickets;
   w.failed = g.failed;
+  w.limit = g.wait_limit >= 0 ? g.wait_limit : kWaitLimit;
   if (g.product == Product::kWeight) return run<128, kImage>(w, s);
   const bool fwd = g.product == Product::kForward;
   switch (p.cols) {

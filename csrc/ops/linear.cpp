@@ -25,23 +25,26 @@ namespace {
     }                                                                        \
   } while (0)
 
-// A word of mapped host memory in which a kernel notes that one of its bounded waits ran out.
-uint32_t* wait_status() {
-  static uint32_t* word = [] {
+// Words of mapped host memory, one per device, in which a kernel notes that one of its bounded waits ran out.
+constexpr int kDevices = 64;
+uint32_t* wait_status(const at::Tensor& t) {
+  static uint32_t* words = [] {
     void* p = nullptr;
     auto mode = cudaStreamCaptureModeRelaxed;  // the first call may be under capture
     LINEAR_CK(cudaThreadExchangeStreamCaptureMode(&mode));
-    const cudaError_t e = cudaHostAlloc(&p, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable);
+    const cudaError_t e = cudaHostAlloc(&p, kDevices * sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable);
     LINEAR_CK(cudaThreadExchangeStreamCaptureMode(&mode));
     LINEAR_CK(e);
-    *static_cast<uint32_t*>(p) = 0;
+    std::fill_n(static_cast<uint32_t*>(p), kDevices, 0u);
     return static_cast<uint32_t*>(p);
   }();
-  return word;
+  return words + t.get_device() % kDevices;
 }
-void check_waits() {
-  if (*static_cast<volatile uint32_t*>(wait_status()) != 0)
-    throw DeviceError("a wait inside a matrix product kernel ran out; results since then are undefined");
+// Reports what a kernel has noted on the device, once.  What it gave up is NaN.
+void check_waits(const at::Tensor& t) {
+  uint32_t* word = wait_status(t);
+  if (*static_cast<volatile uint32_t*>(word) != 0 && __atomic_exchange_n(word, 0u, __ATOMIC_RELAXED) != 0)
+    throw DeviceError("a wait inside an earlier matrix product kernel ran out; what it should have written is NaN");
 }
 
 bool rows_ok(const at::Tensor& t) {
@@ -80,8 +83,8 @@ Scratch scratch_for(std::initializer_list<const kern::GemmPlan*> plans, const at
   return s;
 }
 
-at::Tensor forward_product(const at::Tensor& x, const at::Tensor& w, const at::Tensor& bias) {
-  check_waits();
+at::Tensor forward_product(const at::Tensor& x, const at::Tensor& w, const at::Tensor& bias, int64_t wait_limit = -1) {
+  check_waits(x);
   c10::cuda::CUDAGuard guard(x.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
   const kern::GemmPlan plan = kern::gemm_plan(kern::Product::kForward, x.size(0), w.size(1), w.size(0));
@@ -104,7 +107,8 @@ at::Tensor forward_product(const at::Tensor& x, const at::Tensor& w, const at::T
   g.ldc = w.size(0);
   g.partial = partial;
   g.tickets = tickets;
-  g.failed = wait_status();
+  g.failed = wait_status(x);
+  g.wait_limit = wait_limit;
   LINEAR_CK(kern::launch_gemm_f32(g, stream));
   return y;
 }
@@ -113,8 +117,8 @@ struct Gradients {
   at::Tensor x, w, bias;
 };
 Gradients backward_products(const at::Tensor& grad, const at::Tensor& x, const at::Tensor& w, bool need_x, bool need_w,
-                            bool need_bias) {
-  check_waits();
+                            bool need_bias, int64_t wait_limit = -1) {
+  check_waits(x);
   const int64_t batch = x.size(0), in = w.size(1), out = w.size(0);
   c10::cuda::CUDAGuard guard(x.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
@@ -152,7 +156,8 @@ Gradients backward_products(const at::Tensor& grad, const at::Tensor& x, const a
     g.ldc = in;
     g.partial = partial;
     g.tickets = tickets;
-    g.failed = wait_status();
+    g.failed = wait_status(x);
+    g.wait_limit = wait_limit;
     LINEAR_CK(kern::launch_gemm_f32(g, stream));
   }
   if (own_w) {
@@ -166,7 +171,8 @@ Gradients backward_products(const at::Tensor& grad, const at::Tensor& x, const a
     g.ldc = in;
     g.partial = partial;
     g.tickets = tickets + px.tickets;
-    g.failed = wait_status();
+    g.failed = wait_status(x);
+    g.wait_limit = wait_limit;
     LINEAR_CK(kern::launch_gemm_f32(g, stream));
   }
   return r;
@@ -211,6 +217,16 @@ bool linear_native(const at::Tensor& x, const at::Tensor& w, const c10::optional
   // a program that lets torch round its fp32 products has asked for something else
   if (at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA)) return false;
   return blackwell(x.get_device()) && kern::gemm_pays(kern::Product::kForward, x.size(0), w.size(1), w.size(0));
+}
+
+std::vector<at::Tensor> linear_with_limit(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& grad,
+                                          int64_t wait_limit) {
+  TORCH_CHECK(wait_limit >= 0 && linear_native(x, w, c10::nullopt), "not a call for the kernels");
+  if (!grad) return {forward_product(x, w, at::Tensor(), wait_limit)};
+  TORCH_CHECK(rows_ok(*grad) && grad->device() == x.device() && grad->size(0) == x.size(0) && grad->size(1) == w.size(0),
+              "not a gradient for the kernels");
+  const Gradients g = backward_products(*grad, x, w, true, true, false, wait_limit);
+  return {g.x, g.w};
 }
 
 at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias) {

@@ -171,6 +171,31 @@ def test_linear_under_capture_and_streams():
     assert torch.equal(y, want) and torch.equal(other, want)
 
 
+# A wait that runs out: the kernel ends by itself, everything it should have written is NaN, the next call on the device says so
+# once, and then the layer works as before.  Split and unsplit reductions, one and several tiles per CTA, each tile width.
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,n_in,n_out", [(32, 3072, 3072), (64, 1500, 1500), (256, 3072, 3072), (700, 1000, 4100),
+                                              (2000, 3000, 2900)])
+def test_linear_whose_waits_run_out(batch, n_in, n_out):
+    native = mccl_b200.require_native()
+    torch.manual_seed(0)
+    x, w, g = (torch.randn(*s, device="cuda") for s in ((batch, n_in), (n_out, n_in), (batch, n_out)))
+    want = linear(x, w)
+    (out,) = native._linear_with_limit(x, w, None, 0)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="a wait inside"):
+        linear(x, w)
+    assert out.isnan().all()
+    assert torch.equal(linear(x, w), want)
+    outs = native._linear_with_limit(x, w, g, 0)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="a wait inside"):
+        linear(x, w)
+    own = [t.isnan().any().item() for t in outs]  # a product that does not pay is the library's
+    assert any(own) and all(t.isnan().all() for t, o in zip(outs, own) if o)
+    assert torch.equal(linear(x, w), want)
+
+
 def test_linear_elsewhere_is_torch():
     """What the kernels do not take is torch's own call: other devices, types and orders, scripting and tracing."""
     native = mccl_b200.require_native()
