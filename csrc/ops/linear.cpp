@@ -214,8 +214,9 @@ bool linear_native(const at::Tensor& x, const at::Tensor& w, const c10::optional
   if (bias && bias->defined() &&
       (!ordinary(*bias) || bias->scalar_type() != at::kFloat || bias->dim() != 1 || bias->size(0) != w.size(0) || bias->stride(0) != 1 || bias->device() != x.device()))
     return false;
-  // a program that lets torch round its fp32 products has asked for something else
-  if (at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA)) return false;
+  // a program that lets torch round its fp32 products has asked for something else (the getter that torch's products use: the
+  // older one throws where the newer setting has been used)
+  if (at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) == at::Float32Precision::TF32 || at::autocast::is_autocast_enabled(at::kCUDA)) return false;
   return blackwell(x.get_device()) && kern::gemm_pays(kern::Product::kForward, x.size(0), w.size(1), w.size(0));
 }
 

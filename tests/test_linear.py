@@ -1,5 +1,8 @@
 """The fp32 linear layer on the tensor cores against the same products in 64 bits."""
 import copy
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 import torch
@@ -194,6 +197,25 @@ def test_linear_whose_waits_run_out(batch, n_in, n_out):
     own = [t.isnan().any().item() for t in outs]  # a product that does not pay is the library's
     assert any(own) and all(t.isnan().all() for t, o in zip(outs, own) if o)
     assert torch.equal(linear(x, w), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("setting", ["torch.backends.cuda.matmul.fp32_precision = 'tf32'", "torch.backends.fp32_precision = 'tf32'",
+                                     "torch.set_float32_matmul_precision('high')", "torch.backends.cuda.matmul.allow_tf32 = True"])
+def test_linear_where_tf32_is_allowed(setting):
+    """Each way to allow it leaves the products to torch (in a process of its own: the settings do not mix)."""
+    code = f"""
+import torch, torch.nn.functional as F, mccl_b200
+from mccl_b200.ops.linear import linear
+x, w = torch.randn(64, 2048, device="cuda"), torch.randn(2048, 2048, device="cuda")
+native = mccl_b200.require_native()
+assert native._linear_native(x, w, None)
+{setting}
+assert not native._linear_native(x, w, None)
+assert torch.equal(linear(x, w), F.linear(x, w))
+"""
+    done = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr[-2000:]
 
 
 def test_linear_elsewhere_is_torch():
