@@ -71,6 +71,7 @@ struct Scratch {
     return p;
   }
 };
+// No memory for it: an empty one, and the product is left to torch, which needs less.
 Scratch scratch_for(std::initializer_list<const kern::GemmPlan*> plans, const at::TensorOptions& like) {
   int64_t bytes = 0, partial = 0;
   for (const auto* p : plans) {
@@ -78,8 +79,11 @@ Scratch scratch_for(std::initializer_list<const kern::GemmPlan*> plans, const at
     partial = std::max(partial, p->partial);
   }
   Scratch s;
-  s.buffer = at::empty({bytes + align(partial)}, like.dtype(at::kByte));
-  s.at = static_cast<char*>(s.buffer.data_ptr());
+  try {
+    s.buffer = at::empty({bytes + align(partial)}, like.dtype(at::kByte));
+    s.at = static_cast<char*>(s.buffer.data_ptr());
+  } catch (const c10::OutOfMemoryError&) {
+  }
   return s;
 }
 
@@ -88,8 +92,9 @@ at::Tensor forward_product(const at::Tensor& x, const at::Tensor& w, const at::T
   c10::cuda::CUDAGuard guard(x.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
   const kern::GemmPlan plan = kern::gemm_plan(kern::Product::kForward, x.size(0), w.size(1), w.size(0));
-  at::Tensor y = at::empty({x.size(0), w.size(0)}, x.options());
   Scratch s = scratch_for({&plan}, x.options());
+  if (s.at == nullptr) return at::linear(x, w, bias.defined() ? c10::optional<at::Tensor>(bias) : c10::nullopt);
+  at::Tensor y = at::empty({x.size(0), w.size(0)}, x.options());
   auto* tickets = reinterpret_cast<uint32_t*>(s.take(plan.tickets * 4));
   char* image = s.take(plan.b_image);
   auto* partial = reinterpret_cast<float*>(s.take(plan.partial));
@@ -123,18 +128,20 @@ Gradients backward_products(const at::Tensor& grad, const at::Tensor& x, const a
   c10::cuda::CUDAGuard guard(x.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
   Gradients r;
-  const bool own_x = need_x && kern::gemm_pays(kern::Product::kInput, batch, in, out);
-  const bool own_w = need_w && kern::gemm_pays(kern::Product::kWeight, batch, in, out);
+  bool own_x = need_x && kern::gemm_pays(kern::Product::kInput, batch, in, out);
+  bool own_w = need_w && kern::gemm_pays(kern::Product::kWeight, batch, in, out);
+  kern::GemmPlan px{}, pw{};
+  if (own_x) px = kern::gemm_plan(kern::Product::kInput, batch, in, out);
+  if (own_w) pw = kern::gemm_plan(kern::Product::kWeight, batch, in, out);
+  Scratch s;
+  if (own_x || own_w) s = scratch_for({&px, &pw}, x.options());
+  if (s.at == nullptr) own_x = own_w = false;
   if (need_x && !own_x) r.x = grad.mm(w);
   if (need_w && !own_w) r.w = grad.t().mm(x);
   if (!own_x && !own_w) {
     if (need_bias) r.bias = grad.sum(0);
     return r;
   }
-  kern::GemmPlan px{}, pw{};
-  if (own_x) px = kern::gemm_plan(kern::Product::kInput, batch, in, out);
-  if (own_w) pw = kern::gemm_plan(kern::Product::kWeight, batch, in, out);
-  Scratch s = scratch_for({&px, &pw}, x.options());
   auto* tickets = reinterpret_cast<uint32_t*>(s.take((px.tickets + pw.tickets) * 4));
   char *gx = s.take(px.b_image), *gw = s.take(pw.b_image), *xw = s.take(pw.a_image);
   auto* partial = reinterpret_cast<float*>(s.take(std::max(px.partial, pw.partial)));

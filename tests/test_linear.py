@@ -218,6 +218,33 @@ assert torch.equal(linear(x, w), F.linear(x, w))
     assert done.returncode == 0, done.stderr[-2000:]
 
 
+@pytest.mark.gpu
+def test_linear_without_memory_for_its_images():
+    """Where the images cannot be had the products are torch's."""
+    native = mccl_b200.require_native()
+    torch.manual_seed(0)
+    batch, n_in, n_out = 8192, 4096, 2048  # images of 201 MB forward and of 302 MB backward, tensors of 134, 67 and 34 MB
+    x, w, g = (torch.randn(*s, device="cuda", requires_grad=s[1] == n_in) for s in ((batch, n_in), (n_out, n_in), (batch, n_out)))
+    assert native._linear_native(x, w, None)
+    torch.cuda.empty_cache()
+    _, total = torch.cuda.mem_get_info()
+    try:
+        y = linear(x, w)
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (190 << 20)) / total)
+        with torch.no_grad():
+            z = linear(x, w)
+        assert torch.equal(z, F.linear(x, w)) and not torch.equal(z, y)
+        del z
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (280 << 20)) / total)
+        gx, gw = torch.autograd.grad(y, (x, w), g)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        torch.cuda.empty_cache()
+    assert torch.equal(gx, g.mm(w)) and torch.equal(gw, g.t().mm(x))
+
+
 def test_linear_elsewhere_is_torch():
     """What the kernels do not take is torch's own call: other devices, types and orders, scripting and tracing."""
     native = mccl_b200.require_native()
