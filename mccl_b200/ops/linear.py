@@ -17,7 +17,7 @@ _PLAIN = (torch.Tensor, nn.Parameter)
 
 def linear(input: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``input @ weight.T + bias``."""
-    if (type(input) in _PLAIN and type(weight) in _PLAIN and input.is_cuda and not torch.compiler.is_compiling()
+    if (type(input) in _PLAIN and type(weight) in _PLAIN and (bias is None or type(bias) in _PLAIN) and input.is_cuda and not torch.compiler.is_compiling()
             and torch._C._get_tracing_state() is None and not torch._C._is_torch_function_mode_enabled()):
         from .. import require_native
         return require_native()._linear(input, weight, bias)

@@ -245,6 +245,24 @@ def test_linear_without_memory_for_its_images():
     assert torch.equal(gx, g.mm(w)) and torch.equal(gw, g.t().mm(x))
 
 
+class _Seen(torch.Tensor):
+    """A subclass that sees the functions it is passed to."""
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        cls.seen = func
+        return super().__torch_function__(func, types, args, kwargs or {})
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_linear_of_subclasses(which):
+    args = [torch.randn(64, 1024, device="cuda"), torch.randn(1024, 1024, device="cuda"), torch.randn(1024, device="cuda")]
+    args[which] = args[which].as_subclass(_Seen)
+    _Seen.seen = None
+    assert type(linear(*args)) is _Seen and _Seen.seen is F.linear
+
+
 def test_linear_elsewhere_is_torch():
     """What the kernels do not take is torch's own call: other devices, types and orders, scripting and tracing."""
     native = mccl_b200.require_native()
