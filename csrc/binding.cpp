@@ -839,7 +839,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 #endif
 
   // ---- fp32 linear layer on the tensor cores ----------------------------------------------------------
-  m.def("_linear", &linear, py::arg("input"), py::arg("weight"), py::arg("bias") = py::none());
+  m.def("_linear", &linear, py::arg("input"), py::arg("weight"), py::arg("bias") = py::none(),
+        py::call_guard<py::gil_scoped_release>());
   m.def("_linear_with_limit", &linear_with_limit, py::arg("input"), py::arg("weight"), py::arg("grad"), py::arg("wait_limit"));
   m.def("_linear_native", &linear_native, py::arg("input"), py::arg("weight"), py::arg("bias") = py::none());
 }

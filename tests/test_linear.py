@@ -2,6 +2,8 @@
 import copy
 import subprocess
 import sys
+import threading
+import time
 from pathlib import Path
 
 import pytest
@@ -261,6 +263,26 @@ def test_linear_of_subclasses(which):
     args[which] = args[which].as_subclass(_Seen)
     _Seen.seen = None
     assert type(linear(*args)) is _Seen and _Seen.seen is F.linear
+
+
+def test_linear_lets_other_threads_run():
+    native = mccl_b200.require_native()
+    x, w = torch.randn(4096, 4096), torch.randn(4096, 4096)
+    done, ticks = threading.Event(), set()
+
+    def call():
+        for _ in range(4):
+            native._linear(x, w, None)
+        done.set()
+
+    begin = time.monotonic()
+    thread = threading.Thread(target=call)
+    thread.start()
+    while not done.wait(0.001):
+        ticks.add(int((time.monotonic() - begin) * 100))
+    took = time.monotonic() - begin
+    thread.join()
+    assert len(ticks) > 0.3 * 100 * took  # hundredths of a second in which this thread ran, too
 
 
 def test_linear_elsewhere_is_torch():
