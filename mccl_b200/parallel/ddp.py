@@ -15,6 +15,7 @@ Both return futures that are ordered on the communication stream, so no host
 synchronisation happens between backward and the optimizer step.
 """
 import os
+import weakref
 from typing import Dict, Optional
 
 import torch
@@ -22,6 +23,36 @@ import torch.distributed as dist
 from torch.nn.parallel import DistributedDataParallel
 
 from ..ops.linear import Linear
+
+
+# layers whose products are torch's for the sake of a compressed wrapper: layer -> token of that wrapper
+_torch_product_layers = weakref.WeakKeyDictionary()
+
+
+def _own_products(module, owner=None) -> None:
+    """Undoes :func:`_torch_products` in ``module``: all of it, or what the wrapper ``owner`` has done."""
+    for m in module.modules():
+        token = _torch_product_layers.get(m)
+        if token is not None and (owner is None or token is owner):
+            m.stock = False
+            del _torch_product_layers[m]
+
+
+def _torch_products(ddp, module) -> None:
+    """Compressed training sends what the largest fp32 gradients are, which the last bit of a product can decide: while such
+    a wrapper lives, the module's layers keep torch's products.  Layers whose ``stock`` the program has set stay as they are."""
+    token = object()
+    for m in module.modules():
+        if isinstance(m, Linear) and not m.stock:
+            m.stock = True
+            _torch_product_layers[m] = token
+    module = weakref.ref(module)
+
+    def release():
+        if module() is not None:
+            _own_products(module(), token)
+
+    weakref.finalize(ddp, release).atexit = False
 
 
 def _backend_for(process_group, device):
@@ -218,11 +249,7 @@ def wrap_ddp(module: torch.nn.Module, *, device_ids=None, bucket_cap_mb: Optiona
     ddp_kwargs.setdefault("gradient_as_bucket_view", True)
     on_cuda = next(module.parameters()).is_cuda
     mode = compression if compression is not None else os.environ.get("MCCL_COMPRESSION", "none")
-    if on_cuda and mode == "topk":
-        # which entries are sent is decided by comparing fp32 gradients, where the last bit can count: they stay torch's
-        for m in module.modules():
-            if isinstance(m, Linear):
-                m.stock = True
+    _own_products(module)
     pool = None
     if on_cuda and mode != "topk" and nvls_buckets is not False and dist.is_initialized():
         pool = _nvls_bucket_pool(module, process_group)
@@ -256,6 +283,7 @@ def wrap_ddp(module: torch.nn.Module, *, device_ids=None, bucket_cap_mb: Optiona
         else:
             _install_native_bucket_hook(ddp, optimizer_in_backward, process_group)
     elif on_cuda and mode == "topk":
+        _torch_products(ddp, module)
         ddp._mccl_topk_state = TopKState(process_group)
         ddp.register_comm_hook(ddp._mccl_topk_state, topk_hook)
     elif on_cuda and fused_average:

@@ -1,5 +1,6 @@
 """The fp32 linear layer on the tensor cores against the same products in 64 bits."""
 import copy
+import gc
 import subprocess
 import sys
 import threading
@@ -8,11 +9,13 @@ from pathlib import Path
 
 import pytest
 import torch
+import torch.distributed as dist
 import torch.nn.functional as F
 
 import mccl_b200
 from mccl_b200.models import MLP94M
 from mccl_b200.ops.linear import Linear, linear
+from mccl_b200.parallel import wrap_ddp
 
 
 def _bound(absolute, depth):
@@ -304,3 +307,33 @@ def test_linear_elsewhere_is_torch():
     assert list(model.state_dict())[:2] == ["net.0.weight", "net.0.bias"]
     with pytest.raises(RuntimeError):
         linear(torch.randn(3, 5), torch.randn(4, 6))
+
+
+@pytest.mark.gpu
+def test_compressed_wrapper_gives_its_layers_back():
+    """A module keeps torch's products while a compressed wrapper of it lives, and no longer; the program's own choice stays."""
+    created = not dist.is_initialized()
+    if created:
+        dist.init_process_group("mccl", store=dist.HashStore(), rank=0, world_size=1)
+    try:
+        model = MLP94M(64, 48, 1, 5).cuda()
+        layers = model.net[::2]
+        layers[0].stock = True
+        own = lambda: [not m.stock for m in layers]  # noqa: E731
+        first = wrap_ddp(model, device_ids=[0], compression="topk")
+        assert own() == [False, False, False]
+        dense = wrap_ddp(model, device_ids=[0], compression="none")
+        assert own() == [False, True, True]
+        second = wrap_ddp(model, device_ids=[0], compression="topk")
+        assert own() == [False, False, False]
+        del first, dense
+        gc.collect()
+        assert own() == [False, False, False]
+        del second
+        gc.collect()
+        assert own() == [False, True, True]
+        assert torch.equal(layers[0](torch.ones(2, 64, device="cuda")),
+                           F.linear(torch.ones(2, 64, device="cuda"), layers[0].weight, layers[0].bias))
+    finally:
+        if created:
+            dist.destroy_process_group()
