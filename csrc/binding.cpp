@@ -705,6 +705,21 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     const kern::OlaShape s = kern::ifft_ola_shape(a);
     return py::make_tuple(s.reach, s.batch, s.most, s.begins);
   });
+  m.def("_test_stft_inverse_streams", [](int n_fft, int hop, int64_t length, int batch, bool inverse) {
+    kern::IfftOlaArgs a{};
+    a.n_fft = n_fft;
+    a.hop = hop;
+    a.out_len = length;
+    a.n_frames = static_cast<int>(1 + length / hop);
+    a.batch = batch;
+    a.pad = n_fft / 2;
+    a.stride_f = 1;
+    a.stride_t = n_fft / 2 + 1;
+    a.stride_b = a.stride_t * a.n_frames;
+    a.fold_reflect = inverse ? 0 : 1;
+    a.normalize_envelope = inverse ? 1 : 0;
+    return kern::ifft_ola_streams(a);
+  });
 #endif
 
   // Drives the pool's range allocator with a script of (+bytes | -index) steps: +n allocates n bytes,

@@ -778,6 +778,7 @@ struct OlaGrid {
   OlaPlan plan;
   int batch = 0;      // frames transformed together
   int64_t most = 0;   // segments of one batch entry that are resident together
+  int resident = 1;   // CTAs per SM
   int threads = 0;
   size_t smem = 0;
 };
@@ -824,6 +825,7 @@ OlaGrid ola_grid(const IfftOlaArgs& a) {
     if (segments * a.batch > 0x7FFFFFFF) continue;
     g.batch = static_cast<int>(batch);
     g.most = most;
+    g.resident = resident;
     pl.segments = static_cast<int>(segments);
     pl.ring = static_cast<int>(ring);
     g.threads = 32 * warps;
@@ -833,8 +835,15 @@ OlaGrid ola_grid(const IfftOlaArgs& a) {
   return g;
 }
 
+// What a frame of every lane group takes the stream kernel, forward's gradient and inverse, and what it takes to begin and end,
+// both in tenths of the time of the batch kernel's batch.  Fitted to 230 pairs of times: n_fft 256, 512 and 2048, hop n_fft / 4 and
+// / 2, 1 to 160 signals of 64 Ki to 1 Mi samples.
+constexpr int kStreamFrame[12][2] = {{}, {}, {}, {}, {}, {}, {64, 64}, {64, 64}, {70, 75}, {}, {65, 71}, {}};
+constexpr int kStreamEnds[12] = {0, 0, 0, 0, 0, 0, 5, 5, 9, 0, 32, 0};
+constexpr int kBatchEnds = 20;
+
 // The stream kernel's geometry; threads == 0: not for this problem.  It wants runs of frames that are long against what two
-// neighbours share.
+// neighbours share, and its CTAs, one per SM and in whole numbers per signal, to fill the device about as well as the batch kernel's.
 template <int LH>
 OlaGrid stream_grid(const IfftOlaArgs& a) {
   using F = WarpFft<LH>;
@@ -854,7 +863,17 @@ OlaGrid stream_grid(const IfftOlaArgs& a) {
   const int64_t most = std::max<int64_t>(1, kSms / a.batch);
   const int64_t least = 3ll * (pl.reach - 1) * groups + 2 * pl.edge;  // rows of a CTA
   pl.segments = static_cast<int>(std::min<int64_t>(most, pl.rows / std::max<int64_t>(1, least)));
-  if (pl.segments < 1 || (pl.segments < most && static_cast<int64_t>(pl.segments) * a.batch < kSms * 3 / 4)) return g;
+  if (pl.segments < 1) return g;
+  // Frames of the busiest lane group against batches of the busiest CTA, each as often as its CTAs need turns on the device.
+  // 80 x 1 Mi samples, n_fft 512, hop 128, backward: 612 us in batches, 748 in streams on 80 SMs; 32 x 256 Ki, 2048, 1024: 52
+  // and 65.  32 x 1 Mi, 512, 128: 250 and 211; 120 x 1 Mi, 2048, 512: 1110 and 788.
+  auto ceil_div = [](int64_t x, int64_t y) { return (x + y - 1) / y; };
+  auto longest = [&](int64_t segments, int64_t together) { return ceil_div(ceil_div(pl.rows, segments) + pl.reach - 1, together); };
+  const int64_t turns = ceil_div(static_cast<int64_t>(pl.segments) * a.batch, kSms);
+  const int64_t row_turns = ceil_div(static_cast<int64_t>(rows.plan.segments) * a.batch, static_cast<int64_t>(kSms) * rows.resident);
+  if (turns * (longest(pl.segments, groups) * kStreamFrame[LH][a.normalize_envelope ? 1 : 0] + 10 * (kStreamEnds[LH] + kBatchEnds)) >
+      row_turns * (100 * longest(rows.plan.segments, rows.batch) + 10 * kBatchEnds))
+    return g;
   const size_t kept = F::V - a.hop / (2 * F::L);
   const size_t stream = groups * (F::kHalfSlot * sizeof(float) + kept * F::L * sizeof(float2)) +
                         (a.normalize_envelope ? a.hop * sizeof(float) : 0);
@@ -906,6 +925,9 @@ R for_size(int n_fft, Fn&& f) {
 OlaGrid ola_grid_for(const IfftOlaArgs& a) {
   return for_size<OlaGrid>(a.n_fft, [&](auto lh) { return ola_grid<decltype(lh)::value>(a); });
 }
+OlaGrid stream_grid_for(const IfftOlaArgs& a) {
+  return for_size<OlaGrid>(a.n_fft, [&](auto lh) { return stream_grid<decltype(lh)::value>(a); });
+}
 
 bool valid(const IfftOlaArgs& a) {
   return valid_nfft(a.n_fft) && a.batch > 0 && a.n_frames > 0 && a.hop > 0 && a.out_len > 0;
@@ -939,9 +961,11 @@ int64_t ifft_ola_scratch(const IfftOlaArgs& a) {
   return static_cast<int64_t>(a.batch) * a.n_frames * a.n_fft;
 }
 
+bool ifft_ola_streams(const IfftOlaArgs& a) { return valid(a) && stream_grid_for(a).threads > 0; }
+
 cudaError_t launch_ifft_ola(const IfftOlaArgs& a, float* scratch, cudaStream_t s) {
   if (!valid(a)) return cudaErrorInvalidValue;
-  const OlaGrid stream = for_size<OlaGrid>(a.n_fft, [&](auto lh) { return stream_grid<decltype(lh)::value>(a); });
+  const OlaGrid stream = stream_grid_for(a);
   if (stream.threads > 0) {
     note_launch();
     return for_size<cudaError_t>(a.n_fft, [&](auto lh) -> cudaError_t {

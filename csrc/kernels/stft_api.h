@@ -65,6 +65,8 @@ struct OlaShape {
   std::vector<int64_t> begins;  // first row of every segment, and the end; empty where it cannot run
 };
 OlaShape ifft_ola_shape(const IfftOlaArgs& a);
+// Whether launch_ifft_ola walks the frames in streams (host arithmetic only).
+bool ifft_ola_streams(const IfftOlaArgs& a);
 cudaError_t launch_ifft_ola(const IfftOlaArgs& a, float* scratch, cudaStream_t s);
 
 }  // namespace kern
