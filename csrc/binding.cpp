@@ -30,6 +30,7 @@
 #include "cpu/reduce.h"
 #include "kernels/api.h"
 #include "kernels/launch_count.h"
+#include "kernels/gemm_api.h"
 #include "kernels/optim_api.h"
 #include "kernels/stft_api.h"
 #include "kernels/topk_api.h"
@@ -857,5 +858,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("_linear", &linear, py::arg("input"), py::arg("weight"), py::arg("bias") = py::none(),
         py::call_guard<py::gil_scoped_release>());
   m.def("_linear_with_limit", &linear_with_limit, py::arg("input"), py::arg("weight"), py::arg("grad"), py::arg("wait_limit"));
+  m.def("_linear_pays", [](const std::string& product, int64_t batch, int64_t in, int64_t out) {
+    return kern::gemm_pays(product == "forward" ? kern::Product::kForward : product == "input" ? kern::Product::kInput
+                                                                                                 : kern::Product::kWeight,
+                           batch, in, out);
+  });
   m.def("_linear_native", &linear_native, py::arg("input"), py::arg("weight"), py::arg("bias") = py::none());
 }

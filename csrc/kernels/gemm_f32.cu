@@ -686,17 +686,36 @@ GemmPlan gemm_plan(Product p, int64_t batch, int64_t in, int64_t out) {
   return g;
 }
 
-// From a sweep of 8 to 256 rows over twelve layers of 512 x 256 to 3072 x 3072 (B200, both sides from CUDA graphs; here with
-// the launch that makes the images).  Below these lines the two launches and the empty rows of the tiles cost more than the
-// library's one kernel: 64 x 512 x 256 11.7 and 12.0 us forward, 9.4 and 6.4 input, 7.3 and 3.5 weight gradient; at
-// 24 x 1024 x 1024 10.1 and 13.8, 9.6 and 11.2, 7.0 and 4.7; at 64 x 2048 x 2048 16.3 and 36.9, 15.0 and 39.4, 11.0 and 21.1.
-// The weight gradient of few rows is a matter of writing it.  Images are one and a half times their matrix: none above 1 GB.
+// From sweeps of 1 to 4096 rows over 26 layers, 65536 to 16 features and the reverse among them, and of 8 to 255 rows over 81 of
+// 256 to 3000 (B200, both sides from CUDA graphs; here with the launch that makes the images; weights from memory and, up to 40 MB
+// of them, from the second-level cache).  Of 1139 products taken 13 are slower than the library's, by 3 to 12 %.  What is left to
+// the library, us there and here, rows and features in -> out:
+//  - little to do, less than the two launches cost: 64, 256 -> 512 forward 11.7 and 12.0;
+//  - tiles of 128 rows (of 65 and more) on less than 1000 of the reduction: they take 15 to 17 us at least, the library 8 to 13, 96,
+//    256 -> 3000 forward 9.3 and 14.6; narrower tiles below 512: 33, 256 -> 3000 9.4 and 11.2;
+//  - rows of a tile that the layer does not have: 64, 65536 -> 16 forward 117 and 215; weight gradient of 64, 100000 -> 64 25 and 34;
+//  - few CTAs with long shares of the reduction: 64, 100000 -> 64 forward 180 and 327, 16, 16384 -> 128 21 and 59;
+//  - next to no rows, for which the library reads the weights at 5 TB/s and this kernel at 2.3: 1, 8192 -> 8192 forward 49 and 115;
+//  - weight gradients of less than 75 tiles, half a turn of the device for the library: 255, 850 -> 850 13.1 and 14.1.
+// Images are one and a half times their matrix: none above 1 GB.
 bool gemm_pays(Product p, int64_t batch, int64_t in, int64_t out) {
   constexpr double kImageLimit = 1 << 30;
   const double macs = static_cast<double>(batch) * in * out, layer = static_cast<double>(in) * out;
   if (6.0 * batch * (static_cast<double>(in) + 2.0 * out) > kImageLimit || layer > 1e10) return false;
-  if (p == Product::kWeight) return batch >= 32 && macs >= 1e8;
-  return layer >= 7e5 && macs >= (p == Product::kForward ? 2e7 : 3e7);
+  const bool fwd = p == Product::kForward;
+  if (p == Product::kWeight ? batch < 32 || macs < 1.1e8 : layer < 7e5 || macs < (fwd ? 2e7 : 3e7)) return false;
+  const GemmPlan g = gemm_plan(p, batch, in, out);
+  const int64_t tiles = static_cast<int64_t>(g.tiles_i) * g.tiles_j;
+  if (p == Product::kWeight) {
+    if (4.0 * layer < 3.0 * kRows * kRows * static_cast<double>(tiles)) return false;
+    return tiles > 74 || macs >= (g.splits == 1 ? 1.4e8 : 2.4e8);
+  }
+  if (4 * g.rows_i < 3 * kRows * static_cast<int64_t>(g.tiles_i) || g.depth < 64) return false;
+  const bool deep = layer < 3e7 || g.depth >= (fwd ? 2 : 1) * g.rows_i;
+  if (batch < (deep ? 2 : fwd ? 16 : 8)) return false;
+  if (tiles * g.splits < 24 && (batch < 32 || g.per_split > 64)) return false;
+  if (g.cols == 128 && g.depth < 1000) return macs >= (g.depth < 700 ? 2.7e8 : 2.05e8);
+  return g.depth >= 512 || macs >= 2.4e8;
 }
 
 cudaError_t launch_split_f32(const SplitJob* jobs, int n, float* sums, uint32_t* zero, int64_t zeroed, cudaStream_t s) {
