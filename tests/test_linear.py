@@ -89,6 +89,26 @@ def test_linear_special_values():
     assert ((got.double() - exact).abs()[ok] <= bound[ok]).all()
 
 
+# Error of whole products, 2-norm against 64 bits.  A result is the sum of a group of 64 of the reduction after the other, each rounded
+# to fp32, and the tensor cores cut their sums off at each of a group's four steps: at most some 4 units of 2^-24 of the partial
+# sums, which are no larger than the result's own size.  Without the least of the six products (2^-17 of a number) it is 7e-6.
+# Each tile width, split and unsplit reductions, several tiles per CTA forward and for the input gradient, ragged edges.
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,n_in,n_out", [(24, 1500, 1340), (32, 3072, 3072), (50, 1700, 1027), (64, 2048, 2048),
+                                              (100, 1030, 1410), (256, 3072, 3072), (700, 1000, 4100), (2000, 3000, 2900)])
+def test_linear_error_of_whole_products(batch, n_in, n_out):
+    torch.manual_seed(batch)
+    x = torch.randn(batch, n_in, device="cuda", requires_grad=True)
+    w = (torch.randn(n_out, n_in, device="cuda") / n_in ** 0.5).requires_grad_()
+    b, g = torch.randn(n_out, device="cuda", requires_grad=True), torch.randn(batch, n_out, device="cuda")
+    assert mccl_b200.require_native()._linear_native(x, w, b)
+    y = linear(x, w, b)
+    grads = torch.autograd.grad(y, (x, w, b), g)
+    x, w, b, g = (t.detach().double() for t in (x, w, b, g))
+    for got, want in zip((y, *grads), (x @ w.T + b, g @ w, g.T @ x, g.sum(0))):
+        assert (got.double() - want).norm() <= 4 * 2.0 ** -24 * want.norm()
+
+
 def _floats(gen, rows, cols, exponent):
     """Positive floats of one power of two whose lower 16 bits, what the leading bf16 part leaves, are of every size."""
     upper = torch.randint(0, 128, (rows, cols), generator=gen) << 16
