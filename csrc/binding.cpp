@@ -748,6 +748,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, py::arg("units"), py::arg("nctas"), py::arg("nthreads") = 512, py::arg("tile_bytes") = 0);
   m.def("_mover_tile_bytes", &kern::mover_tile_bytes_host, py::arg("units"), py::arg("nctas"), py::arg("tile_bytes") = 0,
         py::arg("ws") = 2);
+  m.def("_twoshot_tile", [](int64_t chunk_units, int nctas, int nthreads, int64_t tiles) {
+    int64_t batch = 0;
+    const int64_t units = kern::twoshot_tile_units_host(chunk_units, nctas, nthreads, tiles, &batch);
+    return std::make_pair(units, batch);
+  });
   m.attr("MAX_CTAS_PER_LANE") = kern::kMaxCtasPerLane;
 
   // ---- top-k kernels ------------------------------------------------------------------------

@@ -118,6 +118,9 @@ void tile_plan_host(int64_t units, int nctas, int nthreads, int64_t tile_bytes, 
 // rank's block on `nctas` CTAs at world size `ws` (test hook for the rule in coll_common.cuh).
 int64_t mover_tile_bytes_host(int64_t units, int nctas, int64_t tile_bytes, int ws);
 
+// 16-byte units of a tile of the two-shot kernel, and of the batches that its loops move (test hook, likewise).
+int64_t twoshot_tile_units_host(int64_t chunk_units, int nctas, int nthreads, int64_t tiles, int64_t* batch_units);
+
 // All launchers return cudaSuccess or the launch error; none synchronises.
 // dtype: element type of in/out.  wire: element type stored in the arena
 // (== dtype, or F16/BF16 when dtype is F32: fused wire cast).

@@ -210,6 +210,18 @@ template <> struct MultimemSum<__nv_bfloat16> {
   }
 };
 
+// 16-byte units of a two-shot tile; `tiles` per CTA are asked for.  One: bulk phases, whole units per thread.  (Whole batches of
+// nthreads * kTileUnroll units left 3 of 37 CTAs idle, or all but a few of a small chunk's.  Emulated on one GPU, batches and
+// units: 4 x 6553600 fp32 139 and 137 us, 8 x 3000000 fp16 99 and 89, 8 x 100003 fp32 64 and 50, reduce_scatter of 8 x 10007
+// bf16 39 and 29.  kTileUnroll 8: 136 for the first, where 4 took 124.)  Several: whole batches, since a smaller tile's flag
+// round costs more than it overlaps (8 tiles: 8 x 3000000 fp16 121 and 226, 4 x 2000000 fp32 77 and 178).
+constexpr int kTileUnroll = 4;
+__host__ __device__ inline int64_t twoshot_tile_units(int64_t chunk_units, int nctas, int nthreads, int64_t tiles) {
+  const int64_t want = tiles > 1 ? tiles : 1, grain = static_cast<int64_t>(nthreads) * (want > 1 ? kTileUnroll : 1);
+  const int64_t share = ((chunk_units + nctas - 1) / nctas + want - 1) / want;
+  return share > grain ? (share + grain - 1) / grain * grain : grain;
+}
+
 // Tile geometry of the pipelined kernels.  The 16-byte-unit index space [0, units) is cut into
 // tiles of `tile_units` (a whole number of nthreads * kUnroll batches); tile g belongs to CTA
 // g % nctas on EVERY rank, so the CTA that wrote a tile on one rank is the CTA that reads it on

@@ -393,6 +393,11 @@ int64_t mover_tile_bytes_host(int64_t units, int nctas, int64_t tile_bytes, int 
   return mover_tile_bytes(units, nctas, tile_bytes, ws);
 }
 
+int64_t twoshot_tile_units_host(int64_t chunk_units, int nctas, int nthreads, int64_t tiles, int64_t* batch_units) {
+  *batch_units = static_cast<int64_t>(nthreads) * kTileUnroll;
+  return twoshot_tile_units(chunk_units, nctas, nthreads, tiles);
+}
+
 void tile_plan_host(int64_t units, int nctas, int nthreads, int64_t tile_bytes, int64_t* tile_units, int64_t* ntiles) {
   const TilePlan t = TilePlan::make(units, nctas, nthreads, tile_bytes);
   *tile_units = t.tile_units;

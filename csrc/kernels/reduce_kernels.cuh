@@ -177,12 +177,11 @@ __device__ __forceinline__ void reduce_tile(const CtaCtx& k, const T* in_chunk, 
 }
 
 // Tile-pipelined two-shot.  A CTA's share of the chunk index space is cut into
-// tiles of whole 16-byte units per thread; in iteration `it` the CTA
+// tiles (twoshot_tile_units); in iteration `it` the CTA
 // pushes tile it, reduces tile it-1 (whose peer pushes were signalled one
 // iteration ago) and pulls tile it-2, so link traffic, the HBM-bound reduction
 // and the flag round trips overlap instead of forming three bulk-synchronous
 // phases.
-constexpr int kTileUnroll = 4;
 constexpr int kPullUnroll = 8;  // remote loads are round trips: keep more of them in flight
 
 // kSum: SUM/AVG (AVG differs only by the scale); otherwise MIN/MAX/PRODUCT at run time.
@@ -222,15 +221,8 @@ __global__ void __launch_bounds__(512) twoshot_kernel(const __grid_constant__ Co
     return e > b ? e - b : 0;
   };
 
-  // A tile is a whole number of units per thread; the requested tiles per CTA fix its size.  One tile per CTA = bulk phases.
-  // (Whole batches of nthreads * kTileUnroll units left 3 of 37 CTAs idle, or all but a few of a small chunk's.  Emulated on one
-  // GPU, batches and threads: 4 x 6553600 fp32 124 and 121 us, 8 x 3000000 fp16 92 and 84, 8 x 100003 fp32 58 and 44,
-  // reduce_scatter of 8 x 10007 bf16 39 and 29.  kTileUnroll 8: 136 for the first.)
   const int64_t batch_units = static_cast<int64_t>(k.nthreads) * kTileUnroll;
-  const int64_t want_tiles = p.tiles > 1 ? p.tiles : 1;
-  const int64_t per_cta_units = (chunk_units + k.nctas - 1) / k.nctas;
-  int64_t tile_units = ((per_cta_units + want_tiles - 1) / want_tiles + k.nthreads - 1) / k.nthreads * k.nthreads;
-  if (tile_units < k.nthreads) tile_units = k.nthreads;
+  const int64_t tile_units = twoshot_tile_units(chunk_units, k.nctas, k.nthreads, p.tiles);
   const int64_t ntiles_total = (chunk_units + tile_units - 1) / tile_units;
   // tiles g = cta, cta + nctas, ... belong to this CTA
   const int64_t my_tiles = ntiles_total > k.cta ? (ntiles_total - k.cta + k.nctas - 1) / k.nctas : 0;

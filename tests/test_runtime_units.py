@@ -93,6 +93,20 @@ def test_tile_plan_is_a_partition_owned_by_cta_index(native):
                 assert per_cta <= 1024, "12-bit tile counters"
 
 
+def test_twoshot_tiles_are_whole_batches_where_several_are_asked_for(native):
+    # One tile per CTA is whole units per thread, so that no CTA is left without; several are no smaller than a batch.
+    for units in (1, 600, 2049, 46_875, 102_400, 409_600, 1_000_000):
+        for nctas in (1, 18, 37, 64):
+            for threads in (128, 512):
+                share = -(-units // nctas)
+                tile, batch = native._twoshot_tile(units, nctas, threads, 1)
+                assert tile % threads == 0 and share <= tile < share + threads
+                for tiles in (2, 3, 8, 64):
+                    tile, batch = native._twoshot_tile(units, nctas, threads, tiles)
+                    assert batch == 4 * threads and tile % batch == 0
+                    assert tile >= -(-share // tiles) and (tile == batch or tile < -(-share // tiles) + batch)
+
+
 def test_pool_range_allocator_first_fit_and_coalescing(native):
     # steps: +n allocates n bytes, -i releases the block of step i (1-based); 512-byte granules
     offs, used, free_blocks = native._test_range_allocator(1 << 20, [1000, 512, 4096, -2, 300, -1, -3, -5, 1 << 20])
