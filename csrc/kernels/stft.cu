@@ -835,12 +835,19 @@ OlaGrid ola_grid(const IfftOlaArgs& a) {
   return g;
 }
 
-// What a frame of every lane group takes the stream kernel, forward's gradient and inverse, and what it takes to begin and end,
-// both in tenths of the time of the batch kernel's batch.  Fitted to 230 pairs of times: n_fft 256, 512 and 2048, hop n_fft / 4 and
-// / 2, 1 to 160 signals of 64 Ki to 1 Mi samples.
-constexpr int kStreamFrame[12][2] = {{}, {}, {}, {}, {}, {}, {64, 64}, {64, 64}, {70, 75}, {}, {65, 71}, {}};
-constexpr int kStreamEnds[12] = {0, 0, 0, 0, 0, 0, 5, 5, 9, 0, 32, 0};
-constexpr int kBatchEnds = 20;
+// What the stream kernel takes for a frame of every lane group and around them, and what ola_rows takes for a batch of frames of up to
+// two, four and more frames per sample, in tenths of a microsecond; [0] the adjoint, [1] the inverse with its division.  Fitted to 970
+// pairs of times: hop n_fft / 8, / 4, 5 / 16 and / 2, 1 to 200 signals of 64 Ki to 1 Mi samples (B200).
+struct StreamCosts {
+  int frame[2], ends[2], batch[2][3];
+};
+constexpr int kBatchEnds = 140;
+constexpr StreamCosts stream_costs(int lh) {
+  return lh <= 6   ? StreamCosts{{18, 20}, {200, 170}, {{40, 48, 61}, {42, 50, 63}}}
+         : lh == 7 ? StreamCosts{{33, 36}, {240, 240}, {{56, 53, 73}, {61, 55, 76}}}
+         : lh == 8 ? StreamCosts{{29, 34}, {260, 240}, {{46, 40, 39}, {51, 43, 41}}}
+                   : StreamCosts{{59, 77}, {470, 360}, {{86, 85, 87}, {98, 94, 94}}};
+}
 
 // The stream kernel's geometry; threads == 0: not for this problem.  It wants runs of frames that are long against what two
 // neighbours share, and its CTAs, one per SM and in whole numbers per signal, to fill the device about as well as the batch kernel's.
@@ -863,16 +870,21 @@ OlaGrid stream_grid(const IfftOlaArgs& a) {
   const int64_t most = std::max<int64_t>(1, kSms / a.batch);
   const int64_t least = 3ll * (pl.reach - 1) * groups + 2 * pl.edge;  // rows of a CTA
   pl.segments = static_cast<int>(std::min<int64_t>(most, pl.rows / std::max<int64_t>(1, least)));
-  if (pl.segments < 1) return g;
-  // Frames of the busiest lane group against batches of the busiest CTA, each as often as its CTAs need turns on the device.
-  // 80 x 1 Mi samples, n_fft 512, hop 128, backward: 612 us in batches, 748 in streams on 80 SMs; 32 x 256 Ki, 2048, 1024: 52
-  // and 65.  32 x 1 Mi, 512, 128: 250 and 211; 120 x 1 Mi, 2048, 512: 1110 and 788.
+  if (pl.segments < 1 || (pl.segments < most && static_cast<int64_t>(pl.segments) * a.batch < kSms * 3 / 4)) return g;
+  // Frames of the busiest lane group against batches of the busiest CTA, each as often as its CTAs need turns on the device.  Of those
+  // 970 pairs the streams, wherever signals were long, were 4 % or more behind in 186; so in none, and left out where they are as
+  // much ahead in 17.  Us in batches and streams, 80 x 1 Mi samples, 512, hop 128, backward: 612 and 748, on 80 SMs; 32 x 256 Ki, 2048,
+  // 1024: 52 and 65; but 32 x 1 Mi, 512, 128: 250 and 211; 120 x 1 Mi, 2048, 512: 1110 and 788; 80 x 1 Mi, 128, 16: 3591 and 1731.
+  constexpr StreamCosts costs = stream_costs(LH);
+  const int kind = a.normalize_envelope ? 1 : 0;
   auto ceil_div = [](int64_t x, int64_t y) { return (x + y - 1) / y; };
   auto longest = [&](int64_t segments, int64_t together) { return ceil_div(ceil_div(pl.rows, segments) + pl.reach - 1, together); };
   const int64_t turns = ceil_div(static_cast<int64_t>(pl.segments) * a.batch, kSms);
   const int64_t row_turns = ceil_div(static_cast<int64_t>(rows.plan.segments) * a.batch, static_cast<int64_t>(kSms) * rows.resident);
-  if (turns * (longest(pl.segments, groups) * kStreamFrame[LH][a.normalize_envelope ? 1 : 0] + 10 * (kStreamEnds[LH] + kBatchEnds)) >
-      row_turns * (100 * longest(rows.plan.segments, rows.batch) + 10 * kBatchEnds))
+  int batch_cost = costs.batch[kind][pl.reach <= 2 ? 0 : pl.reach <= 4 ? 1 : 2];
+  if (F::n % a.hop != 0) batch_cost = batch_cost * 9 / 8;
+  if (turns * (longest(pl.segments, groups) * costs.frame[kind] + costs.ends[kind]) >
+      row_turns * (longest(rows.plan.segments, rows.batch) * batch_cost + kBatchEnds))
     return g;
   const size_t kept = F::V - a.hop / (2 * F::L);
   const size_t stream = groups * (F::kHalfSlot * sizeof(float) + kept * F::L * sizeof(float2)) +

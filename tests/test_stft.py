@@ -377,10 +377,13 @@ def test_streamed_inverse_matches_64_bits(n_fft, hop, batch, samples, center):
 # Streams, one CTA per SM and whole CTAs per signal, only where they leave no more of the device idle than they gain: times of the
 # two kernels (B200) differ by 5 % at least in every row.
 @pytest.mark.parametrize("n_fft,hop,samples,inverse,streams,batches", [
+    (128, 16, 1 << 20, False, (16, 80), ()), (128, 32, 300000, True, (16, 50, 80), ()), (128, 64, 1 << 16, False, (80, 96, 160), ()),
     (256, 64, 1 << 20, False, (8, 16, 24, 32, 50, 64, 96, 120), (80,)),
+    (256, 32, 300000, True, (50, 80, 160), ()),
     (256, 128, 1 << 16, True, (120, 148), (50, 80, 96, 160)),
     (512, 128, 1 << 20, True, (8, 16, 24, 32, 64, 120), (80, 96)),
-    (512, 256, 1 << 18, False, (24, 32, 64, 120, 148), (80, 96, 160)),
+    (512, 128, 300000, False, (32,), (16, 80)),
+    (512, 256, 1 << 18, False, (64, 120, 148), (80, 96, 160)),
     (2048, 512, 1 << 20, False, (24, 32, 50, 64, 120), (80, 96)),
     (2048, 512, 1 << 18, True, (120, 148, 160), (50, 80, 96)),
     (2048, 1024, 1 << 18, False, (120, 148, 160), (32, 50, 80, 96)),
