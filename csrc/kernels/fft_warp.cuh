@@ -103,42 +103,57 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
   if constexpr (kPacked) return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
   else return make_float2(a.x - b.x, a.y - b.y);
 }
-// d * exp(-2 pi i K / R)
-template <int K, int R>
+// d * exp(-2 pi i K / R); kOpen: at an odd multiple of an eighth turn without the factor sqrt(1/2), which whoever adds the
+// number up next multiplies in (`add_open`): one rounding less, as the compiler has it where sums are not packed.
+constexpr float kHalfRoot = static_cast<float>(root_cos(1, 8));
+template <int K, int R, bool kOpen>
 __device__ __forceinline__ float2 mul_root(float2 d) {
   constexpr float c = static_cast<float>(root_cos(K, R)), s = static_cast<float>(root_sin(K, R));
   if constexpr (K == 0) return d;
   else if constexpr (4 * K == R) return make_float2(d.y, -d.x);
+  else if constexpr (8 * K == R && kOpen) return make_float2(d.x + d.y, d.y - d.x);
+  else if constexpr (8 * K == 3 * R && kOpen) return make_float2(d.y - d.x, -d.x - d.y);
   else if constexpr (8 * K == R) return make_float2(c * (d.x + d.y), c * (d.y - d.x));
   else if constexpr (8 * K == 3 * R) return make_float2(s * (d.y - d.x), -s * (d.x + d.y));
   else return make_float2(d.x * c + d.y * s, d.y * c - d.x * s);
+}
+// a + or - sqrt(1/2) b
+template <int kSign>
+__device__ __forceinline__ float2 add_open(float2 a, float2 b) {
+  return __ffma2_rn(b, make_float2(kSign * kHalfRoot, kSign * kHalfRoot), a);
 }
 
 // Forward FFT of v[O .. O + R), in place, decimation in frequency: X[k] ends up in v[O + bit_reverse(k, R)].
 // Radix 4 (a value meets one twiddle where two radix-2 stages would have two: fewer roundings and fewer
 // instructions), with a last radix-2 stage for odd powers of two.
-template <bool kPacked, int R, int O, int N>
+// kTurn: the values come from a stage that has turned number j by kTurn * j / 4R (0: from elsewhere).  Packed, those at an odd
+// multiple of an eighth are open: j = R / 2 for 1 and 3, j = R / 4 and 3R / 4 for 2.
+template <bool kPacked, int R, int O, int kTurn = 0, int N>
 __device__ __forceinline__ void fft_registers(float2 (&v)[N]) {
+  constexpr bool kOpenHalf = kPacked && (kTurn == 1 || kTurn == 3), kOpenQuarters = kPacked && kTurn == 2 && R >= 4;
   if constexpr (R == 2) {
     const float2 p = v[O], q = v[O + 1];
-    v[O] = add2<kPacked>(p, q);
-    v[O + 1] = sub2<kPacked>(p, q);
+    v[O] = kOpenHalf ? add_open<1>(p, q) : add2<kPacked>(p, q);
+    v[O + 1] = kOpenHalf ? add_open<-1>(p, q) : sub2<kPacked>(p, q);
   } else if constexpr (R >= 4) {
     constexpr int Q = R / 4;
     static_for<0, Q>([&](auto jc) {
       constexpr int j = decltype(jc)::value;
-      const float2 v0 = v[O + j], v1 = v[O + j + Q], v2 = v[O + j + 2 * Q], v3 = v[O + j + 3 * Q];
-      const float2 a0 = add2<kPacked>(v0, v2), a1 = sub2<kPacked>(v0, v2);
-      const float2 a2 = add2<kPacked>(v1, v3), a3 = sub2<kPacked>(v1, v3);
+      constexpr bool half = kOpenHalf && j == 0, quarters = kOpenQuarters && j == 0;
+      const float2 v0 = v[O + j], v2 = v[O + j + 2 * Q], v3 = v[O + j + 3 * Q];
+      const float2 v1 = quarters ? make_float2(kHalfRoot * v[O + j + Q].x, kHalfRoot * v[O + j + Q].y) : v[O + j + Q];
+      const float2 a0 = half ? add_open<1>(v0, v2) : add2<kPacked>(v0, v2), a1 = half ? add_open<-1>(v0, v2) : sub2<kPacked>(v0, v2);
+      const float2 a2 = quarters ? add_open<1>(v1, v3) : add2<kPacked>(v1, v3);
+      const float2 a3 = quarters ? add_open<-1>(v1, v3) : sub2<kPacked>(v1, v3);
       v[O + j] = add2<kPacked>(a0, a2);
-      v[O + j + Q] = mul_root<2 * j, R>(sub2<kPacked>(a0, a2));
-      v[O + j + 2 * Q] = mul_root<j, R>(make_float2(a1.x + a3.y, a1.y - a3.x));
-      v[O + j + 3 * Q] = mul_root<3 * j, R>(make_float2(a1.x - a3.y, a1.y + a3.x));
+      v[O + j + Q] = mul_root<2 * j, R, kPacked>(sub2<kPacked>(a0, a2));
+      v[O + j + 2 * Q] = mul_root<j, R, kPacked>(make_float2(a1.x + a3.y, a1.y - a3.x));
+      v[O + j + 3 * Q] = mul_root<3 * j, R, kPacked>(make_float2(a1.x - a3.y, a1.y + a3.x));
     });
     fft_registers<kPacked, Q, O>(v);
-    fft_registers<kPacked, Q, O + Q>(v);
-    fft_registers<kPacked, Q, O + 2 * Q>(v);
-    fft_registers<kPacked, Q, O + 3 * Q>(v);
+    fft_registers<kPacked, Q, O + Q, 2>(v);
+    fft_registers<kPacked, Q, O + 2 * Q, 1>(v);
+    fft_registers<kPacked, Q, O + 3 * Q, 3>(v);
   }
 }
 
