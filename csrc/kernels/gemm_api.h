@@ -60,7 +60,7 @@ struct GemmArgs {
   float* partial;
   uint32_t* tickets;
   uint32_t* failed;     // set to 1 where a wait runs out, whose tiles then are NaN; or null
-  int64_t wait_limit;   // cycles of a wait; negative: about a second
+  int64_t wait_limit;   // cycles of a quarter of a wait; negative: about a second in all
 };
 cudaError_t launch_gemm_f32(const GemmArgs& g, cudaStream_t s);
 
