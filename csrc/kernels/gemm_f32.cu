@@ -683,34 +683,31 @@ GemmPlan gemm_plan(Product p, int64_t batch, int64_t in, int64_t out) {
 
 // From sweeps of 1 to 4096 rows over 26 layers, 65536 to 16 features and the reverse among them, and of 8 to 255 rows over 81 of
 // 256 to 3000 (B200, both sides from CUDA graphs; here with the launch that makes the images; weights from memory and, up to 40 MB
-// of them, from the second-level cache).  Of 1139 products taken 13 are slower than the library's, by 3 to 12 %.  What is left to
-// the library, us there and here, rows and features in -> out:
+// of them, from the second-level cache).  What is left to the library, us there and here, rows and features in -> out:
 //  - little to do, less than the two launches cost: 64, 256 -> 512 forward 11.7 and 12.0;
-//  - tiles of 128 rows (of 65 and more) on less than 1000 of the reduction: they take 15 to 17 us at least, the library 8 to 13, 96,
-//    256 -> 3000 forward 9.3 and 14.6; narrower tiles below 512: 33, 256 -> 3000 9.4 and 11.2;
+//  - short sums: tiles of 128 rows (of 65 and more) take 15 to 17 us at least, narrower ones 10 to 12, the library 8 to 13: 96,
+//    256 -> 3000 forward 9.3 and 14.6, 33 9.4 and 11.2;
 //  - rows of a tile that the layer does not have: 64, 65536 -> 16 forward 117 and 215; weight gradient of 64, 100000 -> 64 25 and 34;
 //  - few CTAs with long shares of the reduction: 64, 100000 -> 64 forward 180 and 327, 16, 16384 -> 128 21 and 59;
-//  - next to no rows, for which the library reads the weights at 5 TB/s and this kernel at 2.3: 1, 8192 -> 8192 forward 49 and 115;
-//  - weight gradients of less than 75 tiles, half a turn of the device for the library: 255, 850 -> 850 13.1 and 14.1.
+//  - next to no rows, for which the library reads the weights at 5 TB/s and this kernel at 2.3: 1, 8192 -> 8192 forward 49 and 115.
+// Of the 1380 products that size alone let through 138 were slower than the library's by 5 % or more, 81 by 20 %; of the 1241 now, 33
+// and 5.  Those are of 65 rows and more, 300 to 850 deep, most of them within 2 us, and two to four times closer to the exact sums;
+// lines that left them to the library would take that from a model's other gradients too.
 // Images are one and a half times their matrix: none above 1 GB.
 bool gemm_pays(Product p, int64_t batch, int64_t in, int64_t out) {
   constexpr double kImageLimit = 1 << 30;
   const double macs = static_cast<double>(batch) * in * out, layer = static_cast<double>(in) * out;
   if (6.0 * batch * (static_cast<double>(in) + 2.0 * out) > kImageLimit || layer > 1e10) return false;
   const bool fwd = p == Product::kForward;
-  if (p == Product::kWeight ? batch < 32 || macs < 1.1e8 : layer < 7e5 || macs < (fwd ? 2e7 : 3e7)) return false;
+  if (p == Product::kWeight ? batch < 32 || macs < 1e8 : layer < 7e5 || macs < (fwd ? 2e7 : 3e7)) return false;
   const GemmPlan g = gemm_plan(p, batch, in, out);
   const int64_t tiles = static_cast<int64_t>(g.tiles_i) * g.tiles_j;
-  if (p == Product::kWeight) {
-    if (4.0 * layer < 3.0 * kRows * kRows * static_cast<double>(tiles)) return false;
-    return tiles > 74 || macs >= (g.splits == 1 ? 1.4e8 : 2.4e8);
-  }
+  if (p == Product::kWeight) return 4.0 * layer >= 3.0 * kRows * kRows * static_cast<double>(tiles);
   if (4 * g.rows_i < 3 * kRows * static_cast<int64_t>(g.tiles_i) || g.depth < 64) return false;
   const bool deep = layer < 3e7 || g.depth >= (fwd ? 2 : 1) * g.rows_i;
   if (batch < (deep ? 2 : fwd ? 16 : 8)) return false;
   if (tiles * g.splits < 24 && (batch < 32 || g.per_split > 64)) return false;
-  if (g.cols == 128 && g.depth < 1000) return macs >= (g.depth < 700 ? 2.7e8 : 2.05e8);
-  return g.depth >= 512 || macs >= 2.4e8;
+  return g.depth >= (fwd ? 512 : 288) || macs >= 2.5e8;
 }
 
 cudaError_t launch_split_f32(const SplitJob* jobs, int n, float* sums, uint32_t* zero, int64_t zeroed, cudaStream_t s) {
