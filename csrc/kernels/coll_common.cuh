@@ -217,9 +217,10 @@ template <> struct MultimemSum<__nv_bfloat16> {
 // round costs more than it overlaps (8 tiles: 8 x 3000000 fp16 121 and 226, 4 x 2000000 fp32 77 and 178).
 constexpr int kTileUnroll = 4;
 __host__ __device__ inline int64_t twoshot_tile_units(int64_t chunk_units, int nctas, int nthreads, int64_t tiles) {
-  const int64_t want = tiles > 1 ? tiles : 1, grain = static_cast<int64_t>(nthreads) * (want > 1 ? kTileUnroll : 1);
-  const int64_t share = ((chunk_units + nctas - 1) / nctas + want - 1) / want;
-  return share > grain ? (share + grain - 1) / grain * grain : grain;
+  const int64_t want = tiles > 1 ? tiles : 1, grain = static_cast<int64_t>(nthreads) * (tiles > 1 ? kTileUnroll : 1);
+  const int64_t share = (chunk_units + nctas - 1) / nctas;
+  const int64_t tile = ((share + want - 1) / want + grain - 1) / grain * grain;
+  return tile < grain ? grain : tile;
 }
 
 // Tile geometry of the pipelined kernels.  The 16-byte-unit index space [0, units) is cut into
