@@ -157,15 +157,18 @@ def main():
     loss_fn = torch.nn.CrossEntropyLoss()
     warmup = max(args.warmup, 3)
 
-    def run_arm(kind, fused_optim, group):
+    def run_arm(kind, fused_optim, group, torch_products=False):
         """One complete measurement (warm-up, device-timed region, end-to-end region) of one arm.
 
         kind "mccl": this backend + fused-average hook (+ fused AdamW when `fused_optim`);
         kind "nccl": torch's NCCL backend + stock DDP + torch.optim.AdamW(fused=True).
+        `torch_products`: the model's layers use torch's fp32 matrix products (see mccl_b200/ops/linear.py).
         `group` is the process group the arm trains on (None: the default group).
         """
         torch.manual_seed(42)
         model = MLP94M().to(dev)
+        for layer in model.net[::2]:
+            layer.stock = torch_products
         n_params = num_parameters(model)
         in_bw = False
         if kind == "mccl":
@@ -180,8 +183,6 @@ def main():
                            optimizer_in_backward=opt if in_bw else None)
         else:
             from torch.nn.parallel import DistributedDataParallel
-            for layer in model.net:  # torch's own products, like the rest of this arm
-                layer.stock = True
             ddp = DistributedDataParallel(model, device_ids=[local_rank], bucket_cap_mb=args.bucket_mb,
                                           gradient_as_bucket_view=True, process_group=group)
             opt = torch.optim.AdamW(ddp.parameters(), lr=1e-3, fused=True)
@@ -256,14 +257,15 @@ def main():
                 "value": GLOBAL_BATCH / (ms_total / args.steps / 1e3),
                 "e2e_value": GLOBAL_BATCH / (ms_e2e / args.steps / 1e3)}
 
-    main_arm = run_arm(args.impl, not args.no_fused_optim, None)
+    main_arm = run_arm(args.impl, not args.no_fused_optim, None, torch_products=args.impl == "nccl")
     ms_total, ms_e2e = main_arm["ms_total"], main_arm["ms_e2e"]
     clocks, clocks_e2e, launches, loss_b = main_arm["clocks"], main_arm["clocks_e2e"], main_arm["launches"], main_arm["final_loss"]
     n_params, in_bw = main_arm["n_params"], main_arm["in_bw"]
 
     # Comparison arms in the same process, on the same GPUs, with the same steps and warm-up:
     # (a) this backend with torch's own fused AdamW, which isolates the communication path from the
-    # optimizer kernel, and (b) torch's stock NCCL backend + stock DDP + torch AdamW.
+    # optimizer kernel, (b) torch's stock NCCL backend + stock DDP + torch AdamW under the same model, and (c) the same
+    # with torch's own matrix products in the model's layers.
     extra = {}
     if args.impl == "mccl" and not args.no_compare:
         if not args.no_fused_optim:
@@ -272,7 +274,13 @@ def main():
                                        "ms_per_step": round(arm["ms_total"] / args.steps, 4), "clocks": arm["clocks"]}
         try:
             nccl_group = dist.new_group(backend="nccl")
-            arm = run_arm("nccl", False, nccl_group)
+            # the backend's share of the difference: the same layers on either side
+            same = run_arm("nccl", False, nccl_group)
+            extra["nccl_same_layers"] = {"value": round(same["value"], 2), "e2e": round(same["e2e_value"], 2),
+                                         "ms_per_step": round(same["ms_total"] / args.steps, 4), "clocks": same["clocks"]}
+            extra["vs_nccl_same_layers"] = round(main_arm["value"] / same["value"], 4)
+            # and torch alone, its fp32 products included
+            arm = run_arm("nccl", False, nccl_group, torch_products=True)
             extra["nccl_value"] = round(arm["value"], 2)
             extra["nccl_e2e"] = round(arm["e2e_value"], 2)
             extra["nccl_ms_per_step"] = round(arm["ms_total"] / args.steps, 4)
@@ -313,6 +321,9 @@ def main():
             "seq_len": None,
             "parallelism": f"dp{world}",
             "optimizer": "AdamW lr=1e-3",
+            "products": ("fp32 operands, results and sums; each product as six bf16 products on the tensor cores (sums no further "
+                         "from 64 bits than an fp32 kernel's)" if native and native._linear_pays("forward", local_batch, 3072, 3072)
+                         else "torch fp32"),
             "ddp_bucket_mb": args.bucket_mb,
             "l2": "no flush: params+grads+AdamW state are 1.5 GB per step, far above the 126 MB L2",
             "data_plane": plane,
