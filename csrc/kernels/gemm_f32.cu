@@ -55,35 +55,19 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-__device__ __forceinline__ bool bar_test(uint32_t bar, uint32_t parity) {  // a look that never sleeps
-  uint32_t done;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-// Waits for the phase of that parity, for four times `limit` cycles; 0: one look.  A pause of the whole device (another process has it, a
-// debugger stopped it) uses up one of the four at most.
-constexpr long long kWaitLimit = 500000000ll;  // about a quarter of a second
+// Waits for the phase of that parity, for four times `limit` cycles at most.  A pause of the whole device (another process has it, a
+// debugger stopped it) uses up one of the four.
+constexpr long long kWaitLimit = 500000000ll, kLanding = 2000000ll;  // about a quarter of a second and a millisecond
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, long long limit) {
-  if (limit <= 0) return bar_test(bar, parity);
   if (bar_try(bar, parity)) return true;
-  int left = 4;
-  for (long long begin = clock64(); !bar_try(bar, parity);)
-    if (clock64() - begin > limit) {
-      if (--left == 0) return false;
-      begin = clock64();
-    }
-  return true;
-}
-// The same by all lanes of a warp, which agree.  The clock stays out of the way of a wait that one look ends: 256 x 3072 x 3072, forward and
-// input gradient, 40.0 and 39.6 us with bar_wait alone, 39.5 and 38.8 so (with an earlier split2).
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long long limit) {
-  bool ok = limit > 0 && bar_try(bar, parity);
-  if (!__all_sync(0xFFFFFFFFu, ok)) ok = __all_sync(0xFFFFFFFFu, bar_wait(bar, parity, limit));
-  return ok;
+#pragma unroll 1
+  for (int left = 4; left > 0; --left) {
+    const long long begin = clock64();
+    do {
+      if (bar_try(bar, parity)) return true;
+    } while (clock64() - begin <= limit);
+  }
+  return false;
 }
 // Shared-memory matrix descriptors.  k innermost: rows of 64 bytes (32 k), 64-byte swizzle, 512 bytes per eight rows.
 // Own index innermost: rows of 128 bytes (64 rows of the operand, one k), 128-byte swizzle, 1024 bytes per eight k, 4096
@@ -135,7 +119,7 @@ __device__ __forceinline__ bool elect() {
 // A float to be cut off where its bf16 neighbours' middle would round away from zero: half a step further from zero.  At the largest
 // numbers the sum stops, so they don't become infinite as rounding to nearest would make them; infinities and NaN stay.
 // (Rounded to nearest by the conversion, with a look for what that made infinite, 256 x 3072 x 3072 took 41.8 us forward and 41.4 for the
-// input gradient, 40.2 and 39.3 so; cut off, without the half step, 38.5 and 38.7.)
+// input gradient, 40.2 and 39.3 so; the half step itself costs 0.8 us.)
 __device__ __forceinline__ float half_step(float x) {
   return __fmaf_rz(__uint_as_float(__float_as_uint(x) & 0xFF800000u), 0x1p-8f, x);
 }
@@ -300,12 +284,12 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
 
 // One tile of 128 by NT per CTA and, where the tiles do not fill the device, a share of its reduction; tiles in turn where
 // there are more than SMs.  One warp issues all products, eight take acc0 out while the other products of a stage run,
-// the rest cut the weights (once per tile: no pass over them before) or copy images in, four stages ahead (six or seven for
-// the narrow tiles: 20.0 against 19.3 us, 32 x 3072 x 3072 forward; what the stages leave is the weights' cache).
+// the rest cut the weights (once per tile: no pass over them before) or copy images in, four stages ahead (six or seven for the
+// narrow tiles took 20.0 us where four took 19.3, 32 x 3072 x 3072 forward: what the stages leave is the weights' cache).
 // Bound by shared memory: a stage of NT = 128 moves 128 KB through it, 1024 cycles, where its products take 768; measured
 // 870 without the weights' share, 1300 with it.  256 x 3072 x 3072 with weights that come from memory, us, with the images'
-// launch (B200): forward 128.8 with cuBLAS's fp32 kernel, 36.9 so; input gradient 121.7 and 36.2; weight gradient, whose
-// images take the second-level cache 9 TB/s, 98.9 and 30.1: 130 to 160 TFLOP/s of fp32 products, 0.8 to 1 PFLOP/s of bf16.
+// launch (B200): forward 125.9 with cuBLAS's fp32 kernel, 37.8 so; input gradient 122.8 and 37.9; weight gradient, whose
+// images take the second-level cache 9 TB/s, 99.5 and 32.7: 130 to 150 TFLOP/s of fp32 products, 0.8 to 0.9 PFLOP/s of bf16.
 // Tried and left: pairs of CTAs on one tile (92 KB per stage, but each turn waits for both: 47.5 us), weights cut straight
 // into tensor memory (72 KB; a lane's 32 loads per stage cost what that saves: 36.0 and 48.4 us).
 template <int NT, int kSource>
@@ -316,7 +300,6 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
   extern __shared__ char raw[];
   __shared__ alignas(8) uint64_t bars[2 * kStages + 5];
   __shared__ uint32_t tmem_base, last_here;
-  __shared__ int issued, given[kProducers / 32];  // stages that images were asked for, and that each producer warp has filled
   char* smem = raw + ((1024u - (smem_addr(raw) & 1023u)) & 1023u);
   const uint32_t smem0 = smem_addr(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -375,7 +358,6 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
             load_images(tile, c, s);
             if (++s == kStages) s = 0, ++turn;
           }
-        issued = turn * kStages + s;
       }
       __syncwarp();
     } else {
@@ -421,31 +403,32 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
       for (int b = 0; b < kAhead; ++b) fetch(v[b]);
       const bool loads = warp == kIssuer + 1 && elect();
       if (loads) asm volatile("griddepcontrol.wait;" ::: "memory");
-      int tile = first_tile, c = c0;
+      int tile = first_tile, c = c0, missed = 0;
       while (ok && tile < w.tiles) {
 #pragma unroll
         for (int b = 0; b < kAhead; ++b) {
-          if (!ok || tile >= w.tiles) break;
-          ok = warp_wait(empty(s), (turn & 1) ^ 1, w.limit);
-          if (!ok) break;
-          if (loads) load_images(tile, c, s);
+          if (tile >= w.tiles) break;
+          // no branch before the numbers are cut, which needs no stage: warps agree on having given up after a few
+          const bool got = bar_wait(empty(s), (turn & 1) ^ 1, w.limit);
+          if (got && loads) load_images(tile, c, s);
           char* to = mine + s * kStage;
 #pragma unroll
           for (int j = 0; j < 2; ++j) store8(to + j * 4096, kPartA, split8(v[b][j]));
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
-          if (lane == 0) bar_arrive(full(s));
+          if (!got) missed = 1;
+          if (lane == 0 && missed == 0) bar_arrive(full(s));
           fetch(v[b]);
           if (++s == kStages) s = 0, ++turn;
           if (++c == c1) c = c0, tile += tile_step;
         }
+        ok = __all_sync(0xFFFFFFFFu, missed == 0);
       }
-      if (lane == 0) given[warp - kIssuer - 1] = turn * kStages + s;
-      if (loads) issued = turn * kStages + s;
     }
   } else if (warp == kIssuer) {
     issues = elect();
     if (issues) {
+      ok = w.limit > 0;  // a limit of zero, of tests: no product is issued, and all others wait in vain
       constexpr uint32_t one = make_idesc(kAInner, kBInner, NT), two = make_idesc(kAInner, kBInner, 2 * NT);
       constexpr uint32_t step_a = kStep<kAInner>, step_b = kStep<kBInner>;
       const uint32_t acc0 = tmem, acc1 = tmem + NT, acc2 = tmem + 2 * NT;
@@ -493,8 +476,7 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
       for (int i = 0; i < kCols; ++i) sum[i] = 0.f;
       for (int c = c0; ok && c < c1; c += kGroup) {
         // the other five products of the group's last stage run while acc0 is taken out
-        ok = warp_wait(acc0_full, groups++ & 1, w.limit);
-        if (!ok) break;
+        const bool got = bar_wait(acc0_full, groups++ & 1, w.limit);
         fence_after();
 #pragma unroll
         for (int i = 0; i < kCols; i += 16) {
@@ -507,9 +489,9 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
         fence_before();
         __syncwarp();
         if (lane == 0) bar_arrive(acc0_free);
+        ok = __all_sync(0xFFFFFFFFu, got);
       }
-      ok = ok && warp_wait(all_full, done & 1, w.limit);
-      if (!ok) break;
+      const bool got = ok && bar_wait(all_full, done & 1, w.limit);
       fence_after();
 #pragma unroll
       for (int i = 0; i < kCols; i += 16) {
@@ -523,6 +505,8 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
       }
       fence_before();
       __syncwarp();
+      ok = __all_sync(0xFFFFFFFFu, got);
+      if (!ok) break;
       if (lane == 0) bar_arrive(all_free);
       if (w.splits > 1) {
         float* part = w.partial + (static_cast<int64_t>(tile) * w.splits + rank) * (NT * kRows) + half * kCols * kRows + 32 * q + lane;
@@ -549,13 +533,8 @@ __global__ void __launch_bounds__(kThreads<kSource>, 1) gemm_f32_kernel(const Wo
   if (failed) {
     if (tid == 0) {
       if (w.failed) *w.failed = 1u;
-      // The copies in flight end before this CTA's shared memory is another's.  A stage is full when they and all producer
-      // warps have come: for warps that left early this thread does.
-      for (int n = max(issued - kStages, 0); n < issued; ++n) {
-        if (kSource != kImage)
-          for (int p = 0; p < kProducers / 32; ++p)
-            if (given[p] <= n) bar_arrive(full(n % kStages));
-        bar_wait(full(n % kStages), (n / kStages) & 1, kWaitLimit);
+      // The copies in flight, microseconds, end before this CTA's shared memory is another's.
+      for (const long long begin = clock64(); clock64() - begin < kLanding;) {
       }
     }
     if (issues) {  // and the products, before tensor memory is
